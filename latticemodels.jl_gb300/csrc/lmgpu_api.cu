@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "lmgpu_internal.cuh"
+#include "lmgpu_series.cuh"
 
 using namespace lmgpu;
 
@@ -829,6 +830,9 @@ static void free_tables(lm_solver* s) {
     s->d_spack = nullptr;
     s->spack_f4 = 0;
     s->spack_version = ~0ull;
+    if (s->d_sgauge) cudaFree(s->d_sgauge);
+    s->d_sgauge = nullptr;
+    s->sgauge_version = ~0ull;
     s->d_hop2 = nullptr;
     s->d_diag2 = nullptr;
     s->d_hop2f = nullptr;
@@ -1006,6 +1010,68 @@ static int cheb_apply(lm_solver* s, const Geom& g, int precision, int site_fast,
     return LM_OK;
 }
 
+// The ComplexF64 step with whole kets on chip (lmgpu_series.cu); *done = 0 where it does not apply.
+// Kets are replaced in place.  A density matrix takes two launches that each apply U to the columns
+// and store the conjugate transpose: P -> (U P)^dagger -> (U (U P)^dagger)^dagger = U P U^dagger.
+static int series_step(lm_solver* s, lm_state* st, int* done) {
+    lm_ctx* ctx = s->ctx;
+    *done = 0;
+    if (!ctx->fused || st->precision != LM_C64 || s->K > kSeriesMaxK) return LM_OK;
+    const lm_ham* h = s->ham;
+    const Geom& g = h->lat->g;
+    const bool xr = ham_x_real(h);
+    const SeriesPlan plan = series_plan(ctx, g, xr, st->m, false);
+    if (!plan.kt) return LM_OK;
+    if (!xr && s->sgauge_version != s->tab_version) {
+        if (!s->d_sgauge) {
+            int rc = dalloc(ctx, (void**)&s->d_sgauge, sizeof(double2) * 2 * (size_t)g.N, "gauge table");
+            if (rc != LM_OK) return rc;
+        }
+        CUDA_TRY(ctx, launch_gauge_tables(ctx, g, h->d_hop, h->d_onsite, h->t1, s->a, s->b, false, s->d_sgauge,
+                                          s->d_sgauge + g.N, nullptr, nullptr, nullptr),
+                 "gauge tables");
+        s->sgauge_version = s->tab_version;
+    }
+    if (st->kind == LM_DENSITY) {
+        int rc = ensure_scratch(st);
+        if (rc != LM_OK) return rc;
+    }
+    SeriesArgs a;
+    a.Lx = (int)g.Lx;
+    a.Ly = (int)g.Ly;
+    a.per_x = g.per_x;
+    a.per_y = g.per_y;
+    a.K = s->K;
+    a.M = st->m;
+    a.ld_in = a.ld_out = st->ld;
+    a.gauge = xr ? nullptr : s->d_sgauge;
+    a.hy = xr ? s->d_hop2 + g.N : s->d_sgauge + g.N;
+    a.diag = s->d_diag2;
+    a.alpha = 2.0 * h->t1 / s->a;
+    a.phase = make_double2(s->phase_re, s->phase_im);
+    for (int k = 0; k <= s->K; ++k) a.cf[k] = s->coef[(size_t)k].s;
+    cudaEvent_t t0 = nullptr, t1 = nullptr;
+    if (ctx->timing) {
+        int rc = timing_pair(ctx, &t0, &t1);
+        if (rc != LM_OK) return rc;
+        CUDA_TRY(ctx, cudaEventRecord(t0, ctx->stream), "cudaEventRecord");
+    }
+    const int passes = st->kind == LM_DENSITY ? 2 : 1;
+    a.transpose = passes == 2;
+    for (int p = 0; p < passes; ++p) {
+        a.in = (const double2*)(p == 0 ? st->d_data : st->d_a);
+        a.out = (double2*)(p + 1 == passes ? st->d_data : st->d_a);
+        CUDA_TRY(ctx, launch_series_f64(ctx, plan, a), "on-chip chebyshev step");
+    }
+    if (ctx->timing) {
+        CUDA_TRY(ctx, cudaEventRecord(t1, ctx->stream), "cudaEventRecord");
+        ctx->ev_launches[ctx->ev_used] = s->K * passes;
+        ctx->ev_used++;
+    }
+    *done = 1;
+    return LM_OK;
+}
+
 int lm_solver_step(lm_solver* s, lm_state* st) {
     if (!s) return LM_ERR_ARG;
     lm_ctx* ctx = s->ctx;
@@ -1017,7 +1083,10 @@ int lm_solver_step(lm_solver* s, lm_state* st) {
     CHECK_ARG(ctx, st->n == g.N, "lm_solver_step: state size does not match the lattice");
     cudaSetDevice(ctx->device);
     {
-        int rc0 = ensure_scratch(st);
+        int done = 0;
+        int rc0 = series_step(s, st, &done);
+        if (rc0 != LM_OK || done) return rc0;
+        rc0 = ensure_scratch(st);
         if (rc0 != LM_OK) return rc0;
     }
     if (!(ctx->fused && st->kind == LM_KETS && fused_supported(st->precision, s->K) && fused_supported_geom(g))) {

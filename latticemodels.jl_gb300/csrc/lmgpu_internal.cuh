@@ -184,6 +184,9 @@ struct lm_solver {
     size_t spack_f4 = 0;
     uint64_t spack_version = ~0ull;
     int bpack_valid = 0;         // d_spack holds the honeycomb brick planes of the current ELL tables
+    // on-chip ComplexF64 form (lmgpu_series.cu): the gauge and its hops H'[s, s + y], 2 N each
+    double2* d_sgauge = nullptr;
+    uint64_t sgauge_version = ~0ull;
     int has_onsite = 0;
     int fixed_bounds = 0;        // lm_solver_set_bounds: use [fix_emin, fix_emax] instead of Gershgorin
     double fix_emin = 0.0, fix_emax = 0.0;

@@ -22,6 +22,7 @@
 
 #include "lmgpu_internal.cuh"
 #include "lmgpu_order.cuh"
+#include "lmgpu_series.cuh"
 
 namespace lmgpu {
 
@@ -122,7 +123,6 @@ __device__ __forceinline__ DF df_mul(DF x, DF y) {
     e = __fmaf_rn(x.l, y.h, e);
     return df_fast_two_sum(p, e);
 }
-__device__ __forceinline__ DF df_neg(DF x) { return DF{-x.h, -x.l}; }
 __device__ __forceinline__ DF df_re(float4 v) { return DF{v.x, v.y}; }
 __device__ __forceinline__ DF df_im(float4 v) { return DF{v.z, v.w}; }
 __device__ __forceinline__ DF df_from(double x) {
@@ -131,22 +131,38 @@ __device__ __forceinline__ DF df_from(double x) {
 }
 __device__ __forceinline__ double df_value(DF x) { return (double)x.h + (double)x.l; }
 
-// acc += h v on complex df values (h real when RE).
-template <bool RE>
-__device__ __forceinline__ void df_cfma(DF& ar, DF& ai, float4 h, float4 v) {
-    ar = df_add(ar, df_mul(df_re(h), df_re(v)));
-    if (!RE) ar = df_add(ar, df_neg(df_mul(df_im(h), df_im(v))));
-    ai = df_add(ai, df_mul(df_re(h), df_im(v)));
-    if (!RE) ai = df_add(ai, df_mul(df_im(h), df_re(v)));
+// hi + lo of a double: hi the nearest FP32 number, lo the remaining 28 bits rounded to FP32, by
+// integer operations (the conversions of the FP64 pipe run at 1.7 lanes per clock: a block of
+// 268 MB took 240 us with them, 95 us without).  Values below 2^-126 become 0; what overflows FP32
+// (infinities and NaN included) goes through the conversion.
+__device__ __forceinline__ DF df_split(double v) {
+    const int hw = __double2hiint(v);
+    const unsigned lw = (unsigned)__double2loint(v);
+    const int ex = (hw >> 20) & 0x7ff;
+    if (ex >= 1150) return DF{(float)v, 0.f};
+    if (ex <= 896 + 53) return ex <= 896 ? DF{0.f, 0.f} : DF{(float)v, (float)(v - (double)(float)v)};
+    const int sign = hw & 0x80000000;
+    int low = (int)(lw & 0x1fffffffu);
+    const int up = low >> 28;  // round to nearest: the next FP32 number and a negative remainder
+    low -= up << 29;
+    const float h = __int_as_float(sign | ((((hw & 0x7fffffff) - (896 << 20)) << 3 | (int)(lw >> 29)) + up));
+    const float l = __int2float_rn(low) * __int_as_float((ex - 896 - 52) << 23);
+    return DF{h, sign ? -l : l};
 }
 
-// In place: n double2 values -> n float4 df values (same bytes per element).
-__global__ void to_df_kernel(double2* __restrict__ a, int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double2 v = a[i];
-        const DF r = df_from(v.x), m = df_from(v.y);
-        reinterpret_cast<float4*>(a)[i] = make_float4(r.h, r.l, m.h, m.l);
-    }
+// out = in as df values, column by column (ld_in may differ from ld_out; in null: the identity).
+__global__ void to_df_kernel(const double2* __restrict__ in, int64_t ld_in, int64_t n, int64_t M, float4* __restrict__ out,
+                             int64_t ld_out) {
+    for (int64_t m = blockIdx.y; m < M; m += gridDim.y)
+        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+            if (!in) {
+                out[m * ld_out + i] = make_float4(i == m ? 1.f : 0.f, 0.f, 0.f, 0.f);
+                continue;
+            }
+            const double2 v = in[m * ld_in + i];
+            const DF r = df_split(v.x), q = df_split(v.y);
+            out[m * ld_out + i] = make_float4(r.h, r.l, q.h, q.l);
+        }
 }
 
 // The stencil tables in df form: hop (2N double2) -> 2N float4, diag (N double) -> N float2.
@@ -162,50 +178,219 @@ __global__ void df_tables_kernel(const double2* __restrict__ hop2, const double*
     }
 }
 
-// In place: n float4 df values -> n double2 values.
-__global__ void from_df_kernel(double2* __restrict__ a, int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float4 v = reinterpret_cast<const float4*>(a)[i];
-        a[i] = make_double2(df_value(DF{v.x, v.y}), df_value(DF{v.z, v.w}));
+// n x M df values -> ComplexF64 (out) or ComplexF32 (out32), leading dimension ld_out.
+__global__ void from_df_kernel(const float4* __restrict__ in, int64_t ld_in, int64_t n, int64_t M,
+                               double2* __restrict__ out, float2* __restrict__ out32, int64_t ld_out) {
+    for (int64_t m = blockIdx.y; m < M; m += gridDim.y)
+        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+            const float4 v = in[m * ld_in + i];
+            if (out) out[m * ld_out + i] = make_double2(df_value(DF{v.x, v.y}), df_value(DF{v.z, v.w}));
+            else out32[m * ld_out + i] = make_float2(v.x, v.z);
+        }
+}
+
+// One recurrence pass over an N x M block in df arithmetic: out = (2H~) tp - tpp (FIRST: out = H~ tp),
+// out may alias tpp.  A thread owns one row y of KT kets and walks along x: the three columns of tp
+// that a site needs lie in registers, so tp is read once per site from L2 (plus two shared-line reads
+// of the y-neighbours), and the tables once per KT kets.  With DOT the pass also forms
+// Re <tpp, tpp> and Re <tp, tpp> of every ket from the values it holds; with YACC, y += c out.
+// Products enter an unnormalised pair (s, c) by TwoSum, every error term c: 12 FP32 operations per
+// real product and sum; XR (x-hops all equal to the real alpha) adds the two x-neighbours first.
+//
+// What bounds it: HBM (three block passes: read tp and tpp, write out) and the FP32 pipe (about 215
+// operations per element) at about the same time: 119 us of traffic and 108 us of arithmetic for
+// 256 x 256 sites and 256 kets, measured 174 us (209 us with the loads of a column issued when it
+// is used), the dots included.  One thread per site with normalised sums took 258 us, and 113 us
+// more for the dots as a kernel of their own.
+struct MarchArgs {
+    Geom g;
+    const float4* hop;   // 2N: x-hops, then y-hops (2H/a)
+    const float2* diag;  // 2(V - b)/a
+    const float4* tp;
+    const float4* tpp;   // T_{n-1}; FIRST: unused
+    float4* out;
+    int64_t ld, M;
+    int rows, segs, cols;  // rows and x-segments per block, columns per segment
+    float2 alpha;
+    float4* y;
+    float2 c;
+    float2 c0;       // FIRST with YACC: y = c0 tp + c out
+    double* part;    // DOT: partial sums [block][2][pstride]
+    int64_t pstride;
+};
+
+__device__ __forceinline__ void df_madd(DF& a, float ch, float cl, float vh, float vl) {
+    const float p = __fmul_rn(ch, vh);
+    float e = __fmaf_rn(ch, vh, -p);
+    e = __fmaf_rn(ch, vl, e);
+    e = __fmaf_rn(cl, vh, e);
+    const float t = __fadd_rn(a.h, p);
+    const float bb = __fsub_rn(t, a.h);
+    e = __fadd_rn(e, __fadd_rn(__fsub_rn(a.h, __fsub_rn(t, bb)), __fsub_rn(p, bb)));
+    a.l = __fadd_rn(a.l, e);
+    a.h = t;
+}
+__device__ __forceinline__ void df_caddmul(DF& re, DF& im, float4 h, float4 v) {
+    df_madd(re, h.x, h.y, v.x, v.y);
+    df_madd(re, -h.z, -h.w, v.z, v.w);
+    df_madd(im, h.x, h.y, v.z, v.w);
+    df_madd(im, h.z, h.w, v.x, v.y);
+}
+__device__ __forceinline__ DF df_sum2(float uh, float ul, float vh, float vl) {  // u + v, unnormalised
+    const float t = __fadd_rn(uh, vh);
+    const float bb = __fsub_rn(t, uh);
+    const float e = __fadd_rn(__fsub_rn(uh, __fsub_rn(t, bb)), __fsub_rn(vh, bb));
+    return DF{t, __fadd_rn(e, __fadd_rn(ul, vl))};
+}
+
+template <bool XR, bool FIRST, bool DOT, bool YACC, int KT>
+__global__ void __launch_bounds__(256, 2) df_march_kernel(const __grid_constant__ MarchArgs a) {
+    const Geom& g = a.g;
+    const int Ly = (int)g.Ly, Lx = (int)g.Lx;
+    const int t = threadIdx.x, seg = t / a.rows, yl = t - seg * a.rows;
+    const int chunks = (Ly + a.rows - 1) / a.rows;
+    const int chunk = (int)(blockIdx.x % chunks);
+    const int y = chunk * a.rows + yl;
+    const int64_t xa = ((int64_t)(blockIdx.x / chunks) * a.segs + seg) * a.cols;
+    const bool on = seg < a.segs && y < Ly && xa < Lx;
+    const int xb = on ? (int)(xa + a.cols < Lx ? xa + a.cols : Lx) : 0;
+    const int yp = y + 1 < Ly ? 1 : (g.per_y ? 1 - Ly : 0);
+    const int ym = y > 0 ? -1 : (g.per_y ? Ly - 1 : 0);
+    const bool down = y > 0 || g.per_y;
+    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int64_t m0 = (int64_t)blockIdx.y * KT;
+    int64_t off[KT];
+    bool have[KT];
+#pragma unroll
+    for (int q = 0; q < KT; ++q) {
+        have[q] = m0 + q < a.M;
+        off[q] = (have[q] ? m0 + q : m0) * a.ld;
+    }
+    DF aa[KT], ba[KT];
+#pragma unroll
+    for (int q = 0; q < KT; ++q) aa[q] = ba[q] = DF{0.f, 0.f};
+    if (on) {
+        float4 tm[KT], tc[KT];
+        const int x0 = (int)xa;
+        const int xm = x0 > 0 ? x0 - 1 : (g.per_x ? Lx - 1 : -1);
+        float4 hxm = z4;
+        if (!XR && xm >= 0) hxm = a.hop[(int64_t)xm * Ly + y];
+#pragma unroll
+        for (int q = 0; q < KT; ++q) {
+            tm[q] = xm >= 0 ? __ldg(a.tp + off[q] + (int64_t)xm * Ly + y) : z4;
+            tc[q] = __ldg(a.tp + off[q] + (int64_t)x0 * Ly + y);
+        }
+        // the next column and the old value come from L2 or HBM: they are loaded one step ahead
+        float4 tn[KT], t2[KT];
+        const int xn = x0 + 1 < Lx ? x0 + 1 : (g.per_x ? 0 : -1);
+#pragma unroll
+        for (int q = 0; q < KT; ++q) {
+            tn[q] = xn >= 0 ? __ldg(a.tp + off[q] + (int64_t)xn * Ly + y) : z4;
+            t2[q] = FIRST ? z4 : a.tpp[off[q] + (int64_t)x0 * Ly + y];
+        }
+        for (int x = x0; x < xb; ++x) {
+            const int64_t s = (int64_t)x * Ly + y;
+            const int xp = x + 2 < Lx ? x + 2 : (g.per_x ? x + 2 - Lx : -1);
+            float4 up[KT], dn[KT], tn1[KT], t21[KT];
+#pragma unroll
+            for (int q = 0; q < KT; ++q) {
+                tn1[q] = xp >= 0 && x + 1 < xb ? __ldg(a.tp + off[q] + (int64_t)xp * Ly + y) : z4;
+                t21[q] = !FIRST && x + 1 < xb ? a.tpp[off[q] + s + Ly] : z4;
+                up[q] = __ldg(a.tp + off[q] + s + yp);
+                dn[q] = __ldg(a.tp + off[q] + s + ym);
+            }
+            const float4 hu = __ldg(a.hop + g.N + s);
+            float4 hd = down ? __ldg(a.hop + g.N + s + ym) : z4;
+            hd.z = -hd.z;
+            hd.w = -hd.w;
+            const float2 d = __ldg(a.diag + s);
+            float4 hxp = z4;
+            if (!XR) hxp = a.hop[s];
+#pragma unroll
+            for (int q = 0; q < KT; ++q) {
+                DF re = FIRST ? DF{0.f, 0.f} : DF{-t2[q].x, -t2[q].y}, im = FIRST ? DF{0.f, 0.f} : DF{-t2[q].z, -t2[q].w};
+                if (XR) {
+                    DF u = df_sum2(tm[q].x, tm[q].y, tn[q].x, tn[q].y);
+                    df_madd(re, a.alpha.x, a.alpha.y, u.h, u.l);
+                    u = df_sum2(tm[q].z, tm[q].w, tn[q].z, tn[q].w);
+                    df_madd(im, a.alpha.x, a.alpha.y, u.h, u.l);
+                } else {
+                    df_caddmul(re, im, hxp, tn[q]);
+                    df_caddmul(re, im, make_float4(hxm.x, hxm.y, -hxm.z, -hxm.w), tm[q]);
+                }
+                df_caddmul(re, im, hu, up[q]);
+                df_caddmul(re, im, hd, dn[q]);
+                df_madd(re, d.x, d.y, tc[q].x, tc[q].y);
+                df_madd(im, d.x, d.y, tc[q].z, tc[q].w);
+                re = df_fast_two_sum(re.h, re.l);
+                im = df_fast_two_sum(im.h, im.l);
+                if (FIRST) {
+                    re = DF{0.5f * re.h, 0.5f * re.l};
+                    im = DF{0.5f * im.h, 0.5f * im.l};
+                }
+                if (DOT) {
+                    df_madd(aa[q], t2[q].x, t2[q].y, t2[q].x, t2[q].y);
+                    df_madd(aa[q], t2[q].z, t2[q].w, t2[q].z, t2[q].w);
+                    df_madd(ba[q], tc[q].x, tc[q].y, t2[q].x, t2[q].y);
+                    df_madd(ba[q], tc[q].z, tc[q].w, t2[q].z, t2[q].w);
+                    aa[q] = df_fast_two_sum(aa[q].h, aa[q].l);  // long sums: keep the pairs normalised
+                    ba[q] = df_fast_two_sum(ba[q].h, ba[q].l);
+                }
+                if (have[q]) {
+                    a.out[off[q] + s] = make_float4(re.h, re.l, im.h, im.l);
+                    if (YACC) {
+                        DF yr{0.f, 0.f}, yi{0.f, 0.f};
+                        if (FIRST) {
+                            df_madd(yr, a.c0.x, a.c0.y, tc[q].x, tc[q].y);
+                            df_madd(yi, a.c0.x, a.c0.y, tc[q].z, tc[q].w);
+                        } else {
+                            const float4 u = a.y[off[q] + s];
+                            yr = DF{u.x, u.y};
+                            yi = DF{u.z, u.w};
+                        }
+                        df_madd(yr, a.c.x, a.c.y, re.h, re.l);
+                        df_madd(yi, a.c.x, a.c.y, im.h, im.l);
+                        yr = df_fast_two_sum(yr.h, yr.l);
+                        yi = df_fast_two_sum(yi.h, yi.l);
+                        a.y[off[q] + s] = make_float4(yr.h, yr.l, yi.h, yi.l);
+                    }
+                }
+                tm[q] = tc[q];
+                tc[q] = tn[q];
+                tn[q] = tn1[q];
+                t2[q] = t21[q];
+            }
+            if (!XR) hxm = hxp;
+        }
+    }
+    if (DOT) {  // df over the warp, FP64 over the block's warps in order
+        __shared__ double red[8][2 * KT];
+#pragma unroll
+        for (int q = 0; q < 2 * KT; ++q) {
+            DF v = q < KT ? aa[q < KT ? q : 0] : ba[q < KT ? 0 : q - KT];
+            v = df_fast_two_sum(v.h, v.l);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                v = df_add(v, DF{__shfl_xor_sync(0xffffffffu, v.h, o), __shfl_xor_sync(0xffffffffu, v.l, o)});
+            if ((t & 31) == 0) red[t >> 5][q] = df_value(v);
+        }
+        __syncthreads();
+        if (t < 2 * KT && m0 + t % KT < a.M) {
+            double v = 0.0;
+            for (int w = 0; w < (int)(blockDim.x + 31) / 32; ++w) v += red[w][t];
+            a.part[((int64_t)blockIdx.x * 2 + t / KT) * a.pstride + m0 + t % KT] = v;
+        }
     }
 }
 
-// out = (2H~) tp - tpp on df blocks (the tables hold 2H/a and 2(V-b)/a); out may alias tpp.
-// XR: every x-hop is real.  With y non-null also y += c out (c = c_hi + c_lo, the real
-// coefficient of a Chebyshev series, lm_cheb_apply).
-template <bool XR>
-__global__ void __launch_bounds__(256) df_recur_kernel(Geom g, const float4* __restrict__ hopd,
-                                                       const float2* __restrict__ diagd, const float4* tp,
-                                                       const float4* tpp, float4* out, int64_t ld, int64_t M,
-                                                       float4* __restrict__ y, float c_hi, float c_lo) {
-    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= g.N) return;
-    const Nbr nb = neighbours(g, s);
-    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 hxp = nb.hxp ? hopd[s] : z, hyp = nb.hyp ? hopd[g.N + s] : z;
-    float4 t = nb.hxm ? hopd[nb.xm] : z;
-    const float4 hxm = make_float4(t.x, t.y, -t.z, -t.w);  // conj of the hop from x-1
-    t = nb.hym ? hopd[g.N + nb.ym] : z;
-    const float4 hym = make_float4(t.x, t.y, -t.z, -t.w);
-    const float2 dd = diagd[s];
-    const float4 d = make_float4(dd.x, dd.y, 0.f, 0.f);
-    for (int64_t m = blockIdx.y; m < M; m += gridDim.y) {
-        const int64_t o = m * ld;
-        const float4 q = tpp[o + s];
-        DF ar = DF{-q.x, -q.y}, ai = DF{-q.z, -q.w};
-        df_cfma<XR>(ar, ai, hxp, tp[o + nb.xp]);
-        df_cfma<XR>(ar, ai, hxm, tp[o + nb.xm]);
-        df_cfma<false>(ar, ai, hyp, tp[o + nb.yp]);
-        df_cfma<false>(ar, ai, hym, tp[o + nb.ym]);
-        df_cfma<true>(ar, ai, d, tp[o + s]);
-        out[o + s] = make_float4(ar.h, ar.l, ai.h, ai.l);
-        if (y) {
-            const float4 u = y[o + s];
-            const DF c = DF{c_hi, c_lo};
-            const DF yr = df_add(DF{u.x, u.y}, df_mul(c, ar)), yi = df_add(DF{u.z, u.w}, df_mul(c, ai));
-            y[o + s] = make_float4(yr.h, yr.l, yi.h, yi.l);
-        }
-    }
+// out[pass][q][m] = sum of the blocks' partials [pass][block][2][M], in block order.
+__global__ void sum_parts_kernel(const double* __restrict__ part, int nblk, int64_t M, double* __restrict__ out) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= 2 * M) return;
+    const double* p = part + (int64_t)blockIdx.y * nblk * 2 * M + i;
+    double v = 0.0;
+    for (int b = 0; b < nblk; ++b) v += p[(int64_t)b * 2 * M];
+    out[(int64_t)blockIdx.y * 2 * M + i] = v;
 }
 
 // out[col] = Re <A, A>, out[M + col] = Re <B, A> per column, in df per thread and then the
@@ -315,6 +500,112 @@ static double tridiag_eig(const std::vector<double>& a, const std::vector<double
     return 0.5 * (lo + hi);
 }
 
+constexpr int kMarchKets = 2;  // kets per thread of the df passes
+constexpr int64_t kPartPasses = 16;  // passes whose partial dots are summed by one launch
+
+// Rows and segments of a block, columns per segment: the split whose waves of two 256-thread blocks
+// per SM are fullest, counting 1.5 columns for a segment's two shared edges.
+static void march_plan(const lm_ctx* ctx, const Geom& g, int64_t M, MarchArgs& a) {
+    a.rows = (int)std::min<int64_t>(g.Ly, 256);
+    a.segs = std::max(1, 256 / a.rows);
+    const int64_t chunks = (g.Ly + a.rows - 1) / a.rows, groups = (M + kMarchKets - 1) / kMarchKets;
+    const int64_t slots = 2ll * ctx->sm_count;
+    double best = 0.0;
+    a.cols = (int)g.Lx;
+    for (int64_t nseg = 1; nseg <= g.Lx; ++nseg) {
+        const int64_t cols = (g.Lx + nseg - 1) / nseg, n = (g.Lx + cols - 1) / cols;
+        const int64_t blocks = chunks * ((n + a.segs - 1) / a.segs) * groups;
+        const double eff = (double)g.Lx * (double)(chunks * groups) /
+                           ((double)((blocks + slots - 1) / slots * slots) * (double)a.segs * ((double)cols + 1.5));
+        if (eff > best) {
+            best = eff;
+            a.cols = (int)cols;
+        }
+        if (cols <= 4 || blocks > 64 * slots) break;
+    }
+}
+
+static int64_t march_blocks(const MarchArgs& a) {
+    const int64_t chunks = (a.g.Ly + a.rows - 1) / a.rows, n = (a.g.Lx + a.cols - 1) / a.cols;
+    return chunks * ((n + a.segs - 1) / a.segs);
+}
+
+template <bool XR>
+static cudaError_t launch_march(lm_ctx* ctx, const MarchArgs& a, bool first) {
+    const int threads = (a.rows * a.segs + 31) / 32 * 32;
+    for (int64_t m = 0; m < a.M; m += 65535ll * kMarchKets) {  // the grid's y extent is 65535
+        MarchArgs b = a;
+        b.M = std::min<int64_t>(a.M - m, 65535ll * kMarchKets);
+        b.tp += m * a.ld;
+        if (b.tpp) b.tpp += m * a.ld;
+        b.out += m * a.ld;
+        if (b.y) b.y += m * a.ld;
+        if (b.part) b.part += m;
+        const dim3 grid((unsigned)march_blocks(a), (unsigned)((b.M + kMarchKets - 1) / kMarchKets));
+        if (first && a.y) df_march_kernel<XR, true, false, true, kMarchKets><<<grid, threads, 0, ctx->stream>>>(b);
+        else if (first) df_march_kernel<XR, true, false, false, kMarchKets><<<grid, threads, 0, ctx->stream>>>(b);
+        else if (a.part) df_march_kernel<XR, false, true, false, kMarchKets><<<grid, threads, 0, ctx->stream>>>(b);
+        else df_march_kernel<XR, false, false, true, kMarchKets><<<grid, threads, 0, ctx->stream>>>(b);
+        ctx->launches++;
+    }
+    return cudaGetLastError();
+}
+
+static cudaError_t march(lm_ctx* ctx, const MarchArgs& a, bool xr, bool first = false) {
+    return xr ? launch_march<true>(ctx, a, first) : launch_march<false>(ctx, a, first);
+}
+
+// lm_cheb_apply with every column on chip through the whole series (lmgpu_series.cu): no recurrence
+// buffers and one read and one write of the block.
+static int cheb_apply_resident(lm_ham* h, const SeriesPlan& plan, double a, double b, const double* coef, int ncoef,
+                               const double2* in, int64_t ld_in, lm_state* out) {
+    lm_ctx* ctx = h->ctx;
+    const Geom& g = h->lat->g;
+    const size_t N = (size_t)g.N;
+    const bool xr = ham_x_real(h);
+    char* buf = nullptr;  // hops, gauge, diagonal, coefficients
+    const size_t o_g = sizeof(float4) * N, o_d = o_g + (xr ? 0 : sizeof(double2) * N), o_c = o_d + sizeof(float2) * N;
+    cudaError_t e = cudaMalloc((void**)&buf, o_c + sizeof(float2) * (size_t)ncoef);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return check_cuda(ctx, e, "lm_cheb_apply: allocation");
+    }
+    std::vector<float2> cd((size_t)ncoef);
+    for (int k = 0; k < ncoef; ++k) {
+        const float c = (float)coef[k];
+        cd[(size_t)k] = make_float2(c, (float)(coef[k] - (double)c));
+    }
+    double2* gauge = xr ? nullptr : (double2*)(buf + o_g);
+    e = cudaMemcpyAsync(buf + o_c, cd.data(), sizeof(float2) * (size_t)ncoef, cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess)
+        e = launch_gauge_tables(ctx, g, h->d_hop, h->d_onsite, h->t1, a, b, xr, gauge, nullptr, nullptr, (float4*)buf,
+                                (float2*)(buf + o_d));
+    if (e == cudaSuccess) {
+        SeriesArgs r;
+        r.Lx = (int)g.Lx;
+        r.Ly = (int)g.Ly;
+        r.per_x = g.per_x;
+        r.per_y = g.per_y;
+        r.K = ncoef - 1;
+        r.M = out->m;
+        r.in = in;
+        r.ld_in = ld_in;
+        r.ld_out = out->ld;
+        if (out->precision == LM_C64) r.out = (double2*)out->d_data;
+        else r.out32 = (float2*)out->d_data;
+        r.gauge = gauge;
+        r.hy = buf;
+        r.diag = buf + o_d;
+        r.alpha = 2.0 * h->t1 / a;
+        r.cd = (const float2*)(buf + o_c);
+        e = launch_series_df(ctx, plan, r);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    const int rc = e == cudaSuccess ? LM_OK : check_cuda(ctx, e, "lm_cheb_apply: on-chip series");
+    cudaFree(buf);
+    return rc;
+}
+
 extern "C" {
 
 int lm_kpm_moments(lm_ham* h, double emin, double emax, int nmom, const lm_state* vecs, int per_column,
@@ -350,10 +641,18 @@ int lm_kpm_moments(lm_ham* h, double emin, double emax, int nmom, const lm_state
     const bool use_df = ctx->kpm_df != 0;
     const size_t blk = sizeof(double2) * (size_t)ld * (size_t)M;
     const size_t ndots = (size_t)(nsteps + 1) * 2 * (size_t)M;
+    const bool xr = ham_x_real(h);
+    MarchArgs ma{};
+    ma.g = g;
+    ma.ld = ld;
+    ma.M = ma.pstride = M;
+    march_plan(ctx, g, M, ma);
+    const int64_t nblk = march_blocks(ma);
+    double* part = nullptr;  // partial dots of kPartPasses passes
     auto release = [&]() {
         cudaStreamSynchronize(ctx->stream);
         cudaFree(hop2); cudaFree(diag2); cudaFree(hop2f); cudaFree(diag2f);
-        cudaFree(TA); cudaFree(TB); cudaFree(dots); cudaFree(hopd); cudaFree(diagd);
+        cudaFree(TA); cudaFree(TB); cudaFree(dots); cudaFree(hopd); cudaFree(diagd); cudaFree(part);
     };
     cudaError_t e = cudaMalloc((void**)&hop2, sizeof(double2) * 2 * (size_t)N);
     if (e == cudaSuccess) e = cudaMalloc((void**)&diag2, sizeof(double) * (size_t)N);
@@ -364,6 +663,8 @@ int lm_kpm_moments(lm_ham* h, double emin, double emax, int nmom, const lm_state
     if (e == cudaSuccess) e = cudaMalloc((void**)&dots, sizeof(double) * ndots);
     if (e == cudaSuccess && use_df) e = cudaMalloc((void**)&hopd, sizeof(float4) * 2 * (size_t)N);
     if (e == cudaSuccess && use_df) e = cudaMalloc((void**)&diagd, sizeof(float2) * (size_t)N);
+    if (e == cudaSuccess && use_df)
+        e = cudaMalloc((void**)&part, sizeof(double) * (size_t)(kPartPasses * nblk * 2 * M));
     if (e != cudaSuccess) {
         cudaGetLastError();
         release();
@@ -376,64 +677,75 @@ int lm_kpm_moments(lm_ham* h, double emin, double emax, int nmom, const lm_state
     };
     e = launch_normalise(ctx, g, h->d_hop, h->d_onsite, a, b, hop2, diag2, hop2f, diag2f);
     if (e != cudaSuccess) return fail(e, "lm_kpm_moments: tables");
-    if (vecs) {
-        e = cudaMemcpy2DAsync(TA, sizeof(double2) * (size_t)ld, vecs->d_data, sizeof(double2) * (size_t)vecs->ld,
-                              sizeof(double2) * (size_t)N, (size_t)M, cudaMemcpyDeviceToDevice, ctx->stream);
-    } else {
-        const dim3 grid((unsigned)((N + 255) / 256), (unsigned)(N < 65535 ? N : 65535));
-        set_identity_kernel<<<grid, 256, 0, ctx->stream>>>(TA, N, ld);
-        ctx->launches++;
-        e = cudaGetLastError();
-    }
-    if (e != cudaSuccess) return fail(e, "lm_kpm_moments: starting block");
     const unsigned dgrid = (unsigned)(M < 65535 ? M : 65535);
-    // T_1 = H~ T_0
-    const bool xr = ham_x_real(h);
-    e = launch_stencil_recur(ctx, g, LM_C64, hop2, diag2, TA, nullptr, nullptr, TB, ld, M, 0.5, 0.0, 0.0, nullptr, 0.0,
-                             xr);
-    if (e != cudaSuccess) return fail(e, "lm_kpm_moments: recurrence");
-    if (use_df) {  // T_0 and T_1 (FP64) become double-float in place; so do the tables
-        const unsigned cgrid = (unsigned)std::min<int64_t>((ld * M + 255) / 256, 65535);
+    if (use_df) {
         df_tables_kernel<<<(unsigned)std::min<int64_t>((2 * N + 255) / 256, 65535), 256, 0, ctx->stream>>>(
             hop2, diag2, N, hopd, diagd);
-        to_df_kernel<<<cgrid, 256, 0, ctx->stream>>>(TA, ld * M);
-        to_df_kernel<<<cgrid, 256, 0, ctx->stream>>>(TB, ld * M);
-        ctx->launches += 3;
+        to_df_kernel<<<dim3((unsigned)std::min<int64_t>((N + 255) / 256, 65535), dgrid), 256, 0, ctx->stream>>>(
+            vecs ? (const double2*)vecs->d_data : nullptr, ld, N, M, (float4*)TA, ld);
+        ctx->launches += 2;
         e = cudaGetLastError();
         if (e != cudaSuccess) return fail(e, "lm_kpm_moments: double-float conversion");
-    }
-    const dim3 rgrid((unsigned)((N + 255) / 256), (unsigned)(M < 65535 ? M : 65535));
-    double2* Tn = TA;   // T_n
-    double2* Tn1 = TB;  // T_{n+1}
-    for (int64_t n = 0; n <= nsteps; ++n) {
-        double* d = dots + (size_t)n * 2 * (size_t)M;
-        if (use_df) {
-            column_dots2_df_kernel<<<dgrid, 256, 0, ctx->stream>>>((const float4*)Tn, (const float4*)Tn1, N, ld, M, d);
-            ctx->launches += 1;
+        const double al = h->t1 * (2.0 / a);
+        ma.hop = hopd;
+        ma.diag = diagd;
+        ma.alpha = make_float2((float)al, (float)(al - (double)(float)al));
+        ma.tp = (const float4*)TA;
+        ma.out = (float4*)TB;
+        e = march(ctx, ma, xr, true);  // T_1 = H~ T_0
+        if (e != cudaSuccess) return fail(e, "lm_kpm_moments: recurrence");
+        float4* Tn = (float4*)TA;   // T_n
+        float4* Tn1 = (float4*)TB;  // T_{n+1}
+        for (int64_t n = 0; n < nsteps; ++n) {  // T_{n+2} over T_n, and the dots of T_n and T_{n+1}
+            ma.tp = Tn1;
+            ma.tpp = Tn;
+            ma.out = Tn;
+            ma.part = part + (n % kPartPasses) * nblk * 2 * M;
+            e = march(ctx, ma, xr);
+            if (e != cudaSuccess) return fail(e, "lm_kpm_moments: recurrence");
+            std::swap(Tn, Tn1);
+            const int64_t np = n % kPartPasses + 1;
+            if (np == kPartPasses || n + 1 == nsteps) {
+                sum_parts_kernel<<<dim3((unsigned)((2 * M + 127) / 128), (unsigned)np), 128, 0, ctx->stream>>>(
+                    part, (int)nblk, M, dots + (size_t)(n + 1 - np) * 2 * (size_t)M);
+                ctx->launches++;
+            }
+        }
+        column_dots2_df_kernel<<<dgrid, 256, 0, ctx->stream>>>(Tn, Tn1, N, ld, M, dots + (size_t)nsteps * 2 * (size_t)M);
+        ctx->launches++;
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return fail(e, "lm_kpm_moments: dots");
+    } else {
+        if (vecs) {
+            e = cudaMemcpy2DAsync(TA, sizeof(double2) * (size_t)ld, vecs->d_data, sizeof(double2) * (size_t)vecs->ld,
+                                  sizeof(double2) * (size_t)N, (size_t)M, cudaMemcpyDeviceToDevice, ctx->stream);
         } else {
+            const dim3 grid((unsigned)((N + 255) / 256), (unsigned)(N < 65535 ? N : 65535));
+            set_identity_kernel<<<grid, 256, 0, ctx->stream>>>(TA, N, ld);
+            ctx->launches++;
+            e = cudaGetLastError();
+        }
+        if (e != cudaSuccess) return fail(e, "lm_kpm_moments: starting block");
+        // T_1 = H~ T_0
+        e = launch_stencil_recur(ctx, g, LM_C64, hop2, diag2, TA, nullptr, nullptr, TB, ld, M, 0.5, 0.0, 0.0, nullptr,
+                                 0.0, xr);
+        if (e != cudaSuccess) return fail(e, "lm_kpm_moments: recurrence");
+        double2* Tn = TA;   // T_n
+        double2* Tn1 = TB;  // T_{n+1}
+        for (int64_t n = 0; n <= nsteps; ++n) {
+            double* d = dots + (size_t)n * 2 * (size_t)M;
             column_dots_kernel<<<dgrid, 256, 0, ctx->stream>>>(Tn, Tn, N, ld, M, d);
             column_dots_kernel<<<dgrid, 256, 0, ctx->stream>>>(Tn1, Tn, N, ld, M, d + M);
             ctx->launches += 2;
-        }
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return fail(e, "lm_kpm_moments: dots");
-        if (n == nsteps) break;
-        // T_{n+2} = 2 H~ T_{n+1} - T_n, written over T_n
-        if (use_df) {
-            if (xr) df_recur_kernel<true><<<rgrid, 256, 0, ctx->stream>>>(g, hopd, diagd, (const float4*)Tn1,
-                                                                          (const float4*)Tn, (float4*)Tn, ld, M,
-                                                                          nullptr, 0.f, 0.f);
-            else df_recur_kernel<false><<<rgrid, 256, 0, ctx->stream>>>(g, hopd, diagd, (const float4*)Tn1,
-                                                                        (const float4*)Tn, (float4*)Tn, ld, M,
-                                                                        nullptr, 0.f, 0.f);
-            ctx->launches++;
             e = cudaGetLastError();
-        } else {
+            if (e != cudaSuccess) return fail(e, "lm_kpm_moments: dots");
+            if (n == nsteps) break;
+            // T_{n+2} = 2 H~ T_{n+1} - T_n, written over T_n
             e = launch_stencil_recur(ctx, g, LM_C64, hop2, diag2, Tn1, Tn, nullptr, Tn, ld, M, 1.0, 0.0, 0.0, nullptr,
                                      0.0, xr);
+            if (e != cudaSuccess) return fail(e, "lm_kpm_moments: recurrence");
+            std::swap(Tn, Tn1);
         }
-        if (e != cudaSuccess) return fail(e, "lm_kpm_moments: recurrence");
-        std::swap(Tn, Tn1);
     }
     std::vector<double> hd(ndots);
     e = cudaMemcpyAsync(hd.data(), dots, sizeof(double) * ndots, cudaMemcpyDeviceToHost, ctx->stream);
@@ -492,6 +804,12 @@ int lm_cheb_apply(lm_ham* h, double emin, double emax, const double* coef, int n
     float2* diagd = nullptr;
     const bool use_df = ctx->kpm_df != 0 && ncoef > 2;
     const int64_t ld = N;
+    if (use_df && (!in || in->precision == LM_C64)) {
+        const SeriesPlan plan = series_plan(ctx, g, ham_x_real(h), M, true);
+        if (plan.kt)
+            return cheb_apply_resident(h, plan, a, b, coef, ncoef, in ? (const double2*)in->d_data : nullptr,
+                                       in ? in->ld : 0, out);
+    }
     const size_t blk = sizeof(double2) * (size_t)ld * (size_t)M;
     auto release = [&]() {
         cudaStreamSynchronize(ctx->stream);
@@ -519,7 +837,57 @@ int lm_cheb_apply(lm_ham* h, double emin, double emax, const double* coef, int n
     };
     e = launch_normalise(ctx, g, h->d_hop, h->d_onsite, a, b, hop2, diag2, hop2f, diag2f);
     if (e != cudaSuccess) return fail(e, "lm_cheb_apply: tables");
+    const bool xr = ham_x_real(h);
     // T_0
+    const dim3 cgrid((unsigned)std::min<int64_t>((N + 255) / 256, 65535), (unsigned)std::min<int64_t>(M, 65535));
+    if (in && in->precision != LM_C64) {
+        e = launch_convert(ctx, LM_C64, in->d_data, TA, N, M, in->ld, ld);
+        if (e != cudaSuccess) return fail(e, "lm_cheb_apply: input block");
+    }
+    if (use_df) {
+        const bool conv = in && in->precision != LM_C64;
+        df_tables_kernel<<<(unsigned)std::min<int64_t>((2 * N + 255) / 256, 65535), 256, 0, ctx->stream>>>(
+            hop2, diag2, N, hopd, diagd);
+        to_df_kernel<<<cgrid, 256, 0, ctx->stream>>>(conv ? TA : in ? (const double2*)in->d_data : nullptr,
+                                                     conv || !in ? ld : in->ld, N, M, (float4*)TA, ld);
+        ctx->launches += 2;
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return fail(e, "lm_cheb_apply: double-float conversion");
+        auto split = [](double v) { return make_float2((float)v, (float)(v - (double)(float)v)); };
+        MarchArgs ma{};
+        ma.g = g;
+        ma.ld = ld;
+        ma.M = M;
+        march_plan(ctx, g, M, ma);
+        ma.hop = hopd;
+        ma.diag = diagd;
+        ma.alpha = split(h->t1 * (2.0 / a));
+        ma.y = (float4*)Y;
+        ma.c0 = split(coef[0]);
+        ma.c = split(coef[1]);
+        ma.tp = (const float4*)TA;
+        ma.out = (float4*)TB;
+        e = march(ctx, ma, xr, true);  // T_1 = H~ T_0, Y = c_0 T_0 + c_1 T_1
+        float4* Tprev = (float4*)TA;
+        float4* Tn = (float4*)TB;
+        for (int k = 2; k < ncoef && e == cudaSuccess; ++k) {  // T_{n+1} over T_{n-1}, Y += c_{n+1} T_{n+1}
+            ma.tp = Tn;
+            ma.tpp = Tprev;
+            ma.out = Tprev;
+            ma.c = split(coef[k]);
+            e = march(ctx, ma, xr);
+            std::swap(Tprev, Tn);
+        }
+        if (e != cudaSuccess) return fail(e, "lm_cheb_apply: recurrence");
+        from_df_kernel<<<cgrid, 256, 0, ctx->stream>>>((const float4*)Y, ld, N, M,
+                                                       out->precision == LM_C64 ? (double2*)out->d_data : nullptr,
+                                                       (float2*)out->d_data, out->ld);
+        ctx->launches++;
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return fail(e, "lm_cheb_apply: output");
+        release();
+        return LM_OK;
+    }
     if (!in) {
         const dim3 grid((unsigned)((N + 255) / 256), (unsigned)(N < 65535 ? N : 65535));
         set_identity_kernel<<<grid, 256, 0, ctx->stream>>>(TA, N, ld);
@@ -528,8 +896,6 @@ int lm_cheb_apply(lm_ham* h, double emin, double emax, const double* coef, int n
     } else if (in->precision == LM_C64) {
         e = cudaMemcpy2DAsync(TA, sizeof(double2) * (size_t)ld, in->d_data, sizeof(double2) * (size_t)in->ld,
                               sizeof(double2) * (size_t)N, (size_t)M, cudaMemcpyDeviceToDevice, ctx->stream);
-    } else {
-        e = launch_convert(ctx, LM_C64, in->d_data, TA, N, M, in->ld, ld);
     }
     if (e != cudaSuccess) return fail(e, "lm_cheb_apply: input block");
     // Y = c_0 T_0
@@ -538,48 +904,16 @@ int lm_cheb_apply(lm_ham* h, double emin, double emax, const double* coef, int n
     if (e != cudaSuccess) return fail(e, "lm_cheb_apply: first term");
     if (ncoef > 1) {
         // T_1 = H~ T_0, Y += c_1 T_1; then T_{n+1} = 2 H~ T_n - T_{n-1} over T_{n-1}, Y += c_{n+1} T_{n+1}
-        const bool xr = ham_x_real(h);
         e = launch_stencil_recur(ctx, g, LM_C64, hop2, diag2, TA, nullptr, nullptr, TB, ld, M, 0.5, 0.0, 0.0, Y,
                                  coef[1], xr);
-        if (e != cudaSuccess) return fail(e, "lm_cheb_apply: recurrence");
         double2* Tprev = TA;
         double2* Tn = TB;
-        const unsigned cgrid = (unsigned)std::min<int64_t>((ld * M + 255) / 256, 65535);
-        if (use_df) {  // T_0, T_1 and Y (FP64 so far) become double-float in place; so do the tables
-            df_tables_kernel<<<(unsigned)std::min<int64_t>((2 * N + 255) / 256, 65535), 256, 0, ctx->stream>>>(
-                hop2, diag2, N, hopd, diagd);
-            to_df_kernel<<<cgrid, 256, 0, ctx->stream>>>(TA, ld * M);
-            to_df_kernel<<<cgrid, 256, 0, ctx->stream>>>(TB, ld * M);
-            to_df_kernel<<<cgrid, 256, 0, ctx->stream>>>(Y, ld * M);
-            ctx->launches += 4;
-            e = cudaGetLastError();
-            if (e != cudaSuccess) return fail(e, "lm_cheb_apply: double-float conversion");
-        }
-        const dim3 rgrid((unsigned)((N + 255) / 256), (unsigned)(M < 65535 ? M : 65535));
-        for (int k = 2; k < ncoef; ++k) {
-            if (use_df) {
-                const float c_hi = (float)coef[k], c_lo = (float)(coef[k] - (double)c_hi);
-                if (xr) df_recur_kernel<true><<<rgrid, 256, 0, ctx->stream>>>(g, hopd, diagd, (const float4*)Tn,
-                                                                              (const float4*)Tprev, (float4*)Tprev,
-                                                                              ld, M, (float4*)Y, c_hi, c_lo);
-                else df_recur_kernel<false><<<rgrid, 256, 0, ctx->stream>>>(g, hopd, diagd, (const float4*)Tn,
-                                                                            (const float4*)Tprev, (float4*)Tprev,
-                                                                            ld, M, (float4*)Y, c_hi, c_lo);
-                ctx->launches++;
-                e = cudaGetLastError();
-            } else {
-                e = launch_stencil_recur(ctx, g, LM_C64, hop2, diag2, Tn, Tprev, nullptr, Tprev, ld, M, 1.0, 0.0, 0.0,
-                                         Y, coef[k], xr);
-            }
-            if (e != cudaSuccess) return fail(e, "lm_cheb_apply: recurrence");
+        for (int k = 2; k < ncoef && e == cudaSuccess; ++k) {
+            e = launch_stencil_recur(ctx, g, LM_C64, hop2, diag2, Tn, Tprev, nullptr, Tprev, ld, M, 1.0, 0.0, 0.0, Y,
+                                     coef[k], xr);
             std::swap(Tprev, Tn);
         }
-        if (use_df) {
-            from_df_kernel<<<cgrid, 256, 0, ctx->stream>>>(Y, ld * M);
-            ctx->launches++;
-            e = cudaGetLastError();
-            if (e != cudaSuccess) return fail(e, "lm_cheb_apply: double-float conversion");
-        }
+        if (e != cudaSuccess) return fail(e, "lm_cheb_apply: recurrence");
     }
     if (out->precision == LM_C64)
         e = cudaMemcpy2DAsync(out->d_data, sizeof(double2) * (size_t)out->ld, Y, sizeof(double2) * (size_t)ld,
