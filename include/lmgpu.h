@@ -190,6 +190,9 @@ int lm_solver_order(const lm_solver *s, int *K, double *a, double *b);
 /* step!(solver, state, cache) (src/evolution.jl:69-78): psi <- U psi for kets,
  * P <- U P U^dagger for a density matrix. */
 int lm_solver_step(lm_solver *s, lm_state *st);
+/* dst <- U src (two states of the same shape, kind and precision; src is not changed): the state
+ * copy and the step in one pass where the step's form allows it. */
+int lm_solver_step_to(lm_solver *s, const lm_state *src, lm_state *dst);
 
 /* Chebyshev plan (host only, needs no GPU): for x = a*|dt| >= 0 (a = spectral half-width)
  * the order K >= 2 whose neglected tail 2*sum_{k>K}|J_k(x)| is below `tol`, and the

@@ -13,9 +13,11 @@
 // For an on-site potential V_i, < beta, D~ T > = conj(beta_i) T_i / a summed over kets; for a
 // field amplitude A, dH[s, s+e]/dA = -2 pi i LI_e(A = 1) H[s, s+e] on every bond.
 //
-// lm_adjoint_step recomputes T_0 .. T_{K-1} from psi_n, then runs the beta recurrence and the
-// gradient sums in one fused pass per order (FP64 results; c32 sums in double-float); the caller applies U^dagger to lambda with a solver
-// updated for -dt (the same polynomial with conjugate coefficients).
+// lm_adjoint_step recomputes T_0 .. T_{K-1} from psi_n, then runs the beta recurrence and the gradient
+// sums (FP64 results; c32 sums in double-float): ComplexF32 kets that fit on chip take one lattice-resident
+// launch per recurrence and one kernel for the sums over all orders, the others one launch per order,
+// beta and its sums in one pass.  The caller applies U^dagger to lambda with a solver updated for -dt
+// (the same polynomial with conjugate coefficients).
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -25,6 +27,7 @@
 
 #include "lmgpu_internal.cuh"
 #include "lmgpu_order.cuh"
+#include "lmgpu_resident.cuh"
 
 namespace lmgpu {
 
@@ -120,6 +123,47 @@ cudaError_t launch_stencil_recur(lm_ctx* ctx, const Geom& g, int precision, cons
     return cudaGetLastError();
 }
 
+// A block's gradient contributions from the sums of its 8 warps (added in warp order): gV_part of its 32
+// sites and gA_part of the block, one writer per entry and launch.
+__device__ __forceinline__ void grad_block_out(const Geom& g, const Nbr& nb, int64_t s, int lane, int warp,
+                                               const double (&red)[8][10][32], const double2* dhop, double ph_re,
+                                               double ph_im, double f, double* gV_part, double* gA_part) {
+    if (warp != 0) return;
+    double v[10];
+#pragma unroll
+    for (int q = 0; q < 10; ++q) {
+        double t = 0.0;
+        for (int w = 0; w < 8; ++w) t += red[w][q][lane];
+        v[q] = t;
+    }
+    double ga = 0.0;
+    if (s < g.N) {
+        gV_part[(int64_t)blockIdx.y * g.N + s] += f * (ph_re * v[0] - ph_im * v[1]);
+        if (dhop) {
+            const double2 zz = make_double2(0.0, 0.0);
+            const double2 D[4] = {nb.hxp ? dhop[s] : zz, nb.hyp ? dhop[g.N + s] : zz, nb.hxm ? dhop[nb.xm] : zz,
+                                  nb.hym ? dhop[g.N + nb.ym] : zz};
+            double zr = 0.0, zi = 0.0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const double sr = v[2 + 2 * q], si = v[3 + 2 * q];
+                if (q < 2) {  // D S
+                    zr += D[q].x * sr - D[q].y * si;
+                    zi += D[q].x * si + D[q].y * sr;
+                } else {      // conj(D) S
+                    zr += D[q].x * sr + D[q].y * si;
+                    zi += D[q].x * si - D[q].y * sr;
+                }
+            }
+            ga = f * (ph_re * zr - ph_im * zi);
+        }
+    }
+    if (gA_part) {
+        for (int o = 16; o > 0; o >>= 1) ga += __shfl_down_sync(0xffffffffu, ga, o);
+        if (lane == 0) gA_part[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] += ga;
+    }
+}
+
 // One order k of the adjoint, fused: the beta recurrence and the gradient sums in one pass.
 //   beta_k = conj(c_k) lambda + (2H~) beta_{k+1} - beta_{k+2}         (written to bk)
 //   gV[s] += f Re( ph * sum_m conj(beta_k,sm) T_sm )
@@ -200,40 +244,79 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 3 : 2) adj_b
 #pragma unroll
     for (int q = 0; q < 10; ++q) red[warp][q][lane] = a[q].get();
     __syncthreads();
-    if (warp != 0) return;
-    double v[10];
-#pragma unroll
-    for (int q = 0; q < 10; ++q) {
-        double t = 0.0;
-        for (int w = 0; w < 8; ++w) t += red[w][q][lane];
-        v[q] = t;
-    }
-    double ga = 0.0;
+    grad_block_out(g, nb, s, lane, warp, red, dhop, ph_re, ph_im, f, gV_part, gA_part);
+}
+
+// The gradient sums of a whole step from all its T_{k-1} and beta_k (which the lattice-resident kernels
+// wrote to HBM): the sums of adj_beta_grad_kernel<float> over every order at once, so that the ten
+// double-float accumulators of a site are reduced and written once per step.  The orders' factors 1/a
+// and 2/a become 2/a with beta_1 halved (exact).
+//
+// What bounds it: FP32 issue, 20 double-float products (10 operations each) per site, ket and order.  On
+// 64 x 64 sites with 1024 kets and K = 6 a step took 5 recurrence launches of 41 us and 6 fused
+// passes of 102 us; now T_k and beta_k take 62 + 81 us on chip (each writes 200 MB) and the sums 236 us
+// (294 us without the loads one (ket, order) ahead; the products and sums alone are 134 us).
+struct GradOrders {
+    const float2* T[kResMaxK];      // T_0 .. T_{K-1}
+    const float2* b[kResMaxK + 1];  // beta_1 .. beta_K
+};
+
+__global__ void __launch_bounds__(256, 3) adj_sums_kernel(Geom g, const __grid_constant__ GradOrders ord, int K,
+                                                          const double2* __restrict__ dhop, int64_t ld, int64_t M,
+                                                          int64_t mchunk, double ph_re, double ph_im, double f,
+                                                          double* __restrict__ gV_part, double* __restrict__ gA_part) {
+    __shared__ double red[8][10][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t s = (int64_t)blockIdx.x * 32 + lane;
+    const int64_t m0 = (int64_t)blockIdx.y * mchunk, m1 = min(M, m0 + mchunk);
+    Acc<float> a[10];  // conj(b)T_s (re, im); S1x; S1y; S2x; S2y
+    Nbr nb;
     if (s < g.N) {
-        gV_part[(int64_t)blockIdx.y * g.N + s] += f * (ph_re * v[0] - ph_im * v[1]);
-        if (dhop) {
-            const double2 zz = make_double2(0.0, 0.0);
-            const double2 D[4] = {nb.hxp ? dhop[s] : zz, nb.hyp ? dhop[g.N + s] : zz, nb.hxm ? dhop[nb.xm] : zz,
-                                  nb.hym ? dhop[g.N + nb.ym] : zz};
-            double zr = 0.0, zi = 0.0;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const double sr = v[2 + 2 * q], si = v[3 + 2 * q];
-                if (q < 2) {  // D S
-                    zr += D[q].x * sr - D[q].y * si;
-                    zi += D[q].x * si + D[q].y * sr;
-                } else {      // conj(D) S
-                    zr += D[q].x * sr + D[q].y * si;
-                    zi += D[q].x * si - D[q].y * sr;
-                }
+        nb = neighbours(g, s);
+        const int xp = (int)(nb.xp - s), yp = (int)(nb.yp - s), xm = (int)(nb.xm - s), ym = (int)(nb.ym - s);
+        // beta, T and T's neighbours of the next (ket, order) are loaded while this one is summed
+        float2 v[6], w[6];
+        auto load = [&](float2 (&d)[6], int64_t m, int k) {
+            const float2* T = ord.T[k - 1] + m * ld + s;
+            d[0] = ord.b[k][m * ld + s];
+            d[1] = T[0];
+            if (dhop) {
+                d[2] = T[xp];
+                d[3] = T[yp];
+                d[4] = T[xm];
+                d[5] = T[ym];
             }
-            ga = f * (ph_re * zr - ph_im * zi);
+        };
+        auto sum = [&](const float2 (&d)[6], int k) {
+            const float2 b = k == 1 ? make_float2(0.5f * d[0].x, 0.5f * d[0].y) : d[0];
+#pragma unroll
+            for (int q = 0; q < 5; ++q) {  // conj(b) T at the site and its neighbours
+                if (q > 0 && !dhop) break;
+                a[2 * q].add_prod(b.x, d[1 + q].x);
+                a[2 * q].add_prod(b.y, d[1 + q].y);
+                a[2 * q + 1].add_prod(b.x, d[1 + q].y);
+                a[2 * q + 1].add_prod(-b.y, d[1 + q].x);
+            }
+        };
+        int64_t m = m0 + warp;
+        if (m < m1) load(v, m, 1);
+        int k = 1;
+        while (m < m1) {
+            int k2 = k < K ? k + 1 : 1;
+            int64_t m2 = k < K ? m : m + 8;
+            if (m2 < m1) load(w, m2, k2);
+            sum(v, k);
+            if (m2 >= m1) break;
+            k = k2 < K ? k2 + 1 : 1;
+            m = k2 < K ? m2 : m2 + 8;
+            if (m < m1) load(v, m, k);
+            sum(w, k2);
         }
     }
-    if (gA_part) {
-        for (int o = 16; o > 0; o >>= 1) ga += __shfl_down_sync(0xffffffffu, ga, o);
-        if (lane == 0) gA_part[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] += ga;
-    }
+#pragma unroll
+    for (int q = 0; q < 10; ++q) red[warp][q][lane] = a[q].get();
+    __syncthreads();
+    grad_block_out(g, nb, s, lane, warp, red, dhop, ph_re, ph_im, f, gV_part, gA_part);
 }
 
 // rho_s = sum_m |psi_sm|^2; loss = sum_s (rho_s - target_s)^2; lambda = 4 (rho_s - target_s) psi.
@@ -287,14 +370,12 @@ __global__ void flux_derivative_kernel(Geom g, FieldSet f, int comp, const doubl
     one.amp[0] = 1.0;
     const int64_t xi = s / g.Ly, yi = s - xi * g.Ly;
     const double x1 = (double)(xi + 1), y1 = (double)(yi + 1);
-#pragma unroll
-    for (int dir = 0; dir < 2; ++dir) {
-        const double x2 = dir == 0 ? x1 + 1.0 : x1, y2 = dir == 0 ? y1 : y1 + 1.0;
-        const double li = field_line_integral(g, one, x1, y1, x2, y2);
-        const double2 h = hop[dir * g.N + s];
-        const double w = -2.0 * M_PI * li;  // d/dA e^{-2 pi i A li} = -2 pi i li (...)
-        dhop[dir * g.N + s] = make_double2(-w * h.y, w * h.x);  // (i w) h
-    }
+    const int dir = blockIdx.y;  // a direction per thread, as in the assembly
+    const double x2 = dir == 0 ? x1 + 1.0 : x1, y2 = dir == 0 ? y1 : y1 + 1.0;
+    const double li = field_line_integral(g, one, x1, y1, x2, y2);
+    const double2 h = hop[dir * g.N + s];
+    const double w = -2.0 * M_PI * li;  // d/dA e^{-2 pi i A li} = -2 pi i li (...)
+    dhop[dir * g.N + s] = make_double2(-w * h.y, w * h.x);  // (i w) h
 }
 
 }  // namespace lmgpu
@@ -308,7 +389,7 @@ struct lm_adjoint {
     size_t elem = 16;
     int K = 0;
     std::vector<void*> T;  // T_0 .. T_{K-1} (T_0 aliases psi during a step)
-    void* B[3] = {nullptr, nullptr, nullptr};
+    std::vector<void*> B;  // beta_k by order (lattice-resident form) or three rotating blocks
     double* d_gV = nullptr;     // per ket chunk, one partial per site (nchunk x n)
     double* d_gA = nullptr;     // per gradient slot, one partial per (chunk, 32-site block)
     int nslots = 0;
@@ -323,10 +404,9 @@ static void adj_free_stack(lm_adjoint* a) {
     for (size_t i = 1; i < a->T.size(); ++i)
         if (a->T[i]) cudaFree(a->T[i]);
     a->T.clear();
-    for (auto& b : a->B) {
+    for (auto& b : a->B)
         if (b) cudaFree(b);
-        b = nullptr;
-    }
+    a->B.clear();
 }
 
 static int adj_alloc(lm_ctx* ctx, void** p, size_t bytes) {
@@ -338,8 +418,9 @@ static int adj_alloc(lm_ctx* ctx, void** p, size_t bytes) {
     return LM_OK;
 }
 
-static int adj_ensure_stack(lm_adjoint* a, int K) {
-    if (a->K == K && !a->T.empty()) return LM_OK;
+static int adj_ensure_stack(lm_adjoint* a, int K, bool all_beta) {
+    const size_t nb = all_beta ? (size_t)K + 1 : 3;
+    if (a->K == K && !a->T.empty() && a->B.size() == nb) return LM_OK;
     adj_free_stack(a);
     const size_t bytes = a->elem * (size_t)a->n * (size_t)a->m;
     a->T.assign((size_t)K, nullptr);
@@ -347,8 +428,9 @@ static int adj_ensure_stack(lm_adjoint* a, int K) {
         int rc = adj_alloc(a->ctx, &a->T[(size_t)k], bytes);
         if (rc != LM_OK) return rc;
     }
-    for (auto& b : a->B) {
-        int rc = adj_alloc(a->ctx, &b, bytes);
+    a->B.assign(nb, nullptr);
+    for (size_t k = all_beta ? 1 : 0; k < nb; ++k) {
+        int rc = adj_alloc(a->ctx, &a->B[k], bytes);
         if (rc != LM_OK) return rc;
     }
     a->K = K;
@@ -470,9 +552,15 @@ int lm_adjoint_step(lm_adjoint* a, lm_solver* s, lm_ham* h, int component, int s
     cudaSetDevice(ctx->device);
     const Geom& g = h->lat->g;
     const int K = s->K;
-    int rc = adj_ensure_stack(a, K);
-    if (rc != LM_OK) return rc;
     const bool f64 = a->precision == LM_C64;
+    // ComplexF32 kets that fit on chip: T_k and beta_k of all orders in one launch each, then the sums
+    // over all of them.  The recurrences' operation order is that of the per-order kernels.
+    ResidentInst ri{};
+    int cl = 0;
+    const bool resident = !f64 && ctx->fused && K >= 3 && psi->ld == lam->ld &&
+                          resident_single_plan(ctx, g, K, a->m, psi->ld, psi->d_data, lam->d_data, ri, &cl);
+    int rc = adj_ensure_stack(a, K, resident);
+    if (rc != LM_OK) return rc;
     const void* hop2 = f64 ? (const void*)s->d_hop2 : (const void*)s->d_hop2f;
     const void* diag2 = f64 ? (const void*)s->d_diag2 : (const void*)s->d_diag2f;
     const int64_t ld = psi->ld, M = a->m;
@@ -483,7 +571,19 @@ int lm_adjoint_step(lm_adjoint* a, lm_solver* s, lm_ham* h, int component, int s
     };
     // T_0 = psi_n (aliased), T_1 = H~ T_0, T_k = 2 H~ T_{k-1} - T_{k-2}  (k < K)
     a->T[0] = psi->d_data;
-    for (int k = 1; k < K; ++k) {
+    if (resident) {
+        ri.hop2 = s->d_hop2f;
+        ri.diag2 = s->d_diag2f;
+        resident_fill_coef(ri, K, s->coef.data(), s->phase_re, s->phase_im);
+        ResidentOrders ot{}, ob{};
+        for (int k = 1; k < K; ++k) ot.p[k] = (float2*)a->T[(size_t)k];
+        for (int k = 1; k <= K; ++k) ob.p[k] = (float2*)a->B[(size_t)k];
+        rc = resident_single(ctx, K, false, cl, 1, ri, ot);
+        ri.x = (const float2*)lam->d_data;
+        if (rc == LM_OK) rc = resident_single(ctx, K, false, cl, 2, ri, ob);
+        if (rc != LM_OK) return rc;
+    }
+    for (int k = 1; k < K && !resident; ++k) {
         CUDA_TRY(ctx, recur(a->T[(size_t)k - 1], k >= 2 ? a->T[(size_t)k - 2] : nullptr, nullptr, a->T[(size_t)k],
                             k == 1 ? 0.5 : 1.0, 0.0, 0.0),
                  "adjoint forward recurrence");
@@ -491,8 +591,8 @@ int lm_adjoint_step(lm_adjoint* a, lm_solver* s, lm_ham* h, int component, int s
     // field derivative table
     const double2* dhop = nullptr;
     if (component >= 0) {
-        flux_derivative_kernel<<<(unsigned)((g.N + 255) / 256), 256, 0, ctx->stream>>>(g, h->fields, component, h->d_hop,
-                                                                                       a->d_dhop);
+        flux_derivative_kernel<<<dim3((unsigned)((g.N + 127) / 128), 2), 128, 0, ctx->stream>>>(
+            g, h->fields, component, h->d_hop, a->d_dhop);
         ctx->launches++;
         CUDA_TRY(ctx, cudaGetLastError(), "flux derivative kernel");
         dhop = a->d_dhop;
@@ -500,6 +600,18 @@ int lm_adjoint_step(lm_adjoint* a, lm_solver* s, lm_ham* h, int component, int s
     // beta_K .. beta_1 with gradient terms; B[k % 3] rotates
     const dim3 ggrid((unsigned)a->nblk, (unsigned)a->nchunk);
     double* gA = component >= 0 ? a->d_gA + (size_t)slot * (size_t)a->nblk * (size_t)a->nchunk : nullptr;
+    if (resident) {
+        GradOrders go{};
+        for (int k = 1; k <= K; ++k) {
+            go.T[k - 1] = (const float2*)a->T[(size_t)k - 1];
+            go.b[k] = (const float2*)a->B[(size_t)k];
+        }
+        adj_sums_kernel<<<ggrid, 256, 0, ctx->stream>>>(g, go, K, dhop, ld, M, a->mchunk, s->phase_re, s->phase_im,
+                                                        2.0 / s->a, a->d_gV, gA);
+        ctx->launches++;
+        CUDA_TRY(ctx, cudaGetLastError(), "adjoint gradient sums");
+        return LM_OK;
+    }
     for (int k = K; k >= 1; --k) {
         const ChebCoef c = s->coef[(size_t)k];
         const double wre = c.odd ? 0.0 : c.s, wim = c.odd ? c.s : 0.0;  // conj(c_k)

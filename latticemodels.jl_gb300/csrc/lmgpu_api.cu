@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "lmgpu_internal.cuh"
+#include "lmgpu_resident.cuh"
 #include "lmgpu_series.cuh"
 
 using namespace lmgpu;
@@ -224,6 +225,8 @@ int lm_ctx_destroy(lm_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     if (ctx->d_red) cudaFree(ctx->d_red);
     if (ctx->d_ld_part) cudaFree(ctx->d_ld_part);
+    if (ctx->d_res_err) cudaFree(ctx->d_res_err);
+    if (ctx->h_res_err) cudaFreeHost(ctx->h_res_err);
     for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -235,7 +238,7 @@ const char* lm_last_error(const lm_ctx* ctx) { return ctx ? ctx->err.c_str() : "
 int lm_ctx_synchronize(lm_ctx* ctx) {
     if (!ctx) return LM_ERR_ARG;
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize");
-    return LM_OK;
+    return resident_status(ctx);
 }
 
 int lm_ctx_stream(lm_ctx* ctx, void** stream) {
@@ -704,7 +707,7 @@ int lm_state_download(lm_state* s, void* host, int64_t ld) {
                                     (size_t)s->m, cudaMemcpyDeviceToHost, ctx->stream),
              "download state");
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "sync");
-    return LM_OK;
+    return resident_status(ctx);
 }
 
 int lm_state_copy(lm_state* dst, const lm_state* src) {
@@ -940,6 +943,51 @@ int lm_solver_order(const lm_solver* s, int* K, double* a, double* b) {
     return LM_OK;
 }
 
+}  // extern "C"
+
+namespace lmgpu {
+
+int resident_status(lm_ctx* ctx) {
+    if (ctx->h_res_err && *(volatile unsigned long long*)ctx->h_res_err)
+        return set_err(ctx, LM_ERR_TIMEOUT, "lattice-resident step: a halo exchange between two CTAs gave up");
+    return LM_OK;
+}
+
+bool resident_single_plan(const lm_ctx* ctx, const Geom& g, int K, int64_t m, int64_t ld, const void* x, const void* out,
+                          ResidentInst& d, int* cl) {
+    if (!ctx->resident || K < 2 || K > kResMaxK || !resident_plan(g, m, d, cl)) return false;
+    d.x = (const float2*)x;
+    d.out = (float2*)out;
+    d.ld = ld;
+    d.M = m;
+    d.item_begin = 0;
+    d.item_end = (m + d.G - 1) / d.G;
+    d.vec = g.Ly % 2 == 0 && ld % 2 == 0 && (((uintptr_t)x | (uintptr_t)out) & 15) == 0;
+    return true;
+}
+
+int resident_single(lm_ctx* ctx, int K, bool xreal, int cl, int mode, const ResidentInst& d, const ResidentOrders& o) {
+    if (!ctx->d_res_err) {
+        CUDA_TRY(ctx, cudaMalloc((void**)&ctx->d_res_err, sizeof(unsigned long long)), "resident status word");
+        CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_res_err, 0, sizeof(unsigned long long), ctx->stream), "resident status word");
+        CUDA_TRY(ctx, cudaHostAlloc((void**)&ctx->h_res_err, sizeof(unsigned long long), cudaHostAllocDefault),
+                 "resident status word");
+        *ctx->h_res_err = 0;
+    }
+    const int rc = resident_status(ctx);
+    if (rc != LM_OK) return rc;
+    CUDA_TRY(ctx, launch_resident_single(ctx, K, xreal, cl, mode, d, o, ctx->d_res_err), "lattice-resident step");
+    if (cl == 2)  // the word is read by a later call: no wait here
+        CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_res_err, ctx->d_res_err, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                                      ctx->stream),
+                 "resident status word");
+    return LM_OK;
+}
+
+}  // namespace lmgpu
+
+extern "C" {
+
 // One application of the Chebyshev series to the kets laid out by (site_fast, ld, m) in
 // buffers S (input T0), A, Y.  The result lands in S when K is even and in A when K is
 // odd; the return value says which (0 = S, 1 = A).
@@ -976,6 +1024,26 @@ static int cheb_apply(lm_solver* s, const Geom& g, int precision, int site_fast,
             return set_err(ctx, LM_ERR_NOTSUP,
                            "lm_solver_step: a compensated state needs the x-streaming form (Ly even, Lx >= 2K + 3, "
                            "K <= 6; K <= 5 with complex x-hops)");
+        // The region form recomputes a halo around every 32 x 64 tile and holds 16 kets an item; the
+        // lattice-resident form (the same bits) takes about 2400 clocks for a ket, or two half kets, and
+        // order on each SM against 1180 for a tile of a ket and order.  On 97 x 75 sites with 650 kets: 87
+        // against 164 us; on 64 x 64 with 1024: 51 against 114 us.
+        bool resident = false;
+        ResidentInst ri{};
+        int cl = 0;
+        if (!spack && !comp && resident_single_plan(ctx, g, K, m, ld, S, A, ri, &cl)) {
+            int ntx = 0, nty = 0;
+            const int64_t sm = std::max(ctx->sm_count, 1), tiles = fused_items(g, K, m, &ntx, &nty);
+            const int64_t kets = std::min<int64_t>(m, kFusedKetsPerItem);
+            resident = (ri.item_end + sm / cl - 1) / (sm / cl) * 2400 < (tiles + sm - 1) / sm * kets * 1180;
+        }
+        if (resident) {
+            ri.hop2 = (const float2*)hop2;
+            ri.diag2 = (const float*)diag2;
+            resident_fill_coef(ri, K, s->coef.data(), pr, pi);
+            const int rc = resident_single(ctx, K, xr, cl, 0, ri, ResidentOrders{});
+            if (rc != LM_OK) return rc;
+        } else
         CUDA_TRY(ctx, launch_cheb_fused_c32(ctx, g, (const float2*)hop2, (const float*)diag2, (const float2*)S,
                                             (float2*)A, ld, m, K, xr, s->coef.data(), pr, pi, spack, mode, comp),
                  "fused chebyshev step");
@@ -1105,6 +1173,24 @@ int lm_solver_step(lm_solver* s, lm_state* st) {
         if (where == 1) std::swap(st->d_data, st->d_a);
     }
     return LM_OK;
+}
+
+int lm_solver_step_to(lm_solver* s, const lm_state* src, lm_state* dst) {
+    if (!s) return LM_ERR_ARG;
+    lm_ctx* ctx = s->ctx;
+    CHECK_ARG(ctx, src != nullptr && dst != nullptr, "lm_solver_step_to: null state");
+    CHECK_ARG(ctx, src != dst, "lm_solver_step_to: source and destination are the same state");
+    if (s->valid && !s->ell && ctx->fused && src->ctx == ctx && dst->ctx == ctx && src->kind == LM_KETS &&
+        dst->kind == LM_KETS && src->precision == LM_C32 && dst->precision == LM_C32 && src->n == dst->n &&
+        src->m == dst->m && src->ld == dst->ld && src->n == s->ham->lat->g.N && !src->d_lo && !dst->d_lo &&
+        fused_supported(LM_C32, s->K) && fused_supported_geom(s->ham->lat->g)) {
+        // the fused forms read one buffer and write another
+        cudaSetDevice(ctx->device);
+        int where = 0;
+        return cheb_apply(s, s->ham->lat->g, LM_C32, 1, 0, src->d_data, dst->d_data, nullptr, src->ld, src->m, &where);
+    }
+    const int rc = lm_state_copy(dst, src);
+    return rc == LM_OK ? lm_solver_step(s, dst) : rc;
 }
 
 int lm_chebyshev_plan(double x, double tol, int cap, int* K, double* coef) {

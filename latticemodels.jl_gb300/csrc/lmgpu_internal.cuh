@@ -103,6 +103,9 @@ struct lm_ctx {
     int fused_form = 1;                 // LM_OPT_STREAM: 1 = x-streaming form where supported, 0 = region form
     int64_t stream_launches = 0;        // fused steps run in the x-streaming form
     int kpm_df = 1;                     // LM_OPT_KPM: double-float recurrence in lm_kpm_moments
+    unsigned resident_attr = 0;         // shared-memory attributes of the lattice-resident kernels set
+    unsigned long long* d_res_err = nullptr;  // their timeout word (single-lattice launches), and
+    unsigned long long* h_res_err = nullptr;  // its pinned copy, refreshed after every cluster launch
     int resident = 1;                   // LM_OPT_RESIDENT: lattice-resident form in the batch's fused pass
     std::vector<double> h_norms;        // pageable staging of lm_state_renormalize's targets
     std::vector<cudaEvent_t> ev_pool;   // pairs (start, stop) of timed Chebyshev sweeps

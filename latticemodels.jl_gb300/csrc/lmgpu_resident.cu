@@ -466,10 +466,107 @@ __device__ __forceinline__ void res_order(const float2 (&A)[C][R], float2 (&B)[C
     }
 }
 
-template <bool XR, int CL>
+// Column c of a block to a ket block in HBM (rows of the lattice only).
+__device__ __forceinline__ void res_store_col(float2* outk, const ResidentInst& D, const ResMap& m, int c,
+                                              const float2 (&v)[R]) {
+    const int x = m.x0 + c;
+    if (x >= D.Lx) return;
+    float2* o = outk + (int64_t)x * D.Ly + m.y0;
+    if (D.vec) {
+#pragma unroll
+        for (int h = 0; h < R / 2; ++h)
+            if (m.y0 + 2 * h < D.Ly)
+                *reinterpret_cast<float4*>(o + 2 * h) = make_float4(v[2 * h].x, v[2 * h].y, v[2 * h + 1].x, v[2 * h + 1].y);
+    } else {
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+            if (m.y0 + j < D.Ly) o[j] = v[j];
+    }
+}
+
+// One order of the adjoint's recurrences, in the per-order kernels' operation order (the neighbour sum
+// from zero, then alpha, then - B, then + w L), so that both give the same bits:
+//   B <- alpha (2H~) A - B + w L, alpha = 1/2 and no B when FIRST, w L only when LAM (L = lambda).
+// The result goes to outk (HBM) and, when WR, into the exchange buffer.
+template <bool FIRST, bool LAM, bool WR, int CL>
+__device__ __forceinline__ void res_order_adj(const float2 (&A)[C][R], float2 (&B)[C][R], const float2 (&L)[C][R],
+                                              const float2 (&hx)[C][R], const float2 (&hy)[C][R], unsigned Er, unsigned Ew,
+                                              unsigned peerEw, unsigned peerMb, unsigned ct, const ResMap& m, float w_re,
+                                              float w_im, bool has_b, float2* outk, const ResidentInst& D, unsigned mb,
+                                              unsigned parity, unsigned long long* err) {
+    const unsigned ro = Er + m.eo, rb = Er + m.eb, rt = Er + m.et;
+    if (CL == 2 && (m.hw & 1)) res_mbar_wait(mb, parity, err);
+    const float4 l0 = res_lds4(ro - 32u), l1 = res_lds4(ro - 16u);
+    const float2 lft[R] = {make_float2(l0.x, l0.y), make_float2(l0.z, l0.w), make_float2(l1.x, l1.y), make_float2(l1.z, l1.w)};
+    const float4 e0 = res_lds4(ct), e1 = res_lds4(ct + NT * 16u);
+    const float2 hxm0[R] = {make_float2(e0.x, e0.y), make_float2(e0.z, e0.w), make_float2(e1.x, e1.y), make_float2(e1.z, e1.w)};
+    float2 rgt[R];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        const float4 dq = res_lds4(ct + (4u + c) * NT * 16u);
+        const float2 bot = res_lds2(rb + 32u * c + 24u), top = res_lds2(rt + 32u * c);
+        const float2 hym0 = res_lds2(ct + (c < 2 ? 2u : 3u) * NT * 16u + 8u * (c & 1));
+        const float d[R] = {dq.x, dq.y, dq.z, dq.w};
+        if (c == C - 1) {
+            if (CL == 2 && m.hw == 2) res_mbar_wait(mb, parity, err);
+            const float4 r0 = res_lds4(ro + 32u * C), r1 = res_lds4(ro + 32u * C + 16u);
+            rgt[0] = make_float2(r0.x, r0.y);
+            rgt[1] = make_float2(r0.z, r0.w);
+            rgt[2] = make_float2(r1.x, r1.y);
+            rgt[3] = make_float2(r1.z, r1.w);
+        }
+        float2 acc[R];
+#pragma unroll
+        for (int j = 0; j < R; ++j) acc[j] = make_float2(0.f, 0.f);
+        auto add = [&](int j, float2 h, float2 v) {
+            acc[j].x = fmaf(h.x, v.x, acc[j].x); acc[j].x = fmaf(-h.y, v.y, acc[j].x);
+            acc[j].y = fmaf(h.x, v.y, acc[j].y); acc[j].y = fmaf(h.y, v.x, acc[j].y);
+        };
+#pragma unroll
+        for (int j = 0; j < R; ++j) add(j, hx[c][j], c < C - 1 ? A[c + 1 < C ? c + 1 : c][j] : rgt[j]);
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+            add(j, c > 0 ? make_float2(hx[c > 0 ? c - 1 : 0][j].x, -hx[c > 0 ? c - 1 : 0][j].y) : hxm0[j],
+                c > 0 ? A[c > 0 ? c - 1 : 0][j] : lft[j]);
+#pragma unroll
+        for (int j = 0; j < R; ++j) add(j, hy[c][j], j < R - 1 ? A[c][j + 1 < R ? j + 1 : j] : top);
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+            add(j, j > 0 ? make_float2(hy[c][j > 0 ? j - 1 : 0].x, -hy[c][j > 0 ? j - 1 : 0].y) : hym0,
+                j > 0 ? A[c][j > 0 ? j - 1 : 0] : bot);
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            float2 a = acc[j];
+            a.x = fmaf(d[j], A[c][j].x, a.x);
+            a.y = fmaf(d[j], A[c][j].y, a.y);
+            if (FIRST) {
+                a.x *= 0.5f;
+                a.y *= 0.5f;
+            } else if (!LAM || has_b) {
+                a.x -= B[c][j].x;
+                a.y -= B[c][j].y;
+            }
+            if (LAM) {
+                a.x = fmaf(w_re, L[c][j].x, fmaf(-w_im, L[c][j].y, a.x));
+                a.y = fmaf(w_re, L[c][j].y, fmaf(w_im, L[c][j].x, a.y));
+            }
+            B[c][j] = a;
+        }
+        res_store_col(outk, D, m, c, B[c]);
+        if (WR) res_put<CL>(B, c, Ew, peerEw, peerMb, m);
+    }
+}
+
+// MODE 0: the propagator over the instances of a table, items from the queue.  The other modes run one
+// instance, `single`, whose items the CTAs (or clusters) take in turn (a mode of their own: the test
+// for a table cost the batch 0.6 %).  MODE 3: the propagator.  MODE 1: T_1 .. T_{K-1} of the kets, written to
+// orders[k].  MODE 2: the adjoint recurrence beta_K .. beta_1 of the kets (lambda), beta_k = conj(c_k)
+// lambda + 2H~ beta_{k+1} - beta_{k+2}, written to orders[k].
+template <bool XR, int CL, int MODE>
 __global__ void __launch_bounds__(NT, 1)
 cheb_resident_c32_kernel(const ResidentInst* __restrict__ table, int ninst, long long nitems,
-                         unsigned long long* queue, unsigned long long* err, int K) {
+                         unsigned long long* queue, unsigned long long* err, int K,
+                         const __grid_constant__ ResidentInst single, const __grid_constant__ ResidentOrders orders) {
     extern __shared__ float4 smem[];
     __shared__ ResidentInst s_desc[2];
     __shared__ long long s_item[2];
@@ -498,18 +595,23 @@ cheb_resident_c32_kernel(const ResidentInst* __restrict__ table, int ninst, long
     unsigned ph = 0;  // bit b: parity of the next phase of mbarrier b
 
     // next item id: one thread of the cluster takes it from the queue and broadcasts it
-    auto fetch = [&](int slot) {
-        const long long v = (long long)atomicAdd(queue, 1ull);
+    auto fetch = [&](int slot, bool first = false) {
+        const long long v = MODE == 0 ? (long long)atomicAdd(queue, 1ull)
+                                      : first ? blockIdx.x / CL : s_item[slot ^ 1] + gridDim.x / CL;
         s_item[slot] = v;
         if (CL == 2) res_st_peer_s64(res_map_peer(&s_item[slot], peer), v);
     };
     auto load_desc = [&](int slot, long long it) {
+        if (MODE != 0) {
+            if (t < DESC_WORDS) reinterpret_cast<int*>(&s_desc[slot])[t] = reinterpret_cast<const int*>(&single)[t];
+            return;
+        }
         const ResidentInst* src = &table[res_find(table, ninst, it)];
         if (t < DESC_WORDS) reinterpret_cast<int*>(&s_desc[slot])[t] = __ldg(reinterpret_cast<const int*>(src) + t);
     };
 
     if (t == 0 && rank == 0) {
-        fetch(0);
+        fetch(0, true);
         fetch(1);
     }
     res_sync<CL>();
@@ -557,6 +659,17 @@ cheb_resident_c32_kernel(const ResidentInst* __restrict__ table, int ninst, long
                     A[c][j] = (m.on && x < D.Lx && y < D.Ly) ? st[(x - xs0) * D.Ly + y] : make_float2(0.f, 0.f);
                 }
             }
+            if (MODE == 2) {  // beta_K = conj(c_K) lambda; Y keeps lambda
+                const float wr = (K & 1) ? 0.f : D.s[K], wi = (K & 1) ? D.s[K] : 0.f;
+#pragma unroll
+                for (int j = 0; j < R; ++j) {
+                    const float2 l = A[c][j];
+                    Y[c][j] = l;
+                    A[c][j].x = fmaf(wr, l.x, fmaf(-wi, l.y, 0.f));
+                    A[c][j].y = fmaf(wr, l.y, fmaf(wi, l.x, 0.f));
+                }
+                if (live) res_store_col(orders.p[K] + (k0 + m.g) * D.ld, D, m, c, A[c]);
+            }
             if (live) res_put<CL>(A, c, Es, peerE, mb_peer[0], m);
         }
 
@@ -580,6 +693,7 @@ cheb_resident_c32_kernel(const ResidentInst* __restrict__ table, int ninst, long
             if (CL == 2 && t == 0) res_mbar_expect(mb_loc[b], xbytes);
         };
         const unsigned E1 = Es + par, pE1 = peerE + par;
+        if constexpr (MODE == 0 || MODE == 3) {
 #define LM_RES_ORDER(FI, OD, WR, AA, BB, ER, EW, PEW, PMB, SK, MB, PAR) \
     if (live) res_order<XR, FI, OD, WR, CL>(AA, BB, Y, hx, hy, ER, EW, PEW, PMB, cts, m, SK, D.lo, MB, PAR, err)
         // orders k (even): T_{k-1} in B and buffer 1 -> T_k in A and buffer 0; k (odd, k > 1): T_{k-1}
@@ -608,10 +722,39 @@ cheb_resident_c32_kernel(const ResidentInst* __restrict__ table, int ninst, long
             ph ^= 1u;
         }
 #undef LM_RES_ORDER
+        } else {
+            // steps q = 1 .. n: MODE 1 order q (T_q from T_{q-1} and T_{q-2}), MODE 2 order K - q; the input of
+            // step q lies in buffer (q - 1) & 1
+            const int n = K - 1;
+            auto step = [&](auto& P, auto& Q, int q) {
+                const int b = (q - 1) & 1, k = MODE == 1 ? q : K - q;
+                const unsigned er = b ? E1 : Es, ew = b ? Es : E1, pew = b ? peerE : pE1;
+                float2* outk = orders.p[k] + (k0 + m.g) * D.ld;
+                const float wr = (k & 1) ? 0.f : D.s[k], wi = (k & 1) ? D.s[k] : 0.f;  // conj(c_k)
+                xdone(b);
+                if (live) {
+                    const unsigned pa = (ph >> b) & 1u;
+                    if (MODE == 1 && q == 1)
+                        res_order_adj<true, false, true, CL>(P, Q, Y, hx, hy, er, ew, pew, mb_peer[b ^ 1], cts, m, 0.f, 0.f,
+                                                             false, outk, D, mb_loc[b], pa, err);
+                    else if (q < n)
+                        res_order_adj<false, MODE == 2, true, CL>(P, Q, Y, hx, hy, er, ew, pew, mb_peer[b ^ 1], cts, m, wr,
+                                                                  wi, q > 1, outk, D, mb_loc[b], pa, err);
+                    else
+                        res_order_adj<false, MODE == 2, false, CL>(P, Q, Y, hx, hy, er, ew, pew, mb_peer[b ^ 1], cts, m, wr,
+                                                                   wi, q > 1, outk, D, mb_loc[b], pa, err);
+                }
+                ph ^= 1u << b;
+            };
+            for (int q = 1; q <= n; q += 2) {
+                step(A, B, q);
+                if (q + 1 <= n) step(B, A, q + 1);
+            }
+        }
         res_arrive<CL>();  // this item's reads of the exchange buffers are done
 
         // out = e^{-ib dt} y + a0 x (a0 = e^{-ib dt} c_0): the small terms first, the dominant one last
-        if (live) {
+        if ((MODE == 0 || MODE == 3) && live) {
             const float ph_re = D.ph_re, ph_im = D.ph_im, a0_re = D.a0_re, a0_im = D.a0_im;
             float2* outk = D.out + (k0 + m.g) * D.ld;
             auto out_site = [&](float2 yv, float2 x0) {
@@ -711,26 +854,27 @@ void resident_fill_coef(ResidentInst& d, int K, const ChebCoef* coef, double ph_
     d.lo = cheb_lo(ph_re, ph_im, coef[0].s, coef[1].s, true);
 }
 
-template <bool XR, int CL>
+template <bool XR, int CL, int MODE>
 static cudaError_t set_res_attr(lm_ctx* ctx) {
-    const unsigned bit = 1u << (25 + (XR ? 1 : 0) + 2 * (CL - 1));
-    if (ctx->fused_attr & bit) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(cheb_resident_c32_kernel<XR, CL>,
+    const unsigned bit = 1u << ((XR ? 1 : 0) + 2 * (CL - 1) + 4 * MODE);
+    if (ctx->resident_attr & bit) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(cheb_resident_c32_kernel<XR, CL, MODE>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT - STATIC_RESERVE);
-    if (e == cudaSuccess) ctx->fused_attr |= bit;
+    if (e == cudaSuccess) ctx->resident_attr |= bit;
     return e;
 }
 
 cudaError_t ensure_resident_attr(lm_ctx* ctx, bool xreal, int cl) {
-    if (cl == 1) return xreal ? set_res_attr<true, 1>(ctx) : set_res_attr<false, 1>(ctx);
-    return xreal ? set_res_attr<true, 2>(ctx) : set_res_attr<false, 2>(ctx);
+    if (cl == 1) return xreal ? set_res_attr<true, 1, 0>(ctx) : set_res_attr<false, 1, 0>(ctx);
+    return xreal ? set_res_attr<true, 2, 0>(ctx) : set_res_attr<false, 2, 0>(ctx);
 }
 
-template <bool XR, int CL>
+template <bool XR, int CL, int MODE>
 static cudaError_t launch_res(lm_ctx* ctx, const ResidentInst* d_table, int ninst, int64_t nitems,
-                              unsigned long long* d_queue, unsigned long long* d_err, int K, int smem) {
-    auto kern = cheb_resident_c32_kernel<XR, CL>;
-    cudaError_t ea = set_res_attr<XR, CL>(ctx);
+                              unsigned long long* d_queue, unsigned long long* d_err, int K, int smem,
+                              const ResidentInst& single, const ResidentOrders& orders) {
+    auto kern = cheb_resident_c32_kernel<XR, CL, MODE>;
+    cudaError_t ea = set_res_attr<XR, CL, MODE>(ctx);
     if (ea != cudaSuccess) return ea;
     const int sms = ctx->sm_count > 0 ? ctx->sm_count : 152;
     int64_t grid = CL == 2 ? (sms / 2) * 2 : sms;
@@ -750,7 +894,7 @@ static cudaError_t launch_res(lm_ctx* ctx, const ResidentInst* d_table, int nins
         cfg.attrs = attr;
         cfg.numAttrs = 1;
     }
-    return cudaLaunchKernelEx(&cfg, kern, d_table, ninst, (long long)nitems, d_queue, d_err, K);
+    return cudaLaunchKernelEx(&cfg, kern, d_table, ninst, (long long)nitems, d_queue, d_err, K, single, orders);
 }
 
 cudaError_t launch_resident_table(lm_ctx* ctx, int K, bool xreal, int cl, const ResidentInst* d_table, int ninst,
@@ -758,10 +902,29 @@ cudaError_t launch_resident_table(lm_ctx* ctx, int K, bool xreal, int cl, const 
     if (nitems <= 0) return cudaSuccess;
     if (K < 2 || K > kResMaxK || smem > SMEM_LIMIT - STATIC_RESERVE || (cl != 1 && cl != 2)) return cudaErrorInvalidValue;
     cudaError_t e;
-    if (cl == 1) e = xreal ? launch_res<true, 1>(ctx, d_table, ninst, nitems, d_queue, d_err, K, smem)
-                           : launch_res<false, 1>(ctx, d_table, ninst, nitems, d_queue, d_err, K, smem);
-    else e = xreal ? launch_res<true, 2>(ctx, d_table, ninst, nitems, d_queue, d_err, K, smem)
-                   : launch_res<false, 2>(ctx, d_table, ninst, nitems, d_queue, d_err, K, smem);
+    const ResidentInst none{};
+    const ResidentOrders no{};
+    if (cl == 1) e = xreal ? launch_res<true, 1, 0>(ctx, d_table, ninst, nitems, d_queue, d_err, K, smem, none, no)
+                           : launch_res<false, 1, 0>(ctx, d_table, ninst, nitems, d_queue, d_err, K, smem, none, no);
+    else e = xreal ? launch_res<true, 2, 0>(ctx, d_table, ninst, nitems, d_queue, d_err, K, smem, none, no)
+                   : launch_res<false, 2, 0>(ctx, d_table, ninst, nitems, d_queue, d_err, K, smem, none, no);
+    ctx->launches++;
+    return e;
+}
+
+cudaError_t launch_resident_single(lm_ctx* ctx, int K, bool xreal, int cl, int mode, const ResidentInst& inst,
+                                   const ResidentOrders& orders, unsigned long long* d_err) {
+    if (K < 2 || K > kResMaxK || inst.smem > SMEM_LIMIT - STATIC_RESERVE || (cl != 1 && cl != 2) || mode < 0 || mode > 2 ||
+        (mode > 0 && K < 3))  // a first order that is also the last would send a halo nobody reads
+        return cudaErrorInvalidValue;
+    const int64_t n = inst.item_end;
+    cudaError_t e;
+#define LM_RES(X, CLV, MO) launch_res<X, CLV, MO>(ctx, nullptr, 1, n, nullptr, d_err, K, inst.smem, inst, orders)
+    if (mode == 1) e = cl == 1 ? LM_RES(false, 1, 1) : LM_RES(false, 2, 1);
+    else if (mode == 2) e = cl == 1 ? LM_RES(false, 1, 2) : LM_RES(false, 2, 2);
+    else if (xreal) e = cl == 1 ? LM_RES(true, 1, 3) : LM_RES(true, 2, 3);
+    else e = cl == 1 ? LM_RES(false, 1, 3) : LM_RES(false, 2, 3);
+#undef LM_RES
     ctx->launches++;
     return e;
 }

@@ -36,6 +36,11 @@ struct ResidentInst {
     ChebLo lo;            // fused-form second words
 };
 
+// Output blocks of the adjoint's recurrences by order (modes 1 and 2; leading dimension `ld`).
+struct ResidentOrders {
+    float2* p[kResMaxK + 1];
+};
+
 // Lattice-resident form (lmgpu_resident.cu).  resident_plan: whether a lattice of geometry g
 // with m kets runs in it, on one CTA (*cl = 1) or a cluster of two (*cl = 2), and its layout
 // in d (every field but the pointers, items and coefficients).  resident_fill_coef: the
@@ -47,6 +52,18 @@ void resident_fill_coef(ResidentInst& d, int K, const ChebCoef* coef, double ph_
 cudaError_t launch_resident_table(lm_ctx* ctx, int K, bool xreal, int cl, const ResidentInst* d_table, int ninst,
                                   int64_t nitems, unsigned long long* d_queue, unsigned long long* d_err,
                                   int smem);
+// One instance (item_begin = 0, item_end = its number of items), without a queue.  mode 0: the step;
+// mode 1: T_1 .. T_{K-1} of the kets x to orders; mode 2: beta_K .. beta_1 of the co-state x to orders
+// (s[k]: the coefficients; the output pointer is not used).
+cudaError_t launch_resident_single(lm_ctx* ctx, int K, bool xreal, int cl, int mode, const ResidentInst& inst,
+                                   const ResidentOrders& orders, unsigned long long* d_err);
+// The same from a solver or adjoint step (lmgpu_api.cu): the instance of one ket block (every field but
+// tables and coefficients), the launch with the context's timeout word, and that word's state as of
+// the last finished launch (LM_OK or LM_ERR_TIMEOUT).
+bool resident_single_plan(const lm_ctx* ctx, const Geom& g, int K, int64_t m, int64_t ld, const void* x, const void* out,
+                          ResidentInst& d, int* cl);
+int resident_single(lm_ctx* ctx, int K, bool xreal, int cl, int mode, const ResidentInst& d, const ResidentOrders& o);
+int resident_status(lm_ctx* ctx);
 // Sets the kernel's shared-memory attribute (outside stream capture).
 cudaError_t ensure_resident_attr(lm_ctx* ctx, bool xreal, int cl);
 

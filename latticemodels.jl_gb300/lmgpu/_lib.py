@@ -92,6 +92,7 @@ SIGNATURES = {
     "lm_adjoint_step": (_INT, [_P, _P, _P, _INT, _INT, _P, _P]),
     "lm_adjoint_gradients": (_INT, [_P, _PD, _PD]),
     "lm_solver_step": (_INT, [_P, _P]),
+    "lm_solver_step_to": (_INT, [_P, _P, _P]),
     "lm_solver_step_noalloc": (_INT, [_P, _P, _I64, _I64, _I64, _INT]),
     "lm_chebyshev_plan": (_INT, [_D, _D, _INT, _PINT, _PD]),
     "lm_batch_create": (_INT, [_P, _INT, _INT, _D, C.POINTER(_P)]),

@@ -138,8 +138,9 @@ class DensityLossAdjoint:
             ctx.check(lib.lm_state_copy(seg_states[0].handle, cps[c].handle))
             for n in range(n0, n1 - 1):
                 k = n - n0
-                ctx.check(lib.lm_state_copy(seg_states[k + 1].handle, seg_states[k].handle))
-                self._step(self.fwd, V, B[n // self.spi], self.dt, seg_states[k + 1])
+                self._assemble(V, B[n // self.spi])
+                ctx.check(lib.lm_solver_update(self.fwd, self._dh.handle, self.dt, 0))
+                ctx.check(lib.lm_solver_step_to(self.fwd, seg_states[k].handle, seg_states[k + 1].handle))
             for n in range(n1 - 1, n0 - 1, -1):
                 j = n // self.spi
                 self._assemble(V, B[j])
