@@ -392,6 +392,10 @@ int lm_ring_destroy(lm_ring *r);
 int lm_ring_push_localdensity(lm_ring *r, lm_state *st, double t, int64_t *seq);
 /* DensityCurrents(ham, state) on every bond (src/zoo/currents.jl:92-102) at time t. */
 int lm_ring_push_currents(lm_ring *r, lm_ham *ham, lm_state *st, double t, int64_t *seq);
+/* lm_ring_push_localdensity into `rho` and lm_ring_push_currents into `cur` (two rings) of the same
+ * moment, in one read of the kets where the state's form allows it. */
+int lm_ring_push_readouts(lm_ring *rho, lm_ring *cur, lm_ham *ham, lm_state *st, double t, int64_t *seq_rho,
+                          int64_t *seq_cur);
 /* LocalOperatorCurrents (lm_ell_op_currents) of a general Hamiltonian into the next slot:
  * nnz values in CSC order. */
 int lm_ring_push_op_currents(lm_ring *r, lm_ell *h, lm_state *st, int ndof, const double *op, double t,

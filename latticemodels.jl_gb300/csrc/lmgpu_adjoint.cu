@@ -123,19 +123,11 @@ cudaError_t launch_stencil_recur(lm_ctx* ctx, const Geom& g, int precision, cons
     return cudaGetLastError();
 }
 
-// A block's gradient contributions from the sums of its 8 warps (added in warp order): gV_part of its 32
-// sites and gA_part of the block, one writer per entry and launch.
-__device__ __forceinline__ void grad_block_out(const Geom& g, const Nbr& nb, int64_t s, int lane, int warp,
-                                               const double (&red)[8][10][32], const double2* dhop, double ph_re,
-                                               double ph_im, double f, double* gV_part, double* gA_part) {
-    if (warp != 0) return;
-    double v[10];
-#pragma unroll
-    for (int q = 0; q < 10; ++q) {
-        double t = 0.0;
-        for (int w = 0; w < 8; ++w) t += red[w][q][lane];
-        v[q] = t;
-    }
+// A block's gradient contributions of one order from its sums v: gV_part of its 32 sites and gA_part of
+// the block, one writer per entry and launch (one warp calls this).
+__device__ __forceinline__ void grad_block_out(const Geom& g, const Nbr& nb, int64_t s, int lane, const double (&v)[10],
+                                               const double2* dhop, double ph_re, double ph_im, double f,
+                                               double* gV_part, double* gA_part) {
     double ga = 0.0;
     if (s < g.N) {
         gV_part[(int64_t)blockIdx.y * g.N + s] += f * (ph_re * v[0] - ph_im * v[1]);
@@ -244,51 +236,79 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 3 : 2) adj_b
 #pragma unroll
     for (int q = 0; q < 10; ++q) red[warp][q][lane] = a[q].get();
     __syncthreads();
-    grad_block_out(g, nb, s, lane, warp, red, dhop, ph_re, ph_im, f, gV_part, gA_part);
+    if (warp != 0) return;
+    double v[10];
+#pragma unroll
+    for (int q = 0; q < 10; ++q) {
+        double t = 0.0;
+        for (int w = 0; w < 8; ++w) t += red[w][q][lane];
+        v[q] = t;
+    }
+    grad_block_out(g, nb, s, lane, v, dhop, ph_re, ph_im, f, gV_part, gA_part);
 }
 
 // The gradient sums of a whole step from all its T_{k-1} and beta_k (which the lattice-resident kernels
-// wrote to HBM): the sums of adj_beta_grad_kernel<float> over every order at once, so that the ten
-// double-float accumulators of a site are reduced and written once per step.  The orders' factors 1/a
-// and 2/a become 2/a with beta_1 halved (exact).
+// wrote to HBM): order by order the sums of adj_beta_grad_kernel<float>, term for term, so that both forms
+// give the same bits.
 //
-// What bounds it: FP32 issue, 20 double-float products (10 operations each) per site, ket and order.  On
-// 64 x 64 sites with 1024 kets and K = 6 a step took 5 recurrence launches of 41 us and 6 fused
-// passes of 102 us; now T_k and beta_k take 62 + 81 us on chip (each writes 200 MB) and the sums 236 us
-// (294 us without the loads one (ket, order) ahead; the products and sums alone are 134 us).
+// What bounds it: FP32 issue, 20 double-float products (10 operations each) per site, ket and order, and
+// after every order the FP64 pipe (a warp-wide DADD holds a partition for 64 clocks), so each of the
+// 8 warps adds one sum's partials and the pairs become doubles by integer operations.  On 64 x 64 sites
+// with 1024 kets and K = 6 a step took 5 recurrence launches of 41 us and 6 fused passes of 102 us; now
+// T_k and beta_k take 62 + 81 us on chip (each writes 200 MB) and the sums 250 us (134 us of products).
 struct GradOrders {
     const float2* T[kResMaxK];      // T_0 .. T_{K-1}
     const float2* b[kResMaxK + 1];  // beta_1 .. beta_K
 };
 
+// (double)x without the FP64 pipe's conversion
+__device__ __forceinline__ double widen(float x) {
+    const unsigned u = __float_as_uint(x);
+    const unsigned e = u & 0x7f800000u;
+    if (e == 0x7f800000u || (e == 0u && (u << 1) != 0u)) return (double)x;  // infinities, NaN, denormals
+    if (e == 0u) return __hiloint2double((int)u, 0);
+    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))), (int)(u << 29));
+}
+
 __global__ void __launch_bounds__(256, 3) adj_sums_kernel(Geom g, const __grid_constant__ GradOrders ord, int K,
                                                           const double2* __restrict__ dhop, int64_t ld, int64_t M,
-                                                          int64_t mchunk, double ph_re, double ph_im, double f,
+                                                          int64_t mchunk, double ph_re, double ph_im, double inv_a,
                                                           double* __restrict__ gV_part, double* __restrict__ gA_part) {
     __shared__ double red[8][10][32];
+    __shared__ double tot[10][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t s = (int64_t)blockIdx.x * 32 + lane;
     const int64_t m0 = (int64_t)blockIdx.y * mchunk, m1 = min(M, m0 + mchunk);
-    Acc<float> a[10];  // conj(b)T_s (re, im); S1x; S1y; S2x; S2y
+    const int64_t m_first = m0 + warp;
+    const bool on = s < g.N;
     Nbr nb;
-    if (s < g.N) {
+    int xp = 0, yp = 0, xm = 0, ym = 0;
+    if (on) {
         nb = neighbours(g, s);
-        const int xp = (int)(nb.xp - s), yp = (int)(nb.yp - s), xm = (int)(nb.xm - s), ym = (int)(nb.ym - s);
-        // beta, T and T's neighbours of the next (ket, order) are loaded while this one is summed
-        float2 v[6], w[6];
-        auto load = [&](float2 (&d)[6], int64_t m, int k) {
-            const float2* T = ord.T[k - 1] + m * ld + s;
-            d[0] = ord.b[k][m * ld + s];
-            d[1] = T[0];
-            if (dhop) {
-                d[2] = T[xp];
-                d[3] = T[yp];
-                d[4] = T[xm];
-                d[5] = T[ym];
-            }
-        };
-        auto sum = [&](const float2 (&d)[6], int k) {
-            const float2 b = k == 1 ? make_float2(0.5f * d[0].x, 0.5f * d[0].y) : d[0];
+        xp = (int)(nb.xp - s);
+        yp = (int)(nb.yp - s);
+        xm = (int)(nb.xm - s);
+        ym = (int)(nb.ym - s);
+    }
+    // beta, T and T's neighbours of the next ket (of the next order) are loaded while this one is summed
+    auto load = [&](float2 (&d)[6], int64_t m, int k) {
+        if (!on || m >= m1 || k < 1) return;
+        const float2* T = ord.T[k - 1] + m * ld + s;
+        d[0] = ord.b[k][m * ld + s];
+        d[1] = T[0];
+        if (dhop) {
+            d[2] = T[xp];
+            d[3] = T[yp];
+            d[4] = T[xm];
+            d[5] = T[ym];
+        }
+    };
+    float2 v[6], w[6];
+    load(v, m_first, K);
+    for (int k = K; k >= 1; --k) {
+        Acc<float> a[10];  // conj(b)T_s (re, im); S1x; S1y; S2x; S2y
+        auto sum = [&](const float2 (&d)[6]) {
+            const float2 b = d[0];
 #pragma unroll
             for (int q = 0; q < 5; ++q) {  // conj(b) T at the site and its neighbours
                 if (q > 0 && !dhop) break;
@@ -298,25 +318,41 @@ __global__ void __launch_bounds__(256, 3) adj_sums_kernel(Geom g, const __grid_c
                 a[2 * q + 1].add_prod(-b.y, d[1 + q].x);
             }
         };
-        int64_t m = m0 + warp;
-        if (m < m1) load(v, m, 1);
-        int k = 1;
-        while (m < m1) {
-            int k2 = k < K ? k + 1 : 1;
-            int64_t m2 = k < K ? m : m + 8;
-            if (m2 < m1) load(w, m2, k2);
-            sum(v, k);
-            if (m2 >= m1) break;
-            k = k2 < K ? k2 + 1 : 1;
-            m = k2 < K ? m2 : m2 + 8;
-            if (m < m1) load(v, m, k);
-            sum(w, k2);
+        if (on) {
+            int64_t m = m_first;
+            for (; m + 8 < m1; m += 16) {
+                load(w, m + 8, k);
+                sum(v);
+                if (m + 16 < m1) load(v, m + 16, k);
+                else load(v, m_first, k - 1);
+                sum(w);
+            }
+            if (m < m1) {
+                sum(v);
+                load(v, m_first, k - 1);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 10; ++q) red[warp][q][lane] = widen(a[q].hi) + widen(a[q].lo);
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {  // sum q of the block, warps in order
+            const int q = warp + 8 * r;
+            if (q < 10 && (q < 2 || dhop)) {
+                double t = 0.0;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) t += red[u][q][lane];
+                tot[q][lane] = t;
+            }
+        }
+        __syncthreads();
+        if (warp == 0) {  // the other warps go on; tot is rewritten after the next order's first barrier
+            double t[10];
+#pragma unroll
+            for (int q = 0; q < 10; ++q) t[q] = q < 2 || dhop ? tot[q][lane] : 0.0;
+            grad_block_out(g, nb, s, lane, t, dhop, ph_re, ph_im, k == 1 ? inv_a : 2.0 * inv_a, gV_part, gA_part);
         }
     }
-#pragma unroll
-    for (int q = 0; q < 10; ++q) red[warp][q][lane] = a[q].get();
-    __syncthreads();
-    grad_block_out(g, nb, s, lane, warp, red, dhop, ph_re, ph_im, f, gV_part, gA_part);
 }
 
 // rho_s = sum_m |psi_sm|^2; loss = sum_s (rho_s - target_s)^2; lambda = 4 (rho_s - target_s) psi.
@@ -607,7 +643,7 @@ int lm_adjoint_step(lm_adjoint* a, lm_solver* s, lm_ham* h, int component, int s
             go.b[k] = (const float2*)a->B[(size_t)k];
         }
         adj_sums_kernel<<<ggrid, 256, 0, ctx->stream>>>(g, go, K, dhop, ld, M, a->mchunk, s->phase_re, s->phase_im,
-                                                        2.0 / s->a, a->d_gV, gA);
+                                                        1.0 / s->a, a->d_gV, gA);
         ctx->launches++;
         CUDA_TRY(ctx, cudaGetLastError(), "adjoint gradient sums");
         return LM_OK;

@@ -1239,7 +1239,8 @@ int lm_bond_currents(lm_ham* h, lm_state* s, double* out) {
     int rc = ensure_red(ctx, (size_t)std::max<int64_t>(nb, 1));
     if (rc != LM_OK) return rc;
     if (nb == 0) return LM_OK;
-    CUDA_TRY(ctx, launch_bond_currents(ctx, h->lat->g, s->precision, s->kind, h->d_hop, s->d_data, s->m, s->ld, s->d_w, ctx->d_red),
+    CUDA_TRY(ctx, launch_bond_currents(ctx, h->lat->g, s->precision, s->kind, h->d_hop, ham_x_real(h), s->d_data, s->m, s->ld,
+                                       s->d_w, ctx->d_red),
              "bond currents kernel");
     CUDA_TRY(ctx, cudaMemcpyAsync(out, ctx->d_red, sizeof(double) * (size_t)nb, cudaMemcpyDeviceToHost, ctx->stream),
              "download currents");

@@ -275,8 +275,12 @@ cudaError_t launch_scale(lm_ctx* ctx, int precision, void* x, int64_t n, int64_t
                          double re, double im);
 cudaError_t launch_localdensity(lm_ctx* ctx, int precision, int kind, const void* x, int64_t n,
                                 int64_t m, int64_t ld, const double* w, double* out);
-cudaError_t launch_bond_currents(lm_ctx* ctx, const Geom& g, int precision, int kind, const double2* hop,
+// xr: every x-hop of `hop` is real (ham_x_real)
+cudaError_t launch_bond_currents(lm_ctx* ctx, const Geom& g, int precision, int kind, const double2* hop, bool xr,
                                  const void* x, int64_t m, int64_t ld, const double* w, double* out);
+// Density (n values) and bond currents together, in one read of the kets where there is such a kernel.
+cudaError_t launch_readouts(lm_ctx* ctx, const Geom& g, int precision, int kind, const double2* hop, bool xr, const void* x,
+                            int64_t m, int64_t ld, const double* w, double* rho, double* out);
 cudaError_t launch_column_norms(lm_ctx* ctx, int precision, const void* x, int64_t n, int64_t m,
                                 int64_t ld, double* out);
 cudaError_t launch_rescale_columns(lm_ctx* ctx, int precision, void* x, int64_t n, int64_t m,

@@ -409,7 +409,8 @@ __device__ __forceinline__ void bond_write(const Geom& g, const double2* __restr
 
 // Ket blocks: P[j,s] = sum_k w_k psi_jk conj(psi_sk).  A block owns 32 consecutive sites (one
 // per lane); its 8 warps split the kets; partial sums are added in warp order.
-template <typename R, bool WEIGHTED>
+// XR (real x-hops): J of an x-bond needs the imaginary part only, two products fewer of eight.
+template <typename R, bool WEIGHTED, bool XR>
 __global__ void __launch_bounds__(32 * kReadWarps) bond_currents_kets_kernel(
     Geom g, const double2* __restrict__ hop, const typename CT<R>::V* __restrict__ x, int64_t m, int64_t ld,
     const double* __restrict__ w, double* __restrict__ out) {
@@ -431,13 +432,13 @@ __global__ void __launch_bounds__(32 * kReadWarps) bond_currents_kets_kernel(
             const V cx = x[k * ld + jx], cy = x[k * ld + jy];  // c * conj(b)
             if (WEIGHTED) {
                 const double wk = w[k];
-                aw[0] += wk * ((double)cx.x * (double)b.x + (double)cx.y * (double)b.y);
+                if (!XR) aw[0] += wk * ((double)cx.x * (double)b.x + (double)cx.y * (double)b.y);
                 aw[1] += wk * ((double)cx.y * (double)b.x - (double)cx.x * (double)b.y);
                 aw[2] += wk * ((double)cy.x * (double)b.x + (double)cy.y * (double)b.y);
                 aw[3] += wk * ((double)cy.y * (double)b.x - (double)cy.x * (double)b.y);
             } else {
-                a[0].add_prod(cx.x, b.x);
-                a[0].add_prod(cx.y, b.y);
+                if (!XR) a[0].add_prod(cx.x, b.x);
+                if (!XR) a[0].add_prod(cx.y, b.y);
                 a[1].add_prod(cx.y, b.x);
                 a[1].add_prod(-cx.x, b.y);
                 a[2].add_prod(cy.x, b.x);
@@ -478,112 +479,119 @@ __global__ void bond_currents_dm_kernel(Geom g, const double2* __restrict__ hop,
     }
 }
 
-// c32 ket blocks with Ly % 4 == 0: a lane owns 4 consecutive sites of one lattice column, so
-// a warp reads 1 KB of a ket per load (the 256-byte pieces of the kernel above, from kets
-// 512 KB apart, held DRAM to about a quarter of its bandwidth).  The +x neighbours are the
-// same 4 rows of the next column (contiguous); the +y neighbours are the lane's own next sites
-// and, for the fourth, one extra 8-byte load.  Each site gets the products of the kernel above
-// in the same ket order within a slice.  Block y takes the kets of slice y and writes its
-// 4 partial sums per site to plane y of `part`; bond_currents_slices_kernel adds the planes in
-// slice order and writes the bonds.
-template <bool WEIGHTED>
-__global__ void __launch_bounds__(32 * kReadWarps) bond_currents_kets4_kernel(
-    Geom g, const float2* __restrict__ x, int64_t m, int64_t ld, const double* __restrict__ w, int64_t kslice,
-    double* __restrict__ part) {
-    __shared__ double red[kReadWarps][4][128];
+// Bond currents, and with DENS the local density, of c32 ket blocks (no weights) in one read of the kets.
+// A lane owns VEC consecutive sites of one lattice column: 4 where Ly % 4 == 0 and ld is even, so
+// that a warp reads 1 KB of a ket per load (256-byte pieces from kets 512 KB apart hold DRAM to
+// about a quarter of its bandwidth), else 1.  The +x neighbours are the same rows of the next column; the
+// +y neighbours the lane's own next sites and, for the last, one 8-byte load.  A block's 8 warps split
+// the kets of slice blockIdx.y and write the sums of a site to planes of `part`, [slice][sum][site]:
+// the density (DENS), (re, im) of conj(b) c on the x-bond (im only when XR: real x-hops need no
+// more) and on the y-bond; readout_slices_kernel adds the slices in order and writes the readouts.
+//
+// What bounds it: the products, 10 FP32 operations each (exact product, TwoSum; the sums carry 48
+// bits).  256 x 256 sites, 2048 kets, real x-hops: 6 products for the currents and 2 for the density in
+// one pass of 480 us, against 453 us for the currents' 8 and a second pass of 179 us for the density.
+// 97 x 75 sites, 650 kets: 22 us against 44 + 11 us, where one block per 32 sites left SMs idle.
+template <int VEC, bool XR, bool DENS>
+__global__ void __launch_bounds__(32 * kReadWarps) readout_kets_kernel(
+    Geom g, const float2* __restrict__ x, int64_t m, int64_t ld, int64_t kslice, double* __restrict__ part) {
+    constexpr int NQ = (DENS ? 1 : 0) + (XR ? 1 : 2) + 2, QX = DENS ? 1 : 0, QY = QX + (XR ? 1 : 2);
+    __shared__ double red[kReadWarps][32 * VEC];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t s0 = (int64_t)blockIdx.x * 128 + (int64_t)lane * 4;
+    const int64_t s0 = (int64_t)blockIdx.x * (32 * VEC) + (int64_t)lane * VEC;
     const int64_t k0 = (int64_t)blockIdx.y * kslice;
     const int64_t k1 = k0 + kslice < m ? k0 + kslice : m;
-    Acc<float> a[4][4];
-    double aw[4][4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) aw[j][q] = 0.0;
+    Acc<float> a[VEC][NQ];
     if (s0 < g.N) {
         const int64_t xi = s0 / g.Ly, yi0 = s0 - xi * g.Ly;
-        // +x: the same rows of the next column (absent bonds read the sites themselves and are
-        // not written); +y of the fourth site: the next row, the column start, or itself
+        // absent bonds read the sites themselves (always in bounds) and are not written
         const int64_t jx = xi + 1 < g.Lx ? s0 + g.Ly : (g.per_x ? yi0 : s0);
-        const int64_t jy3 = yi0 + 4 < g.Ly ? s0 + 4 : (g.per_y ? s0 - yi0 : s0 + 3);
-#pragma unroll 2
+        const int64_t jy = yi0 + VEC < g.Ly ? s0 + VEC : (g.per_y ? s0 - yi0 : s0 + VEC - 1);
+#pragma unroll (VEC == 4 ? 2 : 4)
         for (int64_t k = k0 + warp; k < k1; k += kReadWarps) {
-            const float4* xb = reinterpret_cast<const float4*>(x + k * ld + s0);
-            const float4* xc = reinterpret_cast<const float4*>(x + k * ld + jx);
-            const float4 b01 = __ldg(xb), b23 = __ldg(xb + 1), c01 = __ldg(xc), c23 = __ldg(xc + 1);
-            const float2 y3 = __ldg(x + k * ld + jy3);
-            const float2 b[4] = {make_float2(b01.x, b01.y), make_float2(b01.z, b01.w), make_float2(b23.x, b23.y),
-                                 make_float2(b23.z, b23.w)};
-            const float2 cxs[4] = {make_float2(c01.x, c01.y), make_float2(c01.z, c01.w), make_float2(c23.x, c23.y),
-                                   make_float2(c23.z, c23.w)};
-            const float2 cys[4] = {b[1], b[2], b[3], y3};
-            const double wk = WEIGHTED ? w[k] : 1.0;
+            float2 b[VEC + 1], c[VEC];
+            if (VEC == 4) {
+                const float4* xb = reinterpret_cast<const float4*>(x + k * ld + s0);
+                const float4* xc = reinterpret_cast<const float4*>(x + k * ld + jx);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float2 bb = b[j], cx = cxs[j], cy = cys[j];  // c * conj(b)
-                if (WEIGHTED) {
-                    aw[j][0] += wk * ((double)cx.x * (double)bb.x + (double)cx.y * (double)bb.y);
-                    aw[j][1] += wk * ((double)cx.y * (double)bb.x - (double)cx.x * (double)bb.y);
-                    aw[j][2] += wk * ((double)cy.x * (double)bb.x + (double)cy.y * (double)bb.y);
-                    aw[j][3] += wk * ((double)cy.y * (double)bb.x - (double)cy.x * (double)bb.y);
-                } else {
-                    a[j][0].add_prod(cx.x, bb.x);
-                    a[j][0].add_prod(cx.y, bb.y);
-                    a[j][1].add_prod(cx.y, bb.x);
-                    a[j][1].add_prod(-cx.x, bb.y);
-                    a[j][2].add_prod(cy.x, bb.x);
-                    a[j][2].add_prod(cy.y, bb.y);
-                    a[j][3].add_prod(cy.y, bb.x);
-                    a[j][3].add_prod(-cy.x, bb.y);
+                for (int h = 0; h < VEC / 2; ++h) {
+                    const float4 u = __ldg(xb + h), v = __ldg(xc + h);
+                    b[2 * h] = make_float2(u.x, u.y);
+                    b[2 * h + 1] = make_float2(u.z, u.w);
+                    c[2 * h] = make_float2(v.x, v.y);
+                    c[2 * h + 1] = make_float2(v.z, v.w);
                 }
+            } else {
+                b[0] = __ldg(x + k * ld + s0);
+                c[0] = __ldg(x + k * ld + jx);
+            }
+            b[VEC] = __ldg(x + k * ld + jy);
+#pragma unroll
+            for (int j = 0; j < VEC; ++j) {
+                const float2 bb = b[j], cx = c[j], cy = b[j + 1];  // c * conj(b)
+                if (DENS) {
+                    a[j][0].add_prod(bb.x, bb.x);
+                    a[j][0].add_prod(bb.y, bb.y);
+                }
+                if (!XR) {
+                    a[j][QX].add_prod(cx.x, bb.x);
+                    a[j][QX].add_prod(cx.y, bb.y);
+                }
+                a[j][QY - 1].add_prod(cx.y, bb.x);
+                a[j][QY - 1].add_prod(-cx.x, bb.y);
+                a[j][QY].add_prod(cy.x, bb.x);
+                a[j][QY].add_prod(cy.y, bb.y);
+                a[j][QY + 1].add_prod(cy.y, bb.x);
+                a[j][QY + 1].add_prod(-cy.x, bb.y);
             }
         }
     }
+    double* pl = part + (int64_t)blockIdx.y * NQ * g.N;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int q = 0; q < NQ; ++q) {
+        if (q > 0) __syncthreads();
 #pragma unroll
-        for (int q = 0; q < 4; ++q) red[warp][q][lane * 4 + j] = WEIGHTED ? aw[j][q] : a[j][q].get();
-    __syncthreads();
-    if (threadIdx.x < 128) {
-        const int64_t s = (int64_t)blockIdx.x * 128 + threadIdx.x;
-        if (s < g.N) {
-            double* pl = part + (int64_t)blockIdx.y * 4 * g.N;
+        for (int j = 0; j < VEC; ++j) red[warp][lane * VEC + j] = a[j][q].get();
+        __syncthreads();
+        const int64_t s = (int64_t)blockIdx.x * (32 * VEC) + threadIdx.x;
+        if (threadIdx.x < 32 * VEC && s < g.N) {
+            double t = 0.0;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                double t = 0.0;
-                for (int r = 0; r < kReadWarps; ++r) t += red[r][q][threadIdx.x];
-                pl[(int64_t)q * g.N + s] = t;
-            }
+            for (int r = 0; r < kReadWarps; ++r) t += red[r][threadIdx.x];
+            pl[(int64_t)q * g.N + s] = t;
         }
     }
 }
 
-// Adds the S slice planes of bond_currents_kets4_kernel in slice order and writes the bonds.
-__global__ void bond_currents_slices_kernel(Geom g, const double2* __restrict__ hop, const double* __restrict__ part,
-                                            int S, double* __restrict__ out) {
+// Adds the S slice planes of readout_kets_kernel in slice order and writes the bonds and the density.
+template <bool XR, bool DENS>
+__global__ void readout_slices_kernel(Geom g, const double2* __restrict__ hop, const double* __restrict__ part, int S,
+                                      double* __restrict__ rho, double* __restrict__ out) {
+    constexpr int NQ = (DENS ? 1 : 0) + (XR ? 1 : 2) + 2, QX = DENS ? 1 : 0, QY = QX + (XR ? 1 : 2);
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= g.N) return;
-    double v[4];
+    double v[NQ];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < NQ; ++q) {
         double t = part[(int64_t)q * g.N + s];
-        for (int y = 1; y < S; ++y) t += part[((int64_t)y * 4 + q) * g.N + s];
+        for (int y = 1; y < S; ++y) t += part[((int64_t)y * NQ + q) * g.N + s];
         v[q] = t;
     }
+    if (DENS) rho[s] = v[0];
     const Nbr nb = neighbours(g, s);
-    if (nb.hxp) bond_write(g, hop, s, 0, nb, v[0], v[1], out);
-    if (nb.hyp) bond_write(g, hop, s, 1, nb, v[2], v[3], out);
+    if (nb.hxp) bond_write(g, hop, s, 0, nb, XR ? 0.0 : v[QX], v[QY - 1], out);
+    if (nb.hyp) bond_write(g, hop, s, 1, nb, v[QY], v[QY + 1], out);
 }
 
-template <bool WEIGHTED>
-static cudaError_t launch_bond_currents4(lm_ctx* ctx, const Geom& g, const double2* hop, const float2* x, int64_t m,
-                                         int64_t ld, const double* w, double* out) {
-    const int64_t chunks = (g.N + 127) / 128;
+template <int VEC, bool XR, bool DENS>
+static cudaError_t launch_readout_t(lm_ctx* ctx, const Geom& g, const double2* hop, const float2* x, int64_t m, int64_t ld,
+                                    double* rho, double* out) {
+    constexpr int NQ = (DENS ? 1 : 0) + (XR ? 1 : 2) + 2;
+    const int64_t chunks = (g.N + 32 * VEC - 1) / (32 * VEC);
     static const int per_sm = [] {  // resident blocks per SM of this instantiation
         int b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, bond_currents_kets4_kernel<WEIGHTED>, 32 * kReadWarps,
-                                                          0) != cudaSuccess) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, readout_kets_kernel<VEC, XR, DENS>, 32 * kReadWarps, 0) !=
+            cudaSuccess) {
             (void)cudaGetLastError();
             b = 0;
         }
@@ -591,46 +599,77 @@ static cudaError_t launch_bond_currents4(lm_ctx* ctx, const Geom& g, const doubl
     }();
     int S = readout_slices(chunks, m, (int64_t)per_sm * ctx->sm_count);
     if (ctx->ld_slices_override > 0) S = ctx->ld_slices_override;
-    cudaError_t e = ensure_readout_part(ctx, (size_t)S * 4 * (size_t)g.N);
-    if (e != cudaSuccess) return e;  // the caller falls back to the one-site-per-lane kernel
+    cudaError_t e = ensure_readout_part(ctx, (size_t)S * NQ * (size_t)g.N);
+    if (e != cudaSuccess) return e;
     const int64_t kslice = (m + S - 1) / S;
-    bond_currents_kets4_kernel<WEIGHTED><<<dim3((unsigned)chunks, (unsigned)S), 32 * kReadWarps, 0, ctx->stream>>>(
-        g, x, m, ld, w, kslice, ctx->d_ld_part);
-    bond_currents_slices_kernel<<<(unsigned)((g.N + 255) / 256), 256, 0, ctx->stream>>>(g, hop, ctx->d_ld_part, S, out);
-    ctx->launches++;
-    return cudaSuccess;
+    readout_kets_kernel<VEC, XR, DENS><<<dim3((unsigned)chunks, (unsigned)S), 32 * kReadWarps, 0, ctx->stream>>>(
+        g, x, m, ld, kslice, ctx->d_ld_part);
+    readout_slices_kernel<XR, DENS><<<(unsigned)((g.N + 127) / 128), 128, 0, ctx->stream>>>(g, hop, ctx->d_ld_part, S, rho,
+                                                                                           out);
+    ctx->launches += 2;
+    return cudaGetLastError();
 }
 
-cudaError_t launch_bond_currents(lm_ctx* ctx, const Geom& g, int precision, int kind, const double2* hop,
+template <int VEC, bool XR>
+static cudaError_t launch_readout_v(lm_ctx* ctx, const Geom& g, const double2* hop, const float2* x, int64_t m, int64_t ld,
+                                    double* rho, double* out) {
+    return rho ? launch_readout_t<VEC, XR, true>(ctx, g, hop, x, m, ld, rho, out)
+               : launch_readout_t<VEC, XR, false>(ctx, g, hop, x, m, ld, rho, out);
+}
+
+// The c32 sums of a block without weights; cudaErrorMemoryAllocation where their scratch does not fit.
+static cudaError_t launch_readout_c32(lm_ctx* ctx, const Geom& g, const double2* hop, bool xr, const float2* x, int64_t m,
+                                      int64_t ld, double* rho, double* out) {
+    const bool wide = g.Ly % 4 == 0 && ld % 2 == 0 && ((uintptr_t)x & 15) == 0 && !ctx->currents_scalar;
+    if (wide) return xr ? launch_readout_v<4, true>(ctx, g, hop, x, m, ld, rho, out)
+                        : launch_readout_v<4, false>(ctx, g, hop, x, m, ld, rho, out);
+    return xr ? launch_readout_v<1, true>(ctx, g, hop, x, m, ld, rho, out)
+              : launch_readout_v<1, false>(ctx, g, hop, x, m, ld, rho, out);
+}
+
+template <typename R, bool XR>
+static void launch_currents_kets(lm_ctx* ctx, const Geom& g, const double2* hop, const void* x, int64_t m, int64_t ld,
+                                 const double* w, double* out) {
+    typedef typename CT<R>::V V;
+    const unsigned blocks = (unsigned)((g.N + 31) / 32);
+    const int thr = 32 * kReadWarps;
+    if (w) bond_currents_kets_kernel<R, true, XR><<<blocks, thr, 0, ctx->stream>>>(g, hop, (const V*)x, m, ld, w, out);
+    else bond_currents_kets_kernel<R, false, XR><<<blocks, thr, 0, ctx->stream>>>(g, hop, (const V*)x, m, ld, w, out);
+    ctx->launches++;
+}
+
+cudaError_t launch_bond_currents(lm_ctx* ctx, const Geom& g, int precision, int kind, const double2* hop, bool xr,
                                  const void* x, int64_t m, int64_t ld, const double* w, double* out) {
     if (g.N <= 0) return cudaSuccess;
     if (kind == LM_DENSITY) {
         const unsigned blocks = (unsigned)((g.N + 127) / 128);
         if (precision == LM_C64) bond_currents_dm_kernel<double><<<blocks, 128, 0, ctx->stream>>>(g, hop, (const double2*)x, ld, out);
         else bond_currents_dm_kernel<float><<<blocks, 128, 0, ctx->stream>>>(g, hop, (const float2*)x, ld, out);
+        ctx->launches++;
+    } else if (precision == LM_C64) {
+        if (xr) launch_currents_kets<double, true>(ctx, g, hop, x, m, ld, w, out);
+        else launch_currents_kets<double, false>(ctx, g, hop, x, m, ld, w, out);
     } else {
-        const unsigned blocks = (unsigned)((g.N + 31) / 32);
-        const int thr = 32 * kReadWarps;
-        if (precision == LM_C64) {
-            if (w) bond_currents_kets_kernel<double, true><<<blocks, thr, 0, ctx->stream>>>(g, hop, (const double2*)x, m, ld, w, out);
-            else bond_currents_kets_kernel<double, false><<<blocks, thr, 0, ctx->stream>>>(g, hop, (const double2*)x, m, ld, w, out);
-        } else if (g.Ly % 4 == 0 && ld % 2 == 0 && ((uintptr_t)x & 15) == 0 && !ctx->currents_scalar) {
-            cudaError_t e = w ? launch_bond_currents4<true>(ctx, g, hop, (const float2*)x, m, ld, w, out)
-                              : launch_bond_currents4<false>(ctx, g, hop, (const float2*)x, m, ld, w, out);
-            if (e == cudaErrorMemoryAllocation) {  // no scratch for the partial sums
-                (void)cudaGetLastError();
-                if (w) bond_currents_kets_kernel<float, true><<<blocks, thr, 0, ctx->stream>>>(g, hop, (const float2*)x, m, ld, w, out);
-                else bond_currents_kets_kernel<float, false><<<blocks, thr, 0, ctx->stream>>>(g, hop, (const float2*)x, m, ld, w, out);
-            } else if (e != cudaSuccess) {
-                return e;
-            }
-        } else {
-            if (w) bond_currents_kets_kernel<float, true><<<blocks, thr, 0, ctx->stream>>>(g, hop, (const float2*)x, m, ld, w, out);
-            else bond_currents_kets_kernel<float, false><<<blocks, thr, 0, ctx->stream>>>(g, hop, (const float2*)x, m, ld, w, out);
+        if (!w) {
+            const cudaError_t e = launch_readout_c32(ctx, g, hop, xr, (const float2*)x, m, ld, nullptr, out);
+            if (e != cudaErrorMemoryAllocation) return e;
+            (void)cudaGetLastError();  // no scratch for the partial sums: one block per 32 sites and all kets
         }
+        if (xr) launch_currents_kets<float, true>(ctx, g, hop, x, m, ld, w, out);
+        else launch_currents_kets<float, false>(ctx, g, hop, x, m, ld, w, out);
     }
-    ctx->launches++;
     return cudaGetLastError();
+}
+
+cudaError_t launch_readouts(lm_ctx* ctx, const Geom& g, int precision, int kind, const double2* hop, bool xr, const void* x,
+                            int64_t m, int64_t ld, const double* w, double* rho, double* out) {
+    if (precision == LM_C32 && kind == LM_KETS && !w && g.N > 0) {
+        const cudaError_t e = launch_readout_c32(ctx, g, hop, xr, (const float2*)x, m, ld, rho, out);
+        if (e != cudaErrorMemoryAllocation) return e;
+        (void)cudaGetLastError();
+    }
+    const cudaError_t e = launch_localdensity(ctx, precision, kind, x, g.N, m, ld, w, rho);
+    return e == cudaSuccess ? launch_bond_currents(ctx, g, precision, kind, hop, xr, x, m, ld, w, out) : e;
 }
 
 // Per-column norms: one block of 512 threads per column, fixed-order tree reduction.
@@ -775,6 +814,13 @@ cudaError_t launch_column_norms_comp(lm_ctx* ctx, const float2* hi, const uint32
 // (hi + lo)[:, k] *= f = target[k] / norms[k]: f as an FP32 pair (fh + fl, formed once per block
 // and column), the product hi fh exact by TwoProd, the small terms hi fl + lo fh added to its
 // error, and the sum split again into hi and its encoded residual.
+//
+// Bound by HBM (24 bytes per element).  A block takes 256 x kRescalePer x VEC elements of a column and a
+// thread has kRescalePer loads in flight; with 256 elements per block the FP64 division at the head of
+// half a million blocks took most of the time: 256 x 256 sites, 2048 kets 1161 -> 520 us.
+constexpr int kRescalePer = 4;
+
+template <int VEC>
 __global__ void __launch_bounds__(256) rescale_columns_comp_kernel(float2* hi, uint32_t* lo, int64_t n, int64_t m,
                                                                    int64_t ld, const double* __restrict__ norms,
                                                                    const double* __restrict__ target) {
@@ -789,22 +835,55 @@ __global__ void __launch_bounds__(256) rescale_columns_comp_kernel(float2* hi, u
         }
         __syncthreads();
         const float fh = fs.x, fl = fs.y;
-        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-            const float2 a = hi[k * ld + i];
-            const unsigned code = lo[k * ld + i];
-            const float l[2] = {res_lo_x(code), res_lo_y(code)};
-            const float h[2] = {a.x, a.y};
-            float o[2], r[2];
+        float2* h = hi + k * ld;
+        uint32_t* l = lo + k * ld;
+        for (int64_t i0 = ((int64_t)blockIdx.x * kRescalePer * 256 + threadIdx.x) * VEC; i0 < n;
+             i0 += (int64_t)gridDim.x * kRescalePer * 256 * VEC) {
+            float v[kRescalePer][2 * VEC];
+            uint32_t code[kRescalePer][VEC];
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                float p, e;
-                two_prod(h[c], fh, p, e);
-                e = fmaf(h[c], fl, fmaf(l[c], fh, e));
-                o[c] = p + e;
-                r[c] = e - (o[c] - p);
+            for (int u = 0; u < kRescalePer; ++u) {
+                const int64_t i = i0 + (int64_t)u * 256 * VEC;
+                if (i >= n) break;
+                if (VEC == 2) {
+                    const float4 q = *reinterpret_cast<const float4*>(h + i);
+                    const uint2 c = *reinterpret_cast<const uint2*>(l + i);
+                    v[u][0] = q.x;
+                    v[u][1] = q.y;
+                    v[u][2 * VEC - 2] = q.z;
+                    v[u][2 * VEC - 1] = q.w;
+                    code[u][0] = c.x;
+                    code[u][VEC - 1] = c.y;
+                } else {
+                    v[u][0] = h[i].x;
+                    v[u][1] = h[i].y;
+                    code[u][0] = l[i];
+                }
             }
-            hi[k * ld + i] = make_float2(o[0], o[1]);
-            lo[k * ld + i] = res_encode(r[0], r[1]);
+#pragma unroll
+            for (int u = 0; u < kRescalePer; ++u) {
+                const int64_t i = i0 + (int64_t)u * 256 * VEC;
+                if (i >= n) break;
+                float r[2 * VEC];
+#pragma unroll
+                for (int c = 0; c < 2 * VEC; ++c) {
+                    const float lw = (c & 1) ? res_lo_y(code[u][c / 2]) : res_lo_x(code[u][c / 2]);
+                    float p, e;
+                    two_prod(v[u][c], fh, p, e);
+                    e = fmaf(v[u][c], fl, fmaf(lw, fh, e));
+                    const float o = p + e;
+                    r[c] = e - (o - p);
+                    v[u][c] = o;
+                }
+                if (VEC == 2) {
+                    *reinterpret_cast<float4*>(h + i) = make_float4(v[u][0], v[u][1], v[u][2 * VEC - 2], v[u][2 * VEC - 1]);
+                    *reinterpret_cast<uint2*>(l + i) =
+                        make_uint2(res_encode(r[0], r[1]), res_encode(r[2 * VEC - 2], r[2 * VEC - 1]));
+                } else {
+                    h[i] = make_float2(v[u][0], v[u][1]);
+                    l[i] = res_encode(r[0], r[1]);
+                }
+            }
         }
     }
 }
@@ -812,9 +891,11 @@ __global__ void __launch_bounds__(256) rescale_columns_comp_kernel(float2* hi, u
 cudaError_t launch_rescale_columns_comp(lm_ctx* ctx, float2* hi, uint32_t* lo, int64_t n, int64_t m, int64_t ld,
                                         const double* norms, const double* target) {
     if (m <= 0) return cudaSuccess;
-    const int64_t bx = std::min<int64_t>((n + 255) / 256, 1024);
-    const dim3 grid((unsigned)bx, (unsigned)(m < 65535 ? m : 65535));
-    rescale_columns_comp_kernel<<<grid, 256, 0, ctx->stream>>>(hi, lo, n, m, ld, norms, target);
+    const bool wide = n % 2 == 0 && ld % 2 == 0 && ((uintptr_t)hi & 15) == 0 && ((uintptr_t)lo & 7) == 0;
+    const int64_t per = 256ll * kRescalePer * (wide ? 2 : 1);
+    const dim3 grid((unsigned)std::min<int64_t>((n + per - 1) / per, 1024), (unsigned)(m < 65535 ? m : 65535));
+    if (wide) rescale_columns_comp_kernel<2><<<grid, 256, 0, ctx->stream>>>(hi, lo, n, m, ld, norms, target);
+    else rescale_columns_comp_kernel<1><<<grid, 256, 0, ctx->stream>>>(hi, lo, n, m, ld, norms, target);
     ctx->launches++;
     return cudaGetLastError();
 }

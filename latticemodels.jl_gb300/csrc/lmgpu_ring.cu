@@ -125,9 +125,30 @@ int lm_ring_push_currents(lm_ring* r, lm_ham* h, lm_state* st, double t, int64_t
     cudaSetDevice(ctx->device);
     return ring_push(r, t, nb, seq, [&](double* d) {
         if (nb == 0) return cudaSuccess;
-        return launch_bond_currents(ctx, h->lat->g, st->precision, st->kind, h->d_hop, st->d_data, st->m, st->ld,
-                                    st->d_w, d);
+        return launch_bond_currents(ctx, h->lat->g, st->precision, st->kind, h->d_hop, ham_x_real(h), st->d_data, st->m,
+                                    st->ld, st->d_w, d);
     });
+}
+
+int lm_ring_push_readouts(lm_ring* rho, lm_ring* cur, lm_ham* h, lm_state* st, double t, int64_t* seq_rho,
+                          int64_t* seq_cur) {
+    if (!rho || !cur) return LM_ERR_ARG;
+    lm_ctx* ctx = rho->ctx;
+    CHECK_ARG(ctx, rho != cur && cur->ctx == ctx, "lm_ring_push_readouts: needs two rings of one context");
+    CHECK_ARG(ctx, h != nullptr && h->ctx == ctx, "lm_ring_push_readouts: Hamiltonian from another context");
+    CHECK_ARG(ctx, st != nullptr && st->ctx == ctx, "lm_ring_push_readouts: state from another context");
+    CHECK_ARG(ctx, st->n == h->lat->g.N, "lm_ring_push_readouts: state size does not match the lattice");
+    if (!h->assembled) return set_err(ctx, LM_ERR_STATE, "lm_ring_push_readouts: Hamiltonian not assembled");
+    const int64_t nb = h->lat->nbonds;
+    CHECK_ARG(ctx, st->n <= rho->len && nb <= cur->len, "lm_ring_push_readouts: slot shorter than the readout");
+    cudaSetDevice(ctx->device);
+    double* d_rho = rho->d_buf + (size_t)(rho->head % rho->nslots) * (size_t)rho->len;
+    int rc = ring_push(cur, t, nb, seq_cur, [&](double* d) {
+        return launch_readouts(ctx, h->lat->g, st->precision, st->kind, h->d_hop, ham_x_real(h), st->d_data, st->m, st->ld,
+                               st->d_w, d_rho, d);
+    });
+    if (rc != LM_OK) return rc;
+    return ring_push(rho, t, st->n, seq_rho, [](double*) { return cudaSuccess; });  // its slot is filled already
 }
 
 int lm_ring_push_op_currents(lm_ring* r, lm_ell* h, lm_state* st, int ndof, const double* op, double t,

@@ -46,6 +46,15 @@ class ReadoutRing:
                                                           C.byref(seq)))
         return seq.value
 
+    def push_both(self, currents: "ReadoutRing", H, state, t: float):
+        """push_density here and push_currents into the ring ``currents``, in one read of the state
+        where its form allows it; the two sequence numbers."""
+        dh = H.device(self.ctx)
+        a, b = C.c_int64(), C.c_int64()
+        self.ctx.check(self.ctx.lib.lm_ring_push_readouts(self.handle, currents.handle, dh.handle, state.handle,
+                                                          float(t), C.byref(a), C.byref(b)))
+        return a.value, b.value
+
     def push_op_currents(self, H, state, t: float, op=None) -> int:
         """DensityCurrents (op None) or LocalOperatorCurrents of a SparseHamiltonian: the value
         of every stored entry, in CSC order."""
@@ -119,6 +128,8 @@ def _collect_rings(pairs, it, nslots):
     from .observables import _site_sum
     from .sparse import SparseHamiltonian
     slots = [None] * len(pairs)  # per readout: (ring, pending sequence numbers, wrap)
+    kinds = [f._lm_readout for f, _ in pairs]
+    both = sorted(kinds) == ["currents", "density"]  # one of each: read out in one pass (square lattices)
     for moment in it:
         st = moment.state
         general = isinstance(moment.H, SparseHamiltonian)
@@ -139,12 +150,19 @@ def _collect_rings(pairs, it, nslots):
             ring, pending, wrap = slots[i]
             if len(pending) == ring.nslots:  # the oldest slot is about to be reused
                 _take(ts, ring, pending.pop(0), wrap)
+            if both and not general:
+                continue
             if kind == "density":
                 pending.append(ring.push_density(st, moment.t))
             elif general:
                 pending.append(ring.push_op_currents(moment.H, st, moment.t))
             else:
                 pending.append(ring.push_currents(moment.H, st, moment.t))
+        if both and not general:
+            d, c = slots[kinds.index("density")], slots[kinds.index("currents")]
+            sd, sc = d[0].push_both(c[0], moment.H, st, moment.t)
+            d[1].append(sd)
+            c[1].append(sc)
     for (f, ts), sl in zip(pairs, slots):
         if sl is None:
             continue

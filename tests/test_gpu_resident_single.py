@@ -1,8 +1,7 @@
 """The lattice-resident kernels on a single lattice: the step of a ket block (one CTA, several kets per
 CTA, a cluster of two, odd sides, a last item that is not full) bit for bit against the region form,
-lm_solver_step_to against copy and step, and the adjoint's recurrences and sums against the
-per-order kernels (the recurrences keep their operation order; the double-float sums differ in the
-order of terms only: 1e-11)."""
+lm_solver_step_to against copy and step, and the adjoint's recurrences and sums bit for bit against the
+per-order kernels."""
 import numpy as np
 import pytest
 
@@ -67,7 +66,7 @@ def test_step_to(lm, Lx, Ly, prec, dt):
 
 
 @pytest.mark.parametrize("Lx,Ly,M,dt", [(12, 10, 37, 0.05), (64, 64, 150, 0.05), (75, 71, 9, 0.05), (9, 7, 200, 0.2),
-                                        (16, 16, 40, 0.02)])
+                                        (16, 16, 256, 0.02)])
 def test_adjoint_forms_agree(lm, Lx, Ly, M, dt):
     lat = lm.SquareLattice(Lx, Ly)
     rng = np.random.default_rng(8)
@@ -84,5 +83,4 @@ def test_adjoint_forms_agree(lm, Lx, Ly, M, dt):
         ctx.set_resident_form(True)
     (l0, v0, b0), (l1, v1, b1) = out
     assert l0 == l1
-    assert np.linalg.norm(v0 - v1) <= 1e-11 * np.linalg.norm(v1)
-    assert np.linalg.norm(b0 - b1) <= 1e-11 * np.linalg.norm(b1)
+    assert np.array_equal(v0, v1) and np.array_equal(b0, b1)
