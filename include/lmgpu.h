@@ -151,6 +151,8 @@ int lm_state_download(lm_state *st, void *host, int64_t ld);
 /* Device-to-device copy of `src` into `dst` (same shape, kind and precision): the state
  * copy `Evolution` makes at construction (src/evolution.jl:190-194). */
 int lm_state_copy(lm_state *dst, const lm_state *src);
+/* A new state with src's shape, kind, precision, values, weights and residual plane. */
+int lm_state_clone(const lm_state *src, lm_state **out);
 /* Current device buffer (it may change after a step) and its leading dimension. */
 int lm_state_device_ptr(lm_state *st, void **ptr, int64_t *ld);
 /* Ket weights w_m, so that P = sum_m w_m |psi_m><psi_m| for the readouts; NULL = all ones. */

@@ -438,15 +438,15 @@ struct lm_adjoint {
 
 static void adj_free_stack(lm_adjoint* a) {
     for (size_t i = 1; i < a->T.size(); ++i)
-        if (a->T[i]) cudaFree(a->T[i]);
+        dev_free(a->ctx, a->T[i]);
     a->T.clear();
     for (auto& b : a->B)
-        if (b) cudaFree(b);
+        dev_free(a->ctx, b);
     a->B.clear();
 }
 
 static int adj_alloc(lm_ctx* ctx, void** p, size_t bytes) {
-    if (cudaMalloc(p, bytes) != cudaSuccess) {
+    if (dev_alloc(ctx, p, bytes) != cudaSuccess) {
         *p = nullptr;
         cudaGetLastError();
         return set_err(ctx, LM_ERR_OOM, "lm_adjoint: device allocation failed");
@@ -504,11 +504,11 @@ int lm_adjoint_create(lm_ctx* ctx, int64_t n, int64_t m, int precision, int nslo
     if (rc == LM_OK) rc = adj_alloc(ctx, (void**)&a->d_target, sizeof(double) * (size_t)n);
     if (rc == LM_OK) rc = adj_alloc(ctx, (void**)&a->d_dhop, sizeof(double2) * 2 * (size_t)n);
     if (rc != LM_OK) {
-        if (a->d_gV) cudaFree(a->d_gV);
-        if (a->d_gA) cudaFree(a->d_gA);
-        if (a->d_loss) cudaFree(a->d_loss);
-        if (a->d_target) cudaFree(a->d_target);
-        if (a->d_dhop) cudaFree(a->d_dhop);
+        dev_free(ctx, a->d_gV);
+        dev_free(ctx, a->d_gA);
+        dev_free(ctx, a->d_loss);
+        dev_free(ctx, a->d_target);
+        dev_free(ctx, a->d_dhop);
         delete a;
         return rc;
     }
@@ -523,11 +523,11 @@ int lm_adjoint_destroy(lm_adjoint* a) {
     cudaSetDevice(a->ctx->device);
     cudaStreamSynchronize(a->ctx->stream);
     adj_free_stack(a);
-    cudaFree(a->d_gV);
-    cudaFree(a->d_gA);
-    cudaFree(a->d_loss);
-    cudaFree(a->d_target);
-    cudaFree(a->d_dhop);
+    dev_free(a->ctx, a->d_gV);
+    dev_free(a->ctx, a->d_gA);
+    dev_free(a->ctx, a->d_loss);
+    dev_free(a->ctx, a->d_target);
+    dev_free(a->ctx, a->d_dhop);
     delete a;
     return LM_OK;
 }

@@ -70,6 +70,65 @@ void bessel_j_all(double x, int kmax, std::vector<double>& out) {
 }  // namespace lmgpu
 
 
+namespace lmgpu {
+cudaError_t dev_alloc(lm_ctx* ctx, void** p, size_t bytes) {
+    *p = nullptr;
+    if (!ctx->pool) return cudaMalloc(p, bytes);
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->stream);
+    if (e == cudaErrorMemoryAllocation) {  // what the pool keeps in pieces may be missing as a whole
+        cudaGetLastError();
+        cudaStreamSynchronize(ctx->stream);
+        cudaMemPoolTrimTo(ctx->pool, 0);
+        e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->stream);
+    }
+    if (e != cudaSuccess) *p = nullptr;
+    return e;
+}
+
+void dev_free(lm_ctx* ctx, void* p) {
+    if (!p) return;
+    if (ctx->pool) cudaFreeAsync(p, ctx->stream);
+    else cudaFree(p);
+}
+
+// A pool of the context's own.  Up to a 64th of the device's memory (4.4 GB) stays with it across
+// synchronisations instead of going back to the driver: allocating and freeing the buffers of a
+// 265 MB state cost 1.1 ms per Evolution.  lm_ctx_destroy gives everything back.
+static void create_pool(lm_ctx* ctx) {
+    int ok = 0;
+    if (cudaDeviceGetAttribute(&ok, cudaDevAttrMemoryPoolsSupported, ctx->device) != cudaSuccess || !ok) {
+        cudaGetLastError();
+        return;
+    }
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = ctx->device;
+    size_t free_b = 0, total = 0;
+    if (cudaMemPoolCreate(&ctx->pool, &props) != cudaSuccess || cudaMemGetInfo(&free_b, &total) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->pool = nullptr;
+        return;
+    }
+    unsigned long long keep = total / 64;
+    cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+}
+}  // namespace lmgpu
+
+static int dalloc_pool(lm_ctx* ctx, void** p, size_t bytes, const char* what) {
+    *p = nullptr;
+    if (bytes == 0) return LM_OK;
+    cudaError_t e = dev_alloc(ctx, p, bytes);
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        cudaGetLastError();
+        return set_err(ctx, e == cudaErrorMemoryAllocation ? LM_ERR_OOM : LM_ERR_CUDA,
+                       std::string("device memory (") + what + "): " + cudaGetErrorString(e));
+    }
+    return LM_OK;
+}
+
 static int dalloc(lm_ctx* ctx, void** p, size_t bytes, const char* what) {
     *p = nullptr;
     if (bytes == 0) return LM_OK;
@@ -87,13 +146,13 @@ namespace lmgpu {
 // Allocates the accumulator buffer of a state on first use (the per-order path needs it).
 int ensure_accumulator(lm_state* s) {
     if (s->d_y) return LM_OK;
-    return dalloc(s->ctx, &s->d_y, s->elem * (size_t)s->ld * (size_t)s->m, "accumulator scratch");
+    return dalloc_pool(s->ctx, &s->d_y, s->elem * (size_t)s->ld * (size_t)s->m, "accumulator scratch");
 }
 // Allocates the recurrence scratch (T_{k-1}/T_k ping-pong) of a state on first use; a state
 // stepped only through a panelled batch never needs it.
 int ensure_scratch(lm_state* s) {
     if (s->d_a) return LM_OK;
-    return dalloc(s->ctx, &s->d_a, s->elem * (size_t)s->ld * (size_t)s->m, "recurrence scratch");
+    return dalloc_pool(s->ctx, &s->d_a, s->elem * (size_t)s->ld * (size_t)s->m, "recurrence scratch");
 }
 }  // namespace lmgpu
 
@@ -213,6 +272,7 @@ int lm_ctx_create(int device, lm_ctx** out) {
         return LM_ERR_CUDA;
     }
     cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
+    create_pool(c);
     if (const char* v = getenv("LMGPU_READOUT_SLICES")) c->ld_slices_override = std::max(0, std::min(64, atoi(v)));
     if (const char* v = getenv("LMGPU_CURRENTS_SCALAR")) c->currents_scalar = atoi(v) != 0;
     *out = c;
@@ -228,6 +288,7 @@ int lm_ctx_destroy(lm_ctx* ctx) {
     if (ctx->d_res_err) cudaFree(ctx->d_res_err);
     if (ctx->h_res_err) cudaFreeHost(ctx->h_res_err);
     for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
+    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
     return LM_OK;
@@ -617,7 +678,7 @@ int lm_ham_bounds(lm_ham* h, double* emin, double* emax) {
 // ------------------------------------------------------------------------------------------
 // states
 // ------------------------------------------------------------------------------------------
-int lm_state_create(lm_ctx* ctx, int64_t n, int64_t m, int kind, int precision, lm_state** out) {
+static int state_alloc(lm_ctx* ctx, int64_t n, int64_t m, int kind, int precision, lm_state** out) {
     if (!ctx) return LM_ERR_ARG;
     CHECK_ARG(ctx, out != nullptr, "lm_state_create: null output");
     *out = nullptr;
@@ -636,26 +697,59 @@ int lm_state_create(lm_ctx* ctx, int64_t n, int64_t m, int kind, int precision, 
     s->elem = precision == LM_C64 ? 16 : 8;
     cudaSetDevice(ctx->device);
     const size_t bytes = s->elem * (size_t)n * (size_t)m;
-    int rc = dalloc(ctx, &s->d_data, bytes, "state");
+    int rc = dalloc_pool(ctx, &s->d_data, bytes, "state");
     // the recurrence scratch and the accumulator are allocated on first use
     if (rc != LM_OK) {
         delete s;
         return rc;
     }
-    cudaMemsetAsync(s->d_data, 0, bytes, ctx->stream);
     *out = s;
     return LM_OK;
+}
+
+int lm_state_create(lm_ctx* ctx, int64_t n, int64_t m, int kind, int precision, lm_state** out) {
+    const int rc = state_alloc(ctx, n, m, kind, precision, out);
+    if (rc != LM_OK) return rc;
+    cudaMemsetAsync((*out)->d_data, 0, (*out)->elem * (size_t)n * (size_t)m, ctx->stream);
+    return LM_OK;
+}
+
+int lm_state_clone(const lm_state* src, lm_state** out) {
+    if (!src) return LM_ERR_ARG;
+    lm_ctx* ctx = src->ctx;
+    CHECK_ARG(ctx, out != nullptr, "lm_state_clone: null output");
+    int rc = state_alloc(ctx, src->n, src->m, src->kind, src->precision, out);
+    if (rc != LM_OK) return rc;
+    lm_state* s = *out;
+    if (src->d_lo) rc = dalloc_pool(ctx, (void**)&s->d_lo, sizeof(uint32_t) * (size_t)s->ld * (size_t)s->m, "compensation plane");
+    if (rc == LM_OK && src->d_w) {
+        rc = dalloc(ctx, (void**)&s->d_w, sizeof(double) * (size_t)s->m, "weights");
+        if (rc == LM_OK)
+            rc = check_cuda(ctx, cudaMemcpyAsync(s->d_w, src->d_w, sizeof(double) * (size_t)s->m, cudaMemcpyDeviceToDevice,
+                                                 ctx->stream),
+                            "copy weights");
+    }
+    if (rc == LM_OK) rc = lm_state_copy(s, src);
+    if (rc != LM_OK) {
+        lm_state_destroy(s);
+        *out = nullptr;
+    }
+    return rc;
 }
 
 int lm_state_destroy(lm_state* s) {
     if (!s) return LM_OK;
     cudaSetDevice(s->ctx->device);
-    cudaStreamSynchronize(s->ctx->stream);
-    if (s->d_data) cudaFree(s->d_data);
-    if (s->d_a) cudaFree(s->d_a);
-    if (s->d_y) cudaFree(s->d_y);
-    if (s->d_w) cudaFree(s->d_w);
-    if (s->d_lo) cudaFree(s->d_lo);
+    // a buffer that was handed out may be in use on any stream; the others only on the context's
+    if (s->exposed) cudaDeviceSynchronize();
+    dev_free(s->ctx, s->d_data);
+    dev_free(s->ctx, s->d_a);
+    dev_free(s->ctx, s->d_y);
+    dev_free(s->ctx, s->d_lo);
+    if (s->d_w) {
+        cudaStreamSynchronize(s->ctx->stream);
+        cudaFree(s->d_w);
+    }
     delete s;
     return LM_OK;
 }
@@ -665,10 +759,7 @@ int lm_state_set_compensation(lm_state* s, int enable) {
     lm_ctx* ctx = s->ctx;
     cudaSetDevice(ctx->device);
     if (!enable) {
-        if (s->d_lo) {
-            cudaStreamSynchronize(ctx->stream);
-            cudaFree(s->d_lo);
-        }
+        dev_free(ctx, s->d_lo);
         s->d_lo = nullptr;
         return LM_OK;
     }
@@ -676,7 +767,7 @@ int lm_state_set_compensation(lm_state* s, int enable) {
               "lm_state_set_compensation: applies to ComplexF32 ket blocks");
     if (s->d_lo) return LM_OK;
     const size_t bytes = sizeof(uint32_t) * (size_t)s->ld * (size_t)s->m;
-    int rc = dalloc(ctx, (void**)&s->d_lo, bytes, "compensation plane");
+    int rc = dalloc_pool(ctx, (void**)&s->d_lo, bytes, "compensation plane");
     if (rc != LM_OK) return rc;
     CUDA_TRY(ctx, cudaMemsetAsync(s->d_lo, 0, bytes, ctx->stream), "clear compensation plane");
     return LM_OK;
@@ -717,14 +808,17 @@ int lm_state_copy(lm_state* dst, const lm_state* src) {
     CHECK_ARG(ctx, dst->n == src->n && dst->m == src->m && dst->kind == src->kind && dst->precision == src->precision,
               "lm_state_copy: states differ in shape, kind or precision");
     cudaSetDevice(ctx->device);
-    CUDA_TRY(ctx, cudaMemcpy2DAsync(dst->d_data, dst->elem * (size_t)dst->ld, src->d_data, src->elem * (size_t)src->ld,
-                                    dst->elem * (size_t)dst->n, (size_t)dst->m, cudaMemcpyDeviceToDevice, ctx->stream),
-             "copy state");
+    // without padding rows one linear copy, which runs at HBM rate (265 MB in 85 us; as a 2D copy 262 us)
+    const size_t count = (size_t)dst->n * (size_t)dst->m;
+    const bool flat = dst->ld == dst->n && src->ld == src->n;
+    auto copy = [&](void* d, const void* p, size_t elem) {
+        return flat ? cudaMemcpyAsync(d, p, elem * count, cudaMemcpyDeviceToDevice, ctx->stream)
+                    : cudaMemcpy2DAsync(d, elem * (size_t)dst->ld, p, elem * (size_t)src->ld, elem * (size_t)dst->n,
+                                        (size_t)dst->m, cudaMemcpyDeviceToDevice, ctx->stream);
+    };
+    CUDA_TRY(ctx, copy(dst->d_data, src->d_data, dst->elem), "copy state");
     if (dst->d_lo && src->d_lo)
-        CUDA_TRY(ctx, cudaMemcpy2DAsync(dst->d_lo, sizeof(uint32_t) * (size_t)dst->ld, src->d_lo,
-                                        sizeof(uint32_t) * (size_t)src->ld, sizeof(uint32_t) * (size_t)dst->n,
-                                        (size_t)dst->m, cudaMemcpyDeviceToDevice, ctx->stream),
-                 "copy compensation plane");
+        CUDA_TRY(ctx, copy(dst->d_lo, src->d_lo, sizeof(uint32_t)), "copy compensation plane");
     else if (dst->d_lo)
         CUDA_TRY(ctx, cudaMemsetAsync(dst->d_lo, 0, sizeof(uint32_t) * (size_t)dst->ld * (size_t)dst->m, ctx->stream),
                  "clear compensation plane");
@@ -735,6 +829,7 @@ int lm_state_device_ptr(lm_state* s, void** ptr, int64_t* ld) {
     if (!s) return LM_ERR_ARG;
     CHECK_ARG(s->ctx, ptr != nullptr, "lm_state_device_ptr: null output");
     *ptr = s->d_data;
+    s->exposed = 1;
     if (ld) *ld = s->ld;
     return LM_OK;
 }

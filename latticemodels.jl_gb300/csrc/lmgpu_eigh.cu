@@ -1032,7 +1032,7 @@ namespace {
 
 template <typename T>
 int dalloc_t(lm_ctx* ctx, T** p, size_t count, const char* what) {
-    cudaError_t e = cudaMalloc((void**)p, sizeof(T) * std::max<size_t>(count, 1));
+    cudaError_t e = dev_alloc(ctx, (void**)p, sizeof(T) * std::max<size_t>(count, 1));
     if (e != cudaSuccess) {
         *p = nullptr;
         cudaGetLastError();
@@ -1053,9 +1053,11 @@ int upload_vec(lm_ctx* ctx, T** dptr, const std::vector<T>& h, const char* what)
 }
 
 struct DevFree {
+    explicit DevFree(lm_ctx* c) : ctx(c) {}
+    lm_ctx* ctx;
     std::vector<void*> ptrs;
     ~DevFree() {
-        for (void* p : ptrs) cudaFree(p);
+        for (void* p : ptrs) dev_free(ctx, p);
     }
     template <typename T>
     T* keep(T* p) {
@@ -1065,10 +1067,10 @@ struct DevFree {
 };
 
 void free_eigsys(lm_eigsys* e) {
-    cudaFree(e->d_A);
-    cudaFree(e->d_tau);
-    cudaFree(e->d_d);
-    cudaFree(e->d_e);
+    dev_free(e->ctx, e->d_A);
+    dev_free(e->ctx, e->d_tau);
+    dev_free(e->ctx, e->d_d);
+    dev_free(e->ctx, e->d_e);
     e->d_A = nullptr;
     e->d_tau = nullptr;
     e->d_d = nullptr;
@@ -1180,7 +1182,7 @@ int reduce_and_solve(lm_eigsys* es) {
     if (rc == LM_OK) rc = dalloc_t(ctx, &es->d_d, (size_t)n, "tridiagonal");
     if (rc == LM_OK) rc = dalloc_t(ctx, &es->d_e, (size_t)std::max<int64_t>(n - 1, 1), "tridiagonal");
     if (rc != LM_OK) return rc;
-    DevFree tmp;
+    DevFree tmp(ctx);
     rc = tri_resident_cols(ctx, n) ? reduce_resident(es, tmp) : reduce_tiles(es, tmp);
     if (rc != LM_OK) return rc;
     es->d.assign((size_t)n, 0.0);
@@ -1375,7 +1377,7 @@ int eigvectors(lm_eigsys* es, const std::vector<int64_t>& idx, double2* X, int64
     const int64_t nmem = (int64_t)mem_lam.size(), ncl = (int64_t)cl_first.size();
     int64_t lmax = 1;
     for (int64_t l : mem_len) lmax = std::max(lmax, l);
-    DevFree tmp;
+    DevFree tmp(ctx);
     int64_t *d_clf = nullptr, *d_clc = nullptr, *d_ms = nullptr, *d_ml = nullptr, *d_seed = nullptr, *d_col = nullptr;
     double *d_lam = nullptr, *d_vec = nullptr, *d_scr = nullptr;
     int rc = upload_vec(ctx, &d_clf, cl_first, "inverse iteration");
@@ -1518,7 +1520,7 @@ int lm_eigsys_vectors(lm_eigsys* e, int64_t first, lm_state* out) {
     if (rc != LM_OK) return rc;
     CHECK_ARG(ctx, first >= 0 && first + out->m <= e->n, "lm_eigsys_vectors: index range outside the spectrum");
     cudaSetDevice(ctx->device);
-    DevFree tmp;
+    DevFree tmp(ctx);
     double2* X = nullptr;
     const bool direct = out->precision == LM_C64;
     for (int64_t c0 = 0; c0 < out->m; c0 += kChunk) {
@@ -1557,7 +1559,7 @@ int lm_eigsys_projector(lm_eigsys* e, const double* weights, lm_state* out) {
         CHECK_ARG(ctx, std::isfinite(weights[k]), "lm_eigsys_projector: non-finite weight");
     cudaSetDevice(ctx->device);
     const int64_t n = e->n;
-    DevFree tmp;
+    DevFree tmp(ctx);
     double2* P = nullptr;
     int64_t ldp = out->ld;
     if (out->precision == LM_C64) {
@@ -1580,8 +1582,8 @@ int lm_eigsys_projector(lm_eigsys* e, const double* weights, lm_state* out) {
         rc = dalloc_t(ctx, &X, (size_t)n * (size_t)cw, "eigenvector chunk");
         if (rc == LM_OK) rc = dalloc_t(ctx, &d_w, (size_t)cw, "weights");
         if (rc != LM_OK) {
-            cudaFree(X);
-            cudaFree(d_w);
+            dev_free(ctx, X);
+            dev_free(ctx, d_w);
             return rc;
         }
         tmp.keep(X);

@@ -235,7 +235,7 @@ int ell_solver_step(lm_solver* s, lm_state* st) {
     }
     if (!st->d_y) {
         const size_t bytes = st->elem * (size_t)st->ld * (size_t)st->m;
-        if (cudaMalloc(&st->d_y, bytes) != cudaSuccess) {
+        if (dev_alloc(ctx, &st->d_y, bytes) != cudaSuccess) {
             st->d_y = nullptr;
             cudaGetLastError();
             return set_err(ctx, LM_ERR_OOM, "lm_solver_step: accumulator allocation");

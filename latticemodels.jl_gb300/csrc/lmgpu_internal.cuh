@@ -103,6 +103,7 @@ struct lm_ctx {
     int fused_form = 1;                 // LM_OPT_STREAM: 1 = x-streaming form where supported, 0 = region form
     int64_t stream_launches = 0;        // fused steps run in the x-streaming form
     int kpm_df = 1;                     // LM_OPT_KPM: double-float recurrence in lm_kpm_moments
+    cudaMemPool_t pool = nullptr;       // device memory of states and temporaries (dev_alloc); null: cudaMalloc
     unsigned resident_attr = 0;         // shared-memory attributes of the lattice-resident kernels set
     unsigned long long* d_res_err = nullptr;  // their timeout word (single-lattice launches), and
     unsigned long long* h_res_err = nullptr;  // its pinned copy, refreshed after every cluster launch
@@ -161,6 +162,7 @@ struct lm_state {
     // significant bits; element i of ket k at d_lo[k ld + i], updated in place by the
     // x-streaming step (null when off)
     uint32_t* d_lo = nullptr;
+    int exposed = 0;   // lm_state_device_ptr handed a buffer out: other streams may be reading it
 };
 
 struct lm_solver {
@@ -261,6 +263,11 @@ namespace lmgpu {
 
 int set_err(lm_ctx* ctx, int code, const std::string& msg);
 int check_cuda(lm_ctx* ctx, cudaError_t e, const char* what);
+// Device memory from the context's pool, ordered on its stream: an allocation is valid for work on that
+// stream, and a free waits for the work queued there before it.  Memory that other streams use is
+// synchronised with them before it is freed.
+cudaError_t dev_alloc(lm_ctx* ctx, void** p, size_t bytes);
+void dev_free(lm_ctx* ctx, void* p);
 
 // Kernel launchers (lmgpu_kernels.cu).  All launch on ctx->stream and return cudaError_t.
 cudaError_t launch_assemble(lm_ctx* ctx, const Geom& g, const FieldSet& f, double t1, double2* hop);

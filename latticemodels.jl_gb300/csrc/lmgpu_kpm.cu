@@ -565,7 +565,7 @@ static int cheb_apply_resident(lm_ham* h, const SeriesPlan& plan, double a, doub
     const bool xr = ham_x_real(h);
     char* buf = nullptr;  // hops, gauge, diagonal, coefficients
     const size_t o_g = sizeof(float4) * N, o_d = o_g + (xr ? 0 : sizeof(double2) * N), o_c = o_d + sizeof(float2) * N;
-    cudaError_t e = cudaMalloc((void**)&buf, o_c + sizeof(float2) * (size_t)ncoef);
+    cudaError_t e = dev_alloc(ctx, (void**)&buf, o_c + sizeof(float2) * (size_t)ncoef);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return check_cuda(ctx, e, "lm_cheb_apply: allocation");
@@ -602,7 +602,7 @@ static int cheb_apply_resident(lm_ham* h, const SeriesPlan& plan, double a, doub
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     const int rc = e == cudaSuccess ? LM_OK : check_cuda(ctx, e, "lm_cheb_apply: on-chip series");
-    cudaFree(buf);
+    dev_free(ctx, buf);
     return rc;
 }
 
@@ -650,21 +650,21 @@ int lm_kpm_moments(lm_ham* h, double emin, double emax, int nmom, const lm_state
     const int64_t nblk = march_blocks(ma);
     double* part = nullptr;  // partial dots of kPartPasses passes
     auto release = [&]() {
-        cudaStreamSynchronize(ctx->stream);
-        cudaFree(hop2); cudaFree(diag2); cudaFree(hop2f); cudaFree(diag2f);
-        cudaFree(TA); cudaFree(TB); cudaFree(dots); cudaFree(hopd); cudaFree(diagd); cudaFree(part);
+        for (void* p : {(void*)hop2, (void*)diag2, (void*)hop2f, (void*)diag2f, (void*)TA, (void*)TB, (void*)dots, (void*)hopd,
+                        (void*)diagd, (void*)part})
+            dev_free(ctx, p);
     };
-    cudaError_t e = cudaMalloc((void**)&hop2, sizeof(double2) * 2 * (size_t)N);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&diag2, sizeof(double) * (size_t)N);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&hop2f, sizeof(float2) * 2 * (size_t)N);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&diag2f, sizeof(float) * (size_t)N);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&TA, blk);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&TB, blk);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&dots, sizeof(double) * ndots);
-    if (e == cudaSuccess && use_df) e = cudaMalloc((void**)&hopd, sizeof(float4) * 2 * (size_t)N);
-    if (e == cudaSuccess && use_df) e = cudaMalloc((void**)&diagd, sizeof(float2) * (size_t)N);
+    cudaError_t e = dev_alloc(ctx, (void**)&hop2, sizeof(double2) * 2 * (size_t)N);
+    if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&diag2, sizeof(double) * (size_t)N);
+    if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&hop2f, sizeof(float2) * 2 * (size_t)N);
+    if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&diag2f, sizeof(float) * (size_t)N);
+    if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&TA, blk);
+    if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&TB, blk);
+    if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&dots, sizeof(double) * ndots);
+    if (e == cudaSuccess && use_df) e = dev_alloc(ctx, (void**)&hopd, sizeof(float4) * 2 * (size_t)N);
+    if (e == cudaSuccess && use_df) e = dev_alloc(ctx, (void**)&diagd, sizeof(float2) * (size_t)N);
     if (e == cudaSuccess && use_df)
-        e = cudaMalloc((void**)&part, sizeof(double) * (size_t)(kPartPasses * nblk * 2 * M));
+        e = dev_alloc(ctx, (void**)&part, sizeof(double) * (size_t)(kPartPasses * nblk * 2 * M));
     if (e != cudaSuccess) {
         cudaGetLastError();
         release();
@@ -813,18 +813,19 @@ int lm_cheb_apply(lm_ham* h, double emin, double emax, const double* coef, int n
     const size_t blk = sizeof(double2) * (size_t)ld * (size_t)M;
     auto release = [&]() {
         cudaStreamSynchronize(ctx->stream);
-        cudaFree(hop2); cudaFree(diag2); cudaFree(hop2f); cudaFree(diag2f);
-        cudaFree(TA); cudaFree(TB); cudaFree(Y); cudaFree(hopd); cudaFree(diagd);
+        for (void* p : {(void*)hop2, (void*)diag2, (void*)hop2f, (void*)diag2f, (void*)TA, (void*)TB, (void*)Y, (void*)hopd,
+                        (void*)diagd})
+            dev_free(ctx, p);
     };
-    cudaError_t e = cudaMalloc((void**)&hop2, sizeof(double2) * 2 * (size_t)N);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&diag2, sizeof(double) * (size_t)N);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&hop2f, sizeof(float2) * 2 * (size_t)N);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&diag2f, sizeof(float) * (size_t)N);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&TA, blk);
-    if (e == cudaSuccess && ncoef > 1) e = cudaMalloc((void**)&TB, blk);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&Y, blk);
-    if (e == cudaSuccess && use_df) e = cudaMalloc((void**)&hopd, sizeof(float4) * 2 * (size_t)N);
-    if (e == cudaSuccess && use_df) e = cudaMalloc((void**)&diagd, sizeof(float2) * (size_t)N);
+    cudaError_t e = dev_alloc(ctx, (void**)&hop2, sizeof(double2) * 2 * (size_t)N);
+    if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&diag2, sizeof(double) * (size_t)N);
+    if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&hop2f, sizeof(float2) * 2 * (size_t)N);
+    if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&diag2f, sizeof(float) * (size_t)N);
+    if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&TA, blk);
+    if (e == cudaSuccess && ncoef > 1) e = dev_alloc(ctx, (void**)&TB, blk);
+    if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&Y, blk);
+    if (e == cudaSuccess && use_df) e = dev_alloc(ctx, (void**)&hopd, sizeof(float4) * 2 * (size_t)N);
+    if (e == cudaSuccess && use_df) e = dev_alloc(ctx, (void**)&diagd, sizeof(float2) * (size_t)N);
     if (e != cudaSuccess) {
         cudaGetLastError();
         release();
@@ -945,14 +946,14 @@ int lm_ham_lanczos_bounds(lm_ham* h, int iters, unsigned long long seed, double*
     double* dot = nullptr;
     auto release = [&]() {
         cudaStreamSynchronize(ctx->stream);
-        cudaFree(hop2); cudaFree(diag2); cudaFree(hop2f); cudaFree(diag2f); cudaFree(buf); cudaFree(dot);
+        for (void* p : {(void*)hop2, (void*)diag2, (void*)hop2f, (void*)diag2f, (void*)buf, (void*)dot}) dev_free(ctx, p);
     };
-    cudaError_t e = cudaMalloc((void**)&hop2, sizeof(double2) * 2 * (size_t)N);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&diag2, sizeof(double) * (size_t)N);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&hop2f, sizeof(float2) * 2 * (size_t)N);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&diag2f, sizeof(float) * (size_t)N);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&buf, sizeof(double2) * 3 * (size_t)N);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&dot, sizeof(double));
+    cudaError_t e = dev_alloc(ctx, (void**)&hop2, sizeof(double2) * 2 * (size_t)N);
+    if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&diag2, sizeof(double) * (size_t)N);
+    if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&hop2f, sizeof(float2) * 2 * (size_t)N);
+    if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&diag2f, sizeof(float) * (size_t)N);
+    if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&buf, sizeof(double2) * 3 * (size_t)N);
+    if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&dot, sizeof(double));
     if (e != cudaSuccess) {
         cudaGetLastError();
         release();

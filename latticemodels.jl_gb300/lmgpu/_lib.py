@@ -74,6 +74,7 @@ SIGNATURES = {
     "lm_state_upload": (_INT, [_P, _P, _I64]),
     "lm_state_download": (_INT, [_P, _P, _I64]),
     "lm_state_copy": (_INT, [_P, _P]),
+    "lm_state_clone": (_INT, [_P, C.POINTER(_P)]),
     "lm_state_device_ptr": (_INT, [_P, C.POINTER(_P), _PI64]),
     "lm_state_set_weights": (_INT, [_P, _PD]),
     "lm_state_norms": (_INT, [_P, _PD]),

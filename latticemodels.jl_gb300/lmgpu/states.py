@@ -126,11 +126,12 @@ class DeviceState:
     def copy(self):
         """Device-to-device copy (the copy Evolution makes at construction)."""
         c = object.__new__(type(self))
-        DeviceState.__init__(c, self.lattice, None, self.kind, self.precision, self.weights, self.ctx,
-                             shape=(self.n, self.m))
-        if self.compensated:
-            c.set_compensation(True)
-        self.ctx.check(self.ctx.lib.lm_state_copy(c.handle, self.handle))
+        c.ctx, c.lattice, c.kind, c.precision = self.ctx, self.lattice, self.kind, self.precision
+        c.n, c.m, c.weights, c.compensated = self.n, self.m, self.weights, self.compensated
+        p = C.c_void_p()
+        self.ctx.check(self.ctx.lib.lm_state_clone(self.handle, C.byref(p)))
+        c.handle = p
+        c._fin = weakref.finalize(c, self.ctx.lib.lm_state_destroy, p)
         return c
 
     def __repr__(self):

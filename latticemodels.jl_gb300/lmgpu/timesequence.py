@@ -73,10 +73,14 @@ class ReadoutRing:
         self.ctx.check(self.ctx.lib.lm_ring_ready(self.handle, int(seq), C.byref(r)))
         return bool(r.value)
 
-    def wait(self, seq: int):
-        """(t, values) of entry ``seq`` (a fresh array)."""
+    def wait(self, seq: int, out=None):
+        """(t, values) of entry ``seq``: a fresh array, or ``out`` (a float64 row of the ring's length)."""
         n = C.c_int64()
         t = C.c_double()
+        if out is not None:
+            self.ctx.check(self.ctx.lib.lm_ring_wait(self.handle, int(seq), C.cast(out.ctypes.data, C.POINTER(C.c_double)),
+                                                     None, C.byref(n), C.byref(t)))
+            return t.value, out[:n.value]
         view = C.POINTER(C.c_double)()
         self.ctx.check(self.ctx.lib.lm_ring_wait(self.handle, int(seq), None, C.byref(view), C.byref(n),
                                                  C.byref(t)))
@@ -128,6 +132,7 @@ def _collect_rings(pairs, it, nslots):
     from .observables import _site_sum
     from .sparse import SparseHamiltonian
     slots = [None] * len(pairs)  # per readout: (ring, pending sequence numbers, wrap)
+    rows = [[] for _ in pairs]   # per readout: unused rows of its current block of results
     kinds = [f._lm_readout for f, _ in pairs]
     both = sorted(kinds) == ["currents", "density"]  # one of each: read out in one pass (square lattices)
     for moment in it:
@@ -149,7 +154,7 @@ def _collect_rings(pairs, it, nslots):
                 slots[i] = (_ring_for(st.ctx, length, nslots, same), [], wrap)
             ring, pending, wrap = slots[i]
             if len(pending) == ring.nslots:  # the oldest slot is about to be reused
-                _take(ts, ring, pending.pop(0), wrap)
+                _take(ts, ring, pending.pop(0), wrap, rows[i])
             if both and not general:
                 continue
             if kind == "density":
@@ -163,16 +168,26 @@ def _collect_rings(pairs, it, nslots):
             sd, sc = d[0].push_both(c[0], moment.H, st, moment.t)
             d[1].append(sd)
             c[1].append(sc)
-    for (f, ts), sl in zip(pairs, slots):
+    for (f, ts), sl, rw in zip(pairs, slots, rows):
         if sl is None:
             continue
         ring, pending, wrap = sl
         for seq in pending:
-            _take(ts, ring, seq, wrap)
+            _take(ts, ring, seq, wrap, rw)
 
 
-def _take(ts, ring, seq, wrap):
-    t, v = ring.wait(seq)
+# Large readouts of a sequence are rows of blocks of this size: numpy backs arrays from 4 MB with huge pages,
+# while every 800 KB array of its own was 200 page faults (55 us)
+_BLOCK_BYTES = 4 << 20
+
+
+def _take(ts, ring, seq, wrap, rows):
+    if 8 * ring.length < (64 << 10):
+        t, v = ring.wait(seq)
+    else:
+        if not rows:
+            rows.extend(np.empty((-(-_BLOCK_BYTES // (8 * ring.length)), ring.length))[::-1])
+        t, v = ring.wait(seq, rows.pop())
     ts.times.append(t)
     ts.values.append(wrap(v))
 
