@@ -285,7 +285,7 @@ int lm_ctx_destroy(lm_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     if (ctx->d_red) cudaFree(ctx->d_red);
     if (ctx->d_ld_part) cudaFree(ctx->d_ld_part);
-    if (ctx->d_res_err) cudaFree(ctx->d_res_err);
+    if (ctx->d_grid) cudaFree(ctx->d_grid);
     if (ctx->h_res_err) cudaFreeHost(ctx->h_res_err);
     for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
@@ -299,7 +299,7 @@ const char* lm_last_error(const lm_ctx* ctx) { return ctx ? ctx->err.c_str() : "
 int lm_ctx_synchronize(lm_ctx* ctx) {
     if (!ctx) return LM_ERR_ARG;
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize");
-    return resident_status(ctx);
+    return wait_status(ctx);
 }
 
 int lm_ctx_stream(lm_ctx* ctx, void** stream) {
@@ -798,7 +798,7 @@ int lm_state_download(lm_state* s, void* host, int64_t ld) {
                                     (size_t)s->m, cudaMemcpyDeviceToHost, ctx->stream),
              "download state");
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "sync");
-    return resident_status(ctx);
+    return wait_status(ctx);
 }
 
 int lm_state_copy(lm_state* dst, const lm_state* src) {
@@ -1042,9 +1042,19 @@ int lm_solver_order(const lm_solver* s, int* K, double* a, double* b) {
 
 namespace lmgpu {
 
-int resident_status(lm_ctx* ctx) {
+int ensure_wait_words(lm_ctx* ctx) {
+    if (ctx->d_grid) return LM_OK;
+    CUDA_TRY(ctx, cudaHostAlloc((void**)&ctx->h_res_err, sizeof(unsigned long long), cudaHostAllocMapped), "status word");
+    *ctx->h_res_err = 0;
+    CUDA_TRY(ctx, cudaHostGetDevicePointer((void**)&ctx->d_res_err, ctx->h_res_err, 0), "status word");
+    CUDA_TRY(ctx, cudaMalloc((void**)&ctx->d_grid, 2 * sizeof(unsigned)), "barrier counters");
+    CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_grid, 0, 2 * sizeof(unsigned), ctx->stream), "barrier counters");
+    return LM_OK;
+}
+
+int wait_status(lm_ctx* ctx) {
     if (ctx->h_res_err && *(volatile unsigned long long*)ctx->h_res_err)
-        return set_err(ctx, LM_ERR_TIMEOUT, "lattice-resident step: a halo exchange between two CTAs gave up");
+        return set_err(ctx, LM_ERR_TIMEOUT, "a bounded wait between thread blocks of a step gave up");
     return LM_OK;
 }
 
@@ -1062,20 +1072,10 @@ bool resident_single_plan(const lm_ctx* ctx, const Geom& g, int K, int64_t m, in
 }
 
 int resident_single(lm_ctx* ctx, int K, bool xreal, int cl, int mode, const ResidentInst& d, const ResidentOrders& o) {
-    if (!ctx->d_res_err) {
-        CUDA_TRY(ctx, cudaMalloc((void**)&ctx->d_res_err, sizeof(unsigned long long)), "resident status word");
-        CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_res_err, 0, sizeof(unsigned long long), ctx->stream), "resident status word");
-        CUDA_TRY(ctx, cudaHostAlloc((void**)&ctx->h_res_err, sizeof(unsigned long long), cudaHostAllocDefault),
-                 "resident status word");
-        *ctx->h_res_err = 0;
-    }
-    const int rc = resident_status(ctx);
+    int rc = ensure_wait_words(ctx);
+    if (rc == LM_OK) rc = wait_status(ctx);
     if (rc != LM_OK) return rc;
     CUDA_TRY(ctx, launch_resident_single(ctx, K, xreal, cl, mode, d, o, ctx->d_res_err), "lattice-resident step");
-    if (cl == 2)  // the word is read by a later call: no wait here
-        CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_res_err, ctx->d_res_err, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                                      ctx->stream),
-                 "resident status word");
     return LM_OK;
 }
 

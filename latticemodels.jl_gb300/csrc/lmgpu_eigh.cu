@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "lmgpu_internal.cuh"
+#include "lmgpu_gridsync.cuh"
 #include "lmgpu_order.cuh"
 
 namespace {
@@ -310,31 +311,6 @@ __global__ void __launch_bounds__(256) her2_tiles_kernel(double2* __restrict__ A
 // ------------------------------------------------------------------------------------------
 constexpr int kTriThreads = 160;      // 4 warps on the pass, 1 on the scalars
 constexpr int kTriMaxCols = 8;        // columns per CTA
-constexpr int kTriPolls = 1 << 21;    // bound of a barrier wait
-
-// Bounded grid barrier over a monotonic counter; false (and *err set) when a wait gave up.
-__device__ __forceinline__ bool grid_barrier(unsigned* ctr, unsigned target, int* err) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int good = 1;
-        unsigned seen;
-        asm volatile("fence.acq_rel.gpu;" ::: "memory");
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
-        int it = 0;
-        do {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(ctr) : "memory");
-            if (++it > kTriPolls) {
-                good = 0;
-                atomicExch(err, 1);
-                break;
-            }
-        } while ((int)(seen - target) < 0);
-        ok = good;
-    }
-    __syncthreads();
-    return ok != 0;
-}
 
 // Sum of NV doubles per lane over the warp; lane k (k < NV, a power of two <= 32) returns the
 // total of value k.  Halving the values with every exchange takes NV + log2(32 / NV) adds per warp.
@@ -418,7 +394,10 @@ __global__ void __launch_bounds__(kTriThreads, 1) tridiag_resident_kernel(TriArg
             __stcg(a.npart + b, nn);
         }
         bar += G;
-        if (!grid_barrier(a.ctr, bar, a.err)) return;
+        if (!grid_barrier(a.ctr, bar)) {
+            if (t == 0) *(volatile int*)a.err = 1;
+            return;
+        }
         if (warp == 4) {
             // the reflector's scalars (the zlarfg convention, as house_kernel)
             double s = 0.0;
@@ -506,7 +485,10 @@ __global__ void __launch_bounds__(kTriThreads, 1) tridiag_resident_kernel(TriArg
             if (t == 0) __stcg(a.dpart + b, dp);
         }
         bar += G;
-        if (!grid_barrier(a.ctr, bar, a.err)) return;
+        if (!grid_barrier(a.ctr, bar)) {
+            if (t == 0) *(volatile int*)a.err = 1;
+            return;
+        }
         if (t == 0) xn[j + 1] = sc_den;
         if (warp == 4) {
             double sx = 0.0, sy = 0.0;

@@ -14,9 +14,12 @@
 #include <vector>
 
 #include "lmgpu_internal.cuh"
+#include "lmgpu_gridsync.cuh"
 #include "lmgpu_order.cuh"
 
 namespace lmgpu {
+
+constexpr int kEllCoopMaxK = 40;  // orders of the cooperative step
 
 // 2H/a off the diagonal and 2(H_ii - b)/a on it, in FP64 and FP32.
 __global__ void ell_normalise_kernel(int64_t n, int w, const double2* __restrict__ vals,
@@ -135,6 +138,122 @@ __global__ void __launch_bounds__(256) cheb_order_ell_rows_kernel(
     }
 }
 
+// All orders of a step in one cooperative launch, for blocks of few elements: a thread owns one (site,
+// ket), keeps its row, T_{k-1}, T_{k-2} and the accumulator in registers, and publishes T_k through the
+// block's two buffers (S: T_0 and even orders, A: odd ones); a grid barrier separates the orders.  The
+// operation order per element is cheb_order_ell_rows_kernel's and cheb_epilogue's.
+//
+// What bounds it: the FP64 pipe (16 DFMAs per site of the honeycomb and order, 3.1 us for 1e5 sites) and
+// a barrier with the gather's latency behind it (about 2 us) per order; a launch per order takes 6.6 us on
+// the device and 2.5 us of the host.  One ket of 100,352 honeycomb sites, K = 11: 58 against 75 us.
+struct EllCoop {
+    int64_t n, total, ld;
+    int w, K;
+    const int* cols;
+    const void* v2;
+    const void* d2;
+    void* S;
+    void* A;
+    double s[kEllCoopMaxK + 1];  // c_k = s[k], or -i s[k] for odd k
+    double ph_re, ph_im;
+    ChebLo lo;
+    unsigned* ctr;
+    unsigned long long* err;
+};
+
+__device__ __forceinline__ double2 load_l2(const double2* p) { return __ldcg(p); }
+__device__ __forceinline__ float2 load_l2(const float2* p) { return __ldcg(p); }
+
+template <typename R, int WMAX>
+__global__ void __launch_bounds__(1024, 1) cheb_ell_coop_kernel(const __grid_constant__ EllCoop a) {
+    typedef typename CT<R>::V V;
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool on = e < a.total;
+    const int64_t ket = on ? e / a.n : 0, site = on ? e - ket * a.n : 0, base = ket * a.ld;
+    V* S = (V*)a.S;
+    V* A = (V*)a.A;
+    int c[WMAX];
+    V hv[WMAX];
+#pragma unroll
+    for (int k = 0; k < WMAX; ++k) {
+        const int64_t i = (int64_t)k * a.n + site;
+        c[k] = on && k < a.w ? __ldg(a.cols + i) : (int)site;
+        hv[k] = on && k < a.w ? __ldg((const V*)a.v2 + i) : CT<R>::make(0, 0);
+    }
+    const R d = on ? __ldg((const R*)a.d2 + site) : R(0);
+    V t1 = on ? load_l2(S + base + site) : CT<R>::make(0, 0);  // T_{k-1}
+    V t2 = t1, y = t1;                                          // T_{k-2}, the sum
+    unsigned bar = 0;
+    for (int k = 1; k <= a.K; ++k) {
+        const V* src = (k & 1) ? S : A;
+        V* dst = (k & 1) ? A : S;
+        if (on) {
+            V v[WMAX];
+#pragma unroll
+            for (int q = 0; q < WMAX; ++q)
+                if (q < a.w) v[q] = load_l2(src + base + c[q]);
+            V acc = k == 1 ? CT<R>::make(0, 0) : CT<R>::make(-t2.x, -t2.y);
+#pragma unroll
+            for (int q = 0; q < WMAX; ++q)
+                if (q < a.w) {
+                    const V h = hv[q];
+                    acc.x = fma(h.x, v[q].x, acc.x); acc.x = fma(-h.y, v[q].y, acc.x);
+                    acc.y = fma(h.x, v[q].y, acc.y); acc.y = fma(h.y, v[q].x, acc.y);
+                }
+            acc.x = fma(d, t1.x, acc.x);
+            acc.y = fma(d, t1.y, acc.y);
+            const R cs = (R)a.s[k], c0 = (R)a.s[0];
+            if (k == 1) {
+                acc = CT<R>::make(acc.x * R(0.5), acc.y * R(0.5));
+                if (sizeof(R) == sizeof(float)) {
+                    const ChebLo& lo = a.lo;
+                    R lx = fma(R(lo.g0_re), t1.x, fma(R(-lo.g0_im), t1.y, fma(R(lo.g1_re), acc.x, R(-lo.g1_im) * acc.y)));
+                    R ly = fma(R(lo.g0_re), t1.y, fma(R(lo.g0_im), t1.x, fma(R(lo.g1_re), acc.y, R(lo.g1_im) * acc.x)));
+                    y.x = fma(c0, t1.x, fma(cs, acc.y, lx));
+                    y.y = fma(c0, t1.y, fma(-cs, acc.x, ly));
+                } else {
+                    y.x = fma(cs, acc.y, c0 * t1.x);
+                    y.y = fma(-cs, acc.x, c0 * t1.y);
+                }
+            } else if (k & 1) {
+                y.x = fma(cs, acc.y, y.x);
+                y.y = fma(-cs, acc.x, y.y);
+            } else {
+                y.x = fma(cs, acc.x, y.x);
+                y.y = fma(cs, acc.y, y.y);
+            }
+            if (k == a.K) {
+                const R pr = (R)a.ph_re, pi = (R)a.ph_im;
+                dst[base + site] = CT<R>::make(fma(pr, y.x, -pi * y.y), fma(pr, y.y, pi * y.x));
+            } else {
+                __stcg(dst + base + site, acc);
+            }
+            t2 = t1;
+            t1 = acc;
+        }
+        if (k < a.K) {
+            bar += gridDim.x;
+            if (!grid_barrier(a.ctr, bar)) {
+                if (threadIdx.x == 0) *(volatile unsigned long long*)a.err = 1ull;
+                return;
+            }
+        }
+    }
+    grid_leave(a.ctr);
+}
+
+template <typename R, int WMAX>
+static cudaError_t launch_ell_coop_t(lm_ctx* ctx, EllCoop a) {
+    // equal shares of the elements per SM
+    const int64_t per = (a.total + ctx->sm_count - 1) / ctx->sm_count;
+    const int threads = (int)((per + 31) / 32 * 32);
+    const int grid = (int)((a.total + threads - 1) / threads);
+    void* args[] = {&a};
+    ctx->launches++;
+    return cudaLaunchCooperativeKernel((const void*)cheb_ell_coop_kernel<R, WMAX>, dim3(grid), dim3(threads), args, 0,
+                                       ctx->stream);
+}
+
 template <typename R, int MODE, bool SF, bool CJ>
 static cudaError_t launch_ell_t(lm_ctx* ctx, const lm_ell* h, const void* v2, const void* d2, const void* tp, void* tq,
                                 void* y, int64_t ld, int64_t m, double c0, ChebCoef ck, double pr, double pi,
@@ -225,6 +344,47 @@ static int ell_apply(lm_solver* s, int precision, int site_fast, int conj, void*
     return LM_OK;
 }
 
+// One cooperative launch for ket blocks of at most one element per thread of a full grid (1024 threads per
+// SM) and at most 8 entries per row; *done = 0 where it does not apply.  Beyond that the orders are
+// bound by the arithmetic or by HBM and a launch each costs little.
+static int ell_coop_step(lm_solver* s, lm_state* st, int* done) {
+    lm_ctx* ctx = s->ctx;
+    const lm_ell* h = s->ell;
+    *done = 0;
+    const int64_t total = st->n * st->m;
+    if (!ctx->fused || st->kind != LM_KETS || h->w > 8 || s->K < 2 || s->K > kEllCoopMaxK ||
+        total > 1024ll * ctx->sm_count)
+        return LM_OK;
+    int rc = ensure_wait_words(ctx);
+    if (rc == LM_OK) rc = wait_status(ctx);
+    if (rc != LM_OK) return rc;
+    const bool f64 = st->precision == LM_C64;
+    EllCoop a{};
+    a.n = st->n;
+    a.total = total;
+    a.ld = st->ld;
+    a.w = h->w;
+    a.K = s->K;
+    a.cols = h->d_cols;
+    a.v2 = f64 ? (const void*)s->d_ev2 : (const void*)s->d_ev2f;
+    a.d2 = f64 ? (const void*)s->d_ed2 : (const void*)s->d_ed2f;
+    a.S = st->d_data;
+    a.A = st->d_a;
+    for (int k = 0; k <= s->K; ++k) a.s[k] = s->coef[(size_t)k].s;
+    a.ph_re = s->phase_re;
+    a.ph_im = s->phase_im;
+    a.lo = cheb_lo(s->phase_re, s->phase_im, s->coef[0].s, s->coef[1].s, false);
+    a.ctr = ctx->d_grid;
+    a.err = ctx->d_res_err;
+    cudaError_t e;
+    if (f64) e = h->w <= 4 ? launch_ell_coop_t<double, 4>(ctx, a) : launch_ell_coop_t<double, 8>(ctx, a);
+    else e = h->w <= 4 ? launch_ell_coop_t<float, 4>(ctx, a) : launch_ell_coop_t<float, 8>(ctx, a);
+    CUDA_TRY(ctx, e, "cooperative ell step");
+    if (s->K & 1) std::swap(st->d_data, st->d_a);
+    *done = 1;
+    return LM_OK;
+}
+
 int ell_solver_step(lm_solver* s, lm_state* st) {
     lm_ctx* ctx = s->ctx;
     CHECK_ARG(ctx, st->n == s->ell->n, "lm_solver_step: state size does not match the Hamiltonian");
@@ -232,14 +392,6 @@ int ell_solver_step(lm_solver* s, lm_state* st) {
     {
         int rc0 = ensure_scratch(st);
         if (rc0 != LM_OK) return rc0;
-    }
-    if (!st->d_y) {
-        const size_t bytes = st->elem * (size_t)st->ld * (size_t)st->m;
-        if (dev_alloc(ctx, &st->d_y, bytes) != cudaSuccess) {
-            st->d_y = nullptr;
-            cudaGetLastError();
-            return set_err(ctx, LM_ERR_OOM, "lm_solver_step: accumulator allocation");
-        }
     }
     int where = 0;
     const lm_ell* h = s->ell;
@@ -278,7 +430,18 @@ int ell_solver_step(lm_solver* s, lm_state* st) {
         return set_err(ctx, LM_ERR_NOTSUP,
                        "lm_solver_step: a compensated state on a general Hamiltonian needs the honeycomb brick layout "
                        "and the x-streaming form");
-    int rc = ell_apply(s, st->precision, 1, 0, st->d_data, st->d_a, st->d_y, st->ld, st->m, &where);
+    int done = 0;
+    int rc = ell_coop_step(s, st, &done);
+    if (rc != LM_OK || done) return rc;
+    if (!st->d_y) {
+        const size_t bytes = st->elem * (size_t)st->ld * (size_t)st->m;
+        if (dev_alloc(ctx, &st->d_y, bytes) != cudaSuccess) {
+            st->d_y = nullptr;
+            cudaGetLastError();
+            return set_err(ctx, LM_ERR_OOM, "lm_solver_step: accumulator allocation");
+        }
+    }
+    rc = ell_apply(s, st->precision, 1, 0, st->d_data, st->d_a, st->d_y, st->ld, st->m, &where);
     if (rc != LM_OK) return rc;
     if (where == 1) std::swap(st->d_data, st->d_a);
     if (st->kind == LM_DENSITY) {  // P <- X U^dagger: conj(U) on every row of X

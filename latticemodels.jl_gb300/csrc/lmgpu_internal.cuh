@@ -105,8 +105,9 @@ struct lm_ctx {
     int kpm_df = 1;                     // LM_OPT_KPM: double-float recurrence in lm_kpm_moments
     cudaMemPool_t pool = nullptr;       // device memory of states and temporaries (dev_alloc); null: cudaMalloc
     unsigned resident_attr = 0;         // shared-memory attributes of the lattice-resident kernels set
-    unsigned long long* d_res_err = nullptr;  // their timeout word (single-lattice launches), and
-    unsigned long long* h_res_err = nullptr;  // its pinned copy, refreshed after every cluster launch
+    unsigned long long* h_res_err = nullptr;  // timeout word of the kernels that wait (mapped host memory)
+    unsigned long long* d_res_err = nullptr;  // and its device address
+    unsigned* d_grid = nullptr;         // barrier counters of cooperative launches (zero between launches)
     int resident = 1;                   // LM_OPT_RESIDENT: lattice-resident form in the batch's fused pass
     std::vector<double> h_norms;        // pageable staging of lm_state_renormalize's targets
     std::vector<cudaEvent_t> ev_pool;   // pairs (start, stop) of timed Chebyshev sweeps
@@ -360,6 +361,10 @@ bool ham_uniform_columns(const lm_ham* h);
 // raised (by at most one FP32 ulp, relative 6e-8) until 2 t_exact / a is an FP32 number, so a
 // hop of magnitude t_exact has no rounding error in the FP32 stencil tables.
 void plan_propagator(lm_solver* s, double emin, double emax, double dt, double t_exact = 0.0);
+// The context's timeout word and barrier counters, created on first use; the word's state as of the last
+// finished launch (LM_OK or LM_ERR_TIMEOUT).
+int ensure_wait_words(lm_ctx* ctx);
+int wait_status(lm_ctx* ctx);
 // lm_solver_step / destroy for a solver updated with an lm_ell Hamiltonian (lmgpu_ell.cu).
 int ell_solver_step(lm_solver* s, lm_state* st);
 void ell_free_tables(lm_solver* s);

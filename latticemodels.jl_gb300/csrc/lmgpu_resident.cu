@@ -103,7 +103,7 @@ __device__ __forceinline__ void res_mbar_wait(unsigned a, unsigned parity, unsig
             : "=r"(done) : "r"(a), "r"(parity) : "memory");
         if (done) return;
     }
-    atomicOr(err, 1ull);
+    *(volatile unsigned long long*)err = 1ull;  // device memory (a batch) or mapped host memory
 }
 template <int CL>
 __device__ __forceinline__ void res_sync() {

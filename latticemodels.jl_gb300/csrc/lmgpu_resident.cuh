@@ -58,12 +58,10 @@ cudaError_t launch_resident_table(lm_ctx* ctx, int K, bool xreal, int cl, const 
 cudaError_t launch_resident_single(lm_ctx* ctx, int K, bool xreal, int cl, int mode, const ResidentInst& inst,
                                    const ResidentOrders& orders, unsigned long long* d_err);
 // The same from a solver or adjoint step (lmgpu_api.cu): the instance of one ket block (every field but
-// tables and coefficients), the launch with the context's timeout word, and that word's state as of
-// the last finished launch (LM_OK or LM_ERR_TIMEOUT).
+// tables and coefficients) and the launch with the context's timeout word.
 bool resident_single_plan(const lm_ctx* ctx, const Geom& g, int K, int64_t m, int64_t ld, const void* x, const void* out,
                           ResidentInst& d, int* cl);
 int resident_single(lm_ctx* ctx, int K, bool xreal, int cl, int mode, const ResidentInst& d, const ResidentOrders& o);
-int resident_status(lm_ctx* ctx);
 // Sets the kernel's shared-memory attribute (outside stream capture).
 cudaError_t ensure_resident_attr(lm_ctx* ctx, bool xreal, int cl);
 
