@@ -123,6 +123,32 @@ cudaError_t launch_stencil_recur(lm_ctx* ctx, const Geom& g, int precision, cons
     return cudaGetLastError();
 }
 
+// The on-site and field terms of one order at a site from its sums v, before the factor f; the field
+// term is f times the real part.
+__device__ __forceinline__ double grad_site_V(const double (&v)[10], double ph_re, double ph_im) {
+    return ph_re * v[0] - ph_im * v[1];
+}
+
+__device__ __forceinline__ double grad_site_A(const Geom& g, const Nbr& nb, int64_t s, const double (&v)[10],
+                                              const double2* dhop, double ph_re, double ph_im, double f) {
+    const double2 zz = make_double2(0.0, 0.0);
+    const double2 D[4] = {nb.hxp ? dhop[s] : zz, nb.hyp ? dhop[g.N + s] : zz, nb.hxm ? dhop[nb.xm] : zz,
+                          nb.hym ? dhop[g.N + nb.ym] : zz};
+    double zr = 0.0, zi = 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const double sr = v[2 + 2 * q], si = v[3 + 2 * q];
+        if (q < 2) {  // D S
+            zr += D[q].x * sr - D[q].y * si;
+            zi += D[q].x * si + D[q].y * sr;
+        } else {      // conj(D) S
+            zr += D[q].x * sr + D[q].y * si;
+            zi += D[q].x * si - D[q].y * sr;
+        }
+    }
+    return f * (ph_re * zr - ph_im * zi);
+}
+
 // A block's gradient contributions of one order from its sums v: gV_part of its 32 sites and gA_part of
 // the block, one writer per entry and launch (one warp calls this).
 __device__ __forceinline__ void grad_block_out(const Geom& g, const Nbr& nb, int64_t s, int lane, const double (&v)[10],
@@ -130,25 +156,9 @@ __device__ __forceinline__ void grad_block_out(const Geom& g, const Nbr& nb, int
                                                double* gV_part, double* gA_part) {
     double ga = 0.0;
     if (s < g.N) {
-        gV_part[(int64_t)blockIdx.y * g.N + s] += f * (ph_re * v[0] - ph_im * v[1]);
-        if (dhop) {
-            const double2 zz = make_double2(0.0, 0.0);
-            const double2 D[4] = {nb.hxp ? dhop[s] : zz, nb.hyp ? dhop[g.N + s] : zz, nb.hxm ? dhop[nb.xm] : zz,
-                                  nb.hym ? dhop[g.N + nb.ym] : zz};
-            double zr = 0.0, zi = 0.0;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const double sr = v[2 + 2 * q], si = v[3 + 2 * q];
-                if (q < 2) {  // D S
-                    zr += D[q].x * sr - D[q].y * si;
-                    zi += D[q].x * si + D[q].y * sr;
-                } else {      // conj(D) S
-                    zr += D[q].x * sr + D[q].y * si;
-                    zi += D[q].x * si - D[q].y * sr;
-                }
-            }
-            ga = f * (ph_re * zr - ph_im * zi);
-        }
+        double* gv = gV_part + (int64_t)blockIdx.y * g.N + s;
+        *gv = fma(f, grad_site_V(v, ph_re, ph_im), *gv);
+        if (dhop) ga = grad_site_A(g, nb, s, v, dhop, ph_re, ph_im, f);
     }
     if (gA_part) {
         for (int o = 16; o > 0; o >>= 1) ga += __shfl_down_sync(0xffffffffu, ga, o);
@@ -251,11 +261,14 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 3 : 2) adj_b
 // wrote to HBM): order by order the sums of adj_beta_grad_kernel<float>, term for term, so that both forms
 // give the same bits.
 //
-// What bounds it: FP32 issue, 20 double-float products (10 operations each) per site, ket and order, and
-// after every order the FP64 pipe (a warp-wide DADD holds a partition for 64 clocks), so each of the
-// 8 warps adds one sum's partials and the pairs become doubles by integer operations.  On 64 x 64 sites
-// with 1024 kets and K = 6 a step took 5 recurrence launches of 41 us and 6 fused passes of 102 us; now
-// T_k and beta_k take 62 + 81 us on chip (each writes 200 MB) and the sums 250 us (134 us of products).
+// What bounds it: the FP32 pipe, 20 double-float products (10 operations each) per site, ket and order, as
+// packed pairs (re, im): 140 us at that pipe's rate on 64 x 64 sites with 1024 kets and K = 6, and at a
+// block's end the FP64 pipe's latency (a warp-wide DADD holds a partition for 64 clocks), so each of the
+// 8 warps adds one sum's partials and the pairs become doubles by integer operations.  An order is a block of
+// its own (6144 blocks; all orders in turn made 1024, whose last wave was a quarter full) and
+// adj_fold_kernel adds them.  The step took 5 recurrence launches of 41 us and 6 fused passes of 102 us; now
+// T_k and beta_k take 61 + 66 us on chip (each writes 200 MB) and the sums 214 + 5 us (293 us with the
+// orders in turn and scalar products; 227 to 253 us with the loads by cp.async; 272 us with 2 blocks per SM).
 struct GradOrders {
     const float2* T[kResMaxK];      // T_0 .. T_{K-1}
     const float2* b[kResMaxK + 1];  // beta_1 .. beta_K
@@ -270,88 +283,108 @@ __device__ __forceinline__ double widen(float x) {
     return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))), (int)(u << 29));
 }
 
-__global__ void __launch_bounds__(256, 3) adj_sums_kernel(Geom g, const __grid_constant__ GradOrders ord, int K,
+__global__ void __launch_bounds__(256, 3) adj_sums_kernel(Geom g, const __grid_constant__ GradOrders ord,
                                                           const double2* __restrict__ dhop, int64_t ld, int64_t M,
                                                           int64_t mchunk, double ph_re, double ph_im, double inv_a,
-                                                          double* __restrict__ gV_part, double* __restrict__ gA_part) {
+                                                          double* __restrict__ sums_V, double* __restrict__ sums_A) {
     __shared__ double red[8][10][32];
     __shared__ double tot[10][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int k = (int)blockIdx.z + 1;
     const int64_t s = (int64_t)blockIdx.x * 32 + lane;
     const int64_t m0 = (int64_t)blockIdx.y * mchunk, m1 = min(M, m0 + mchunk);
-    const int64_t m_first = m0 + warp;
     const bool on = s < g.N;
     Nbr nb;
-    int xp = 0, yp = 0, xm = 0, ym = 0;
+    Acc2 a[5];  // (re, im) of conj(b)T_s; S1x; S1y; S2x; S2y
     if (on) {
         nb = neighbours(g, s);
-        xp = (int)(nb.xp - s);
-        yp = (int)(nb.yp - s);
-        xm = (int)(nb.xm - s);
-        ym = (int)(nb.ym - s);
-    }
-    // beta, T and T's neighbours of the next ket (of the next order) are loaded while this one is summed
-    auto load = [&](float2 (&d)[6], int64_t m, int k) {
-        if (!on || m >= m1 || k < 1) return;
-        const float2* T = ord.T[k - 1] + m * ld + s;
-        d[0] = ord.b[k][m * ld + s];
-        d[1] = T[0];
-        if (dhop) {
-            d[2] = T[xp];
-            d[3] = T[yp];
-            d[4] = T[xm];
-            d[5] = T[ym];
-        }
-    };
-    float2 v[6], w[6];
-    load(v, m_first, K);
-    for (int k = K; k >= 1; --k) {
-        Acc<float> a[10];  // conj(b)T_s (re, im); S1x; S1y; S2x; S2y
+        const int xp = (int)(nb.xp - s), yp = (int)(nb.yp - s), xm = (int)(nb.xm - s), ym = (int)(nb.ym - s);
+        // beta, T and T's neighbours of the next ket are loaded while this one is summed
+        int n = m0 + warp < m1 ? (int)((m1 - m0 - warp + 7) / 8) : 0;
+        const float2* T = ord.T[k - 1] + (m0 + warp) * ld + s;
+        const float2* bk = ord.b[k] + (m0 + warp) * ld + s;
+        auto load = [&](float2 (&d)[6]) {
+            d[0] = __ldg(bk);
+            d[1] = __ldg(T);
+            if (dhop) {
+                d[2] = __ldg(T + xp);
+                d[3] = __ldg(T + yp);
+                d[4] = __ldg(T + xm);
+                d[5] = __ldg(T + ym);
+            }
+            T += 8 * ld;
+            bk += 8 * ld;
+        };
         auto sum = [&](const float2 (&d)[6]) {
             const float2 b = d[0];
+            const float2 b1 = make_float2(b.x, b.x), n1 = make_float2(-b.x, -b.x);
+            const float2 b2 = make_float2(b.y, -b.y), n2 = make_float2(-b.y, b.y);
 #pragma unroll
             for (int q = 0; q < 5; ++q) {  // conj(b) T at the site and its neighbours
                 if (q > 0 && !dhop) break;
-                a[2 * q].add_prod(b.x, d[1 + q].x);
-                a[2 * q].add_prod(b.y, d[1 + q].y);
-                a[2 * q + 1].add_prod(b.x, d[1 + q].y);
-                a[2 * q + 1].add_prod(-b.y, d[1 + q].x);
+                const float2 t = d[1 + q];
+                a[q].add_prod(b1, n1, t);
+                a[q].add_prod(b2, n2, make_float2(t.y, t.x));
             }
         };
-        if (on) {
-            int64_t m = m_first;
-            for (; m + 8 < m1; m += 16) {
-                load(w, m + 8, k);
-                sum(v);
-                if (m + 16 < m1) load(v, m + 16, k);
-                else load(v, m_first, k - 1);
-                sum(w);
-            }
-            if (m < m1) {
-                sum(v);
-                load(v, m_first, k - 1);
-            }
+        float2 v[6], w[6];
+        if (n > 0) load(v);
+        while (n > 0) {
+            if (n > 1) load(w);
+            sum(v);
+            if (--n == 0) break;
+            if (n > 1) load(v);
+            sum(w);
+            --n;
         }
+    }
 #pragma unroll
-        for (int q = 0; q < 10; ++q) red[warp][q][lane] = widen(a[q].hi) + widen(a[q].lo);
-        __syncthreads();
+    for (int q = 0; q < 5; ++q) {
+        red[warp][2 * q][lane] = widen(a[q].hi.x) + widen(a[q].lo.x);
+        red[warp][2 * q + 1][lane] = widen(a[q].hi.y) + widen(a[q].lo.y);
+    }
+    __syncthreads();
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {  // sum q of the block, warps in order
-            const int q = warp + 8 * r;
-            if (q < 10 && (q < 2 || dhop)) {
-                double t = 0.0;
+    for (int r = 0; r < 2; ++r) {  // sum q of the block, warps in order
+        const int q = warp + 8 * r;
+        if (q < 10 && (q < 2 || dhop)) {
+            double t = red[0][q][lane];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) t += red[u][q][lane];
-                tot[q][lane] = t;
-            }
+            for (int u = 1; u < 8; ++u) t += red[u][q][lane];
+            tot[q][lane] = t;
         }
-        __syncthreads();
-        if (warp == 0) {  // the other warps go on; tot is rewritten after the next order's first barrier
-            double t[10];
+    }
+    __syncthreads();
+    if (warp != 0) return;
+    double t[10], ga = 0.0;
 #pragma unroll
-            for (int q = 0; q < 10; ++q) t[q] = q < 2 || dhop ? tot[q][lane] : 0.0;
-            grad_block_out(g, nb, s, lane, t, dhop, ph_re, ph_im, k == 1 ? inv_a : 2.0 * inv_a, gV_part, gA_part);
-        }
+    for (int q = 0; q < 10; ++q) t[q] = q < 2 || dhop ? tot[q][lane] : 0.0;
+    const int64_t row = (int64_t)(k - 1) * gridDim.y + blockIdx.y;
+    if (on) {
+        sums_V[row * g.N + s] = grad_site_V(t, ph_re, ph_im);
+        if (dhop) ga = grad_site_A(g, nb, s, t, dhop, ph_re, ph_im, k == 1 ? inv_a : 2.0 * inv_a);
+    }
+    if (dhop) {
+        for (int o = 16; o > 0; o >>= 1) ga += __shfl_down_sync(0xffffffffu, ga, o);
+        if (lane == 0) sums_A[row * gridDim.x + blockIdx.x] = ga;
+    }
+}
+
+// Adds the orders' terms to the gradients' parts, K first, as the per-order kernels do: nV entries of gV_part
+// and nA of gA_part (null without a field derivative).
+__global__ void adj_fold_kernel(int K, int64_t nV, int64_t nA, double inv_a, const double* __restrict__ sums_V,
+                                const double* __restrict__ sums_A, double* __restrict__ gV_part,
+                                double* __restrict__ gA_part) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nV) {
+        double t = gV_part[i];
+        for (int k = K; k >= 1; --k) t = fma(k == 1 ? inv_a : 2.0 * inv_a, sums_V[(int64_t)(k - 1) * nV + i], t);
+        gV_part[i] = t;
+    }
+    if (gA_part && i < nA) {
+        double t = gA_part[i];
+        for (int k = K; k >= 1; --k) t += sums_A[(int64_t)(k - 1) * nA + i];
+        gA_part[i] = t;
     }
 }
 
@@ -434,6 +467,7 @@ struct lm_adjoint {
     double* d_loss = nullptr;   // one partial per 32-site block (nblk)
     double* d_target = nullptr;
     double2* d_dhop = nullptr;
+    double* d_sums = nullptr;   // lattice-resident form: the orders' terms of gV and gA before they are added
 };
 
 static void adj_free_stack(lm_adjoint* a) {
@@ -443,6 +477,9 @@ static void adj_free_stack(lm_adjoint* a) {
     for (auto& b : a->B)
         dev_free(a->ctx, b);
     a->B.clear();
+    dev_free(a->ctx, a->d_sums);
+    a->d_sums = nullptr;
+    a->K = 0;
 }
 
 static int adj_alloc(lm_ctx* ctx, void** p, size_t bytes) {
@@ -467,6 +504,10 @@ static int adj_ensure_stack(lm_adjoint* a, int K, bool all_beta) {
     a->B.assign(nb, nullptr);
     for (size_t k = all_beta ? 1 : 0; k < nb; ++k) {
         int rc = adj_alloc(a->ctx, &a->B[k], bytes);
+        if (rc != LM_OK) return rc;
+    }
+    if (all_beta) {
+        int rc = adj_alloc(a->ctx, (void**)&a->d_sums, sizeof(double) * (size_t)K * (size_t)a->nchunk * (size_t)(a->n + a->nblk));
         if (rc != LM_OK) return rc;
     }
     a->K = K;
@@ -642,10 +683,17 @@ int lm_adjoint_step(lm_adjoint* a, lm_solver* s, lm_ham* h, int component, int s
             go.T[k - 1] = (const float2*)a->T[(size_t)k - 1];
             go.b[k] = (const float2*)a->B[(size_t)k];
         }
-        adj_sums_kernel<<<ggrid, 256, 0, ctx->stream>>>(g, go, K, dhop, ld, M, a->mchunk, s->phase_re, s->phase_im,
-                                                        1.0 / s->a, a->d_gV, gA);
+        const int64_t nV = a->n * a->nchunk, nA = a->nblk * a->nchunk;
+        double* sums_V = a->d_sums;
+        double* sums_A = a->d_sums + nV * K;
+        adj_sums_kernel<<<dim3(ggrid.x, ggrid.y, (unsigned)K), 256, 0, ctx->stream>>>(
+            g, go, dhop, ld, M, a->mchunk, s->phase_re, s->phase_im, 1.0 / s->a, sums_V, sums_A);
         ctx->launches++;
         CUDA_TRY(ctx, cudaGetLastError(), "adjoint gradient sums");
+        adj_fold_kernel<<<(unsigned)((nV + 255) / 256), 256, 0, ctx->stream>>>(K, nV, nA, 1.0 / s->a, sums_V, sums_A,
+                                                                               a->d_gV, gA);
+        ctx->launches++;
+        CUDA_TRY(ctx, cudaGetLastError(), "adjoint gradient fold");
         return LM_OK;
     }
     for (int k = K; k >= 1; --k) {

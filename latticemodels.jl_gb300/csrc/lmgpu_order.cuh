@@ -43,6 +43,50 @@ template <> struct Acc<float> {
     __device__ __forceinline__ double get() const { return (double)hi + (double)lo; }
 };
 
+// d = a * b + c on both halves of a float pair in one instruction (two round-to-nearest FMAs:
+// the same results as two fmaf calls).
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
+        "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+        "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+
+// Packed FP32 pairs: one instruction each for both halves, the same rounding as the scalar
+// operation on each half.
+#define LM_F32X2_BINOP(NAME, OP)                                                                     \
+    __device__ __forceinline__ float2 NAME(float2 a, float2 b) {                                     \
+        float2 d;                                                                                    \
+        asm("{\n\t.reg .b64 ra, rb, rd;\n\t"                                                          \
+            "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t" OP                                   \
+            " rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"                                               \
+            : "=f"(d.x), "=f"(d.y)                                                                   \
+            : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));                                               \
+        return d;                                                                                    \
+    }
+LM_F32X2_BINOP(fadd2, "add.rn.f32x2")
+LM_F32X2_BINOP(fsub2, "sub.rn.f32x2")
+LM_F32X2_BINOP(fmul2, "mul.rn.f32x2")
+#undef LM_F32X2_BINOP
+
+// Two Acc<float> side by side, on packed instructions: half the issue slots, and the bits of two separate
+// accumulators (signs are moved between exact operations only).  na = -a.
+struct Acc2 {
+    float2 hi = {0.f, 0.f}, lo = {0.f, 0.f};
+    __device__ __forceinline__ void add_prod(float2 a, float2 na, float2 b) {
+        const float2 np = fmul2(na, b);       // -p
+        const float2 pe = ffma2(a, b, np);    // a*b = p + pe exactly
+        const float2 s = fsub2(hi, np);       // TwoSum(hi, p) = s + e exactly
+        const float2 bp = fsub2(s, hi);
+        const float2 e = fsub2(fsub2(hi, fsub2(s, bp)), fadd2(np, bp));
+        hi = s;
+        lo = fadd2(lo, fadd2(e, pe));
+    }
+};
+
 // ------------------------------------------------------------------------------------------
 // Neighbour routing on the square lattice (src/core/boundaries.jl:251-289 for the periodic
 // case: a destination one step outside is wrapped by the axis translation).

@@ -40,6 +40,7 @@
 #include <cstdint>
 
 #include "lmgpu_internal.cuh"
+#include "lmgpu_order.cuh"
 
 namespace lmgpu {
 
@@ -121,36 +122,8 @@ __device__ __forceinline__ void cp_async8s(float2* dst_smem, const void* src, bo
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src), "r"(n));
 }
 __device__ __forceinline__ void cp_async_commit_s() { asm volatile("cp.async.commit_group;\n" ::); }
-// d = a * b + c on both halves of a float pair in one instruction (two round-to-nearest FMAs:
-// the same results as two fmaf calls).
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
-        "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
-        "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return d;
-}
 template <int N>
 __device__ __forceinline__ void cp_async_wait_s() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
-// Packed FP32 pairs: one instruction each for both halves, the same rounding as the scalar
-// operation on each half.
-#define LM_F32X2_BINOP(NAME, OP)                                                                     \
-    __device__ __forceinline__ float2 NAME(float2 a, float2 b) {                                     \
-        float2 d;                                                                                    \
-        asm("{\n\t.reg .b64 ra, rb, rd;\n\t"                                                          \
-            "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t" OP                                   \
-            " rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"                                               \
-            : "=f"(d.x), "=f"(d.y)                                                                   \
-            : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));                                               \
-        return d;                                                                                    \
-    }
-LM_F32X2_BINOP(fadd2, "add.rn.f32x2")
-LM_F32X2_BINOP(fsub2, "sub.rn.f32x2")
-LM_F32X2_BINOP(fmul2, "mul.rn.f32x2")
-#undef LM_F32X2_BINOP
 
 // (hi + lo) = a1 x1 + a2 x2 + r + a1 l on both components of a compensated output at once:
 // a1 x1 (the dominant term for the workloads' small spectral centres: a1 + i a2 = e^{-ib dt} c_0)
