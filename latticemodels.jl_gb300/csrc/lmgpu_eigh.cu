@@ -29,7 +29,6 @@
 #include <vector>
 
 #include "lmgpu_internal.cuh"
-#include "lmgpu_gridsync.cuh"
 #include "lmgpu_order.cuh"
 
 namespace {
@@ -295,19 +294,23 @@ __global__ void __launch_bounds__(256) her2_tiles_kernel(double2* __restrict__ A
 // memory of all SMs together (n <= 8 SMs).  CTA b keeps the columns b, b + G, ... (at most 8, full
 // columns, both triangles), so a product p_c = sum_r conj(A[r, c]) v_r needs no sum over CTAs and
 // the row x_c = conj(A[j, c]) of the next reflector is spread over all of them.  Per column j:
-//   barrier 1 publishes x and the partial norms; every CTA forms the reflector's scalars (one
-//   warp, beside the others' pass), applies the pending rank-2 update to its columns and
-//   multiplies them by the new v in the same pass (12 DFMAs per element);
-//   barrier 2 publishes p and the partial dots p^H v; the update of column set r > j waits for
-//   the next pass, only row j + 1 is updated at once (it is the next x).
+//   warp 4 updates row j of the own columns (the next x) and posts x and a partial norm; the pass
+//   warps apply the pending rank-2 update to rows r > j meanwhile (8 DFMAs per element);
+//   exchange 1; the pass warps multiply the columns by x (4 DFMAs), warp 4 forms the reflector's
+//   scalars; warp 4 posts p and a partial dot p^H v; exchange 2.
 // v is never formed: v = scal xt with xt = x, xt[0] = alpha - beta, so scal folds into the
 // per-column factors.  The update uses w = p + al v, v w^H + w v^H = v (p + 2 Re(al) v)^H + p v^H.
-// What bounds it: GB300's FP64 rate of about 2 DFMAs per clock and SM.  Storing both triangles
-// costs 12 instead of 8 DFMAs per element, but 4 launches per column become two grid barriers, and
-// no warp repeats another's scalar FP64 work (a warp-wide FP64 instruction holds the pipe for 16
-// clocks: the reflector's square root and divisions in 32 warps took 20 us per column).  N = 864:
-// 13.6 ms (4.1 ms of DFMAs, the rest barriers and the serial scalar chain), the launches per column
-// 49.8 ms.
+// An exchange: every value has a word of its own per column, set to a sentinel before the launch; a CTA
+// posts its values, adds 1 to a counter without a fence, waits for the counter and loads what it
+// needs, looking again at a word that still holds the sentinel.  A barrier with a fence took 5100
+// clocks with the loads after it, this 3700; polling the words without the counter 12600 (each of the
+// 152 stores into a line that all SMs poll costs a round trip between the dies).
+// What bounds it: GB300's FP64 rate of about 2 DFMAs per clock and SM in the early columns (storing
+// both triangles costs 12 instead of 8 DFMAs per element, but no sum over CTAs), the exchanges and warp 4's
+// chain in the late ones.  A warp-wide FP64 instruction holds a partition's pipe for 64 clocks even
+// for one lane, so warp 4 has a lane per component of a complex scalar, and takes its root and
+// reciprocals by Newton's iteration.  N = 864: 11.4 ms (5 ms of DFMAs); 13.5 ms with two fenced
+// barriers and the update and product in one pass after the first, 49.8 ms with launches per column.
 // ------------------------------------------------------------------------------------------
 constexpr int kTriThreads = 160;      // 4 warps on the pass, 1 on the scalars
 constexpr int kTriMaxCols = 8;        // columns per CTA
@@ -339,13 +342,138 @@ struct TriArgs {
     double* d;
     double* e;
     double2* tau;
-    double2* xg;           // n: x of the current column
-    double2* pg;           // n: p
-    double* npart;         // G partial norms
-    double2* dpart;        // G partial dots
-    unsigned* ctr;         // barrier counter (zeroed)
+    // Exchanged values, each written once per launch over the sentinel (all bits set):
+    double2* xg;           // n x n: x of column j at j n
+    double2* pg;           // n x n: p
+    double* ng;            // G x n: partial norms
+    double* dg;            // G x n: partial dots
+    unsigned* ctr;         // columns' exchanges done, by all CTAs (zeroed)
     int* err;
 };
+
+// A value of the exchange is there when its bits are no longer the sentinel's; a NaN is stored as the
+// plain quiet NaN.  Values are single 8-byte words, so no barrier or fence orders them.
+__device__ __forceinline__ void post_word(double* p, double v) {
+    long long u = __double_as_longlong(v);
+    if (u == -1ll) u = 0x7ff8000000000000ll;
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(u) : "memory");
+}
+__device__ __forceinline__ long long peek_word(const double* p) {
+    long long u;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(u) : "l"(p) : "memory");
+    return u;
+}
+__device__ __forceinline__ void peek_pair(const double2* p, long long& x, long long& y) {
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "l"(p) : "memory");
+}
+
+constexpr int kTriPolls = 1 << 20;  // bound of a wait for posted values (about half a second)
+
+// One thread: adds this CTA to the exchange's counter and waits until all have come.  Most values are
+// there then; no fence orders them, so each is still checked.
+__device__ __forceinline__ bool meet(unsigned* ctr, unsigned target) {
+    asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
+    unsigned seen;
+    int it = 0;
+    do {
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(ctr) : "memory");
+        if (++it > kTriPolls) return false;
+    } while ((int)(seen - target) < 0);
+    return true;
+}
+// The pass warps wait here until warp 4 has seen an exchange complete: polling the values themselves meanwhile
+// slows their arrival, and polling a word of shared memory takes issue slots from warp 4 (11.4, 13.3 and
+// 13.8 ms for N = 864).
+__device__ __forceinline__ void gate_arrive(int id) {
+    __syncwarp();
+    asm volatile("barrier.arrive %0, %1;" ::"r"(id), "n"(kTriThreads) : "memory");
+}
+__device__ __forceinline__ void gate_wait(int id) {
+    __syncwarp();
+    asm volatile("barrier.sync %0, %1;" ::"r"(id), "n"(kTriThreads) : "memory");
+}
+
+// Waits for the pairs q[row[i]] with row[i] < n.  False when the wait gave up.
+template <int U>
+__device__ __forceinline__ bool wait_pairs(const double2* q, const int (&row)[U], int n, double2 (&v)[U]) {
+    long long x[U], y[U];
+#pragma unroll
+    for (int i = 0; i < U; ++i) {
+        x[i] = y[i] = 0;
+        if (row[i] < n) peek_pair(q + row[i], x[i], y[i]);
+    }
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < U; ++i) {
+        int it = 0;
+        while (x[i] == -1ll || y[i] == -1ll) {
+            if (++it > kTriPolls) {
+                ok = false;
+                break;
+            }
+            peek_pair(q + row[i], x[i], y[i]);
+        }
+        v[i] = make_double2(__longlong_as_double(x[i]), __longlong_as_double(y[i]));
+    }
+    return ok;
+}
+
+// Sum over the warp of the words q[0 .. G), G <= 256, in a fixed order.
+__device__ __forceinline__ bool wait_sum(const double* q, int G, int lane, double& sum) {
+    constexpr int U = 8;
+    long long x[U];
+#pragma unroll
+    for (int i = 0; i < U; ++i) {
+        x[i] = 0;
+        if (lane + 32 * i < G) x[i] = peek_word(q + lane + 32 * i);
+    }
+    bool ok = true;
+    double s = 0.0;
+#pragma unroll
+    for (int i = 0; i < U; ++i) {
+        int it = 0;
+        while (x[i] == -1ll) {
+            if (++it > kTriPolls) {
+                ok = false;
+                break;
+            }
+            x[i] = peek_word(q + lane + 32 * i);
+        }
+        if (32 * i < G) s = i == 0 ? __longlong_as_double(x[i]) : s + __longlong_as_double(x[i]);
+    }
+#pragma unroll
+    for (int w = 16; w >= 1; w /= 2) s += __shfl_xor_sync(0xffffffffu, s, w);
+    sum = s;
+    return ok;
+}
+
+// 1 / sqrt(t) and 1 / d by Newton's iteration from the FP32 approximations, on arguments scaled into
+// [1, 4) and [1, 2): two steps take their 22 bits beyond FP64's 53.  A quarter of the FP64 instructions of
+// sqrt and a division.  Zero, subnormal and extreme arguments go the plain way.
+__device__ __forceinline__ double newton_rsqrt(double t) {
+    const int hi = __double2hiint(t), lo = __double2loint(t);
+    const int ex = (hi >> 20) - 1023;
+    if (ex < -900 || ex > 900) return 1.0 / sqrt(t);
+    const int sc = ex & ~1, mh = hi - (sc << 20);
+    const unsigned y = __float_as_uint(rsqrtf(__uint_as_float(((unsigned)(mh - (896 << 20)) << 3) | ((unsigned)lo >> 29))));
+    const double m = __hiloint2double(mh, lo);
+    double r = __hiloint2double((int)((y >> 3) + (896u << 20)), (int)(y << 29));
+#pragma unroll
+    for (int i = 0; i < 2; ++i) r = fma(0.5 * r, fma(-(m * r), r, 1.0), r);
+    return __hiloint2double(__double2hiint(r) - ((sc / 2) << 20), __double2loint(r));
+}
+__device__ __forceinline__ double newton_recip(double d) {  // d > 0
+    const int hi = __double2hiint(d), lo = __double2loint(d);
+    const int ex = (hi >> 20) - 1023;
+    if (ex < -900 || ex > 900) return 1.0 / d;
+    const int mh = hi - (ex << 20);
+    const unsigned y = __float_as_uint(__frcp_rn(__uint_as_float(((unsigned)(mh - (896 << 20)) << 3) | ((unsigned)lo >> 29))));
+    const double m = __hiloint2double(mh, lo);
+    double r = __hiloint2double((int)((y >> 3) + (896u << 20)), (int)(y << 29));
+#pragma unroll
+    for (int i = 0; i < 2; ++i) r = fma(r, fma(-m, r, 1.0), r);
+    return __hiloint2double(__double2hiint(r) - (ex << 20), __double2loint(r));
+}
 
 template <int NC>
 __global__ void __launch_bounds__(kTriThreads, 1) tridiag_resident_kernel(TriArgs a) {
@@ -354,10 +482,7 @@ __global__ void __launch_bounds__(kTriThreads, 1) tridiag_resident_kernel(TriArg
     const int warp = t >> 5, lane = t & 31;
     double2* S = sm;                  // column k at S + k n
     double2* ps = sm + (size_t)(NC + 2) * n;
-    __shared__ double2 sc_tau, sc_scal, sc_den;
     __shared__ double2 Gk[NC], Fk[NC], acc_sh[4][NC];
-    __shared__ double sc_s;
-    __shared__ double part_sh[NC];
     for (int k = 0; k < NC; ++k) {
         const int c = b + k * G;
         if (c < n)
@@ -366,77 +491,95 @@ __global__ void __launch_bounds__(kTriThreads, 1) tridiag_resident_kernel(TriArg
     if (t < NC) Gk[t] = Fk[t] = make_double2(0.0, 0.0);
     for (int r = t; r < n; r += kTriThreads) ps[r] = sm[(size_t)NC * n + r] = sm[(size_t)(NC + 1) * n + r] = make_double2(0.0, 0.0);
     __syncthreads();
-    unsigned bar = 0;
+    constexpr int U = NC + 2;  // rows of a pass thread (n <= 152 NC takes one batch)
+    constexpr int kFold = NC > 4 ? 8 : NC > 2 ? 4 : NC > 1 ? 2 : 1;  // a power of two >= NC
+    // warp 4: lane 2 k + i holds component i of column k's complex scalars (a warp-wide FP64 instruction
+    // costs the same for one lane as for 32)
+    const int kk = (lane >> 1) & (kFold - 1), im = lane & 1;
+    const int kc = kk < NC ? kk : 0;
+    const int c = b + kk * G;
+    const bool own = warp == 4 && lane < 2 * NC && c < n;
+    auto mul_part = [&](double2 u, double w0, double w1) {  // component im of u w: w0 this lane's part, w1 the other
+        return fma(u.x, w0, im ? u.y * w1 : -u.y * w1);
+    };
+    auto other = [](double v) { return __shfl_xor_sync(0xffffffffu, v, 1); };
+    unsigned met = 0;
     for (int j = 0; j + 1 < n; ++j) {
         double2* xp = sm + (size_t)(NC + ((j & 1) ^ 1)) * n;  // xt of the previous column
         double2* xn = sm + (size_t)(NC + (j & 1)) * n;        // x, then xt, of this one
-        // row j of the own columns, updated: x_c = conj(A[j, c])
-        if (t < NC) {
-            const int c = b + t * G;
-            double nn = 0.0;
-            if (c >= j && c < n) {
-                double2 v = S[(size_t)t * n + j];
-                v = cfma(make_double2(-xp[j].x, -xp[j].y), Gk[t], v);
-                v = cfma(make_double2(-ps[j].x, -ps[j].y), Fk[t], v);
-                if (c == j) a.d[j] = v.x;
-                else {
-                    __stcg(a.xg + c, make_double2(v.x, -v.y));
-                    if (c > j + 1) nn = fma(v.x, v.x, v.y * v.y);
-                }
-            }
-            part_sh[t] = nn;
-        }
-        __syncwarp();
-        if (t == 0) {
-            double nn = 0.0;
-#pragma unroll
-            for (int k = 0; k < NC; ++k) nn += part_sh[k];
-            __stcg(a.npart + b, nn);
-        }
-        bar += G;
-        if (!grid_barrier(a.ctr, bar)) {
-            if (t == 0) *(volatile int*)a.err = 1;
-            return;
-        }
+        const double2* xj = a.xg + (int64_t)j * n;
+        const double2* pj = a.pg + (int64_t)j * n;
+        bool ok = true;
+        double2 tv = make_double2(0.0, 0.0), scal = tv, den = tv, ts = tv;
+        double vc = 0.0, tvc = 0.0;  // component im of v_c and of tau v_c
+        auto row = [&](int q) { return j + 1 + 32 * (((warp + 3) & 3) + 4 * q) + lane; };  // of a pass thread
         if (warp == 4) {
-            // the reflector's scalars (the zlarfg convention, as house_kernel)
-            double s = 0.0;
-            for (int i = lane; i < G; i += 32) s += __ldcg(a.npart + i);
-#pragma unroll
-            for (int w = 16; w >= 1; w /= 2) s += __shfl_xor_sync(0xffffffffu, s, w);
-            if (lane == 0) {
-                const double2 alpha = __ldcg(a.xg + j + 1);
-                double2 tv = make_double2(0.0, 0.0), scal = make_double2(0.0, 0.0), den = make_double2(0.0, 0.0);
-                double beta = alpha.x;
-                if (s != 0.0 || alpha.y != 0.0) {
-                    const double nrm = sqrt(fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, s)));
-                    beta = alpha.x >= 0.0 ? -nrm : nrm;
-                    const double rb = 1.0 / beta;
-                    tv = make_double2((beta - alpha.x) * rb, -alpha.y * rb);
-                    den = make_double2(alpha.x - beta, alpha.y);
-                    const double rd = 1.0 / fma(den.x, den.x, den.y * den.y);
-                    scal = make_double2(den.x * rd, -den.y * rd);
-                }
-                sc_tau = tv;
-                sc_scal = scal;
-                sc_den = den;
-                if (b == 0) {
-                    a.e[j] = beta;
-                    a.tau[j] = tv;
-                }
+            // row j of the own columns, updated: x_c = conj(A[j, c])
+            double x = 0.0;
+            if (own && c >= j) {
+                const double2 v = S[(size_t)kc * n + j], xo = xp[j], po = ps[j], g = Gk[kc], f = Fk[kc];
+                x = im ? v.y : v.x;
+                x = fma(-xo.x, im ? g.y : g.x, x);
+                x = fma(im ? -xo.y : xo.y, im ? g.x : g.y, x);
+                x = fma(-po.x, im ? f.y : f.x, x);
+                x = fma(im ? -po.y : po.y, im ? f.x : f.y, x);
+                if (im) x = -x;
+                if (c > j) post_word((double*)(xj + c) + im, x);
+                else if (!im) a.d[j] = x;
             }
-        } else {
-            // pending update of the own columns, rows r > j, and their products with the new x (row
-            // j + 1 enters with xt = den once the scalars are known)
-            double2 acc[NC];
+            double nn = own && c > j + 1 ? x * x : 0.0;
 #pragma unroll
-            for (int k = 0; k < NC; ++k) acc[k] = make_double2(0.0, 0.0);
-            // rows of a thread are those of its index mod 128 in every column, so xp, ps and xn are
-            // read by the thread that wrote them
-            for (int r = t + ((j + 1 - t + 127) / 128) * 128 * (j + 1 > t); r < n; r += 128) {
-                double2 x = __ldcg(a.xg + r);
-                xn[r] = x;
-                if (r == j + 1) x = make_double2(0.0, 0.0);
+            for (int w = kFold; w >= 1; w /= 2) nn += __shfl_xor_sync(0xffffffffu, nn, w);
+            met += G;
+            __syncwarp();
+            if (lane == 0) {
+                post_word(a.ng + (int64_t)j * G + b, nn);
+                ok = meet(a.ctr, met);
+            }
+            gate_arrive(1);
+            // the reflector's scalars (the zlarfg convention, as house_kernel), by every lane
+            double s;
+            long long ax, ay;
+            peek_pair(xj + j + 1, ax, ay);
+            ok = wait_sum(a.ng + (int64_t)j * G, G, lane, s) && ok;
+            for (int it = 0; ax == -1ll || ay == -1ll;) {
+                if (++it > kTriPolls) {
+                    ok = false;
+                    break;
+                }
+                peek_pair(xj + j + 1, ax, ay);
+            }
+            const double2 alpha = make_double2(__shfl_sync(0xffffffffu, __longlong_as_double(ax), 0),
+                                               __shfl_sync(0xffffffffu, __longlong_as_double(ay), 0));
+            double beta = alpha.x;
+            if (s != 0.0 || alpha.y != 0.0) {
+                const double nn2 = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, s));
+                const double rs = newton_rsqrt(nn2);
+                double nrm = nn2 * rs;
+                nrm = fma(fma(-nrm, nrm, nn2), 0.5 * rs, nrm);
+                beta = alpha.x >= 0.0 ? -nrm : nrm;
+                const double rb = alpha.x >= 0.0 ? -rs : rs;  // 1 / beta
+                den = make_double2(alpha.x - beta, alpha.y);
+                const double rd = newton_recip(fma(den.x, den.x, den.y * den.y));
+                tv = make_double2(-den.x * rb, -alpha.y * rb);
+                scal = make_double2(den.x * rd, -den.y * rd);
+                const double tp = mul_part(tv, im ? scal.y : scal.x, im ? scal.x : scal.y), tq = other(tp);
+                ts = make_double2(im ? tq : tp, im ? tp : tq);
+            }
+            if (b == 0 && lane == 0) {
+                a.e[j] = beta;
+                a.tau[j] = tv;
+            }
+            // v_c = scal xt_c and tau v_c
+            const double xc = c == j + 1 ? (im ? den.y : den.x) : x;
+            const double xo = other(xc);
+            vc = mul_part(scal, xc, xo);
+            const double vo = other(vc);
+            tvc = mul_part(tv, vc, vo);
+            if (!own || c <= j) vc = tvc = 0.0;
+        } else {
+            // the pending update of the own columns, rows r > j, while x travels
+            for (int q = 0, r; (r = row(q)) < n; ++q) {
                 const double2 xo = make_double2(-xp[r].x, -xp[r].y), po = make_double2(-ps[r].x, -ps[r].y);
 #pragma unroll
                 for (int k = 0; k < NC; ++k) {
@@ -445,10 +588,33 @@ __global__ void __launch_bounds__(kTriThreads, 1) tridiag_resident_kernel(TriArg
                     v = cfma(xo, Gk[k], v);
                     v = cfma(po, Fk[k], v);
                     S[(size_t)k * n + r] = v;
-                    acc[k] = cfma_conj(v, x, acc[k]);
                 }
             }
-            constexpr int NV = NC <= 1 ? 2 : NC <= 2 ? 4 : NC <= 4 ? 8 : 16;
+            // products with the new x (row j + 1 enters with xt = den once the scalars are known)
+            double2 acc[NC];
+#pragma unroll
+            for (int k = 0; k < NC; ++k) acc[k] = make_double2(0.0, 0.0);
+            gate_wait(1);
+            for (int q = 0; row(q) < n; q += U) {
+                double2 x[U];
+                int rows[U];
+#pragma unroll
+                for (int i = 0; i < U; ++i) rows[i] = row(q + i);
+                ok = wait_pairs(xj, rows, n, x) && ok;
+#pragma unroll
+                for (int i = 0; i < U; ++i) {
+                    const int r = rows[i];
+                    if (r >= n) break;
+                    xn[r] = x[i];
+                    if (r == j + 1) x[i] = make_double2(0.0, 0.0);
+#pragma unroll
+                    for (int k = 0; k < NC; ++k) {
+                        if (b + k * G <= j || b + k * G >= n) continue;
+                        acc[k] = cfma_conj(S[(size_t)k * n + r], x[i], acc[k]);
+                    }
+                }
+            }
+            constexpr int NV = 2 * kFold;
             double v[NV];
 #pragma unroll
             for (int i = 0; i < NV; ++i) v[i] = i / 2 < NC ? ((i & 1) ? acc[i / 2 < NC ? i / 2 : 0].y : acc[i / 2 < NC ? i / 2 : 0].x) : 0.0;
@@ -458,61 +624,65 @@ __global__ void __launch_bounds__(kTriThreads, 1) tridiag_resident_kernel(TriArg
                 dst[lane & 1] = tot;
             }
         }
-        __syncthreads();
-        if (t < 32) {
-            double2 dp = make_double2(0.0, 0.0);
-            const int c = b + t * G;
-            if (t < NC && c > j && c < n) {
-                const double2 den = sc_den, scal = sc_scal, tv = sc_tau;
-                double2 q = cadd(cadd(acc_sh[0][t], acc_sh[1][t]), cadd(acc_sh[2][t], acc_sh[3][t]));
-                q = cfma_conj(S[(size_t)t * n + j + 1], den, q);
-                const double2 xc = c == j + 1 ? den : xn[c];
-                const double2 vc = cmul(scal, xc);
-                const double2 pc = cmul(tv, cmul(scal, q));
-                __stcg(a.pg + c, pc);
-                a.A[c + (int64_t)j * a.n] = vc;
-                Fk[t] = make_double2(vc.x, -vc.y);
-                Gk[t] = make_double2(pc.x, -pc.y);  // completed below
-                dp = cfma_conj(pc, vc, dp);
-            } else if (t < NC) {
-                Fk[t] = Gk[t] = make_double2(0.0, 0.0);
-            }
-#pragma unroll
-            for (int w = (NC > 4 ? 4 : NC > 2 ? 2 : NC > 1 ? 1 : 0); w >= 1; w /= 2) {
-                dp.x += __shfl_xor_sync(0xffffffffu, dp.x, w);
-                dp.y += __shfl_xor_sync(0xffffffffu, dp.y, w);
-            }
-            if (t == 0) __stcg(a.dpart + b, dp);
-        }
-        bar += G;
-        if (!grid_barrier(a.ctr, bar)) {
+        if (__syncthreads_or(!ok)) {
             if (t == 0) *(volatile int*)a.err = 1;
             return;
         }
-        if (t == 0) xn[j + 1] = sc_den;
         if (warp == 4) {
-            double sx = 0.0, sy = 0.0;
-            for (int i = lane; i < G; i += 32) {
-                const double2 q = __ldcg(a.dpart + i);
-                sx += q.x;
-                sy += q.y;
+            double pc = 0.0;
+            if (own && c > j) {
+                const double2 s1 = S[(size_t)kc * n + j + 1];
+                const double* q0 = (const double*)&acc_sh[0][kc] + im;
+                double q = (q0[0] + q0[2 * NC]) + (q0[4 * NC] + q0[6 * NC]);
+                q = fma(s1.x, im ? den.y : den.x, q);
+                pc = fma(im ? -s1.y : s1.y, im ? den.x : den.y, q);
             }
+            const double qo = other(pc);
+            pc = mul_part(ts, pc, qo);
+            if (own && c > j) {
+                post_word((double*)(pj + c) + im, pc);
+                ((double*)(a.A + c + (int64_t)j * n))[im] = vc;
+            }
+            double dp = own && c > j ? pc * tvc : 0.0;  // Re(tau conj(p) v), summed over both components
 #pragma unroll
-            for (int w = 16; w >= 1; w /= 2) {
-                sx += __shfl_xor_sync(0xffffffffu, sx, w);
-                sy += __shfl_xor_sync(0xffffffffu, sy, w);
+            for (int w = kFold; w >= 1; w /= 2) dp += __shfl_xor_sync(0xffffffffu, dp, w);
+            met += G;
+            __syncwarp();
+            if (lane == 0) {
+                post_word(a.dg + (int64_t)j * G + b, dp);
+                ok = meet(a.ctr, met);
             }
-            if (lane == 0) sc_s = -fma(sc_tau.x, sx, -sc_tau.y * sy);  // 2 Re(al), al = -(tau / 2) p^H v
+            gate_arrive(2);
+            double s;
+            ok = wait_sum(a.dg + (int64_t)j * G, G, lane, s) && ok;  // -2 Re(al), al = -(tau / 2) p^H v
+            // F = conj(v), G = scal (conj(p) + 2 Re(al) conj(v))
+            const double f = im ? -vc : vc;
+            const double g = fma(-s, f, im ? -pc : pc);
+            const double go = other(g);
+            const double gs = mul_part(scal, g, go);
+            if (lane < 2 * NC) {
+                const bool on = own && c > j;
+                ((double*)&Fk[kc])[im] = on ? f : 0.0;
+                ((double*)&Gk[kc])[im] = on ? gs : 0.0;
+            }
+            if (lane == 0) xn[j + 1] = den;
         } else {
-            for (int r = t + ((j + 1 - t + 127) / 128) * 128 * (j + 1 > t); r < n; r += 128) ps[r] = __ldcg(a.pg + r);
+            gate_wait(2);
+            for (int q = 0; row(q) < n; q += U) {
+                double2 p[U];
+                int rows[U];
+#pragma unroll
+                for (int i = 0; i < U; ++i) rows[i] = row(q + i);
+                ok = wait_pairs(pj, rows, n, p) && ok;
+#pragma unroll
+                for (int i = 0; i < U; ++i)
+                    if (rows[i] < n) ps[rows[i]] = p[i];
+            }
         }
-        __syncthreads();
-        if (t < NC) {
-            const double s = sc_s;
-            const double2 g = make_double2(fma(s, Fk[t].x, Gk[t].x), fma(s, Fk[t].y, Gk[t].y));
-            Gk[t] = cmul(sc_scal, g);
+        if (__syncthreads_or(!ok)) {
+            if (t == 0) *(volatile int*)a.err = 1;
+            return;
         }
-        __syncthreads();
     }
     // the last diagonal entry: column n - 1, row n - 1, with the last update
     if (t < NC && b + t * G == n - 1) {
@@ -1076,50 +1246,6 @@ cudaError_t launch_tri(lm_ctx* ctx, TriArgs a, int grid) {
                                        ctx->stream);
 }
 
-int reduce_resident(lm_eigsys* es, DevFree& tmp) {
-    lm_ctx* ctx = es->ctx;
-    const int64_t n = es->n;
-    // two or more columns per CTA: fewer CTAs make the barriers cheaper, and below 300 rows the
-    // pass over a column is shorter than a barrier
-    const int nc = std::max(tri_resident_cols(ctx, n), (int)std::min<int64_t>(n, 2));
-    const int grid = (int)((n + nc - 1) / nc);
-    double2* buf = nullptr;  // x, p, partial dots, partial norms, barrier counter and error word
-    int rc = dalloc_t(ctx, &buf, (size_t)(2 * n + 2 * grid + 1), "tridiagonalisation exchange");
-    tmp.keep(buf);
-    if (rc != LM_OK) return rc;
-    TriArgs a;
-    a.A = es->d_A;
-    a.n = n;
-    a.d = es->d_d;
-    a.e = es->d_e;
-    a.tau = es->d_tau;
-    a.xg = buf;
-    a.pg = buf + n;
-    a.dpart = buf + 2 * n;
-    a.npart = (double*)(buf + 2 * n + grid);
-    a.ctr = (unsigned*)(buf + 2 * n + 2 * grid);
-    a.err = (int*)(a.ctr + 1);
-    CUDA_TRY(ctx, cudaMemsetAsync(buf, 0, sizeof(double2) * (size_t)(2 * n + 2 * grid + 1), ctx->stream),
-             "eigensolver: clear exchange");
-    cudaError_t e;
-    switch (nc) {
-        case 2: e = launch_tri<2>(ctx, a, grid); break;
-        case 3: e = launch_tri<3>(ctx, a, grid); break;
-        case 4: e = launch_tri<4>(ctx, a, grid); break;
-        case 5: e = launch_tri<5>(ctx, a, grid); break;
-        case 6: e = launch_tri<6>(ctx, a, grid); break;
-        case 7: e = launch_tri<7>(ctx, a, grid); break;
-        default: e = launch_tri<8>(ctx, a, grid); break;
-    }
-    CUDA_TRY(ctx, e, "eigensolver: tridiagonalisation");
-    ctx->launches++;
-    int err = 0;
-    CUDA_TRY(ctx, cudaMemcpyAsync(&err, a.err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream), "eigensolver: status");
-    CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "eigensolver: synchronize");
-    if (err) return set_err(ctx, LM_ERR_TIMEOUT, "eigensolver: a grid barrier of the tridiagonalisation gave up");
-    return LM_OK;
-}
-
 // One launch sequence per column on the lower tiles: matrices beyond the resident form.
 int reduce_tiles(lm_eigsys* es, DevFree& tmp) {
     lm_ctx* ctx = es->ctx;
@@ -1153,6 +1279,52 @@ int reduce_tiles(lm_eigsys* es, DevFree& tmp) {
         if ((j & 255) == 0) CUDA_TRY(ctx, cudaGetLastError(), "eigensolver: tridiagonalisation");
     }
     CUDA_TRY(ctx, cudaGetLastError(), "eigensolver: tridiagonalisation");
+    return LM_OK;
+}
+
+int reduce_resident(lm_eigsys* es, DevFree& tmp) {
+    lm_ctx* ctx = es->ctx;
+    const int64_t n = es->n;
+    // two or more columns per CTA: fewer CTAs make the barriers cheaper, and below 300 rows the
+    // pass over a column is shorter than a barrier
+    const int nc = std::max(tri_resident_cols(ctx, n), (int)std::min<int64_t>(n, 2));
+    const int grid = (int)((n + nc - 1) / nc);
+    // x, p, partial norms and dots of every column, over the sentinel; and the error word
+    const size_t words = 4 * (size_t)n * (size_t)n + 2 * (size_t)grid * (size_t)n;
+    double* buf = nullptr;
+    int rc = dalloc_t(ctx, &buf, words + 2, "tridiagonalisation exchange");
+    tmp.keep(buf);
+    if (rc != LM_OK) return reduce_tiles(es, tmp);  // its buffers are smaller
+    TriArgs a;
+    a.A = es->d_A;
+    a.n = n;
+    a.d = es->d_d;
+    a.e = es->d_e;
+    a.tau = es->d_tau;
+    a.err = (int*)buf;
+    a.ctr = (unsigned*)(buf + 1);
+    a.xg = (double2*)(buf + 2);
+    a.pg = a.xg + n * n;
+    a.ng = (double*)(a.pg + n * n);
+    a.dg = a.ng + (size_t)grid * n;
+    CUDA_TRY(ctx, cudaMemsetAsync(buf, 0, 16, ctx->stream), "eigensolver: clear status");
+    CUDA_TRY(ctx, cudaMemsetAsync(buf + 2, 0xff, sizeof(double) * words, ctx->stream), "eigensolver: clear exchange");
+    cudaError_t e;
+    switch (nc) {
+        case 2: e = launch_tri<2>(ctx, a, grid); break;
+        case 3: e = launch_tri<3>(ctx, a, grid); break;
+        case 4: e = launch_tri<4>(ctx, a, grid); break;
+        case 5: e = launch_tri<5>(ctx, a, grid); break;
+        case 6: e = launch_tri<6>(ctx, a, grid); break;
+        case 7: e = launch_tri<7>(ctx, a, grid); break;
+        default: e = launch_tri<8>(ctx, a, grid); break;
+    }
+    CUDA_TRY(ctx, e, "eigensolver: tridiagonalisation");
+    ctx->launches++;
+    int err = 0;
+    CUDA_TRY(ctx, cudaMemcpyAsync(&err, a.err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream), "eigensolver: status");
+    CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "eigensolver: synchronize");
+    if (err) return set_err(ctx, LM_ERR_TIMEOUT, "eigensolver: a wait of the tridiagonalisation gave up");
     return LM_OK;
 }
 

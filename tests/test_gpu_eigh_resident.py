@@ -34,3 +34,16 @@ def test_eigensystem_edges(Lx, Ly, clean):
     P = eig.projector(wt).to_numpy()
     Pr = (X * wt) @ X.conj().T
     assert np.linalg.norm(P - Pr) <= 1e-12 * np.linalg.norm(Pr)
+
+
+@pytest.mark.parametrize("ex", [-470, -300, 300, 470])
+def test_eigenvalues_scaled(ex):
+    """Scaling H by a power of two scales the eigenvalues: the reflectors' roots and reciprocals inside
+    and beyond the range of their scaled iteration."""
+    import lmgpu
+    ol, ll = o.SquareLattice(11, 13), lmgpu.SquareLattice(11, 13)
+    V, sc = o.anderson_disorder(ol.N, 2.0, 7), 2.0 ** ex
+    pt = (6.0, 7.0)
+    w = np.linalg.eigvalsh(o.tightbinding_hamiltonian(ol, field=o.PointFlux(0.2, pt), onsite=V).toarray())
+    eig = lmgpu.diagonalize(lmgpu.tightbinding_hamiltonian(ll, V * sc, t1=sc, field=lmgpu.PointFlux(0.2, pt)))
+    assert np.abs(eig.values / sc - w).max() <= 1e-13 * np.abs(w).max()
