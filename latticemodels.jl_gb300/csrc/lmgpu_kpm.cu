@@ -95,7 +95,7 @@ __global__ void start_vector_kernel(double2* __restrict__ v, int64_t n, unsigned
 // Double-float ("df") form of the moment recurrence (LM_OPT_KPM = 1, the default).  A real number is an
 // unevaluated sum hi + lo of two FP32 values (about 48 significant bits), so the recurrence
 // runs on the FP32 pipe instead of GB300's 1/64-rate FP64 pipe.  A complex df value is a float4
-// {re.hi, re.lo, im.hi, im.lo}, the size of a double2, so the FP64 buffers are reused in place.
+// {re.hi, im.hi, re.lo, im.lo}, the size of a double2, so the FP64 buffers are reused in place.
 // Products take the exact FMA error term (p + e = a*b exactly); sums use the double-word
 // addition of Dekker and of Knuth's TwoSum.  Every step is an explicit round-to-nearest
 // intrinsic, which nvcc never contracts into an FMA or reorders, so the error-free
@@ -123,8 +123,8 @@ __device__ __forceinline__ DF df_mul(DF x, DF y) {
     e = __fmaf_rn(x.l, y.h, e);
     return df_fast_two_sum(p, e);
 }
-__device__ __forceinline__ DF df_re(float4 v) { return DF{v.x, v.y}; }
-__device__ __forceinline__ DF df_im(float4 v) { return DF{v.z, v.w}; }
+__device__ __forceinline__ DF df_re(float4 v) { return DF{v.x, v.z}; }
+__device__ __forceinline__ DF df_im(float4 v) { return DF{v.y, v.w}; }
 __device__ __forceinline__ DF df_from(double x) {
     const float h = (float)x;
     return DF{h, (float)(x - (double)h)};
@@ -161,7 +161,7 @@ __global__ void to_df_kernel(const double2* __restrict__ in, int64_t ld_in, int6
             }
             const double2 v = in[m * ld_in + i];
             const DF r = df_split(v.x), q = df_split(v.y);
-            out[m * ld_out + i] = make_float4(r.h, r.l, q.h, q.l);
+            out[m * ld_out + i] = make_float4(r.h, q.h, r.l, q.l);
         }
 }
 
@@ -184,8 +184,8 @@ __global__ void from_df_kernel(const float4* __restrict__ in, int64_t ld_in, int
     for (int64_t m = blockIdx.y; m < M; m += gridDim.y)
         for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
             const float4 v = in[m * ld_in + i];
-            if (out) out[m * ld_out + i] = make_double2(df_value(DF{v.x, v.y}), df_value(DF{v.z, v.w}));
-            else out32[m * ld_out + i] = make_float2(v.x, v.z);
+            if (out) out[m * ld_out + i] = make_double2(df_value(df_re(v)), df_value(df_im(v)));
+            else out32[m * ld_out + i] = make_float2(v.x, v.y);
         }
 }
 
@@ -219,30 +219,6 @@ struct MarchArgs {
     int64_t pstride;
 };
 
-__device__ __forceinline__ void df_madd(DF& a, float ch, float cl, float vh, float vl) {
-    const float p = __fmul_rn(ch, vh);
-    float e = __fmaf_rn(ch, vh, -p);
-    e = __fmaf_rn(ch, vl, e);
-    e = __fmaf_rn(cl, vh, e);
-    const float t = __fadd_rn(a.h, p);
-    const float bb = __fsub_rn(t, a.h);
-    e = __fadd_rn(e, __fadd_rn(__fsub_rn(a.h, __fsub_rn(t, bb)), __fsub_rn(p, bb)));
-    a.l = __fadd_rn(a.l, e);
-    a.h = t;
-}
-__device__ __forceinline__ void df_caddmul(DF& re, DF& im, float4 h, float4 v) {
-    df_madd(re, h.x, h.y, v.x, v.y);
-    df_madd(re, -h.z, -h.w, v.z, v.w);
-    df_madd(im, h.x, h.y, v.z, v.w);
-    df_madd(im, h.z, h.w, v.x, v.y);
-}
-__device__ __forceinline__ DF df_sum2(float uh, float ul, float vh, float vl) {  // u + v, unnormalised
-    const float t = __fadd_rn(uh, vh);
-    const float bb = __fsub_rn(t, uh);
-    const float e = __fadd_rn(__fsub_rn(uh, __fsub_rn(t, bb)), __fsub_rn(vh, bb));
-    return DF{t, __fadd_rn(e, __fadd_rn(ul, vl))};
-}
-
 template <bool XR, bool FIRST, bool DOT, bool YACC, int KT>
 __global__ void __launch_bounds__(256, 2) df_march_kernel(const __grid_constant__ MarchArgs a) {
     const Geom& g = a.g;
@@ -266,9 +242,7 @@ __global__ void __launch_bounds__(256, 2) df_march_kernel(const __grid_constant_
         have[q] = m0 + q < a.M;
         off[q] = (have[q] ? m0 + q : m0) * a.ld;
     }
-    DF aa[KT], ba[KT];
-#pragma unroll
-    for (int q = 0; q < KT; ++q) aa[q] = ba[q] = DF{0.f, 0.f};
+    DF2 aa[KT], ba[KT];  // the real and imaginary products side by side
     if (on) {
         float4 tm[KT], tc[KT];
         const int x0 = (int)xa;
@@ -308,51 +282,39 @@ __global__ void __launch_bounds__(256, 2) df_march_kernel(const __grid_constant_
             if (!XR) hxp = a.hop[s];
 #pragma unroll
             for (int q = 0; q < KT; ++q) {
-                DF re = FIRST ? DF{0.f, 0.f} : DF{-t2[q].x, -t2[q].y}, im = FIRST ? DF{0.f, 0.f} : DF{-t2[q].z, -t2[q].w};
+                const DF2 u2(t2[q]), uc(tc[q]);
+                DF2 r;
+                if (!FIRST) r = DF2(make_float4(-t2[q].x, -t2[q].y, -t2[q].z, -t2[q].w));
                 if (XR) {
-                    DF u = df_sum2(tm[q].x, tm[q].y, tn[q].x, tn[q].y);
-                    df_madd(re, a.alpha.x, a.alpha.y, u.h, u.l);
-                    u = df_sum2(tm[q].z, tm[q].w, tn[q].z, tn[q].w);
-                    df_madd(im, a.alpha.x, a.alpha.y, u.h, u.l);
+                    r.madd(a.alpha, df2_sum(DF2(tm[q]), DF2(tn[q])));
                 } else {
-                    df_caddmul(re, im, hxp, tn[q]);
-                    df_caddmul(re, im, make_float4(hxm.x, hxm.y, -hxm.z, -hxm.w), tm[q]);
+                    r.maddc(hxp, DF2(tn[q]));
+                    r.maddc(make_float4(hxm.x, hxm.y, -hxm.z, -hxm.w), DF2(tm[q]));
                 }
-                df_caddmul(re, im, hu, up[q]);
-                df_caddmul(re, im, hd, dn[q]);
-                df_madd(re, d.x, d.y, tc[q].x, tc[q].y);
-                df_madd(im, d.x, d.y, tc[q].z, tc[q].w);
-                re = df_fast_two_sum(re.h, re.l);
-                im = df_fast_two_sum(im.h, im.l);
+                r.maddc(hu, DF2(up[q]));
+                r.maddc(hd, DF2(dn[q]));
+                r.madd(d, uc);
+                r.normalise();
                 if (FIRST) {
-                    re = DF{0.5f * re.h, 0.5f * re.l};
-                    im = DF{0.5f * im.h, 0.5f * im.l};
+                    r.h = make_float2(0.5f * r.h.x, 0.5f * r.h.y);
+                    r.l = make_float2(0.5f * r.l.x, 0.5f * r.l.y);
                 }
                 if (DOT) {
-                    df_madd(aa[q], t2[q].x, t2[q].y, t2[q].x, t2[q].y);
-                    df_madd(aa[q], t2[q].z, t2[q].w, t2[q].z, t2[q].w);
-                    df_madd(ba[q], tc[q].x, tc[q].y, t2[q].x, t2[q].y);
-                    df_madd(ba[q], tc[q].z, tc[q].w, t2[q].z, t2[q].w);
-                    aa[q] = df_fast_two_sum(aa[q].h, aa[q].l);  // long sums: keep the pairs normalised
-                    ba[q] = df_fast_two_sum(ba[q].h, ba[q].l);
+                    const float2 nh = make_float2(-u2.h.x, -u2.h.y), nl = make_float2(-u2.l.x, -u2.l.y);
+                    aa[q].madd(u2.h, nh, nl, u2.h, u2.l);
+                    ba[q].madd(u2.h, nh, nl, uc.h, uc.l);
+                    aa[q].normalise();  // long sums: keep the pairs normalised
+                    ba[q].normalise();
                 }
                 if (have[q]) {
-                    a.out[off[q] + s] = make_float4(re.h, re.l, im.h, im.l);
+                    a.out[off[q] + s] = r.word();
                     if (YACC) {
-                        DF yr{0.f, 0.f}, yi{0.f, 0.f};
-                        if (FIRST) {
-                            df_madd(yr, a.c0.x, a.c0.y, tc[q].x, tc[q].y);
-                            df_madd(yi, a.c0.x, a.c0.y, tc[q].z, tc[q].w);
-                        } else {
-                            const float4 u = a.y[off[q] + s];
-                            yr = DF{u.x, u.y};
-                            yi = DF{u.z, u.w};
-                        }
-                        df_madd(yr, a.c.x, a.c.y, re.h, re.l);
-                        df_madd(yi, a.c.x, a.c.y, im.h, im.l);
-                        yr = df_fast_two_sum(yr.h, yr.l);
-                        yi = df_fast_two_sum(yi.h, yi.l);
-                        a.y[off[q] + s] = make_float4(yr.h, yr.l, yi.h, yi.l);
+                        DF2 yv;
+                        if (FIRST) yv.madd(a.c0, uc);
+                        else yv = DF2(a.y[off[q] + s]);
+                        yv.madd(a.c, r);
+                        yv.normalise();
+                        a.y[off[q] + s] = yv.word();
                     }
                 }
                 tm[q] = tc[q];
@@ -367,8 +329,8 @@ __global__ void __launch_bounds__(256, 2) df_march_kernel(const __grid_constant_
         __shared__ double red[8][2 * KT];
 #pragma unroll
         for (int q = 0; q < 2 * KT; ++q) {
-            DF v = q < KT ? aa[q < KT ? q : 0] : ba[q < KT ? 0 : q - KT];
-            v = df_fast_two_sum(v.h, v.l);
+            const DF2 w = q < KT ? aa[q < KT ? q : 0] : ba[q < KT ? 0 : q - KT];
+            DF v = df_add(DF{w.h.x, w.l.x}, DF{w.h.y, w.l.y});
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1)
                 v = df_add(v, DF{__shfl_xor_sync(0xffffffffu, v.h, o), __shfl_xor_sync(0xffffffffu, v.l, o)});

@@ -87,6 +87,46 @@ struct Acc2 {
     }
 };
 
+// A complex double-float number or sum on packed instructions, (re, im) side by side: half the issue
+// slots of scalar ones, the same bits.  In memory {re.hi, im.hi, re.lo, im.lo}.
+struct DF2 {
+    float2 h = {0.f, 0.f}, l = {0.f, 0.f};
+    __device__ __forceinline__ DF2() {}
+    __device__ __forceinline__ DF2(float2 hi, float2 lo) : h(hi), l(lo) {}
+    __device__ __forceinline__ explicit DF2(float4 v) : h(make_float2(v.x, v.y)), l(make_float2(v.z, v.w)) {}
+    __device__ __forceinline__ float4 word() const { return make_float4(h.x, h.y, l.x, l.y); }
+    // += c v componentwise, as an unnormalised pair: v enters h by TwoSum, all error terms l.  The negated
+    // parts of c turn the product's error around, so that no operand needs a change of sign.
+    __device__ __forceinline__ void madd(float2 ch, float2 nch, float2 ncl, float2 vh, float2 vl) {
+        const float2 p = fmul2(ch, vh);
+        const float2 ne = ffma2(ncl, vh, ffma2(nch, vl, ffma2(nch, vh, p)));
+        const float2 t = fadd2(h, p);
+        const float2 bb = fsub2(t, h);
+        const float2 e = fadd2(fsub2(h, fsub2(t, bb)), fsub2(p, bb));
+        l = fadd2(l, fsub2(e, ne));
+        h = t;
+    }
+    __device__ __forceinline__ void madd(float2 c, DF2 v) {  // real c = {hi, lo}
+        madd(make_float2(c.x, c.x), make_float2(-c.x, -c.x), make_float2(-c.y, -c.y), v.h, v.l);
+    }
+    __device__ __forceinline__ void maddc(float4 c, DF2 v) {  // complex c = {re.hi, re.lo, im.hi, im.lo}
+        madd(make_float2(c.x, c.y), v);
+        madd(make_float2(-c.z, c.z), make_float2(c.z, -c.z), make_float2(c.w, -c.w), make_float2(v.h.y, v.h.x),
+             make_float2(v.l.y, v.l.x));
+    }
+    __device__ __forceinline__ void normalise() {
+        const float2 s = fadd2(h, l);
+        l = fsub2(l, fsub2(s, h));
+        h = s;
+    }
+};
+__device__ __forceinline__ DF2 df2_sum(DF2 u, DF2 v) {  // unnormalised
+    const float2 t = fadd2(u.h, v.h);
+    const float2 bb = fsub2(t, u.h);
+    const float2 e = fadd2(fsub2(u.h, fsub2(t, bb)), fsub2(v.h, bb));
+    return DF2(t, fadd2(e, fadd2(u.l, v.l)));
+}
+
 // ------------------------------------------------------------------------------------------
 // Neighbour routing on the square lattice (src/core/boundaries.jl:251-289 for the periodic
 // case: a destination one step outside is wrapped by the axis translation).

@@ -22,6 +22,7 @@
 
 #include <algorithm>
 
+#include "lmgpu_order.cuh"
 #include "lmgpu_series.cuh"
 
 namespace lmgpu {
@@ -77,85 +78,43 @@ struct ArithF64 {
     __device__ static Elem zero() { return make_double2(0.0, 0.0); }
 };
 
-// ... and double-float: a real number is hi + lo, {re.hi, re.lo, im.hi, im.lo}.  An accumulator is an
-// unnormalised pair (s, c): products enter s by TwoSum, every error term c.  All operations are
-// round-to-nearest intrinsics, which the compiler neither contracts nor reorders.
+// ... and double-float, real and imaginary part side by side.  An accumulator is an unnormalised pair:
+// products enter h by TwoSum, every error term l.  All operations round to nearest, and the compiler
+// neither contracts nor reorders them.
 struct ArithDF {
-    typedef float4 Elem;
-    typedef float4 CCoef;
+    typedef float4 Elem;   // {re.hi, im.hi, re.lo, im.lo}
+    typedef float4 CCoef;  // {re.hi, re.lo, im.hi, im.lo}
     typedef float2 Coef;
-    struct Acc {
-        float rs, rc, is, ic;
-    };
-    __device__ static void two_sum(float& s, float& c, float p) {
-        const float t = __fadd_rn(s, p);
-        const float bb = __fsub_rn(t, s);
-        c = __fadd_rn(c, __fadd_rn(__fsub_rn(s, __fsub_rn(t, bb)), __fsub_rn(p, bb)));
-        s = t;
-    }
-    __device__ static void madd(float& s, float& c, float ch, float cl, float vh, float vl) {
-        const float p = __fmul_rn(ch, vh);
-        float e = __fmaf_rn(ch, vh, -p);
-        e = __fmaf_rn(ch, vl, e);
-        e = __fmaf_rn(cl, vh, e);
-        const float t = __fadd_rn(s, p);
-        const float bb = __fsub_rn(t, s);
-        e = __fadd_rn(e, __fadd_rn(__fsub_rn(s, __fsub_rn(t, bb)), __fsub_rn(p, bb)));
-        c = __fadd_rn(c, e);
-        s = t;
-    }
+    typedef DF2 Acc;
     __device__ static Elem from(double2 v) {
         const float2 r = dsplit(v.x), i = dsplit(v.y);
-        return make_float4(r.x, r.y, i.x, i.y);
+        return make_float4(r.x, i.x, r.y, i.y);
     }
     __device__ static double2 to(const Acc& a) {
-        return make_double2((double)a.rs + (double)a.rc, (double)a.is + (double)a.ic);
+        return make_double2((double)a.h.x + (double)a.l.x, (double)a.h.y + (double)a.l.y);
     }
     __device__ static Coef coef(double v) { return dsplit(v); }
-    __device__ static void clear(Acc& a) { a.rs = a.rc = a.is = a.ic = 0.f; }
-    __device__ static void neg(Acc& a, Elem v) {
-        a.rs = -v.x;
-        a.rc = -v.y;
-        a.is = -v.z;
-        a.ic = -v.w;
-    }
-    __device__ static void add(Acc& a, Coef c, Elem v) {
-        madd(a.rs, a.rc, c.x, c.y, v.x, v.y);
-        madd(a.is, a.ic, c.x, c.y, v.z, v.w);
-    }
+    __device__ static void clear(Acc& a) { a = DF2(); }
+    __device__ static void neg(Acc& a, Elem v) { a = DF2(make_float4(-v.x, -v.y, -v.z, -v.w)); }
+    __device__ static void add(Acc& a, Coef c, Elem v) { a.madd(c, DF2(v)); }
     __device__ static void add2(Acc& a, Coef c, Elem u, Elem v) {  // the sum first: one product for two neighbours
-        float s = u.x, l = __fadd_rn(u.y, v.y);
-        two_sum(s, l, v.x);
-        madd(a.rs, a.rc, c.x, c.y, s, l);
-        s = u.z;
-        l = __fadd_rn(u.w, v.w);
-        two_sum(s, l, v.z);
-        madd(a.is, a.ic, c.x, c.y, s, l);
+        a.madd(c, df2_sum(DF2(u), DF2(v)));
     }
-    __device__ static void addc(Acc& a, CCoef h, Elem v) {
-        madd(a.rs, a.rc, h.x, h.y, v.x, v.y);
-        madd(a.rs, a.rc, -h.z, -h.w, v.z, v.w);
-        madd(a.is, a.ic, h.x, h.y, v.z, v.w);
-        madd(a.is, a.ic, h.z, h.w, v.x, v.y);
-    }
+    __device__ static void addc(Acc& a, CCoef h, Elem v) { a.maddc(h, DF2(v)); }
     // the sum over the orders: hundreds of terms, so the pair is normalised after each (left as it is,
     // the compensation word grows and the series ends 4 times as far off, 1.7e-13 at 48 x 48)
     __device__ static void addy(Acc& a, Coef c, Elem v) {
         add(a, c, v);
-        const float r = __fadd_rn(a.rs, a.rc), i = __fadd_rn(a.is, a.ic);
-        a.rc = __fsub_rn(a.rc, __fsub_rn(r, a.rs));
-        a.ic = __fsub_rn(a.ic, __fsub_rn(i, a.is));
-        a.rs = r;
-        a.is = i;
+        a.normalise();
     }
     __device__ static CCoef conj(CCoef h) { return make_float4(h.x, h.y, -h.z, -h.w); }
     __device__ static CCoef czero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
-    __device__ static Elem finish(const Acc& a) {
-        const float r = __fadd_rn(a.rs, a.rc), i = __fadd_rn(a.is, a.ic);
-        return make_float4(r, __fsub_rn(a.rc, __fsub_rn(r, a.rs)), i, __fsub_rn(a.ic, __fsub_rn(i, a.is)));
+    __device__ static Elem finish(Acc a) {
+        a.normalise();
+        return a.word();
     }
     __device__ static Elem half(Elem v) { return make_float4(0.5f * v.x, 0.5f * v.y, 0.5f * v.z, 0.5f * v.w); }
-    __device__ static Elem mul_mi(Elem v) { return make_float4(v.z, v.w, -v.x, -v.y); }
+    __device__ static Elem mul_mi(Elem v) { return make_float4(v.y, -v.x, v.w, -v.z); }
     __device__ static Elem zero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
 };
 
