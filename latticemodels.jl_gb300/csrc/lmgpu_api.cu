@@ -920,15 +920,15 @@ int lm_solver_create(lm_ctx* ctx, double tol, lm_solver** out) {
 }
 
 static void free_tables(lm_solver* s) {
-    if (s->d_hop2) cudaFree(s->d_hop2);
-    if (s->d_diag2) cudaFree(s->d_diag2);
-    if (s->d_hop2f) cudaFree(s->d_hop2f);
-    if (s->d_diag2f) cudaFree(s->d_diag2f);
-    if (s->d_spack) cudaFree(s->d_spack);
+    dev_free(s->ctx, s->d_hop2);
+    dev_free(s->ctx, s->d_diag2);
+    dev_free(s->ctx, s->d_hop2f);
+    dev_free(s->ctx, s->d_diag2f);
+    dev_free(s->ctx, s->d_spack);
     s->d_spack = nullptr;
     s->spack_f4 = 0;
     s->spack_version = ~0ull;
-    if (s->d_sgauge) cudaFree(s->d_sgauge);
+    dev_free(s->ctx, s->d_sgauge);
     s->d_sgauge = nullptr;
     s->sgauge_version = ~0ull;
     s->d_hop2 = nullptr;
@@ -963,10 +963,10 @@ int lm_solver_update(lm_solver* s, lm_ham* h, double dt, int force) {
     const Geom& g = h->lat->g;
     if (s->tab_n != g.N) {
         free_tables(s);
-        int rc = dalloc(ctx, (void**)&s->d_hop2, sizeof(double2) * 2 * (size_t)g.N, "hop table");
-        if (rc == LM_OK) rc = dalloc(ctx, (void**)&s->d_diag2, sizeof(double) * (size_t)g.N, "diag table");
-        if (rc == LM_OK) rc = dalloc(ctx, (void**)&s->d_hop2f, sizeof(float2) * 2 * (size_t)g.N, "hop table f32");
-        if (rc == LM_OK) rc = dalloc(ctx, (void**)&s->d_diag2f, sizeof(float) * (size_t)g.N, "diag table f32");
+        int rc = dalloc_pool(ctx, (void**)&s->d_hop2, sizeof(double2) * 2 * (size_t)g.N, "hop table");
+        if (rc == LM_OK) rc = dalloc_pool(ctx, (void**)&s->d_diag2, sizeof(double) * (size_t)g.N, "diag table");
+        if (rc == LM_OK) rc = dalloc_pool(ctx, (void**)&s->d_hop2f, sizeof(float2) * 2 * (size_t)g.N, "hop table f32");
+        if (rc == LM_OK) rc = dalloc_pool(ctx, (void**)&s->d_diag2f, sizeof(float) * (size_t)g.N, "diag table f32");
         if (rc != LM_OK) {
             free_tables(s);
             s->valid = 0;
@@ -1187,7 +1187,7 @@ static int series_step(lm_solver* s, lm_state* st, int* done) {
     if (!plan.kt) return LM_OK;
     if (!xr && s->sgauge_version != s->tab_version) {
         if (!s->d_sgauge) {
-            int rc = dalloc(ctx, (void**)&s->d_sgauge, sizeof(double2) * 2 * (size_t)g.N, "gauge table");
+            int rc = dalloc_pool(ctx, (void**)&s->d_sgauge, sizeof(double2) * 2 * (size_t)g.N, "gauge table");
             if (rc != LM_OK) return rc;
         }
         CUDA_TRY(ctx, launch_gauge_tables(ctx, g, h->d_hop, h->d_onsite, h->t1, s->a, s->b, false, s->d_sgauge,

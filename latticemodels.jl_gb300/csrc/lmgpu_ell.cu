@@ -453,10 +453,10 @@ int ell_solver_step(lm_solver* s, lm_state* st) {
 }
 
 void ell_free_tables(lm_solver* s) {
-    cudaFree(s->d_ev2);
-    cudaFree(s->d_ed2);
-    cudaFree(s->d_ev2f);
-    cudaFree(s->d_ed2f);
+    dev_free(s->ctx, s->d_ev2);
+    dev_free(s->ctx, s->d_ed2);
+    dev_free(s->ctx, s->d_ev2f);
+    dev_free(s->ctx, s->d_ed2f);
     s->d_ev2 = nullptr;
     s->d_ed2 = nullptr;
     s->d_ev2f = nullptr;
@@ -1042,10 +1042,10 @@ int lm_ell_solver_update(lm_solver* s, lm_ell* h, double dt, int force) {
     const int64_t tab = h->n * (int64_t)h->w;
     if (s->ell_tab != tab + h->n) {
         ell_free_tables(s);
-        cudaError_t e = cudaMalloc((void**)&s->d_ev2, sizeof(double2) * (size_t)tab);
-        if (e == cudaSuccess) e = cudaMalloc((void**)&s->d_ed2, sizeof(double) * (size_t)h->n);
-        if (e == cudaSuccess) e = cudaMalloc((void**)&s->d_ev2f, sizeof(float2) * (size_t)tab);
-        if (e == cudaSuccess) e = cudaMalloc((void**)&s->d_ed2f, sizeof(float) * (size_t)h->n);
+        cudaError_t e = dev_alloc(ctx, (void**)&s->d_ev2, sizeof(double2) * (size_t)tab);
+        if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&s->d_ed2, sizeof(double) * (size_t)h->n);
+        if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&s->d_ev2f, sizeof(float2) * (size_t)tab);
+        if (e == cudaSuccess) e = dev_alloc(ctx, (void**)&s->d_ed2f, sizeof(float) * (size_t)h->n);
         if (e != cudaSuccess) {
             cudaGetLastError();
             ell_free_tables(s);

@@ -107,6 +107,10 @@ struct lm_ctx {
     unsigned resident_attr = 0;         // shared-memory attributes of the lattice-resident kernels set
     unsigned long long* h_res_err = nullptr;  // timeout word of the kernels that wait (mapped host memory)
     unsigned long long* d_res_err = nullptr;  // and its device address
+    struct {
+        int threads = 0, fit = 0;
+        size_t smem = 0;
+    } series_fit[9];                    // CTAs per SM of the on-chip series kernels at their last block and shared size
     unsigned* d_grid = nullptr;         // barrier counters of cooperative launches (zero between launches)
     int resident = 1;                   // LM_OPT_RESIDENT: lattice-resident form in the batch's fused pass
     std::vector<double> h_norms;        // pageable staging of lm_state_renormalize's targets

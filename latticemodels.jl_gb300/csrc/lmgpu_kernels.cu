@@ -467,9 +467,10 @@ __global__ void __launch_bounds__(32 * kReadWarps) bond_currents_kets_kernel(
 // Density matrices: P[j,s] read directly.
 template <typename R>
 __global__ void bond_currents_dm_kernel(Geom g, const double2* __restrict__ hop, const typename CT<R>::V* __restrict__ x,
-                                        int64_t ld, double* __restrict__ out) {
+                                        int64_t ld, double* __restrict__ rho, double* __restrict__ out) {
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= g.N) return;
+    if (rho) rho[s] = (double)x[s * ld + s].x;  // the density of the same readout: one launch for both
     const Nbr nb = neighbours(g, s);
 #pragma unroll
     for (int dir = 0; dir < 2; ++dir) {
@@ -638,14 +639,21 @@ static void launch_currents_kets(lm_ctx* ctx, const Geom& g, const double2* hop,
     ctx->launches++;
 }
 
+// Bond currents of a density matrix, with rho also its local density.
+static cudaError_t launch_bond_currents_dm(lm_ctx* ctx, const Geom& g, int precision, const double2* hop, const void* x,
+                                           int64_t ld, double* rho, double* out) {
+    const unsigned blocks = (unsigned)((g.N + 127) / 128);
+    if (precision == LM_C64) bond_currents_dm_kernel<double><<<blocks, 128, 0, ctx->stream>>>(g, hop, (const double2*)x, ld, rho, out);
+    else bond_currents_dm_kernel<float><<<blocks, 128, 0, ctx->stream>>>(g, hop, (const float2*)x, ld, rho, out);
+    ctx->launches++;
+    return cudaGetLastError();
+}
+
 cudaError_t launch_bond_currents(lm_ctx* ctx, const Geom& g, int precision, int kind, const double2* hop, bool xr,
                                  const void* x, int64_t m, int64_t ld, const double* w, double* out) {
     if (g.N <= 0) return cudaSuccess;
     if (kind == LM_DENSITY) {
-        const unsigned blocks = (unsigned)((g.N + 127) / 128);
-        if (precision == LM_C64) bond_currents_dm_kernel<double><<<blocks, 128, 0, ctx->stream>>>(g, hop, (const double2*)x, ld, out);
-        else bond_currents_dm_kernel<float><<<blocks, 128, 0, ctx->stream>>>(g, hop, (const float2*)x, ld, out);
-        ctx->launches++;
+        return launch_bond_currents_dm(ctx, g, precision, hop, x, ld, nullptr, out);
     } else if (precision == LM_C64) {
         if (xr) launch_currents_kets<double, true>(ctx, g, hop, x, m, ld, w, out);
         else launch_currents_kets<double, false>(ctx, g, hop, x, m, ld, w, out);
@@ -668,6 +676,7 @@ cudaError_t launch_readouts(lm_ctx* ctx, const Geom& g, int precision, int kind,
         if (e != cudaErrorMemoryAllocation) return e;
         (void)cudaGetLastError();
     }
+    if (kind == LM_DENSITY && g.N > 0) return launch_bond_currents_dm(ctx, g, precision, hop, x, ld, rho, out);
     const cudaError_t e = launch_localdensity(ctx, precision, kind, x, g.N, m, ld, w, rho);
     return e == cudaSuccess ? launch_bond_currents(ctx, g, precision, kind, hop, xr, x, m, ld, w, out) : e;
 }

@@ -296,16 +296,23 @@ __global__ void __launch_bounds__(32) gauge_tables_kernel(Geom g, const double2*
 }
 
 template <class A, int KT, int S, bool PROP>
-cudaError_t launch_t(lm_ctx* ctx, const SeriesPlan& p, const SeriesArgs& a) {
-    cudaError_t e = cudaFuncSetAttribute(series_resident_kernel<A, KT, S, PROP>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
-    if (e != cudaSuccess) return e;
+cudaError_t launch_t(lm_ctx* ctx, const SeriesPlan& p, const SeriesArgs& a, int variant) {
     const int64_t items = (a.M + KT - 1) / KT;
     const int threads = (a.Ly * a.nseg + 31) / 32 * 32;
     // several CTAs of a small lattice share an SM, each taking an equal share of the kets
-    int fit = 1;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, series_resident_kernel<A, KT, S, PROP>, threads, p.smem);
-    if (e != cudaSuccess) return e;
+    auto& f = ctx->series_fit[variant];
+    if (f.threads != threads || f.smem != p.smem) {
+        cudaError_t e = cudaFuncSetAttribute(series_resident_kernel<A, KT, S, PROP>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+        int fit = 1;
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, series_resident_kernel<A, KT, S, PROP>, threads, p.smem);
+        if (e != cudaSuccess) return e;
+        f.threads = threads;
+        f.smem = p.smem;
+        f.fit = fit;
+    }
+    const int fit = f.fit;
     const int64_t slots = (int64_t)std::max(fit, 1) * ctx->sm_count, waves = (items + slots - 1) / slots;
     series_resident_kernel<A, KT, S, PROP><<<(unsigned)((items + waves - 1) / waves), threads, p.smem, ctx->stream>>>(a);
     ctx->launches++;
@@ -357,19 +364,19 @@ cudaError_t launch_gauge_tables(lm_ctx* ctx, const Geom& g, const double2* hop, 
 cudaError_t launch_series_f64(lm_ctx* ctx, const SeriesPlan& p, SeriesArgs a) {
     a.nseg = p.nseg;
     a.cols = p.cols;
-    if (p.cols <= 2) return launch_t<ArithF64, 1, 2, true>(ctx, p, a);
-    if (p.cols <= 4) return launch_t<ArithF64, 1, 4, true>(ctx, p, a);
-    if (p.cols <= 8) return launch_t<ArithF64, 1, 8, true>(ctx, p, a);
-    return launch_t<ArithF64, 1, 12, true>(ctx, p, a);
+    if (p.cols <= 2) return launch_t<ArithF64, 1, 2, true>(ctx, p, a, 0);
+    if (p.cols <= 4) return launch_t<ArithF64, 1, 4, true>(ctx, p, a, 1);
+    if (p.cols <= 8) return launch_t<ArithF64, 1, 8, true>(ctx, p, a, 2);
+    return launch_t<ArithF64, 1, 12, true>(ctx, p, a, 3);
 }
 
 cudaError_t launch_series_df(lm_ctx* ctx, const SeriesPlan& p, SeriesArgs a) {
     a.nseg = p.nseg;
     a.cols = p.cols;
-    if (p.kt == 2) return p.cols <= 2 ? launch_t<ArithDF, 2, 2, false>(ctx, p, a) : launch_t<ArithDF, 2, 6, false>(ctx, p, a);
-    if (p.cols <= 2) return launch_t<ArithDF, 1, 2, false>(ctx, p, a);
-    if (p.cols <= 6) return launch_t<ArithDF, 1, 6, false>(ctx, p, a);
-    return launch_t<ArithDF, 1, 12, false>(ctx, p, a);
+    if (p.kt == 2) return p.cols <= 2 ? launch_t<ArithDF, 2, 2, false>(ctx, p, a, 4) : launch_t<ArithDF, 2, 6, false>(ctx, p, a, 5);
+    if (p.cols <= 2) return launch_t<ArithDF, 1, 2, false>(ctx, p, a, 6);
+    if (p.cols <= 6) return launch_t<ArithDF, 1, 6, false>(ctx, p, a, 7);
+    return launch_t<ArithDF, 1, 12, false>(ctx, p, a, 8);
 }
 
 }  // namespace lmgpu

@@ -727,11 +727,11 @@ int ensure_stream_pack(lm_solver* s, const Geom& g) {
     pack_dims(g, &npair, &Xp, &plane);
     const size_t need = pack_f4(g);
     if (s->spack_f4 != need) {
-        if (s->d_spack) cudaFree(s->d_spack);
+        dev_free(ctx, s->d_spack);
         s->d_spack = nullptr;
         s->spack_f4 = 0;
         s->spack_version = ~0ull;
-        const cudaError_t e = cudaMalloc((void**)&s->d_spack, sizeof(float4) * need);
+        const cudaError_t e = dev_alloc(ctx, (void**)&s->d_spack, sizeof(float4) * need);
         if (e != cudaSuccess) {
             s->d_spack = nullptr;
             cudaGetLastError();
@@ -791,10 +791,10 @@ int ensure_brick_pack(lm_solver* s, const Geom& g, const int* d_bmap) {
     pack_dims(g, &npair, &Xp, &plane);
     const size_t need = pack_f4(g);
     if (s->spack_f4 != need) {
-        if (s->d_spack) cudaFree(s->d_spack);
+        dev_free(ctx, s->d_spack);
         s->d_spack = nullptr;
         s->spack_f4 = 0;
-        const cudaError_t e = cudaMalloc((void**)&s->d_spack, sizeof(float4) * need);
+        const cudaError_t e = dev_alloc(ctx, (void**)&s->d_spack, sizeof(float4) * need);
         if (e != cudaSuccess) {
             s->d_spack = nullptr;
             cudaGetLastError();
