@@ -202,18 +202,25 @@ __global__ void __launch_bounds__(1024, 1) cheb_ell_coop_kernel(const __grid_con
                 }
             acc.x = fma(d, t1.x, acc.x);
             acc.y = fma(d, t1.y, acc.y);
+            if (k == 1) acc = CT<R>::make(acc.x * R(0.5), acc.y * R(0.5));
+            if (k < a.K) __stcg(dst + base + site, acc);
+            t2 = t1;
+            t1 = acc;
+        }
+        if (k < a.K) grid_arrive(a.ctr);
+        if (on) {  // the sum, while the other CTAs arrive
+            const V acc = t1;
             const R cs = (R)a.s[k], c0 = (R)a.s[0];
             if (k == 1) {
-                acc = CT<R>::make(acc.x * R(0.5), acc.y * R(0.5));
                 if (sizeof(R) == sizeof(float)) {
                     const ChebLo& lo = a.lo;
-                    R lx = fma(R(lo.g0_re), t1.x, fma(R(-lo.g0_im), t1.y, fma(R(lo.g1_re), acc.x, R(-lo.g1_im) * acc.y)));
-                    R ly = fma(R(lo.g0_re), t1.y, fma(R(lo.g0_im), t1.x, fma(R(lo.g1_re), acc.y, R(lo.g1_im) * acc.x)));
-                    y.x = fma(c0, t1.x, fma(cs, acc.y, lx));
-                    y.y = fma(c0, t1.y, fma(-cs, acc.x, ly));
+                    R lx = fma(R(lo.g0_re), t2.x, fma(R(-lo.g0_im), t2.y, fma(R(lo.g1_re), acc.x, R(-lo.g1_im) * acc.y)));
+                    R ly = fma(R(lo.g0_re), t2.y, fma(R(lo.g0_im), t2.x, fma(R(lo.g1_re), acc.y, R(lo.g1_im) * acc.x)));
+                    y.x = fma(c0, t2.x, fma(cs, acc.y, lx));
+                    y.y = fma(c0, t2.y, fma(-cs, acc.x, ly));
                 } else {
-                    y.x = fma(cs, acc.y, c0 * t1.x);
-                    y.y = fma(-cs, acc.x, c0 * t1.y);
+                    y.x = fma(cs, acc.y, c0 * t2.x);
+                    y.y = fma(-cs, acc.x, c0 * t2.y);
                 }
             } else if (k & 1) {
                 y.x = fma(cs, acc.y, y.x);
@@ -225,15 +232,11 @@ __global__ void __launch_bounds__(1024, 1) cheb_ell_coop_kernel(const __grid_con
             if (k == a.K) {
                 const R pr = (R)a.ph_re, pi = (R)a.ph_im;
                 dst[base + site] = CT<R>::make(fma(pr, y.x, -pi * y.y), fma(pr, y.y, pi * y.x));
-            } else {
-                __stcg(dst + base + site, acc);
             }
-            t2 = t1;
-            t1 = acc;
         }
         if (k < a.K) {
             bar += gridDim.x;
-            if (!grid_barrier(a.ctr, bar)) {
+            if (!grid_wait(a.ctr, bar)) {
                 if (threadIdx.x == 0) *(volatile unsigned long long*)a.err = 1ull;
                 return;
             }

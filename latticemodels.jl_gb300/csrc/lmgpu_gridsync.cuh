@@ -9,14 +9,19 @@ constexpr int kGridPolls = 1 << 21;  // bound of a barrier wait (about a second)
 // Every CTA adds 1 to the counter and waits until it has reached `target` (the launch's CTAs times the
 // barriers so far); what a CTA wrote before is visible to all after.  False for every thread of a CTA
 // whose wait gave up: it leaves the kernel, and so do the others, whose counter cannot fill up.
-__device__ __forceinline__ bool grid_barrier(unsigned* ctr, unsigned target) {
-    __shared__ int ok;
+// In two halves, with work between them that the other CTAs do not wait for.
+__device__ __forceinline__ void grid_arrive(unsigned* ctr) {
     __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
+    }
+}
+__device__ __forceinline__ bool grid_wait(unsigned* ctr, unsigned target) {
+    __shared__ int ok;
     if (threadIdx.x == 0) {
         int good = 1, it = 0;
         unsigned seen;
-        asm volatile("fence.acq_rel.gpu;" ::: "memory");
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(ctr) : "memory");
             if (++it > kGridPolls) {
