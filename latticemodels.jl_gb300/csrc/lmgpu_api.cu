@@ -91,7 +91,7 @@ void dev_free(lm_ctx* ctx, void* p) {
     else cudaFree(p);
 }
 
-// A pool of the context's own.  Up to a 64th of the device's memory (4.4 GB) stays with it across
+// A pool of the context's own.  Up to a 32nd of the device's memory (9 GB) stays with it across
 // synchronisations instead of going back to the driver: allocating and freeing the buffers of a
 // 265 MB state cost 1.1 ms per Evolution.  lm_ctx_destroy gives everything back.
 static void create_pool(lm_ctx* ctx) {
@@ -111,7 +111,7 @@ static void create_pool(lm_ctx* ctx) {
         ctx->pool = nullptr;
         return;
     }
-    unsigned long long keep = total / 64;
+    unsigned long long keep = total / 32;
     cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
 }
 }  // namespace lmgpu

@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(256) cheb_order_ell_rows_kernel(
 //
 // What bounds it: the FP64 pipe (16 DFMAs per site of the honeycomb and order, 3.1 us for 1e5 sites) and
 // a barrier with the gather's latency behind it (about 2 us) per order; a launch per order takes 6.6 us on
-// the device and 2.5 us of the host.  One ket of 100,352 honeycomb sites, K = 11: 58 against 75 us.
+// the device and 2.5 us of the host.  One ket of 100,352 honeycomb sites, K = 11: 61.5 against 75 us (65.9 us with the sum ahead of the barrier).
 struct EllCoop {
     int64_t n, total, ld;
     int w, K;

@@ -490,11 +490,13 @@ __global__ void bond_currents_dm_kernel(Geom g, const double2* __restrict__ hop,
 // more) and on the y-bond; readout_slices_kernel adds the slices in order and writes the readouts.
 //
 // What bounds it: the products, 10 FP32 operations each (exact product, TwoSum; the sums carry 48
-// bits).  256 x 256 sites, 2048 kets, real x-hops: 6 products for the currents and 2 for the density in
-// one pass of 480 us, against 453 us for the currents' 8 and a second pass of 179 us for the density.
-// 97 x 75 sites, 650 kets: 22 us against 44 + 11 us, where one block per 32 sites left SMs idle.
+// bits), two at a time on packed pairs.  256 x 256 sites, 2048 kets, real x-hops: 6 products for the
+// currents and 2 for the density in one pass of 426 us (scalar products 478 us, packed ones without the
+// bound of three blocks per SM 558 us), against 453 us for the currents' 8 and a second pass of 179 us for
+// the density.  97 x 75 sites, 650 kets: 31 us (33 us with scalar products) against 44 + 11 us, where one
+// block per 32 sites left SMs idle.
 template <int VEC, bool XR, bool DENS>
-__global__ void __launch_bounds__(32 * kReadWarps) readout_kets_kernel(
+__global__ void __launch_bounds__(32 * kReadWarps, VEC == 4 ? 3 : 4) readout_kets_kernel(
     Geom g, const float2* __restrict__ x, int64_t m, int64_t ld, int64_t kslice, double* __restrict__ part) {
     constexpr int NQ = (DENS ? 1 : 0) + (XR ? 1 : 2) + 2, QX = DENS ? 1 : 0, QY = QX + (XR ? 1 : 2);
     __shared__ double red[kReadWarps][32 * VEC];
@@ -502,7 +504,7 @@ __global__ void __launch_bounds__(32 * kReadWarps) readout_kets_kernel(
     const int64_t s0 = (int64_t)blockIdx.x * (32 * VEC) + (int64_t)lane * VEC;
     const int64_t k0 = (int64_t)blockIdx.y * kslice;
     const int64_t k1 = k0 + kslice < m ? k0 + kslice : m;
-    Acc<float> a[VEC][NQ];
+    Acc2 ad[VEC], ax[VEC], ay[VEC];  // |b|^2 by component; x-bond (XR: the two products of im; else re, im); y-bond (re, im)
     if (s0 < g.N) {
         const int64_t xi = s0 / g.Ly, yi0 = s0 - xi * g.Ly;
         // absent bonds read the sites themselves (always in bounds) and are not written
@@ -530,20 +532,17 @@ __global__ void __launch_bounds__(32 * kReadWarps) readout_kets_kernel(
 #pragma unroll
             for (int j = 0; j < VEC; ++j) {
                 const float2 bb = b[j], cx = c[j], cy = b[j + 1];  // c * conj(b)
-                if (DENS) {
-                    a[j][0].add_prod(bb.x, bb.x);
-                    a[j][0].add_prod(bb.y, bb.y);
+                const float2 b1 = make_float2(bb.x, bb.x), n1 = make_float2(-bb.x, -bb.x);
+                const float2 b2 = make_float2(bb.y, -bb.y), n2 = make_float2(-bb.y, bb.y);
+                if (DENS) ad[j].add_prod(bb, make_float2(-bb.x, -bb.y), bb);
+                if (XR) {
+                    ax[j].add_prod(make_float2(-bb.y, bb.x), make_float2(bb.y, -bb.x), cx);
+                } else {
+                    ax[j].add_prod(b1, n1, cx);
+                    ax[j].add_prod(b2, n2, make_float2(cx.y, cx.x));
                 }
-                if (!XR) {
-                    a[j][QX].add_prod(cx.x, bb.x);
-                    a[j][QX].add_prod(cx.y, bb.y);
-                }
-                a[j][QY - 1].add_prod(cx.y, bb.x);
-                a[j][QY - 1].add_prod(-cx.x, bb.y);
-                a[j][QY].add_prod(cy.x, bb.x);
-                a[j][QY].add_prod(cy.y, bb.y);
-                a[j][QY + 1].add_prod(cy.y, bb.x);
-                a[j][QY + 1].add_prod(-cy.x, bb.y);
+                ay[j].add_prod(b1, n1, cy);
+                ay[j].add_prod(b2, n2, make_float2(cy.y, cy.x));
             }
         }
     }
@@ -552,7 +551,11 @@ __global__ void __launch_bounds__(32 * kReadWarps) readout_kets_kernel(
     for (int q = 0; q < NQ; ++q) {
         if (q > 0) __syncthreads();
 #pragma unroll
-        for (int j = 0; j < VEC; ++j) red[warp][lane * VEC + j] = a[j][q].get();
+        for (int j = 0; j < VEC; ++j) {
+            const Acc2& v = DENS && q == 0 ? ad[j] : q < QY ? ax[j] : ay[j];
+            const double re = (double)v.hi.x + (double)v.lo.x, im = (double)v.hi.y + (double)v.lo.y;
+            red[warp][lane * VEC + j] = (DENS && q == 0) || (XR && q < QY) ? re + im : q == QX || q == QY ? re : im;
+        }
         __syncthreads();
         const int64_t s = (int64_t)blockIdx.x * (32 * VEC) + threadIdx.x;
         if (threadIdx.x < 32 * VEC && s < g.N) {
