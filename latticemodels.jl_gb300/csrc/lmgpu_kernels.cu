@@ -113,14 +113,15 @@ static void launch_cheb_t(lm_ctx* ctx, const Geom& g, const void* hop2, const vo
                           void* tq, void* y, int64_t ld, int64_t m, double c0, ChebCoef ck, double ph_re,
                           double ph_im, ChebLo lo) {
     typedef typename CT<R>::V V;
-    constexpr int INNER = 4;
     const int thr = SF ? 256 : 128;
     const int64_t nfast = SF ? g.N : m;
     const int64_t nslow = SF ? m : g.N;
     const int64_t gx = (nfast + thr - 1) / thr;
-    int64_t gy = (nslow + INNER - 1) / INNER;
-    if (gy > 65535) gy = 65535;
-    dim3 grid((unsigned)gx, (unsigned)gy);
+    // FP64: a ket per thread.  Four in turn left the FP64 pipe idle behind their loads and filled the SMs
+    // unevenly (256 x 256 sites, 384 kets: 675 against 757 us per order; 96 x 41 sites, 41 kets: 7.2 against
+    // 10.2 us).  FP32 is bound by memory, where a thread's stencil row serves four kets.
+    constexpr int INNER = sizeof(R) == sizeof(double) ? 1 : 4;
+    const dim3 grid((unsigned)gx, (unsigned)std::min<int64_t>((nslow + INNER - 1) / INNER, 65535));
     cheb_order_kernel<R, MODE, SF, CJ, INNER, XR><<<grid, thr, 0, ctx->stream>>>(
         g, (const V*)hop2, (const R*)diag2, (const V*)tp, (V*)tq, (V*)y, ld, m, (R)c0, (R)ck.s, ck.odd,
         (R)ph_re, (R)ph_im, lo);
