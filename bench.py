@@ -500,8 +500,8 @@ def run_kpm_workload(args):
     passes = (nmom + 1) // 2 + 1
     # per pass, FP64 path: the recurrence reads T_{n+1} and T_n and writes T_{n+2}; the two
     # dot products read T_n (twice) and T_{n+1}: six block passes of N*R*16 bytes.  The
-    # double-float path forms both dots in one read of T_n and T_{n+1}: five passes.
-    alg = 5.0 * N * R * 16 * passes
+    # double-float path forms both dots from the values the recurrence holds: three passes.
+    alg = 3.0 * N * R * 16 * passes
     alg64 = 6.0 * N * R * 16 * passes
     peak, peak_kind = measured_peak_hbm()
     line = {"metric": "KPM vector-moments/s (Chebyshev moments, double-float recurrence)",
@@ -515,8 +515,8 @@ def run_kpm_workload(args):
                          "frac": alg / (ms / 1000.0) / 1e9 / peak, "traffic": None,
                          "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)",
                          "alg_bytes_per_call": alg,
-                         "note": "whole call (recurrence + dot kernels): 5 block passes per pass (the double-float "
-                                 "dots read T_n and T_n+1 once for both moments)"},
+                         "note": "whole call: 3 block passes per pass (both moment dots from the values the "
+                                 "double-float recurrence holds)"},
             "mu0_over_N": float(mu[0] / (N * R)), "clocks": clocks,
             "fp64": {"value": R * nmom / (ms64 / 1000.0), "ms_per_step": ms64, "speedup_of_default": ms64 / ms,
                      "roofline_frac": alg64 / (ms64 / 1000.0) / 1e9 / peak,

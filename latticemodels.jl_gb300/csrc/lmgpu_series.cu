@@ -15,9 +15,10 @@
 // What bounds it: the arithmetic.  FP64 runs at 1.7 lane operations per clock and SM, so the
 // 16 of a site and order are all that counts; a double-float product and sum takes 12 FP32
 // operations (error-free product, TwoSum, one compensation word that is folded in once per site)
-// instead of 18 with a normalised sum.  Measured: a dense 10 x 10 step 21 us against 18 launches of
-// 6 us, a dense 47 x 31 step 1.45 ms (1.25 ms of DFMAs) against 1.57 ms, the Fermi operator of a 48 x 48
-// lattice (470 terms) 20 ms against 54 ms with a launch per term.
+// instead of 18 with a normalised sum, on packed pairs (re, im).  Measured: a dense 10 x 10 step 21 us
+// against 18 launches of 3 us and their host time (67 us), a dense 47 x 31 step 1.31 ms as with a launch per
+// order, the Fermi operator of a 48 x 48 lattice (470 terms) 16.9 ms (19.4 ms with scalar operations)
+// against 54 ms with a launch per term.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -339,15 +340,18 @@ SeriesPlan series_plan(const lm_ctx* ctx, const Geom& g, bool x_real, int64_t M,
     const int kt = df && p.cols <= 6 && M >= 2 * ctx->sm_count && 2 * ket + tables <= kMaxSmem ? 2 : 1;
     p.smem = kt * ket + tables;
     if (p.smem > kMaxSmem) return p;
-    // Against one launch per order: here an order takes the longest SM's share of the kets (N sites at
-    // 16 DFMAs of 1.7 a clock, or 190 FP32 operations at about 100 a clock), there a launch of about
-    // 5 us and the whole block at the same rate or at its memory traffic.  Few kets on a large lattice
-    // leave SMs idle here; elsewhere this form is ahead (10 x 10 dense: 1.4 against 6 us an order;
-    // 47 x 31 dense: 62 against 82 us; double-float 48 x 48: 39 against 111 us).
-    const double sites = (double)g.N, cyc = df ? 1.9 : 16.0 / 1.7, mhz = 2000.0;
+    // Against one launch per order: here an order takes the longest SM's share of the kets (10.8 clocks a
+    // site in FP64, the gauge included, or 1.9 in double-float), there a launch of about 5 us and the whole
+    // block at 16 or 20 DFMAs of 1.87 a clock and SM (double-float: at its memory traffic).  Few kets on a
+    // large lattice leave SMs idle here, and from about 1500 sites a dense FP64 step is ahead there; elsewhere
+    // this form is (dense steps here / there: 10 x 10 22.5 / 66.7 us, 30 x 30 505 / 555 us, 47 x 31 1309 /
+    // 1314 us, 48 x 48 3208 / 3078 us; 200 kets of 48 x 48 204 / 171 us; double-float 48 x 48: 34 / 111 us an
+    // order).
+    const double sites = (double)g.N, mhz = 2000.0;
     const int64_t per_sm = (M + (int64_t)kt * ctx->sm_count - 1) / ((int64_t)kt * ctx->sm_count) * kt;
-    const double here = 0.5 + (double)per_sm * sites * cyc / mhz;
-    const double there = 5.0 + (double)M * sites * (df ? 2.0e-5 : cyc / mhz / ctx->sm_count * (x_real ? 1.0 : 1.25));
+    const double here = 0.5 + (double)per_sm * sites * (df ? 1.9 : 10.8) / mhz;
+    const double there =
+        5.0 + (double)M * sites * (df ? 2.0e-5 : (x_real ? 16.0 : 20.0) / 1.87 / mhz / ctx->sm_count);
     if (here < there) p.kt = kt;
     return p;
 }
