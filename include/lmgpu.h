@@ -68,8 +68,10 @@ int lm_ctx_synchronize(lm_ctx *ctx);
  * CUDA events against the library's launches. */
 int lm_ctx_stream(lm_ctx *ctx, void **stream);
 /* Context options.  LM_OPT_FUSED (default 1): a ComplexF32 ket-block step whose Chebyshev
- * order is at most 8 runs as one temporally blocked launch; 0 selects one launch per order
- * (same results to FP32 rounding; kept for comparison). */
+ * order is at most 8 runs as one temporally blocked launch; the ComplexF64 step of a small
+ * lattice with an open x axis keeps whole kets on chip for all orders; a general Hamiltonian's
+ * step on a small block and the ComplexF32 adjoint on chip take one launch for all orders.
+ * 0 selects one launch per order for all of them (same results to rounding; kept for comparison). */
 #define LM_OPT_FUSED 1
 /* LM_OPT_STREAM (default 1): a single lattice with even Ly, Lx >= 2K + 3 and K <= 6 runs the
  * fused step in its x-streaming form (a warp walks one ket along x with a halo only in y);
@@ -77,12 +79,15 @@ int lm_ctx_stream(lm_ctx *ctx, void **stream);
 #define LM_OPT_STREAM 2
 /* LM_OPT_KPM (default 1): the recurrences of lm_kpm_moments and lm_cheb_apply run in
  * double-float arithmetic (pairs of FP32 values, about 48 significant bits) on the FP32 pipe;
- * 0 selects FP64.  KPM moments agree to about 1e-15 mu_0. */
+ * 0 selects FP64.  KPM moments agree to about 1e-15 mu_0.  lm_cheb_apply keeps columns that fit in
+ * shared memory on chip through the whole series. */
 #define LM_OPT_KPM 3
 /* LM_OPT_RESIDENT (default 1): in a ComplexF32 batch's fused pass, lattices of up to 4608
  * sites (one CTA; smaller ones several kets per CTA) or 9216 sites (a cluster of two CTAs)
  * keep a whole ket on chip for all K orders (K <= 40); 0 runs them in the region form.  Both
- * give bit-identical results.  Takes effect at the next lm_batch_update. */
+ * give bit-identical results.  Takes effect at the next lm_batch_update.  Also the form of a single
+ * lattice's ComplexF32 step where the streaming form does not apply, and of the ComplexF32 adjoint's
+ * recurrences (0: the region form, and a launch per order). */
 #define LM_OPT_RESIDENT 4
 int lm_ctx_set_option(lm_ctx *ctx, int option, int value);
 /* Number of fused steps that ran in the x-streaming form on this context so far. */
