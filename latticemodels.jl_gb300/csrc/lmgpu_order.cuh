@@ -158,16 +158,6 @@ __device__ __forceinline__ Nbr neighbours(const Geom& g, int64_t s) {
     return n;
 }
 
-// x / 2.  FP64 by the exponent, beside the FP64 pipe that bounds those kernels; zeros, subnormals, infinities
-// and NaN by a product.
-__device__ __forceinline__ float halved(float x) { return 0.5f * x; }
-__device__ __forceinline__ double halved(double x) {
-    const int hi = __double2hiint(x), ex = hi & 0x7ff00000;
-    if (ex <= 0x00100000 || ex == 0x7ff00000) return 0.5 * x;
-    return __hiloint2double(hi - 0x00100000, __double2loint(x));
-}
-
-
 // ------------------------------------------------------------------------------------------
 // One order of the Chebyshev recurrence for exp(-i H dt), H~ = (H - b)/a:
 //   FIRST: T1 = H~ T0            -> tq;   y  = c0 T0 + c1 T1 (+ g0 T0 + g1 T1 in FP32, see ChebLo)
@@ -190,7 +180,7 @@ __device__ __forceinline__ void cheb_epilogue(typename CT<R>::V acc, typename CT
     typedef typename CT<R>::V V;
     if (MODE == CHEB_FIRST) {
         // T1 = (sum)/2 exactly, y = c0 T0 + c1 T1 with c1 = -i s (or +i s when conj)
-        const V t1 = CT<R>::make(halved(acc.x), halved(acc.y));
+        const V t1 = CT<R>::make(acc.x * R(0.5), acc.y * R(0.5));
         tq[i] = t1;
         V yy;
         if (sizeof(R) == sizeof(float)) {
