@@ -99,3 +99,10 @@ def test_real_series_doublefloat(lm, Lx, Ly, field, per, M, precision):
         ctx.set_kpm_doublefloat(True)
     assert rel(out[0], out[2]) <= (1e-12 if precision == "c64" else 1e-7)
     assert np.abs(out[1] - out[3]).max() <= 1e-13 * np.abs(out[3][:, 0]).max()
+
+
+@pytest.mark.parametrize("Lx,Ly,per,M", [(24, 130, {"axis1": True, "axis2": True}, 200), (16, 300, {"axis2": True}, 200),
+                                         (24, 300, None, 201), (5, 259, {"axis2": True}, 199)])
+def test_doublefloat_chunks_of_rows(lm, Lx, Ly, per, M):
+    """Blocks that hold a part of a column's rows (chunks of 44, 100, 50 and 87 here, the last ones shorter)."""
+    test_real_series_doublefloat(lm, Lx, Ly, "landau", per, M, "c64")
