@@ -991,6 +991,9 @@ int lm_solver_update(lm_solver* s, lm_ham* h, double dt, int force) {
     s->dt = dt;
     s->valid = 1;
     s->has_onsite = h->d_onsite != nullptr;
+    s->x_real = ham_x_real(h);
+    s->uniform_columns = ham_uniform_columns(h);
+    s->t1 = h->t1;
     return LM_OK;
 }
 
@@ -1107,8 +1110,8 @@ static int cheb_apply(lm_solver* s, const Geom& g, int precision, int site_fast,
     }
     if (ctx->fused && site_fast && !conj && fused_supported(precision, K) && fused_supported_geom(g)) {
         // whole series in one temporally blocked pass; result lands in A
-        const bool xr = ham_x_real(s->ham);
-        const int mode = ham_uniform_columns(s->ham) ? 2 : (xr ? 1 : 0);
+        const bool xr = s->x_real;
+        const int mode = s->uniform_columns ? 2 : (xr ? 1 : 0);
         const float4* spack = nullptr;
         if (ctx->fused_form == 1 && stream_supported(g, K, mode, S, A, ld)) {
             const int rc = ensure_stream_pack(s, g);
@@ -1154,7 +1157,7 @@ static int cheb_apply(lm_solver* s, const Geom& g, int precision, int site_fast,
         return set_err(ctx, LM_ERR_NOTSUP,
                        "lm_solver_step: a compensated state needs the x-streaming form (fused step enabled)");
     const ChebLo lo = cheb_lo(pr, pi, c0, coef(1).s, false);
-    const bool xr = ham_x_real(s->ham);
+    const bool xr = s->x_real;
     CUDA_TRY(ctx, launch_cheb_order(ctx, g, precision, site_fast, conj, CHEB_FIRST, hop2, diag2, S, A, Y, ld, m, c0, coef(1), pr, pi, lo, xr),
              "chebyshev order 1");
     for (int k = 2; k <= K; ++k) {
@@ -1180,9 +1183,8 @@ static int series_step(lm_solver* s, lm_state* st, int* done) {
     lm_ctx* ctx = s->ctx;
     *done = 0;
     if (!ctx->fused || st->precision != LM_C64 || s->K > kSeriesMaxK) return LM_OK;
-    const lm_ham* h = s->ham;
-    const Geom& g = h->lat->g;
-    const bool xr = ham_x_real(h);
+    const Geom& g = s->ham->lat->g;
+    const bool xr = s->x_real;
     const SeriesPlan plan = series_plan(ctx, g, xr, st->m, false);
     if (!plan.kt) return LM_OK;
     if (!xr && s->sgauge_version != s->tab_version) {
@@ -1190,7 +1192,8 @@ static int series_step(lm_solver* s, lm_state* st, int* done) {
             int rc = dalloc_pool(ctx, (void**)&s->d_sgauge, sizeof(double2) * 2 * (size_t)g.N, "gauge table");
             if (rc != LM_OK) return rc;
         }
-        CUDA_TRY(ctx, launch_gauge_tables(ctx, g, h->d_hop, h->d_onsite, h->t1, s->a, s->b, false, s->d_sgauge,
+        // from the solver's own 2H/a: x-hops of modulus 2 t1/a, y-hops already scaled
+        CUDA_TRY(ctx, launch_gauge_tables(ctx, g, s->d_hop2, nullptr, 2.0 * s->t1 / s->a, 2.0, 0.0, false, s->d_sgauge,
                                           s->d_sgauge + g.N, nullptr, nullptr, nullptr),
                  "gauge tables");
         s->sgauge_version = s->tab_version;
@@ -1210,7 +1213,7 @@ static int series_step(lm_solver* s, lm_state* st, int* done) {
     a.gauge = xr ? nullptr : s->d_sgauge;
     a.hy = xr ? s->d_hop2 + g.N : s->d_sgauge + g.N;
     a.diag = s->d_diag2;
-    a.alpha = 2.0 * h->t1 / s->a;
+    a.alpha = 2.0 * s->t1 / s->a;
     a.phase = make_double2(s->phase_re, s->phase_im);
     for (int k = 0; k <= s->K; ++k) a.cf[k] = s->coef[(size_t)k].s;
     cudaEvent_t t0 = nullptr, t1 = nullptr;

@@ -198,6 +198,9 @@ struct lm_solver {
     double2* d_sgauge = nullptr;
     uint64_t sgauge_version = ~0ull;
     int has_onsite = 0;
+    // of H at the update, like the tables (the lm_ham may hold another H by the time of a step)
+    int x_real = 0, uniform_columns = 0;  // ham_x_real, ham_uniform_columns
+    double t1 = 0.0;
     int fixed_bounds = 0;        // lm_solver_set_bounds: use [fix_emin, fix_emax] instead of Gershgorin
     double fix_emin = 0.0, fix_emax = 0.0;
     // general sparse Hamiltonian (lm_ell_*): set by lm_ell_solver_update, cleared by

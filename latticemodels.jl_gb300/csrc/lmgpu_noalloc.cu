@@ -84,7 +84,7 @@ extern "C" int lm_solver_step_noalloc(lm_solver* s, void* kets, int64_t n, int64
     const double c0 = s->coef[0].s;
     const ChebLo lo = cheb_lo(s->phase_re, s->phase_im, c0, s->coef[1].s, false);
     // T_k overwrites T_{k-2}: even orders land in the caller's block, odd orders in A
-    const bool xr = ham_x_real(s->ham);
+    const bool xr = s->x_real;
     rc = check_cuda(ctx, launch_cheb_order(ctx, g, precision, 1, 0, CHEB_FIRST, hop2, diag2, kets, A, Y, ld, m, c0,
                                            s->coef[1], s->phase_re, s->phase_im, lo, xr),
                     "lm_solver_step_noalloc: order 1");

@@ -33,7 +33,7 @@ struct SeriesPlan {
 };
 SeriesPlan series_plan(const lm_ctx* ctx, const Geom& g, bool x_real, int64_t M, bool df);
 
-// Gauge and stencil tables of H (raw hops and on-site term): gauge may be null when x_real.  Double
+// Gauge and stencil tables of H (hops of modulus t1 and on-site term; 2/a scales them): gauge may be null when x_real.  Double
 // tables (hy, diag) or double-float ones (hyd, diagd); null pointers are skipped.
 cudaError_t launch_gauge_tables(lm_ctx* ctx, const Geom& g, const double2* hop, const double* onsite, double t1, double a,
                                 double b, bool x_real, double2* gauge, double2* hy, double* diag, float4* hyd,
