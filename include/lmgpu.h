@@ -64,6 +64,13 @@ int lm_ctx_create(int device, lm_ctx **out);
 int lm_ctx_destroy(lm_ctx *ctx);
 const char *lm_last_error(const lm_ctx *ctx);
 int lm_ctx_synchronize(lm_ctx *ctx);
+/* Some steps run in one launch whose thread blocks wait for one another (lattices held by a pair
+ * of blocks, a general Hamiltonian's step on a small block).  Every such wait is bounded.  When one gives
+ * up, the state is unfinished, and lm_ctx_synchronize, downloads, readouts, norms, ring waits, KPM moments
+ * and the adjoint's loss and gradients return LM_ERR_TIMEOUT from then on.  The context stays in that
+ * condition: which of its states are sound is not known, so a program goes on with a new context.
+ * lm_ctx_raise_timeout puts a context into it from the host, for tests of a program's reaction. */
+int lm_ctx_raise_timeout(lm_ctx *ctx);
 /* The context's CUDA stream (cudaStream_t), for callers that order their own work or
  * CUDA events against the library's launches. */
 int lm_ctx_stream(lm_ctx *ctx, void **stream);

@@ -613,7 +613,7 @@ int lm_adjoint_seed(lm_adjoint* a, lm_state* psi, const double* target, lm_state
     double tot = 0.0;
     for (double v : part) tot += v;  // block order
     *loss = tot;
-    return LM_OK;
+    return wait_status(ctx);
 }
 
 int lm_adjoint_step(lm_adjoint* a, lm_solver* s, lm_ham* h, int component, int slot, lm_state* psi, lm_state* lam) {
@@ -748,7 +748,7 @@ int lm_adjoint_gradients(lm_adjoint* a, double* gV, double* gA) {
         for (size_t q = 0; q < nb * nc; ++q) tot += p[q];  // chunk-major block order
         gA[j] = tot;
     }
-    return LM_OK;
+    return wait_status(ctx);
 }
 
 int lm_solver_set_bounds(lm_solver* s, double emin, double emax) {

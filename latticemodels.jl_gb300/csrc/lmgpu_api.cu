@@ -302,6 +302,16 @@ int lm_ctx_synchronize(lm_ctx* ctx) {
     return wait_status(ctx);
 }
 
+int lm_ctx_raise_timeout(lm_ctx* ctx) {
+    if (!ctx) return LM_ERR_ARG;
+    cudaSetDevice(ctx->device);
+    const int rc = ensure_wait_words(ctx);
+    if (rc != LM_OK) return rc;
+    CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize");
+    *(volatile unsigned long long*)ctx->h_res_err = 1;
+    return LM_OK;
+}
+
 int lm_ctx_stream(lm_ctx* ctx, void** stream) {
     if (!ctx) return LM_ERR_ARG;
     CHECK_ARG(ctx, stream != nullptr, "lm_ctx_stream: null output");
@@ -871,7 +881,7 @@ int lm_state_norms(lm_state* s, double* out) {
         CUDA_TRY(ctx, launch_column_norms(ctx, s->precision, s->d_data, s->n, s->m, s->ld, ctx->d_red), "column norms");
     CUDA_TRY(ctx, cudaMemcpyAsync(out, ctx->d_red, sizeof(double) * (size_t)s->m, cudaMemcpyDeviceToHost, ctx->stream), "download norms");
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "sync");
-    return LM_OK;
+    return wait_status(ctx);
 }
 
 int lm_state_renormalize(lm_state* s, const double* target) {
@@ -1047,9 +1057,11 @@ namespace lmgpu {
 
 int ensure_wait_words(lm_ctx* ctx) {
     if (ctx->d_grid) return LM_OK;
-    CUDA_TRY(ctx, cudaHostAlloc((void**)&ctx->h_res_err, sizeof(unsigned long long), cudaHostAllocMapped), "status word");
-    *ctx->h_res_err = 0;
-    CUDA_TRY(ctx, cudaHostGetDevicePointer((void**)&ctx->d_res_err, ctx->h_res_err, 0), "status word");
+    if (!ctx->h_res_err) {
+        CUDA_TRY(ctx, cudaHostAlloc((void**)&ctx->h_res_err, sizeof(unsigned long long), cudaHostAllocMapped), "status word");
+        *ctx->h_res_err = 0;
+        CUDA_TRY(ctx, cudaHostGetDevicePointer((void**)&ctx->d_res_err, ctx->h_res_err, 0), "status word");
+    }
     CUDA_TRY(ctx, cudaMalloc((void**)&ctx->d_grid, 2 * sizeof(unsigned)), "barrier counters");
     CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_grid, 0, 2 * sizeof(unsigned), ctx->stream), "barrier counters");
     return LM_OK;
@@ -1322,7 +1334,7 @@ int lm_localdensity(lm_state* s, double* out) {
     CUDA_TRY(ctx, cudaMemcpyAsync(out, ctx->d_red, sizeof(double) * (size_t)s->n, cudaMemcpyDeviceToHost, ctx->stream),
              "download density");
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "sync");
-    return LM_OK;
+    return wait_status(ctx);
 }
 
 int lm_bond_currents(lm_ham* h, lm_state* s, double* out) {
@@ -1343,7 +1355,7 @@ int lm_bond_currents(lm_ham* h, lm_state* s, double* out) {
     CUDA_TRY(ctx, cudaMemcpyAsync(out, ctx->d_red, sizeof(double) * (size_t)nb, cudaMemcpyDeviceToHost, ctx->stream),
              "download currents");
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "sync");
-    return LM_OK;
+    return wait_status(ctx);
 }
 
 int lm_trace(lm_state* s, double* out) {
@@ -1358,7 +1370,7 @@ int lm_trace(lm_state* s, double* out) {
     CUDA_TRY(ctx, launch_sum(ctx, ctx->d_red, s->n, ctx->d_red + s->n), "sum kernel");
     CUDA_TRY(ctx, cudaMemcpyAsync(out, ctx->d_red + s->n, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream), "download trace");
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "sync");
-    return LM_OK;
+    return wait_status(ctx);
 }
 
 }  // extern "C"

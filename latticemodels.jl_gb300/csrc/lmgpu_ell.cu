@@ -1095,7 +1095,7 @@ int lm_ell_currents(lm_ell* h, lm_state* st, double* out) {
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, d_out, sizeof(double) * (size_t)h->nnz, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     cudaFree(d_out);
-    return check_cuda(ctx, e, "lm_ell_currents");
+    return e == cudaSuccess ? wait_status(ctx) : check_cuda(ctx, e, "lm_ell_currents");
 }
 
 int lm_ell_op_currents(lm_ell* h, lm_state* st, int ndof, const double* op, double* out) {
@@ -1114,7 +1114,7 @@ int lm_ell_op_currents(lm_ell* h, lm_state* st, int ndof, const double* op, doub
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, d_out, sizeof(double) * (size_t)h->nnz, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     cudaFree(d_out);
-    return check_cuda(ctx, e, "lm_ell_op_currents");
+    return e == cudaSuccess ? wait_status(ctx) : check_cuda(ctx, e, "lm_ell_op_currents");
 }
 
 }  // extern "C"

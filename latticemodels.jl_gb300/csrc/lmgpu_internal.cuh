@@ -369,7 +369,8 @@ bool ham_uniform_columns(const lm_ham* h);
 // hop of magnitude t_exact has no rounding error in the FP32 stencil tables.
 void plan_propagator(lm_solver* s, double emin, double emax, double dt, double t_exact = 0.0);
 // The context's timeout word and barrier counters, created on first use; the word's state as of the last
-// finished launch (LM_OK or LM_ERR_TIMEOUT).
+// finished launch (LM_OK or LM_ERR_TIMEOUT).  Every call that hands a value computed from device states to
+// the host ends with it, and a launch that would wait does not start once it is set.
 int ensure_wait_words(lm_ctx* ctx);
 int wait_status(lm_ctx* ctx);
 // lm_solver_step / destroy for a solver updated with an lm_ell Hamiltonian (lmgpu_ell.cu).

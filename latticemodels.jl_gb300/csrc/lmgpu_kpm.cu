@@ -719,6 +719,8 @@ int lm_kpm_moments(lm_ham* h, double emin, double emax, int nmom, const lm_state
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return fail(e, "lm_kpm_moments: download");
     release();
+    const int waited = vecs ? wait_status(ctx) : LM_OK;
+    if (waited != LM_OK) return waited;
     // assemble the moments column by column (sums over columns in column order)
     const double* d0 = hd.data();
     for (int64_t col = 0; col < (per_column ? M : 1); ++col) {

@@ -192,7 +192,7 @@ int lm_ring_wait(lm_ring* r, int64_t seq, double* out, const double** view, int6
     if (view) *view = h;
     if (n) *n = cnt;
     if (t) *t = r->t[(size_t)k];
-    return LM_OK;
+    return wait_status(r->ctx);
 }
 
 int lm_ring_head(const lm_ring* r, int64_t* head) {
