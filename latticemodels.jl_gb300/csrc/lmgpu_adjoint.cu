@@ -274,15 +274,6 @@ struct GradOrders {
     const float2* b[kResMaxK + 1];  // beta_1 .. beta_K
 };
 
-// (double)x without the FP64 pipe's conversion
-__device__ __forceinline__ double widen(float x) {
-    const unsigned u = __float_as_uint(x);
-    const unsigned e = u & 0x7f800000u;
-    if (e == 0x7f800000u || (e == 0u && (u << 1) != 0u)) return (double)x;  // infinities, NaN, denormals
-    if (e == 0u) return __hiloint2double((int)u, 0);
-    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))), (int)(u << 29));
-}
-
 __global__ void __launch_bounds__(256, 3) adj_sums_kernel(Geom g, const __grid_constant__ GradOrders ord,
                                                           const double2* __restrict__ dhop, int64_t ld, int64_t M,
                                                           int64_t mchunk, double ph_re, double ph_im, double inv_a,

@@ -413,14 +413,18 @@ __device__ __forceinline__ void bond_write(const Geom& g, const double2* __restr
 // Ket blocks: P[j,s] = sum_k w_k psi_jk conj(psi_sk).  A block owns 32 consecutive sites (one
 // per lane); its 8 warps split the kets; partial sums are added in warp order.
 // XR (real x-hops): J of an x-bond needs the imaginary part only, two products fewer of eight.
+// With `part` a block takes the kets of slice blockIdx.y and writes its sums to planes
+// [slice][sum][site] instead, (re unless XR, im) of the x-bond and (re, im) of the y-bond;
+// readout_slices_kernel adds the slices in order and writes the bonds.
 template <typename R, bool WEIGHTED, bool XR>
 __global__ void __launch_bounds__(32 * kReadWarps) bond_currents_kets_kernel(
     Geom g, const double2* __restrict__ hop, const typename CT<R>::V* __restrict__ x, int64_t m, int64_t ld,
-    const double* __restrict__ w, double* __restrict__ out) {
+    const double* __restrict__ w, double* __restrict__ out, int64_t kslice, double* __restrict__ part) {
     typedef typename CT<R>::V V;
     __shared__ double red[kReadWarps][4][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t s = (int64_t)blockIdx.x * 32 + lane;
+    const int64_t k0 = (int64_t)blockIdx.y * kslice, k1 = k0 + kslice < m ? k0 + kslice : m;
     Nbr nb;
     Acc<R> a[4];  // (re, im) of the +x bond, then of the +y bond
     double aw[4] = {0.0, 0.0, 0.0, 0.0};
@@ -430,15 +434,16 @@ __global__ void __launch_bounds__(32 * kReadWarps) bond_currents_kets_kernel(
         const int64_t jx = nb.hxp ? nb.xp : s, jy = nb.hyp ? nb.yp : s;
         // unrolled so that four kets' loads are in flight per thread; the sums keep their order
 #pragma unroll 4
-        for (int64_t k = warp; k < m; k += kReadWarps) {
+        for (int64_t k = k0 + warp; k < k1; k += kReadWarps) {
             const V b = x[k * ld + s];
             const V cx = x[k * ld + jx], cy = x[k * ld + jy];  // c * conj(b)
             if (WEIGHTED) {
-                const double wk = w[k];
-                if (!XR) aw[0] += wk * ((double)cx.x * (double)b.x + (double)cx.y * (double)b.y);
-                aw[1] += wk * ((double)cx.y * (double)b.x - (double)cx.x * (double)b.y);
-                aw[2] += wk * ((double)cy.x * (double)b.x + (double)cy.y * (double)b.y);
-                aw[3] += wk * ((double)cy.y * (double)b.x - (double)cy.x * (double)b.y);
+                const double wk = w[k], br = widen(b.x), bi = widen(b.y);
+                const double xr = widen(cx.x), xi = widen(cx.y), yr = widen(cy.x), yi = widen(cy.y);
+                if (!XR) aw[0] += wk * (xr * br + xi * bi);
+                aw[1] += wk * (xi * br - xr * bi);
+                aw[2] += wk * (yr * br + yi * bi);
+                aw[3] += wk * (yi * br - yr * bi);
             } else {
                 if (!XR) a[0].add_prod(cx.x, b.x);
                 if (!XR) a[0].add_prod(cx.y, b.y);
@@ -461,6 +466,12 @@ __global__ void __launch_bounds__(32 * kReadWarps) bond_currents_kets_kernel(
             double t = 0.0;
             for (int r = 0; r < kReadWarps; ++r) t += red[r][q][lane];
             v[q] = t;
+        }
+        if (part) {
+            constexpr int Q0 = XR ? 1 : 0;
+#pragma unroll
+            for (int q = Q0; q < 4; ++q) part[((int64_t)blockIdx.y * (4 - Q0) + q - Q0) * g.N + s] = v[q];
+            return;
         }
         if (nb.hxp) bond_write(g, hop, s, 0, nb, v[0], v[1], out);
         if (nb.hyp) bond_write(g, hop, s, 1, nb, v[2], v[3], out);
@@ -640,9 +651,47 @@ static void launch_currents_kets(lm_ctx* ctx, const Geom& g, const double2* hop,
     typedef typename CT<R>::V V;
     const unsigned blocks = (unsigned)((g.N + 31) / 32);
     const int thr = 32 * kReadWarps;
-    if (w) bond_currents_kets_kernel<R, true, XR><<<blocks, thr, 0, ctx->stream>>>(g, hop, (const V*)x, m, ld, w, out);
-    else bond_currents_kets_kernel<R, false, XR><<<blocks, thr, 0, ctx->stream>>>(g, hop, (const V*)x, m, ld, w, out);
+    if (w) bond_currents_kets_kernel<R, true, XR><<<blocks, thr, 0, ctx->stream>>>(g, hop, (const V*)x, m, ld, w, out, m, nullptr);
+    else bond_currents_kets_kernel<R, false, XR><<<blocks, thr, 0, ctx->stream>>>(g, hop, (const V*)x, m, ld, w, out, m, nullptr);
     ctx->launches++;
+}
+
+// The same with weights over S slices of the kets.  Bound by the FP64 pipe (12 multiplications and additions
+// per site and ket with complex x-hops; FP32 amplitudes are widened by integer operations, which left 12 of
+// 18), so a lattice whose blocks leave SMs idle is split further.  Complex x-hops, readout and download:
+// 48 x 48 sites, 1024 kets 71 us (in one slice, converting on the FP64 pipe 173 us; four sites per
+// lane in slices 92 us), 97 x 76, 650 kets 124 us (222; 173), 256 x 256, 2048 kets 2.77 ms (4.54; 4.74).
+// cudaErrorMemoryAllocation where the planes do not fit.
+template <bool XR>
+static cudaError_t launch_currents_weighted(lm_ctx* ctx, const Geom& g, const double2* hop, const float2* x, int64_t m,
+                                            int64_t ld, const double* w, double* out, int S) {
+    cudaError_t e = ensure_readout_part(ctx, (size_t)S * (XR ? 3 : 4) * (size_t)g.N);
+    if (e != cudaSuccess) return e;
+    bond_currents_kets_kernel<float, true, XR><<<dim3((unsigned)((g.N + 31) / 32), (unsigned)S), 32 * kReadWarps, 0,
+                                                 ctx->stream>>>(g, hop, x, m, ld, w, out, (m + S - 1) / S, ctx->d_ld_part);
+    readout_slices_kernel<XR, false><<<(unsigned)((g.N + 127) / 128), 128, 0, ctx->stream>>>(g, hop, ctx->d_ld_part, S, nullptr,
+                                                                                            out);
+    ctx->launches += 2;
+    return cudaGetLastError();
+}
+
+// Slices of the weighted sums: as readout_slices, but a block on each SM almost fills the FP64 pipe already, so
+// what counts is the share of the SM with the most blocks (a lone one at 1.5 times its work).  S = 1 where
+// that is within 2 % per slice of the best: few kets, or a lattice that fills the device.
+static int weighted_slices(const lm_ctx* ctx, const Geom& g, int64_t m) {
+    if (ctx->ld_slices_override > 0) return ctx->ld_slices_override;
+    const int64_t chunks = (g.N + 31) / 32, sms = std::max(ctx->sm_count, 1);
+    const int smax = (int)std::max<int64_t>(1, std::min<int64_t>(8, m / 64));
+    int best = 1;
+    double tbest = 1e300;
+    for (int S = 1; S <= smax; ++S) {
+        const double t = std::max((double)((chunks * S + sms - 1) / sms), 1.5) / S * (1.0 + 0.02 * S);
+        if (t < tbest * (1.0 - 1e-9)) {
+            tbest = t;
+            best = S;
+        }
+    }
+    return best;
 }
 
 // Bond currents of a density matrix, with rho also its local density.
@@ -668,6 +717,11 @@ cudaError_t launch_bond_currents(lm_ctx* ctx, const Geom& g, int precision, int 
             const cudaError_t e = launch_readout_c32(ctx, g, hop, xr, (const float2*)x, m, ld, nullptr, out);
             if (e != cudaErrorMemoryAllocation) return e;
             (void)cudaGetLastError();  // no scratch for the partial sums: one block per 32 sites and all kets
+        } else if (const int S = weighted_slices(ctx, g, m); S > 1) {
+            const cudaError_t e = xr ? launch_currents_weighted<true>(ctx, g, hop, (const float2*)x, m, ld, w, out, S)
+                                     : launch_currents_weighted<false>(ctx, g, hop, (const float2*)x, m, ld, w, out, S);
+            if (e != cudaErrorMemoryAllocation) return e;
+            (void)cudaGetLastError();
         }
         if (xr) launch_currents_kets<float, true>(ctx, g, hop, x, m, ld, w, out);
         else launch_currents_kets<float, false>(ctx, g, hop, x, m, ld, w, out);

@@ -43,6 +43,16 @@ template <> struct Acc<float> {
     __device__ __forceinline__ double get() const { return (double)hi + (double)lo; }
 };
 
+// (double)x without the FP64 pipe's conversion
+__device__ __forceinline__ double widen(float x) {
+    const unsigned u = __float_as_uint(x);
+    const unsigned e = u & 0x7f800000u;
+    if (e == 0x7f800000u || (e == 0u && (u << 1) != 0u)) return (double)x;  // infinities, NaN, denormals
+    if (e == 0u) return __hiloint2double((int)u, 0);
+    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))), (int)(u << 29));
+}
+__device__ __forceinline__ double widen(double x) { return x; }
+
 // d = a * b + c on both halves of a float pair in one instruction (two round-to-nearest FMAs:
 // the same results as two fmaf calls).
 __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
