@@ -494,6 +494,17 @@ __global__ void bond_currents_dm_kernel(Geom g, const double2* __restrict__ hop,
     }
 }
 
+// The readouts of a site from its sums v: the density (DENS), the x-bond and the y-bond.
+template <bool XR, bool DENS, int NQ>
+__device__ __forceinline__ void readout_write(const Geom& g, const double2* __restrict__ hop, int64_t s,
+                                              const double (&v)[NQ], double* __restrict__ rho, double* __restrict__ out) {
+    constexpr int QX = DENS ? 1 : 0, QY = QX + (XR ? 1 : 2);
+    if (DENS) rho[s] = v[0];
+    const Nbr nb = neighbours(g, s);
+    if (nb.hxp) bond_write(g, hop, s, 0, nb, XR ? 0.0 : v[QX], v[QY - 1], out);
+    if (nb.hyp) bond_write(g, hop, s, 1, nb, v[QY], v[QY + 1], out);
+}
+
 // Bond currents, and with DENS the local density, of c32 ket blocks (no weights) in one read of the kets.
 // A lane owns VEC consecutive sites of one lattice column: 4 where Ly % 4 == 0 and ld is even, so
 // that a warp reads 1 KB of a ket per load (256-byte pieces from kets 512 KB apart hold DRAM to
@@ -501,7 +512,9 @@ __global__ void bond_currents_dm_kernel(Geom g, const double2* __restrict__ hop,
 // +y neighbours the lane's own next sites and, for the last, one 8-byte load.  A block's 8 warps split
 // the kets of slice blockIdx.y and write the sums of a site to planes of `part`, [slice][sum][site]:
 // the density (DENS), (re, im) of conj(b) c on the x-bond (im only when XR: real x-hops need no
-// more) and on the y-bond; readout_slices_kernel adds the slices in order and writes the readouts.
+// more) and on the y-bond; readout_slices_kernel adds the slices in order and writes the readouts.  A single
+// slice (`out` not null) writes them itself, with the same values: one launch for a block of few kets (97 x 75
+// sites, 8 kets, with the download: 14 us, 19 us in two).
 //
 // What bounds it: the products, 10 FP32 operations each (exact product, TwoSum; the sums carry 48
 // bits), two at a time on packed pairs.  256 x 256 sites, 2048 kets, real x-hops: 6 products for the
@@ -511,7 +524,8 @@ __global__ void bond_currents_dm_kernel(Geom g, const double2* __restrict__ hop,
 // block per 32 sites left SMs idle.
 template <int VEC, bool XR, bool DENS>
 __global__ void __launch_bounds__(32 * kReadWarps, VEC == 4 ? 3 : 4) readout_kets_kernel(
-    Geom g, const float2* __restrict__ x, int64_t m, int64_t ld, int64_t kslice, double* __restrict__ part) {
+    Geom g, const float2* __restrict__ x, int64_t m, int64_t ld, int64_t kslice, double* __restrict__ part,
+    const double2* __restrict__ hop, double* __restrict__ rho, double* __restrict__ out) {
     constexpr int NQ = (DENS ? 1 : 0) + (XR ? 1 : 2) + 2, QX = DENS ? 1 : 0, QY = QX + (XR ? 1 : 2);
     __shared__ double red[kReadWarps][32 * VEC];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -560,7 +574,9 @@ __global__ void __launch_bounds__(32 * kReadWarps, VEC == 4 ? 3 : 4) readout_ket
             }
         }
     }
-    double* pl = part + (int64_t)blockIdx.y * NQ * g.N;
+    const int64_t s = (int64_t)blockIdx.x * (32 * VEC) + threadIdx.x;
+    const bool own = threadIdx.x < 32 * VEC && s < g.N;
+    double tot[NQ];
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
         if (q > 0) __syncthreads();
@@ -571,21 +587,26 @@ __global__ void __launch_bounds__(32 * kReadWarps, VEC == 4 ? 3 : 4) readout_ket
             red[warp][lane * VEC + j] = (DENS && q == 0) || (XR && q < QY) ? re + im : q == QX || q == QY ? re : im;
         }
         __syncthreads();
-        const int64_t s = (int64_t)blockIdx.x * (32 * VEC) + threadIdx.x;
-        if (threadIdx.x < 32 * VEC && s < g.N) {
-            double t = 0.0;
+        tot[q] = 0.0;
+        if (own) {
 #pragma unroll
-            for (int r = 0; r < kReadWarps; ++r) t += red[r][threadIdx.x];
-            pl[(int64_t)q * g.N + s] = t;
+            for (int r = 0; r < kReadWarps; ++r) tot[q] += red[r][threadIdx.x];
         }
     }
+    if (!own) return;
+    if (out) {
+        readout_write<XR, DENS>(g, hop, s, tot, rho, out);
+        return;
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) part[((int64_t)blockIdx.y * NQ + q) * g.N + s] = tot[q];
 }
 
 // Adds the S slice planes of readout_kets_kernel in slice order and writes the bonds and the density.
 template <bool XR, bool DENS>
 __global__ void readout_slices_kernel(Geom g, const double2* __restrict__ hop, const double* __restrict__ part, int S,
                                       double* __restrict__ rho, double* __restrict__ out) {
-    constexpr int NQ = (DENS ? 1 : 0) + (XR ? 1 : 2) + 2, QX = DENS ? 1 : 0, QY = QX + (XR ? 1 : 2);
+    constexpr int NQ = (DENS ? 1 : 0) + (XR ? 1 : 2) + 2;
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= g.N) return;
     double v[NQ];
@@ -595,10 +616,7 @@ __global__ void readout_slices_kernel(Geom g, const double2* __restrict__ hop, c
     for (int y = 1; y < S; ++y)  // the loads of a few slices are under way together
 #pragma unroll
         for (int q = 0; q < NQ; ++q) v[q] += part[((int64_t)y * NQ + q) * g.N + s];
-    if (DENS) rho[s] = v[0];
-    const Nbr nb = neighbours(g, s);
-    if (nb.hxp) bond_write(g, hop, s, 0, nb, XR ? 0.0 : v[QX], v[QY - 1], out);
-    if (nb.hyp) bond_write(g, hop, s, 1, nb, v[QY], v[QY + 1], out);
+    readout_write<XR, DENS>(g, hop, s, v, rho, out);
 }
 
 template <int VEC, bool XR, bool DENS>
@@ -615,13 +633,21 @@ static cudaError_t launch_readout_t(lm_ctx* ctx, const Geom& g, const double2* h
         }
         return b;
     }();
-    int S = readout_slices(chunks, m, (int64_t)per_sm * ctx->sm_count);
+    // with a site per lane slices pay from 256 kets (25 x 25 sites, 200 kets 16 against 20 us; 300 kets 20 us either
+    // way; 150 x 151, 200 kets 34 against 44 us)
+    int S = VEC == 1 && m < 256 ? 1 : readout_slices(chunks, m, (int64_t)per_sm * ctx->sm_count);
     if (ctx->ld_slices_override > 0) S = ctx->ld_slices_override;
+    if (S == 1) {
+        readout_kets_kernel<VEC, XR, DENS><<<(unsigned)chunks, 32 * kReadWarps, 0, ctx->stream>>>(g, x, m, ld, m, nullptr, hop,
+                                                                                                  rho, out);
+        ctx->launches++;
+        return cudaGetLastError();
+    }
     cudaError_t e = ensure_readout_part(ctx, (size_t)S * NQ * (size_t)g.N);
     if (e != cudaSuccess) return e;
     const int64_t kslice = (m + S - 1) / S;
     readout_kets_kernel<VEC, XR, DENS><<<dim3((unsigned)chunks, (unsigned)S), 32 * kReadWarps, 0, ctx->stream>>>(
-        g, x, m, ld, kslice, ctx->d_ld_part);
+        g, x, m, ld, kslice, ctx->d_ld_part, nullptr, nullptr, nullptr);
     readout_slices_kernel<XR, DENS><<<(unsigned)((g.N + 127) / 128), 128, 0, ctx->stream>>>(g, hop, ctx->d_ld_part, S, rho,
                                                                                            out);
     ctx->launches += 2;
