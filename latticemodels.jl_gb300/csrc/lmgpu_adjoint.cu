@@ -448,6 +448,7 @@ struct lm_adjoint {
     int precision = LM_C64;
     size_t elem = 16;
     int K = 0;
+    int lean_K = 1 << 30;  // from this order on the blocks of the lattice-resident form did not fit
     std::vector<void*> T;  // T_0 .. T_{K-1} (T_0 aliases psi during a step)
     std::vector<void*> B;  // beta_k by order (lattice-resident form) or three rotating blocks
     double* d_gV = nullptr;     // per ket chunk, one partial per site (nchunk x n)
@@ -500,6 +501,11 @@ static int adj_ensure_stack(lm_adjoint* a, int K, bool all_beta) {
     if (all_beta) {
         int rc = adj_alloc(a->ctx, (void**)&a->d_sums, sizeof(double) * (size_t)K * (size_t)a->nchunk * (size_t)(a->n + a->nblk));
         if (rc != LM_OK) return rc;
+        // the other form takes K - 3 blocks less: what a program still allocates (the scratch of its states,
+        // a checkpoint) must not fail for them
+        size_t free_b = 0, total = 0;
+        if (cudaMemGetInfo(&free_b, &total) == cudaSuccess && free_b < 4 * bytes)
+            return set_err(a->ctx, LM_ERR_OOM, "lm_adjoint: no room beside the blocks of all orders");
     }
     a->K = K;
     return LM_OK;
@@ -625,9 +631,14 @@ int lm_adjoint_step(lm_adjoint* a, lm_solver* s, lm_ham* h, int component, int s
     // over all of them.  The recurrences' operation order is that of the per-order kernels.
     ResidentInst ri{};
     int cl = 0;
-    const bool resident = !f64 && ctx->fused && K >= 3 && psi->ld == lam->ld &&
-                          resident_single_plan(ctx, g, K, a->m, psi->ld, psi->d_data, lam->d_data, ri, &cl);
+    bool resident = !f64 && ctx->fused && K >= 3 && K < a->lean_K && psi->ld == lam->ld &&
+                    resident_single_plan(ctx, g, K, a->m, psi->ld, psi->d_data, lam->d_data, ri, &cl);
     int rc = adj_ensure_stack(a, K, resident);
+    if (rc == LM_ERR_OOM && resident) {  // K + 2 blocks instead of 2K - 1, and the same bits
+        a->lean_K = K;
+        resident = false;
+        rc = adj_ensure_stack(a, K, false);
+    }
     if (rc != LM_OK) return rc;
     const void* hop2 = f64 ? (const void*)s->d_hop2 : (const void*)s->d_hop2f;
     const void* diag2 = f64 ? (const void*)s->d_diag2 : (const void*)s->d_diag2f;
