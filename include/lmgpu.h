@@ -62,6 +62,10 @@ int lm_version(void);
  * the reference runs on the CPU (src/evolution.jl:183-196 holds no device state). */
 int lm_ctx_create(int device, lm_ctx **out);
 int lm_ctx_destroy(lm_ctx *ctx);
+/* A context keeps the memory of destroyed objects for the next ones, up to a 32nd of the device's.  Its own
+ * allocations give it back when memory runs short; lm_ctx_trim gives it back for other programs' or
+ * other libraries' use (and waits for the context's stream). */
+int lm_ctx_trim(lm_ctx *ctx);
 const char *lm_last_error(const lm_ctx *ctx);
 int lm_ctx_synchronize(lm_ctx *ctx);
 /* Some steps run in one launch whose thread blocks wait for one another (lattices held by a pair

@@ -73,12 +73,11 @@ void bessel_j_all(double x, int kmax, std::vector<double>& out) {
 namespace lmgpu {
 cudaError_t dev_alloc(lm_ctx* ctx, void** p, size_t bytes) {
     *p = nullptr;
-    if (!ctx->pool) return cudaMalloc(p, bytes);
+    if (!ctx->pool) return dev_malloc(ctx, p, bytes);
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->stream);
-    if (e == cudaErrorMemoryAllocation) {  // what the pool keeps in pieces may be missing as a whole
+    if (e == cudaErrorMemoryAllocation) {  // what is kept in pieces may be missing as a whole
         cudaGetLastError();
-        cudaStreamSynchronize(ctx->stream);
-        cudaMemPoolTrimTo(ctx->pool, 0);
+        release_kept(ctx);
         e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->stream);
     }
     if (e != cudaSuccess) *p = nullptr;
@@ -91,10 +90,73 @@ void dev_free(lm_ctx* ctx, void* p) {
     else cudaFree(p);
 }
 
-// A pool of the context's own.  Up to a 32nd of the device's memory (9 GB) stays with it across
-// synchronisations instead of going back to the driver: allocating and freeing the buffers of a
-// 265 MB state cost 1.1 ms per Evolution.  lm_ctx_destroy gives everything back.
+cudaError_t dev_malloc(lm_ctx* ctx, void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        release_kept(ctx);
+        e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) *p = nullptr;
+    return e;
+}
+
+cudaError_t state_mem_alloc(lm_ctx* ctx, void** p, size_t bytes) {
+    {
+        std::lock_guard<std::mutex> lock(ctx->kept_mutex);
+        for (auto it = ctx->kept.begin(); it != ctx->kept.end(); ++it)
+            if (it->first == bytes) {
+                *p = it->second;
+                ctx->kept_bytes -= bytes;
+                ctx->kept.erase(it);
+                return cudaSuccess;
+            }
+    }
+    return dev_malloc(ctx, p, bytes);
+}
+
+void state_mem_free(lm_ctx* ctx, void* p, size_t bytes) {
+    if (!p) return;
+    std::vector<void*> drop;  // the oldest ones beyond the limit
+    {
+        std::lock_guard<std::mutex> lock(ctx->kept_mutex);
+        ctx->kept.emplace_back(bytes, p);
+        ctx->kept_bytes += bytes;
+        while (ctx->kept_bytes > ctx->kept_max) {
+            drop.push_back(ctx->kept.front().second);
+            ctx->kept_bytes -= ctx->kept.front().first;
+            ctx->kept.pop_front();
+        }
+    }
+    if (drop.empty()) return;
+    cudaStreamSynchronize(ctx->stream);
+    for (void* q : drop) cudaFree(q);
+}
+
+void release_kept(lm_ctx* ctx) {
+    std::list<std::pair<size_t, void*>> drop;
+    {
+        std::lock_guard<std::mutex> lock(ctx->kept_mutex);
+        drop.swap(ctx->kept);
+        ctx->kept_bytes = 0;
+    }
+    cudaStreamSynchronize(ctx->stream);
+    for (auto& b : drop) cudaFree(b.second);
+    if (ctx->pool) cudaMemPoolTrimTo(ctx->pool, 0);
+}
+
+// A pool of the context's own for tables and temporaries, and the limit of the states' buffers kept for
+// reuse: up to a 64th of the device's memory each (4.4 GB) stays with the context instead of going back to
+// the driver, as allocating and freeing the buffers of a 265 MB state cost 1.1 ms per Evolution.  An
+// allocation of the library that fails gives it back and tries again; lm_ctx_trim and lm_ctx_destroy give
+// it back too, and the driver takes what the pool keeps for other allocations of the process by itself.
 static void create_pool(lm_ctx* ctx) {
+    size_t free_b = 0, total = 0;
+    if (cudaMemGetInfo(&free_b, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    ctx->kept_max = total / 64;
     int ok = 0;
     if (cudaDeviceGetAttribute(&ok, cudaDevAttrMemoryPoolsSupported, ctx->device) != cudaSuccess || !ok) {
         cudaGetLastError();
@@ -105,21 +167,21 @@ static void create_pool(lm_ctx* ctx) {
     props.handleTypes = cudaMemHandleTypeNone;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = ctx->device;
-    size_t free_b = 0, total = 0;
-    if (cudaMemPoolCreate(&ctx->pool, &props) != cudaSuccess || cudaMemGetInfo(&free_b, &total) != cudaSuccess) {
+    if (cudaMemPoolCreate(&ctx->pool, &props) != cudaSuccess) {
         cudaGetLastError();
         ctx->pool = nullptr;
         return;
     }
-    unsigned long long keep = total / 32;
+    unsigned long long keep = total / 64;
     cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
 }
 }  // namespace lmgpu
 
-static int dalloc_pool(lm_ctx* ctx, void** p, size_t bytes, const char* what) {
+static int dalloc_with(cudaError_t (*alloc)(lm_ctx*, void**, size_t), lm_ctx* ctx, void** p, size_t bytes,
+                       const char* what) {
     *p = nullptr;
     if (bytes == 0) return LM_OK;
-    cudaError_t e = dev_alloc(ctx, p, bytes);
+    cudaError_t e = alloc(ctx, p, bytes);
     if (e != cudaSuccess) {
         *p = nullptr;
         cudaGetLastError();
@@ -128,18 +190,14 @@ static int dalloc_pool(lm_ctx* ctx, void** p, size_t bytes, const char* what) {
     }
     return LM_OK;
 }
-
+static int dalloc_pool(lm_ctx* ctx, void** p, size_t bytes, const char* what) {
+    return dalloc_with(dev_alloc, ctx, p, bytes, what);
+}
 static int dalloc(lm_ctx* ctx, void** p, size_t bytes, const char* what) {
-    *p = nullptr;
-    if (bytes == 0) return LM_OK;
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaSuccess) {
-        *p = nullptr;
-        cudaGetLastError();
-        return set_err(ctx, e == cudaErrorMemoryAllocation ? LM_ERR_OOM : LM_ERR_CUDA,
-                       std::string("cudaMalloc(") + what + "): " + cudaGetErrorString(e));
-    }
-    return LM_OK;
+    return dalloc_with(dev_malloc, ctx, p, bytes, what);
+}
+static int dalloc_state(lm_ctx* ctx, void** p, size_t bytes, const char* what) {
+    return dalloc_with(state_mem_alloc, ctx, p, bytes, what);
 }
 
 namespace lmgpu {
@@ -152,7 +210,7 @@ int ensure_accumulator(lm_state* s) {
 // stepped only through a panelled batch never needs it.
 int ensure_scratch(lm_state* s) {
     if (s->d_a) return LM_OK;
-    return dalloc_pool(s->ctx, &s->d_a, s->elem * (size_t)s->ld * (size_t)s->m, "recurrence scratch");
+    return dalloc_state(s->ctx, &s->d_a, s->elem * (size_t)s->ld * (size_t)s->m, "recurrence scratch");
 }
 }  // namespace lmgpu
 
@@ -288,6 +346,7 @@ int lm_ctx_destroy(lm_ctx* ctx) {
     if (ctx->d_grid) cudaFree(ctx->d_grid);
     if (ctx->h_res_err) cudaFreeHost(ctx->h_res_err);
     for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
+    release_kept(ctx);
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -300,6 +359,13 @@ int lm_ctx_synchronize(lm_ctx* ctx) {
     if (!ctx) return LM_ERR_ARG;
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize");
     return wait_status(ctx);
+}
+
+int lm_ctx_trim(lm_ctx* ctx) {
+    if (!ctx) return LM_ERR_ARG;
+    cudaSetDevice(ctx->device);
+    release_kept(ctx);
+    return LM_OK;
 }
 
 int lm_ctx_raise_timeout(lm_ctx* ctx) {
@@ -707,7 +773,7 @@ static int state_alloc(lm_ctx* ctx, int64_t n, int64_t m, int kind, int precisio
     s->elem = precision == LM_C64 ? 16 : 8;
     cudaSetDevice(ctx->device);
     const size_t bytes = s->elem * (size_t)n * (size_t)m;
-    int rc = dalloc_pool(ctx, &s->d_data, bytes, "state");
+    int rc = dalloc_state(ctx, &s->d_data, bytes, "state");
     // the recurrence scratch and the accumulator are allocated on first use
     if (rc != LM_OK) {
         delete s;
@@ -752,8 +818,9 @@ int lm_state_destroy(lm_state* s) {
     cudaSetDevice(s->ctx->device);
     // a buffer that was handed out may be in use on any stream; the others only on the context's
     if (s->exposed) cudaDeviceSynchronize();
-    dev_free(s->ctx, s->d_data);
-    dev_free(s->ctx, s->d_a);
+    const size_t bytes = s->elem * (size_t)s->ld * (size_t)s->m;
+    state_mem_free(s->ctx, s->d_data, bytes);
+    state_mem_free(s->ctx, s->d_a, bytes);
     dev_free(s->ctx, s->d_y);
     dev_free(s->ctx, s->d_lo);
     if (s->d_w) {
@@ -1062,7 +1129,7 @@ int ensure_wait_words(lm_ctx* ctx) {
         *ctx->h_res_err = 0;
         CUDA_TRY(ctx, cudaHostGetDevicePointer((void**)&ctx->d_res_err, ctx->h_res_err, 0), "status word");
     }
-    CUDA_TRY(ctx, cudaMalloc((void**)&ctx->d_grid, 2 * sizeof(unsigned)), "barrier counters");
+    CUDA_TRY(ctx, dev_malloc(ctx, (void**)&ctx->d_grid, 2 * sizeof(unsigned)), "barrier counters");
     CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_grid, 0, 2 * sizeof(unsigned), ctx->stream), "barrier counters");
     return LM_OK;
 }

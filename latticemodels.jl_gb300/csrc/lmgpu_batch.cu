@@ -373,7 +373,7 @@ static int upload_table(lm_ctx* ctx, T** dptr, size_t* cap, const std::vector<T>
         if (*dptr) cudaFree(*dptr);
         *dptr = nullptr;
         *cap = 0;
-        cudaError_t e = cudaMalloc((void**)dptr, need);
+        cudaError_t e = dev_malloc(ctx, (void**)dptr, need);
         if (e != cudaSuccess) {
             *dptr = nullptr;
             cudaGetLastError();
@@ -515,7 +515,7 @@ static int build_tables(lm_batch* b) {
 template <typename T>
 static int upload_new(lm_ctx* ctx, T** dptr, const std::vector<T>& host) {
     *dptr = nullptr;
-    cudaError_t e = cudaMalloc((void**)dptr, std::max<size_t>(host.size(), 1) * sizeof(T));
+    cudaError_t e = dev_malloc(ctx, (void**)dptr, std::max<size_t>(host.size(), 1) * sizeof(T));
     if (e == cudaSuccess && !host.empty())
         e = cudaMemcpy(*dptr, host.data(), host.size() * sizeof(T), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
@@ -554,8 +554,8 @@ static int build_panel_tables(lm_batch* b) {
         b->pa.assign(n, nullptr);
         b->py.assign(n, nullptr);
         for (size_t i = 0; i < n; ++i) {
-            cudaError_t e = cudaMalloc(&b->pa[i], need[i]);
-            if (e == cudaSuccess) e = cudaMalloc(&b->py[i], need[i]);
+            cudaError_t e = dev_malloc(ctx, (void**)&b->pa[i], need[i]);
+            if (e == cudaSuccess) e = dev_malloc(ctx, (void**)&b->py[i], need[i]);
             if (e != cudaSuccess) {
                 cudaGetLastError();
                 free_panel(b);
@@ -776,7 +776,7 @@ int lm_batch_create(lm_ctx* ctx, int kind, int precision, double tol, lm_batch**
     b->precision = precision;
     b->tol = tol;
     cudaSetDevice(ctx->device);
-    if (cudaMalloc((void**)&b->dqueue, 7 * sizeof(unsigned long long)) != cudaSuccess ||
+    if (dev_malloc(ctx, (void**)&b->dqueue, 7 * sizeof(unsigned long long)) != cudaSuccess ||
         cudaMemset(b->dqueue, 0, 7 * sizeof(unsigned long long)) != cudaSuccess) {
         cudaGetLastError();
         if (b->dqueue) cudaFree(b->dqueue);

@@ -745,12 +745,12 @@ int lm_ell_create_csc(lm_ctx* ctx, int64_t n, const int64_t* colptr, const int64
         ccol[(size_t)p] = (int)h->csc_col[(size_t)p];
     }
     cudaSetDevice(ctx->device);
-    cudaError_t e = cudaMalloc((void**)&h->d_cols, sizeof(int) * cols.size());
-    if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_vals, sizeof(double2) * h->h_vals.size());
-    if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_diag, sizeof(double) * (size_t)n);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_crow, sizeof(int) * (size_t)std::max<int64_t>(nnz, 1));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_ccol, sizeof(int) * (size_t)std::max<int64_t>(nnz, 1));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_cval, sizeof(double2) * (size_t)std::max<int64_t>(nnz, 1));
+    cudaError_t e = dev_malloc(ctx, (void**)&h->d_cols, sizeof(int) * cols.size());
+    if (e == cudaSuccess) e = dev_malloc(ctx, (void**)&h->d_vals, sizeof(double2) * h->h_vals.size());
+    if (e == cudaSuccess) e = dev_malloc(ctx, (void**)&h->d_diag, sizeof(double) * (size_t)n);
+    if (e == cudaSuccess) e = dev_malloc(ctx, (void**)&h->d_crow, sizeof(int) * (size_t)std::max<int64_t>(nnz, 1));
+    if (e == cudaSuccess) e = dev_malloc(ctx, (void**)&h->d_ccol, sizeof(int) * (size_t)std::max<int64_t>(nnz, 1));
+    if (e == cudaSuccess) e = dev_malloc(ctx, (void**)&h->d_cval, sizeof(double2) * (size_t)std::max<int64_t>(nnz, 1));
     if (e == cudaSuccess)
         e = cudaMemcpy(h->d_cols, cols.data(), sizeof(int) * cols.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && nnz > 0) e = cudaMemcpy(h->d_crow, crow.data(), sizeof(int) * crow.size(), cudaMemcpyHostToDevice);
@@ -834,7 +834,7 @@ int lm_ell_set_layout(lm_ell* h, int layout, int64_t a, int64_t b, int periodic_
     }
     cudaSetDevice(ctx->device);
     int* d = nullptr;
-    if (cudaMalloc((void**)&d, sizeof(int) * bm.size()) != cudaSuccess) {
+    if (dev_malloc(ctx, (void**)&d, sizeof(int) * bm.size()) != cudaSuccess) {
         cudaGetLastError();
         return set_err(ctx, LM_ERR_OOM, "lm_ell_set_layout: bond map");
     }
@@ -941,11 +941,11 @@ int lm_ell_create_bonds(lm_ctx* ctx, int64_t n, int64_t nbonds, const int64_t* s
     }
     h->nbonds = nbonds;
     cudaSetDevice(ctx->device);
-    cudaError_t e = cudaMalloc((void**)&h->d_bxy, sizeof(double) * (size_t)std::max<int64_t>(4 * nbonds, 1));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_bbase, sizeof(double2) * (size_t)std::max<int64_t>(nbonds, 1));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_eptr, sizeof(int64_t) * (size_t)(nnz + 1));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_eterm, sizeof(int64_t) * (size_t)std::max<int64_t>(2 * nbonds, 1));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_emap, sizeof(int64_t) * (size_t)nnz);
+    cudaError_t e = dev_malloc(ctx, (void**)&h->d_bxy, sizeof(double) * (size_t)std::max<int64_t>(4 * nbonds, 1));
+    if (e == cudaSuccess) e = dev_malloc(ctx, (void**)&h->d_bbase, sizeof(double2) * (size_t)std::max<int64_t>(nbonds, 1));
+    if (e == cudaSuccess) e = dev_malloc(ctx, (void**)&h->d_eptr, sizeof(int64_t) * (size_t)(nnz + 1));
+    if (e == cudaSuccess) e = dev_malloc(ctx, (void**)&h->d_eterm, sizeof(int64_t) * (size_t)std::max<int64_t>(2 * nbonds, 1));
+    if (e == cudaSuccess) e = dev_malloc(ctx, (void**)&h->d_emap, sizeof(int64_t) * (size_t)nnz);
     if (e == cudaSuccess && nbonds > 0) {
         e = cudaMemcpy(h->d_bxy, xy, sizeof(double) * (size_t)(4 * nbonds), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(h->d_bbase, base, sizeof(double2) * (size_t)nbonds, cudaMemcpyHostToDevice);
@@ -996,7 +996,7 @@ int lm_ell_set_onsite(lm_ell* h, const double* v) {
     } else {
         for (int64_t i = 0; i < h->n; ++i) CHECK_ARG(ctx, isfinite(v[i]), "lm_ell_set_onsite: non-finite value");
         if (!h->d_onsite) {
-            cudaError_t e = cudaMalloc((void**)&h->d_onsite, sizeof(double) * (size_t)h->n);
+            cudaError_t e = dev_malloc(ctx, (void**)&h->d_onsite, sizeof(double) * (size_t)h->n);
             if (e != cudaSuccess) {
                 cudaGetLastError();
                 h->d_onsite = nullptr;
@@ -1082,7 +1082,7 @@ int lm_ell_currents(lm_ell* h, lm_state* st, double* out) {
     if (h->nnz == 0) return LM_OK;
     cudaSetDevice(ctx->device);
     double* d_out = nullptr;
-    CUDA_TRY(ctx, cudaMalloc((void**)&d_out, sizeof(double) * (size_t)h->nnz), "lm_ell_currents: allocation");
+    CUDA_TRY(ctx, dev_malloc(ctx, (void**)&d_out, sizeof(double) * (size_t)h->nnz), "lm_ell_currents: allocation");
     const unsigned grid = (unsigned)std::min<int64_t>((h->nnz + 255) / 256, 65535);
     if (st->precision == LM_C64)
         ell_currents_kernel<double><<<grid, 256, 0, ctx->stream>>>(h->nnz, h->d_crow, h->d_ccol, h->d_cval, st->kind,
@@ -1109,7 +1109,7 @@ int lm_ell_op_currents(lm_ell* h, lm_state* st, int ndof, const double* op, doub
     if (h->nnz == 0) return LM_OK;
     cudaSetDevice(ctx->device);
     double* d_out = nullptr;
-    CUDA_TRY(ctx, cudaMalloc((void**)&d_out, sizeof(double) * (size_t)h->nnz), "lm_ell_op_currents: allocation");
+    CUDA_TRY(ctx, dev_malloc(ctx, (void**)&d_out, sizeof(double) * (size_t)h->nnz), "lm_ell_op_currents: allocation");
     cudaError_t e = launch_ell_op_currents(ctx, h, st, ndof, lop, d_out);
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, d_out, sizeof(double) * (size_t)h->nnz, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);

@@ -3,7 +3,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <list>
+#include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/lmgpu.h"
@@ -103,7 +106,11 @@ struct lm_ctx {
     int fused_form = 1;                 // LM_OPT_STREAM: 1 = x-streaming form where supported, 0 = region form
     int64_t stream_launches = 0;        // fused steps run in the x-streaming form
     int kpm_df = 1;                     // LM_OPT_KPM: double-float recurrence in lm_kpm_moments
-    cudaMemPool_t pool = nullptr;       // device memory of states and temporaries (dev_alloc); null: cudaMalloc
+    cudaMemPool_t pool = nullptr;       // device memory of tables and temporaries (dev_alloc); null: cudaMalloc
+    // buffers of destroyed states, oldest first, for the next state of the same size (state_alloc)
+    std::mutex kept_mutex;
+    std::list<std::pair<size_t, void*>> kept;
+    size_t kept_bytes = 0, kept_max = 0;
     unsigned resident_attr = 0;         // shared-memory attributes of the lattice-resident kernels set
     unsigned long long* h_res_err = nullptr;  // timeout word of the kernels that wait (mapped host memory)
     unsigned long long* d_res_err = nullptr;  // and its device address
@@ -276,6 +283,15 @@ int check_cuda(lm_ctx* ctx, cudaError_t e, const char* what);
 // synchronised with them before it is freed.
 cudaError_t dev_alloc(lm_ctx* ctx, void** p, size_t bytes);
 void dev_free(lm_ctx* ctx, void* p);
+// The two buffers of a state that lm_state_device_ptr hands out: cudaMalloc memory, which can be exported
+// to other processes (cudaIpcGetMemHandle) and reached by peers, as a pool's cannot.  A freed buffer is kept for
+// the next state of its size; only the context's stream uses it, so the order of that stream is enough.
+cudaError_t state_mem_alloc(lm_ctx* ctx, void** p, size_t bytes);
+void state_mem_free(lm_ctx* ctx, void* p, size_t bytes);
+// cudaMalloc after giving back what the context keeps, if it has to.
+cudaError_t dev_malloc(lm_ctx* ctx, void** p, size_t bytes);
+// Gives back what the context keeps of freed memory.
+void release_kept(lm_ctx* ctx);
 
 // Kernel launchers (lmgpu_kernels.cu).  All launch on ctx->stream and return cudaError_t.
 cudaError_t launch_assemble(lm_ctx* ctx, const Geom& g, const FieldSet& f, double t1, double2* hop);

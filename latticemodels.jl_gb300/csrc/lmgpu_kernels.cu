@@ -327,7 +327,7 @@ static cudaError_t ensure_readout_part(lm_ctx* ctx, size_t n) {
     if (ctx->d_ld_part) cudaFree(ctx->d_ld_part);
     ctx->d_ld_part = nullptr;
     ctx->ld_part_cap = 0;
-    cudaError_t e = cudaMalloc((void**)&ctx->d_ld_part, n * sizeof(double));
+    cudaError_t e = dev_malloc(ctx, (void**)&ctx->d_ld_part, n * sizeof(double));
     if (e == cudaSuccess) ctx->ld_part_cap = n;
     return e;
 }

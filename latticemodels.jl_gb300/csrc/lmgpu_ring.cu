@@ -41,7 +41,7 @@ int lm_ring_create(lm_ctx* ctx, int nslots, int64_t len, lm_ring** out) {
     r->nslots = nslots;
     r->len = len;
     const size_t bytes = sizeof(double) * (size_t)len * (size_t)nslots;
-    cudaError_t e = cudaMalloc((void**)&r->d_buf, bytes);
+    cudaError_t e = dev_malloc(ctx, (void**)&r->d_buf, bytes);
     if (e == cudaSuccess) e = cudaHostAlloc((void**)&r->h_buf, bytes, cudaHostAllocDefault);
     r->ev.assign((size_t)nslots, nullptr);
     for (int i = 0; e == cudaSuccess && i < nslots; ++i)

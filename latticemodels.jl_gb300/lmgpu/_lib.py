@@ -49,6 +49,7 @@ SIGNATURES = {
     "lm_ctx_destroy": (_INT, [_P]),
     "lm_last_error": (C.c_char_p, [_P]),
     "lm_ctx_synchronize": (_INT, [_P]),
+    "lm_ctx_trim": (_INT, [_P]),
     "lm_ctx_raise_timeout": (_INT, [_P]),
     "lm_ctx_stream": (_INT, [_P, C.POINTER(_P)]),
     "lm_ctx_set_option": (_INT, [_P, _INT, _INT]),
