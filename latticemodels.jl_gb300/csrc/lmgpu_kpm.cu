@@ -133,14 +133,14 @@ __device__ __forceinline__ double df_value(DF x) { return (double)x.h + (double)
 
 // hi + lo of a double: hi the nearest FP32 number, lo the remaining 28 bits rounded to FP32, by
 // integer operations (the conversions of the FP64 pipe run at 1.7 lanes per clock: a block of
-// 268 MB took 240 us with them, 95 us without).  Values below 2^-126 become 0; what overflows FP32
-// (infinities and NaN included) goes through the conversion.
+// 268 MB took 240 us with them, 95 us without).  What is or leaves an FP32 subnormal, and what overflows FP32
+// (infinities and NaN included), goes through the conversion; below 2^-150 that gives 0.
 __device__ __forceinline__ DF df_split(double v) {
     const int hw = __double2hiint(v);
     const unsigned lw = (unsigned)__double2loint(v);
     const int ex = (hw >> 20) & 0x7ff;
     if (ex >= 1150) return DF{(float)v, 0.f};
-    if (ex <= 896 + 53) return ex <= 896 ? DF{0.f, 0.f} : DF{(float)v, (float)(v - (double)(float)v)};
+    if (ex <= 896 + 53) return ex < 1023 - 150 ? DF{0.f, 0.f} : DF{(float)v, (float)(v - (double)(float)v)};
     const int sign = hw & 0x80000000;
     int low = (int)(lw & 0x1fffffffu);
     const int up = low >> 28;  // round to nearest: the next FP32 number and a negative remainder
