@@ -384,6 +384,8 @@ typedef struct lm_eigsys lm_eigsys;
 int lm_eigsys_create(lm_ham *ham, lm_eigsys **out);
 int lm_eigsys_create_ell(lm_ell *ham, lm_eigsys **out);
 int lm_eigsys_destroy(lm_eigsys *e);
+/* 1 / sqrt(x) and 1 / x as the reduction forms them (Newton's iteration), for tests of their accuracy. */
+int lm_newton_reciprocals(lm_ctx *ctx, int64_t n, const double *x, double *rsqrt, double *recip);
 int lm_eigsys_size(const lm_eigsys *e, int64_t *n);
 /* The N eigenvalues in ascending order (host array of N doubles). */
 int lm_eigsys_values(const lm_eigsys *e, double *out);

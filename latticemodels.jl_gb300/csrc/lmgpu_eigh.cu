@@ -449,7 +449,8 @@ __device__ __forceinline__ bool wait_sum(const double* q, int G, int lane, doubl
 
 // 1 / sqrt(t) and 1 / d by Newton's iteration from the FP32 approximations, on arguments scaled into
 // [1, 4) and [1, 2): two steps take their 22 bits beyond FP64's 53.  A quarter of the FP64 instructions of
-// sqrt and a division.  Zero, subnormal and extreme arguments go the plain way.
+// sqrt and a division.  Zero, subnormal and extreme arguments go the plain way.  Within 1.5 and 1 units in the
+// last place of the exact values by the last step's roundings; 1.28 and 0.50 are the largest found.
 __device__ __forceinline__ double newton_rsqrt(double t) {
     const int hi = __double2hiint(t), lo = __double2loint(t);
     const int ex = (hi >> 20) - 1023;
@@ -473,6 +474,13 @@ __device__ __forceinline__ double newton_recip(double d) {  // d > 0
 #pragma unroll
     for (int i = 0; i < 2; ++i) r = fma(r, fma(-m, r, 1.0), r);
     return __hiloint2double(__double2hiint(r) - (ex << 20), __double2loint(r));
+}
+
+__global__ void newton_kernel(const double* __restrict__ x, int64_t n, double* __restrict__ rs, double* __restrict__ rd) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    rs[i] = newton_rsqrt(x[i]);
+    rd[i] = newton_recip(x[i]);
 }
 
 template <int NC>
@@ -560,9 +568,14 @@ __global__ void __launch_bounds__(kTriThreads, 1) tridiag_resident_kernel(TriArg
                 beta = alpha.x >= 0.0 ? -nrm : nrm;
                 const double rb = alpha.x >= 0.0 ? -rs : rs;  // 1 / beta
                 den = make_double2(alpha.x - beta, alpha.y);
-                const double rd = newton_recip(fma(den.x, den.x, den.y * den.y));
+                const double dd = fma(den.x, den.x, den.y * den.y);
                 tv = make_double2(-den.x * rb, -alpha.y * rb);
-                scal = make_double2(den.x * rd, -den.y * rd);
+                if (dd < 0x1p-1000) {  // 1 / dd may overflow where den / dd does not
+                    scal = make_double2(den.x / dd, -den.y / dd);
+                } else {
+                    const double rd = newton_recip(dd);
+                    scal = make_double2(den.x * rd, -den.y * rd);
+                }
                 const double tp = mul_part(tv, im ? scal.y : scal.x, im ? scal.x : scal.y), tq = other(tp);
                 ts = make_double2(im ? tq : tp, im ? tp : tq);
             }
@@ -1583,6 +1596,25 @@ int eigsys_from_dense(lm_ctx* ctx, int64_t n, lm_eigsys** out) {
 }  // namespace
 
 extern "C" {
+
+int lm_newton_reciprocals(lm_ctx* ctx, int64_t n, const double* x, double* rsqrt, double* recip) {
+    if (!ctx) return LM_ERR_ARG;
+    CHECK_ARG(ctx, n >= 1 && x && rsqrt && recip, "lm_newton_reciprocals: bad argument");
+    cudaSetDevice(ctx->device);
+    DevFree tmp(ctx);
+    double* d = nullptr;
+    const int rc = dalloc_t(ctx, &d, 3 * (size_t)n, "arguments");
+    tmp.keep(d);
+    if (rc != LM_OK) return rc;
+    const size_t bytes = sizeof(double) * (size_t)n;
+    CUDA_TRY(ctx, cudaMemcpyAsync(d, x, bytes, cudaMemcpyHostToDevice, ctx->stream), "upload");
+    newton_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(d, n, d + n, d + 2 * n);
+    CUDA_TRY(ctx, cudaGetLastError(), "lm_newton_reciprocals");
+    CUDA_TRY(ctx, cudaMemcpyAsync(rsqrt, d + n, bytes, cudaMemcpyDeviceToHost, ctx->stream), "download");
+    CUDA_TRY(ctx, cudaMemcpyAsync(recip, d + 2 * n, bytes, cudaMemcpyDeviceToHost, ctx->stream), "download");
+    CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "sync");
+    return LM_OK;
+}
 
 int lm_eigsys_create(lm_ham* h, lm_eigsys** out) {
     if (!h || !out) return LM_ERR_ARG;

@@ -128,6 +128,7 @@ SIGNATURES = {
     "lm_ham_lanczos_bounds": (_INT, [_P, _INT, C.c_ulonglong, _PD, _PD]),
     "lm_eigsys_create": (_INT, [_P, C.POINTER(_P)]),
     "lm_eigsys_create_ell": (_INT, [_P, C.POINTER(_P)]),
+    "lm_newton_reciprocals": (_INT, [_P, _I64, _PD, _PD, _PD]),
     "lm_eigsys_destroy": (_INT, [_P]),
     "lm_eigsys_size": (_INT, [_P, _PI64]),
     "lm_eigsys_values": (_INT, [_P, _PD]),
