@@ -314,6 +314,10 @@ __global__ void __launch_bounds__(256) her2_tiles_kernel(double2* __restrict__ A
 // ------------------------------------------------------------------------------------------
 constexpr int kTriThreads = 160;      // 4 warps on the pass, 1 on the scalars
 constexpr int kTriMaxCols = 8;        // columns per CTA
+// Shared-memory limits of the resident kernels.  They are also the kernels' attribute, which is the device's,
+// not a context's: a value that followed the matrix could be lowered by another thread before the launch.
+constexpr int kTriMaxSmem = 224 * 1024;
+constexpr int kBackMaxSmem = 220 * 1024;
 
 // Sum of NV doubles per lane over the warp; lane k (k < NV, a power of two <= 32) returns the
 // total of value k.  Halving the values with every exchange takes NV + log2(32 / NV) adds per warp.
@@ -1246,13 +1250,13 @@ void free_eigsys(lm_eigsys* e) {
 // three more vectors of n complex numbers have to fit in an SM's shared memory.
 int tri_resident_cols(const lm_ctx* ctx, int64_t n) {
     const int64_t c = (n + ctx->sm_count - 1) / ctx->sm_count;
-    return n >= 2 && c <= kTriMaxCols && (c + 3) * n * (int64_t)sizeof(double2) <= 224 * 1024 ? (int)c : 0;
+    return n >= 2 && c <= kTriMaxCols && (c + 3) * n * (int64_t)sizeof(double2) <= kTriMaxSmem ? (int)c : 0;
 }
 
 template <int NC>
 cudaError_t launch_tri(lm_ctx* ctx, TriArgs a, int grid) {
     const size_t smem = sizeof(double2) * (size_t)(NC + 3) * (size_t)a.n;
-    cudaError_t e = cudaFuncSetAttribute(tridiag_resident_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(tridiag_resident_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTriMaxSmem);
     if (e != cudaSuccess) return e;
     void* args[] = {&a};
     return cudaLaunchCooperativeKernel((const void*)tridiag_resident_kernel<NC>, dim3(grid), dim3(kTriThreads), args, smem,
@@ -1274,8 +1278,8 @@ int reduce_tiles(lm_eigsys* es, DevFree& tmp) {
     if (rc == LM_OK) rc = dalloc_t(ctx, &d_pdot, (size_t)(m0 + 255) / 256, "partial dots");
     tmp.keep(d_v); tmp.keep(d_p); tmp.keep(d_part1); tmp.keep(d_part2); tmp.keep(d_pdot);
     if (rc != LM_OK) return rc;
-    const size_t smem = sizeof(double2) * kTile * (kTile + 1);
-    CUDA_TRY(ctx, cudaFuncSetAttribute(hemv_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    constexpr int kSmem = (int)sizeof(double2) * kTile * (kTile + 1);
+    CUDA_TRY(ctx, cudaFuncSetAttribute(hemv_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem),
              "eigensolver: shared memory attribute");
     for (int64_t j = 0; j + 1 < n; ++j) {
         const int64_t m = n - 1 - j, o = j + 1;
@@ -1283,7 +1287,7 @@ int reduce_tiles(lm_eigsys* es, DevFree& tmp) {
         const int64_t ntiles = (int64_t)nt * (nt + 1) / 2;
         const int nb = (int)((m + 255) / 256);
         house_kernel<<<1, 1024, 0, ctx->stream>>>(es->d_A, n, n, j, es->d_d, es->d_e, es->d_tau, d_v);
-        hemv_tiles_kernel<<<(unsigned)ntiles, 256, smem, ctx->stream>>>(es->d_A, n, o, m, nt, d_v, es->d_tau + j,
+        hemv_tiles_kernel<<<(unsigned)ntiles, 256, kSmem, ctx->stream>>>(es->d_A, n, o, m, nt, d_v, es->d_tau + j,
                                                                        d_part1, d_part2);
         hemv_reduce_kernel<<<nb, 256, 0, ctx->stream>>>(m, nt, d_part1, d_part2, d_v, es->d_tau + j, d_p, d_pdot);
         her2_tiles_kernel<<<(unsigned)ntiles, 256, 0, ctx->stream>>>(es->d_A, n, o, m, d_v, d_p, d_pdot, nb,
@@ -1469,7 +1473,7 @@ int check_lm_state_dense(lm_ctx* ctx, const lm_state* st, int64_t n, int kind, c
 // Columns per CTA of the resident back-transformation: one wave over the SMs where shared memory
 // allows it (C columns and two reflectors of n complex numbers); 0 where not one column fits.
 int back_resident_cols(const lm_ctx* ctx, int64_t n, int64_t nv) {
-    const int64_t fit = 220 * 1024 / (n * (int64_t)sizeof(double2)) - 2;
+    const int64_t fit = kBackMaxSmem / (n * (int64_t)sizeof(double2)) - 2;
     const int64_t want = (nv + ctx->sm_count - 1) / ctx->sm_count;
     return n >= 2 && fit >= 1 ? (int)std::min<int64_t>({want, fit, (int64_t)kBackMaxCols}) : 0;
 }
@@ -1477,7 +1481,7 @@ int back_resident_cols(const lm_ctx* ctx, int64_t n, int64_t nv) {
 template <int C>
 cudaError_t launch_back_t(lm_eigsys* es, double2* X, int64_t ldx, int64_t nv) {
     const size_t smem = sizeof(double2) * (size_t)(C + 2) * (size_t)es->n;
-    cudaError_t e = cudaFuncSetAttribute(back_resident_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(back_resident_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBackMaxSmem);
     if (e != cudaSuccess) return e;
     back_resident_kernel<C><<<(unsigned)((nv + C - 1) / C), kBackThreads, smem, es->ctx->stream>>>(
         es->d_A, es->n, (int)es->n, es->d_tau, X, ldx, nv);
