@@ -296,33 +296,63 @@ __global__ void __launch_bounds__(32) gauge_tables_kernel(Geom g, const double2*
     }
 }
 
+// CTAs of this block and shared size that fit an SM, remembered for the last ones.
 template <class A, int KT, int S, bool PROP>
-cudaError_t launch_t(lm_ctx* ctx, const SeriesPlan& p, const SeriesArgs& a, int variant) {
-    const int64_t items = (a.M + KT - 1) / KT;
-    const int threads = (a.Ly * a.nseg + 31) / 32 * 32;
-    // several CTAs of a small lattice share an SM, each taking an equal share of the kets
+cudaError_t fit_t(lm_ctx* ctx, int variant, int threads, size_t smem, int* fit) {
     auto& f = ctx->series_fit[variant];
-    if (f.threads != threads || f.smem != p.smem) {
+    if (f.threads != threads || f.smem != smem) {
         cudaError_t e = cudaFuncSetAttribute(series_resident_kernel<A, KT, S, PROP>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
-        int fit = 1;
+        int n = 1;
         if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, series_resident_kernel<A, KT, S, PROP>, threads, p.smem);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, series_resident_kernel<A, KT, S, PROP>, threads, smem);
         if (e != cudaSuccess) return e;
         f.threads = threads;
-        f.smem = p.smem;
-        f.fit = fit;
+        f.smem = smem;
+        f.fit = std::max(n, 1);
     }
-    const int fit = f.fit;
-    const int64_t slots = (int64_t)std::max(fit, 1) * ctx->sm_count, waves = (items + slots - 1) / slots;
-    series_resident_kernel<A, KT, S, PROP><<<(unsigned)((items + waves - 1) / waves), threads, p.smem, ctx->stream>>>(a);
+    *fit = f.fit;
+    return cudaSuccess;
+}
+
+// Several CTAs of a small lattice share an SM, each taking an equal share of the items.
+struct Share {
+    int64_t waves, grid;
+};
+Share share(int64_t items, int fit, int sm_count) {
+    const int64_t slots = (int64_t)fit * sm_count, waves = (items + slots - 1) / slots;
+    return {waves, (items + waves - 1) / waves};
+}
+
+int block_threads(int Ly, int nseg) { return (Ly * nseg + 31) / 32 * 32; }
+
+template <class A, int KT, int S, bool PROP>
+cudaError_t launch_t(lm_ctx* ctx, const SeriesPlan& p, const SeriesArgs& a, int variant) {
+    const int threads = block_threads(a.Ly, a.nseg);
+    int fit = 1;
+    const cudaError_t e = fit_t<A, KT, S, PROP>(ctx, variant, threads, p.smem, &fit);
+    if (e != cudaSuccess) return e;
+    const Share sh = share((a.M + KT - 1) / KT, fit, ctx->sm_count);
+    series_resident_kernel<A, KT, S, PROP><<<(unsigned)sh.grid, threads, p.smem, ctx->stream>>>(a);
     ctx->launches++;
     return cudaGetLastError();
 }
 
+// CTAs per SM of a plan's FP64 kernel (0 on an error).
+int fit_f64(lm_ctx* ctx, const SeriesPlan& p, int threads) {
+    int fit = 0;
+    const cudaError_t e = p.cols <= 2   ? fit_t<ArithF64, 1, 2, true>(ctx, 0, threads, p.smem, &fit)
+                          : p.cols <= 4 ? fit_t<ArithF64, 1, 4, true>(ctx, 1, threads, p.smem, &fit)
+                          : p.cols <= 8 ? fit_t<ArithF64, 1, 8, true>(ctx, 2, threads, p.smem, &fit)
+                                        : fit_t<ArithF64, 1, 12, true>(ctx, 3, threads, p.smem, &fit);
+    if (e == cudaSuccess) return fit;
+    cudaGetLastError();
+    return 0;
+}
+
 }  // namespace
 
-SeriesPlan series_plan(const lm_ctx* ctx, const Geom& g, bool x_real, int64_t M, bool df) {
+SeriesPlan series_plan(lm_ctx* ctx, const Geom& g, bool x_real, int64_t M, bool df) {
     SeriesPlan p;
     // a periodic x axis has no such gauge in general; there the FP64 form stays with the per-order
     // kernels also where the x-hops are real, so that both kinds of field round alike
@@ -340,18 +370,29 @@ SeriesPlan series_plan(const lm_ctx* ctx, const Geom& g, bool x_real, int64_t M,
     const int kt = df && p.cols <= 6 && M >= 2 * ctx->sm_count && 2 * ket + tables <= kMaxSmem ? 2 : 1;
     p.smem = kt * ket + tables;
     if (p.smem > kMaxSmem) return p;
-    // Against one launch per order: here an order takes the longest SM's share of the kets (10.8 clocks a
-    // site in FP64, the gauge included, or 1.9 in double-float), there a launch of about 5 us and the whole
-    // block at 16 or 20 DFMAs of 1.87 a clock and SM (double-float: at its memory traffic).  Few kets on a
-    // large lattice leave SMs idle here, and from about 1500 sites a dense FP64 step is ahead there; elsewhere
-    // this form is (dense steps here / there: 10 x 10 22.5 / 66.7 us, 30 x 30 505 / 555 us, 47 x 31 1309 /
-    // 1314 us, 48 x 48 3208 / 3078 us; 200 kets of 48 x 48 204 / 171 us; double-float 48 x 48: 34 / 111 us an
-    // order).
+    // Against one launch per order.
     const double sites = (double)g.N, mhz = 2000.0;
-    const int64_t per_sm = (M + (int64_t)kt * ctx->sm_count - 1) / ((int64_t)kt * ctx->sm_count) * kt;
-    const double here = 0.5 + (double)per_sm * sites * (df ? 1.9 : 10.8) / mhz;
-    const double there =
-        5.0 + (double)M * sites * (df ? 2.0e-5 : (x_real ? 16.0 : 20.0) / 1.87 / mhz / ctx->sm_count);
+    double here, there;
+    if (df) {
+        // An order takes the longest SM's share of the kets at 1.9 clocks a site, a launch per order about 5 us
+        // and its memory traffic (48 x 48: 34 against 111 us an order).
+        const int64_t per_sm = (M + (int64_t)kt * ctx->sm_count - 1) / ((int64_t)kt * ctx->sm_count) * kt;
+        here = 0.5 + (double)per_sm * sites * 1.9 / mhz;
+        there = 5.0 + (double)M * sites * 2.0e-5;
+    } else {
+        // A launch per order takes 4.25 us and the block's 16 or 20 DFMAs a site at 1.84 a clock and SM.  Here the
+        // kets of the SM with the most of them count, in whole CTAs and waves, at 9.4 or 10.1 clocks for a
+        // thread's column, idle lanes included.  Fitted to 330 steps of 13 lattices from 6 x 6 to 64 x 62 with 1 to
+        // 1500 kets and dense (here within 20 %, there within 10 %).  Complex x-hops, K = 9, here / there: dense
+        // 10 x 10 25 / 74 us, 24 x 24 229 / 296 us, 40 x 33 1476 / 1207 us; 32 x 27 with 304 kets 96 / 126 us, with 330,
+        // whose third CTA makes it four kets an SM, 187 / 133 us; 31 x 47 with 700 436 / 367 us.
+        const int threads = block_threads((int)g.Ly, p.nseg), fit = fit_f64(ctx, p, threads);
+        if (!fit) return p;
+        const Share sh = share(M, fit, ctx->sm_count);
+        const int64_t kets = (sh.grid + ctx->sm_count - 1) / ctx->sm_count * sh.waves;
+        here = 0.55 + 0.2 * (double)sh.waves + (double)kets * threads * p.cols * (x_real ? 9.4 : 10.1) / mhz;
+        there = 4.25 + (double)M * sites * (x_real ? 16.0 : 20.0) / 1.84 / mhz / ctx->sm_count;
+    }
     if (here < there) p.kt = kt;
     return p;
 }

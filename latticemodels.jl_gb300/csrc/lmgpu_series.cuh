@@ -31,7 +31,7 @@ struct SeriesPlan {
     int kt = 0, nseg = 0, cols = 0;
     size_t smem = 0;
 };
-SeriesPlan series_plan(const lm_ctx* ctx, const Geom& g, bool x_real, int64_t M, bool df);
+SeriesPlan series_plan(lm_ctx* ctx, const Geom& g, bool x_real, int64_t M, bool df);
 
 // Gauge and stencil tables of H (hops of modulus t1 and on-site term; 2/a scales them): gauge may be null when x_real.  Double
 // tables (hy, diag) or double-float ones (hyd, diagd); null pointers are skipped.
