@@ -210,6 +210,7 @@ struct MarchArgs {
     const float4* tpp;   // T_{n-1}; FIRST: unused
     float4* out;
     int64_t ld, M;
+    int kt;                // kets per thread
     int rows, segs, cols;  // rows and x-segments per block, columns per segment
     float2 alpha;
     float4* y;
@@ -351,6 +352,7 @@ __global__ void sum_parts_kernel(const double* __restrict__ part, int nblk, int6
     if (i >= 2 * M) return;
     const double* p = part + (int64_t)blockIdx.y * nblk * 2 * M + i;
     double v = 0.0;
+#pragma unroll 16  // that many loads under way together: with few kets this chain is all the kernel does
     for (int b = 0; b < nblk; ++b) v += p[(int64_t)b * 2 * M];
     out[(int64_t)blockIdx.y * 2 * M + i] = v;
 }
@@ -462,32 +464,37 @@ static double tridiag_eig(const std::vector<double>& a, const std::vector<double
     return 0.5 * (lo + hi);
 }
 
-constexpr int kMarchKets = 2;  // kets per thread of the df passes
 constexpr int64_t kPartPasses = 16;  // passes whose partial dots are summed by one launch
 
-// Rows and segments of a block, columns per segment: the split whose waves of two blocks of up to 256
-// threads per SM are fullest, counting 1.5 columns for a segment's two shared edges and half a row for
-// those of a chunk of rows (96 rows in one chunk leave a quarter of a block's threads out: 1.97 ms a pass of
-// 9216 x 9216 against 1.66 ms in chunks of 32).
+// Kets per thread, rows and segments of a block, columns per segment: the split with the shortest waves of two
+// blocks of up to 256 threads per SM, counting 1.5 columns for a segment's two shared edges and half a
+// row for those of a chunk of rows (96 rows in one chunk leave a quarter of a block's threads out: 1.97 ms a
+// pass of 9216 x 9216 against 1.66 ms in chunks of 32).  Two kets share the table loads, so one alone costs
+// 0.8 of two; where a thread has three columns or less, its chain of loads and sums is what counts, and one ket
+// costs 0.6 (64 x 64 sites, complex x-hops, a series of 64 terms on one / two / eight kets: 295 us each, the
+// launches' pace; with two kets and at least four columns per thread 471 / 554 / 562 us).
 static void march_plan(const lm_ctx* ctx, const Geom& g, int64_t M, MarchArgs& a) {
-    const int64_t groups = (M + kMarchKets - 1) / kMarchKets, slots = 2ll * ctx->sm_count;
-    const int64_t chunks0 = (g.Ly + 255) / 256;
-    double best = 0.0;
-    for (int64_t c = chunks0; c <= std::max<int64_t>(chunks0, g.Ly / 32); ++c) {
-        const int64_t rows = (g.Ly + c - 1) / c, segs = std::max<int64_t>(1, 256 / rows), chunks = (g.Ly + rows - 1) / rows;
-        for (int64_t nseg = 1; nseg <= g.Lx; ++nseg) {
-            const int64_t cols = (g.Lx + nseg - 1) / nseg, n = (g.Lx + cols - 1) / cols;
-            const int64_t blocks = chunks * ((n + segs - 1) / segs) * groups;
-            const double eff = (double)g.Lx * (double)(g.Ly * groups) /
-                               ((double)((blocks + slots - 1) / slots * slots) * 256.0 * ((double)cols + 1.5) *
-                                (1.0 + (c > 1 ? 0.5 / (double)rows : 0.0)));
-            if (eff > best) {
-                best = eff;
-                a.rows = (int)rows;
-                a.segs = (int)segs;
-                a.cols = (int)cols;
+    const int64_t slots = 2ll * ctx->sm_count, chunks0 = (g.Ly + 255) / 256;
+    double best = 1e300;
+    for (int kt = 2; kt >= 1; --kt) {
+        const int64_t groups = (M + kt - 1) / kt;
+        for (int64_t c = chunks0; c <= std::max<int64_t>(chunks0, g.Ly / 32); ++c) {
+            const int64_t rows = (g.Ly + c - 1) / c, segs = std::max<int64_t>(1, 256 / rows), chunks = (g.Ly + rows - 1) / rows;
+            // the fewest columns whose blocks make w waves, for the first w that hold them all and on
+            const int64_t w0 = (chunks * groups + slots - 1) / slots;
+            for (int64_t w = w0; w <= std::max<int64_t>(w0, 64); ++w) {
+                const int64_t cols = (g.Lx + w * slots / (chunks * groups) * segs - 1) / (w * slots / (chunks * groups) * segs);
+                const double t = (double)w * ((double)cols + 1.5) * (1.0 + (c > 1 ? 0.5 / (double)rows : 0.0)) *
+                                 (kt == 2 ? 1.0 : cols <= 3 ? 0.6 : 0.8);
+                if (t < best) {
+                    best = t;
+                    a.kt = kt;
+                    a.rows = (int)rows;
+                    a.segs = (int)segs;
+                    a.cols = (int)cols;
+                }
+                if (cols <= 1) break;
             }
-            if (cols <= 4 || blocks > 64 * slots) break;
         }
     }
 }
@@ -497,29 +504,30 @@ static int64_t march_blocks(const MarchArgs& a) {
     return chunks * ((n + a.segs - 1) / a.segs);
 }
 
-template <bool XR>
+template <bool XR, int KT>
 static cudaError_t launch_march(lm_ctx* ctx, const MarchArgs& a, bool first) {
     const int threads = (a.rows * a.segs + 31) / 32 * 32;
-    for (int64_t m = 0; m < a.M; m += 65535ll * kMarchKets) {  // the grid's y extent is 65535
+    for (int64_t m = 0; m < a.M; m += 65535ll * KT) {  // the grid's y extent is 65535
         MarchArgs b = a;
-        b.M = std::min<int64_t>(a.M - m, 65535ll * kMarchKets);
+        b.M = std::min<int64_t>(a.M - m, 65535ll * KT);
         b.tp += m * a.ld;
         if (b.tpp) b.tpp += m * a.ld;
         b.out += m * a.ld;
         if (b.y) b.y += m * a.ld;
         if (b.part) b.part += m;
-        const dim3 grid((unsigned)march_blocks(a), (unsigned)((b.M + kMarchKets - 1) / kMarchKets));
-        if (first && a.y) df_march_kernel<XR, true, false, true, kMarchKets><<<grid, threads, 0, ctx->stream>>>(b);
-        else if (first) df_march_kernel<XR, true, false, false, kMarchKets><<<grid, threads, 0, ctx->stream>>>(b);
-        else if (a.part) df_march_kernel<XR, false, true, false, kMarchKets><<<grid, threads, 0, ctx->stream>>>(b);
-        else df_march_kernel<XR, false, false, true, kMarchKets><<<grid, threads, 0, ctx->stream>>>(b);
+        const dim3 grid((unsigned)march_blocks(a), (unsigned)((b.M + KT - 1) / KT));
+        if (first && a.y) df_march_kernel<XR, true, false, true, KT><<<grid, threads, 0, ctx->stream>>>(b);
+        else if (first) df_march_kernel<XR, true, false, false, KT><<<grid, threads, 0, ctx->stream>>>(b);
+        else if (a.part) df_march_kernel<XR, false, true, false, KT><<<grid, threads, 0, ctx->stream>>>(b);
+        else df_march_kernel<XR, false, false, true, KT><<<grid, threads, 0, ctx->stream>>>(b);
         ctx->launches++;
     }
     return cudaGetLastError();
 }
 
 static cudaError_t march(lm_ctx* ctx, const MarchArgs& a, bool xr, bool first = false) {
-    return xr ? launch_march<true>(ctx, a, first) : launch_march<false>(ctx, a, first);
+    if (a.kt == 2) return xr ? launch_march<true, 2>(ctx, a, first) : launch_march<false, 2>(ctx, a, first);
+    return xr ? launch_march<true, 1>(ctx, a, first) : launch_march<false, 1>(ctx, a, first);
 }
 
 // lm_cheb_apply with every column on chip through the whole series (lmgpu_series.cu): no recurrence
