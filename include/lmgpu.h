@@ -103,6 +103,9 @@ int lm_ctx_stream(lm_ctx *ctx, void **stream);
 int lm_ctx_set_option(lm_ctx *ctx, int option, int value);
 /* Number of fused steps that ran in the x-streaming form on this context so far. */
 int lm_ctx_stream_launches(lm_ctx *ctx, int64_t *n);
+/* Number of launches of the lattice-resident form for a single lattice (a ComplexF32 step, one recurrence of an
+ * adjoint step) on this context so far. */
+int lm_ctx_resident_launches(lm_ctx *ctx, int64_t *n);
 /* Opt-in CUDA-event timing of the Chebyshev-order launches (for measurement); events are
  * resolved lazily by lm_ctx_timing, so timing adds no host synchronisation per step. */
 int lm_ctx_set_timing(lm_ctx *ctx, int enable);

@@ -445,6 +445,12 @@ int lm_ctx_stream_launches(lm_ctx* ctx, int64_t* n) {
     return LM_OK;
 }
 
+int lm_ctx_resident_launches(lm_ctx* ctx, int64_t* n) {
+    if (!ctx || !n) return LM_ERR_ARG;
+    *n = ctx->resident_launches;
+    return LM_OK;
+}
+
 int lm_ctx_set_timing(lm_ctx* ctx, int enable) {
     if (!ctx) return LM_ERR_ARG;
     ctx->timing = enable ? 1 : 0;

@@ -105,6 +105,7 @@ struct lm_ctx {
     unsigned long long stream_attr_comp = 0;  // the same for its compensated-state variant
     int fused_form = 1;                 // LM_OPT_STREAM: 1 = x-streaming form where supported, 0 = region form
     int64_t stream_launches = 0;        // fused steps run in the x-streaming form
+    int64_t resident_launches = 0;      // launches of the lattice-resident form for a single lattice
     int kpm_df = 1;                     // LM_OPT_KPM: double-float recurrence in lm_kpm_moments
     cudaMemPool_t pool = nullptr;       // device memory of tables and temporaries (dev_alloc); null: cudaMalloc
     // buffers of destroyed states, oldest first, for the next state of the same size (state_alloc)

@@ -926,6 +926,7 @@ cudaError_t launch_resident_single(lm_ctx* ctx, int K, bool xreal, int cl, int m
     else e = cl == 1 ? LM_RES(false, 1, 3) : LM_RES(false, 2, 3);
 #undef LM_RES
     ctx->launches++;
+    ctx->resident_launches++;
     return e;
 }
 

@@ -54,6 +54,7 @@ SIGNATURES = {
     "lm_ctx_stream": (_INT, [_P, C.POINTER(_P)]),
     "lm_ctx_set_option": (_INT, [_P, _INT, _INT]),
     "lm_ctx_stream_launches": (_INT, [_P, _PI64]),
+    "lm_ctx_resident_launches": (_INT, [_P, _PI64]),
     "lm_ctx_set_timing": (_INT, [_P, _INT]),
     "lm_ctx_timing": (_INT, [_P, _PD, _PI64, _PI64]),
     "lm_ctx_reset_timing": (_INT, [_P]),

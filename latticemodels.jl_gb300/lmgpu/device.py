@@ -56,6 +56,12 @@ class Context:
         self.check(self.lib.lm_ctx_stream_launches(self.handle, C.byref(n)))
         return n.value
 
+    def resident_launches(self) -> int:
+        """Launches of the lattice-resident form for a single lattice so far."""
+        n = C.c_int64()
+        self.check(self.lib.lm_ctx_resident_launches(self.handle, C.byref(n)))
+        return n.value
+
     def set_timing(self, on: bool):
         self.check(self.lib.lm_ctx_set_timing(self.handle, 1 if on else 0))
 
