@@ -89,7 +89,8 @@ int lm_ctx_stream(lm_ctx *ctx, void **stream);
  * 0 selects the region form (a halo on both axes).  Both give bit-identical results. */
 #define LM_OPT_STREAM 2
 /* LM_OPT_KPM (default 1): the recurrences of lm_kpm_moments and lm_cheb_apply run in
- * double-float arithmetic (pairs of FP32 values, about 48 significant bits) on the FP32 pipe;
+ * double-float arithmetic (pairs of FP32 values) on the FP32 pipe: stored values have 48 significant
+ * bits, the sum of a site's terms one or two less until its pair is normalised, once per site;
  * 0 selects FP64.  KPM moments agree to about 1e-15 mu_0.  lm_cheb_apply keeps columns that fit in
  * shared memory on chip through the whole series. */
 #define LM_OPT_KPM 3

@@ -18,7 +18,7 @@
 //      per launch where a column does not fit), and the weighted projector P = sum_k w_k x_k x_k^H
 //      over lower tiles, accumulated over vector chunks.
 //
-// GB300 runs FP64 at about two FMAs per clock per SM, so every stage is bound by its FP64
+// GB300 runs FP64 at two FMAs per clock per SM (1.84 reached), so every stage is bound by its FP64
 // FMAs: the kernels spend none on anything else (complex products are four DFMAs).
 #include <cuda_runtime.h>
 
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(256) her2_tiles_kernel(double2* __restrict__ A
 // needs, looking again at a word that still holds the sentinel.  A barrier with a fence took 5100
 // clocks with the loads after it, this 3700; polling the words without the counter 12600 (each of the
 // 152 stores into a line that all SMs poll costs a round trip between the dies).
-// What bounds it: GB300's FP64 rate of about 2 DFMAs per clock and SM in the early columns (storing
+// What bounds it: GB300's FP64 rate of 2 DFMAs per clock and SM in the early columns (storing
 // both triangles costs 12 instead of 8 DFMAs per element, but no sum over CTAs), the exchanges and warp 4's
 // chain in the late ones.  A warp-wide FP64 instruction holds a partition's pipe for 64 clocks even
 // for one lane, so warp 4 has a lane per component of a complex scalar, and takes its root and
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(kTriThreads, 1) tridiag_resident_kernel(TriArg
     for (int r = t; r < n; r += kTriThreads) ps[r] = sm[(size_t)NC * n + r] = sm[(size_t)(NC + 1) * n + r] = make_double2(0.0, 0.0);
     __syncthreads();
     constexpr int U = NC + 2;  // rows of a pass thread (n <= 152 NC takes one batch)
-    constexpr int kFold = NC > 4 ? 8 : NC > 2 ? 4 : NC > 1 ? 2 : 1;  // a power of two >= NC
+    constexpr int kFold = NC > 4 ? 8 : NC > 2 ? 4 : 2;  // a power of two >= NC (2 to 8)
     // warp 4: lane 2 k + i holds component i of column k's complex scalars (a warp-wide FP64 instruction
     // costs the same for one lane as for 32)
     const int kk = (lane >> 1) & (kFold - 1), im = lane & 1;
@@ -804,7 +804,7 @@ __device__ __forceinline__ double hash_unit(uint64_t a, uint64_t b) {  // determ
 // Thread-per-cluster arrays are interleaved (row i of cluster q at [i ncl + q], of member mi at
 // [i nmem + mi]), so a warp's accesses are consecutive, and every sweep loads kSteinRows rows
 // before it uses them.  The pivots are kept as reciprocals: one division per row in the
-// factorisation and none in the three solves 432 vectors of N = 864 take 2.1 ms (5.6 ms with a
+// factorisation and none in the three solves.  432 vectors of N = 864 take 1.9 ms (5.6 ms with a
 // division per row and solve and a vector per thread in memory order).
 constexpr int kSteinRows = 8;
 

@@ -145,7 +145,12 @@ __global__ void __launch_bounds__(256) cheb_order_ell_rows_kernel(
 //
 // What bounds it: the FP64 pipe (16 DFMAs per site of the honeycomb and order, 3.1 us for 1e5 sites) and
 // a barrier with the gather's latency behind it (about 2 us) per order; a launch per order takes 6.6 us on
-// the device and 2.5 us of the host.  One ket of 100,352 honeycomb sites, K = 11: 61.5 against 75 us (65.9 us with the sum ahead of the barrier).
+// the device and 2.5 us of the host.  One ket of 100,352 honeycomb sites, K = 11: 61.5 against 75 us (65.9 us
+// with the sum ahead of the barrier).  Rows of up to 8 entries in FP64 keep about 200 bytes of a thread's row in
+// local memory (64 registers at 1024 threads), and the launch still wins up to the full grid: one launch
+// / a launch per order, us, one ket: triangular lattice (6 entries, K = 11) 10,000 sites 41 / 68, 40,000 56 /
+// 93, 144,400 141 / 160; 8 entries, 150,000 sites 146 / 160; kagome (4), 145,200 sites 78 / 103; FP32 1.8 to 2.4
+// times as fast at every size.
 struct EllCoop {
     int64_t n, total, ld;
     int w, K;

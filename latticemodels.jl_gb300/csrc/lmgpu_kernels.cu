@@ -912,7 +912,7 @@ cudaError_t launch_column_norms_comp(lm_ctx* ctx, const float2* hi, const uint32
 //
 // Bound by HBM (24 bytes per element).  A block takes 256 x kRescalePer x VEC elements of a column and a
 // thread has kRescalePer loads in flight; with 256 elements per block the FP64 division at the head of
-// half a million blocks took most of the time: 256 x 256 sites, 2048 kets 1161 -> 520 us.
+// half a million blocks took most of the time: 256 x 256 sites, 2048 kets 1161 -> 455 us.
 constexpr int kRescalePer = 4;
 
 template <int VEC>

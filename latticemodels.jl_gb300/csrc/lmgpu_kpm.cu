@@ -132,7 +132,7 @@ __device__ __forceinline__ DF df_from(double x) {
 __device__ __forceinline__ double df_value(DF x) { return (double)x.h + (double)x.l; }
 
 // hi + lo of a double: hi the nearest FP32 number, lo the remaining 28 bits rounded to FP32, by
-// integer operations (the conversions of the FP64 pipe run at 1.7 lanes per clock: a block of
+// integer operations (conversions run on the FP64 pipe, at its rate: a block of
 // 268 MB took 240 us with them, 95 us without).  What is or leaves an FP32 subnormal, and what overflows FP32
 // (infinities and NaN included), goes through the conversion; below 2^-150 that gives 0.
 __device__ __forceinline__ DF df_split(double v) {
@@ -197,10 +197,10 @@ __global__ void from_df_kernel(const float4* __restrict__ in, int64_t ld_in, int
 // Products enter an unnormalised pair (s, c) by TwoSum, every error term c: 12 FP32 operations per
 // real product and sum; XR (x-hops all equal to the real alpha) adds the two x-neighbours first.
 //
-// What bounds it: HBM (three block passes: read tp and tpp, write out) and the FP32 pipe (about 215
-// operations per element) at about the same time: 119 us of traffic and 108 us of arithmetic for
-// 256 x 256 sites and 256 kets, measured 174 us (209 us with the loads of a column issued when it
-// is used), the dots included.  One thread per site with normalised sums took 258 us, and 113 us
+// What bounds it: the FP32 pipe (about 215 operations per element) and HBM (three block passes: read tp and
+// tpp, write out), which do not overlap fully at 14 warps per SM: 119 us of traffic and 135 us without
+// any memory access for 256 x 256 sites and 256 kets, measured 176 us (209 us with the loads of a column
+// issued when it is used), the dots included.  One thread per site with normalised sums took 258 us, and 113 us
 // more for the dots as a kernel of their own.
 struct MarchArgs {
     Geom g;

@@ -12,8 +12,8 @@
 // Landau field without an x twist is in it, g = 1).  A site and order then takes 16 real
 // multiply-adds instead of 20, for 8 more per ket and launch at the load and the store.
 //
-// What bounds it: the arithmetic.  FP64 runs at 1.7 lane operations per clock and SM, so the
-// 16 of a site and order are all that counts; a double-float product and sum takes 12 FP32
+// What bounds it: the arithmetic.  FP64 runs at 2 lane operations per clock and SM (1.84 reached; its pipe is
+// 79 % busy with one CTA per SM), so the 16 of a site and order are all that counts; a double-float product and sum takes 12 FP32
 // operations (error-free product, TwoSum, one compensation word that is folded in once per site)
 // instead of 18 with a normalised sum, on packed pairs (re, im).  Measured: a dense 10 x 10 step 21 us
 // against 18 launches of 3 us and their host time (67 us), a dense 47 x 31 step 1.31 ms as with a launch per

@@ -176,8 +176,8 @@ def _collect_rings(pairs, it, nslots):
             _take(ts, ring, seq, wrap, rw)
 
 
-# Large readouts of a sequence are rows of blocks of this size: numpy backs arrays from 4 MB with huge pages,
-# while every 800 KB array of its own was 200 page faults (55 us)
+# Large readouts (from 64 KB) of a sequence are rows of blocks of this size: numpy backs arrays from 4 MB with huge
+# pages, while every 800 KB array of its own was 200 page faults (55 us).  A value kept alone keeps its block.
 _BLOCK_BYTES = 4 << 20
 
 
@@ -198,7 +198,8 @@ def timesequences(fs, it, nslots: int = 8):
     ``localdensity(P)`` and ``DensityCurrents(H, P)`` at every moment of ``ev(times)``.
 
     ``moment_density`` and ``moment_currents`` go through device readout rings (asynchronous
-    downloads); any other callable is applied to each moment as it is yielded."""
+    downloads); any other callable is applied to each moment as it is yielded.  Values of 64 KB and
+    more are rows of shared 4 MB arrays: a program that keeps a few of a long run copies them."""
     out = [TimeSequence() for _ in fs]
     ring_pairs = [(f, ts) for f, ts in zip(fs, out) if getattr(f, "_lm_readout", None) is not None]
     plain = [(f, ts) for f, ts in zip(fs, out) if getattr(f, "_lm_readout", None) is None]
