@@ -413,10 +413,11 @@ __device__ __forceinline__ void bond_write(const Geom& g, const double2* __restr
 // Ket blocks: P[j,s] = sum_k w_k psi_jk conj(psi_sk).  A block owns 32 consecutive sites (one
 // per lane); its 8 warps split the kets; partial sums are added in warp order.
 // XR (real x-hops): J of an x-bond needs the imaginary part only, two products fewer of eight.
-// With `part` a block takes the kets of slice blockIdx.y and writes its sums to planes
+// SLICED: a block takes the kets of slice blockIdx.y and writes its sums to planes
 // [slice][sum][site] instead, (re unless XR, im) of the x-bond and (re, im) of the y-bond;
-// readout_slices_kernel adds the slices in order and writes the bonds.
-template <typename R, bool WEIGHTED, bool XR>
+// readout_slices_kernel adds the slices in order and writes the bonds.  (A form of its own: the tests for it
+// cost the readout of a single ket 0.4 of 5.9 us.)
+template <typename R, bool WEIGHTED, bool XR, bool SLICED>
 __global__ void __launch_bounds__(32 * kReadWarps) bond_currents_kets_kernel(
     Geom g, const double2* __restrict__ hop, const typename CT<R>::V* __restrict__ x, int64_t m, int64_t ld,
     const double* __restrict__ w, double* __restrict__ out, int64_t kslice, double* __restrict__ part) {
@@ -424,7 +425,7 @@ __global__ void __launch_bounds__(32 * kReadWarps) bond_currents_kets_kernel(
     __shared__ double red[kReadWarps][4][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t s = (int64_t)blockIdx.x * 32 + lane;
-    const int64_t k0 = (int64_t)blockIdx.y * kslice, k1 = k0 + kslice < m ? k0 + kslice : m;
+    const int64_t k0 = SLICED ? (int64_t)blockIdx.y * kslice : 0, k1 = SLICED && k0 + kslice < m ? k0 + kslice : m;
     Nbr nb;
     Acc<R> a[4];  // (re, im) of the +x bond, then of the +y bond
     double aw[4] = {0.0, 0.0, 0.0, 0.0};
@@ -467,7 +468,7 @@ __global__ void __launch_bounds__(32 * kReadWarps) bond_currents_kets_kernel(
             for (int r = 0; r < kReadWarps; ++r) t += red[r][q][lane];
             v[q] = t;
         }
-        if (part) {
+        if constexpr (SLICED) {
             constexpr int Q0 = XR ? 1 : 0;
 #pragma unroll
             for (int q = Q0; q < 4; ++q) part[((int64_t)blockIdx.y * (4 - Q0) + q - Q0) * g.N + s] = v[q];
@@ -661,10 +662,15 @@ static cudaError_t launch_readout_v(lm_ctx* ctx, const Geom& g, const double2* h
                : launch_readout_t<VEC, XR, false>(ctx, g, hop, x, m, ld, rho, out);
 }
 
+// Whether a lane of the c32 sums can take four sites of a column.
+static bool readout_wide(const lm_ctx* ctx, const Geom& g, const void* x, int64_t ld) {
+    return g.Ly % 4 == 0 && ld % 2 == 0 && ((uintptr_t)x & 15) == 0 && !ctx->currents_scalar;
+}
+
 // The c32 sums of a block without weights; cudaErrorMemoryAllocation where their scratch does not fit.
 static cudaError_t launch_readout_c32(lm_ctx* ctx, const Geom& g, const double2* hop, bool xr, const float2* x, int64_t m,
                                       int64_t ld, double* rho, double* out) {
-    const bool wide = g.Ly % 4 == 0 && ld % 2 == 0 && ((uintptr_t)x & 15) == 0 && !ctx->currents_scalar;
+    const bool wide = readout_wide(ctx, g, x, ld);
     if (wide) return xr ? launch_readout_v<4, true>(ctx, g, hop, x, m, ld, rho, out)
                         : launch_readout_v<4, false>(ctx, g, hop, x, m, ld, rho, out);
     return xr ? launch_readout_v<1, true>(ctx, g, hop, x, m, ld, rho, out)
@@ -677,8 +683,8 @@ static void launch_currents_kets(lm_ctx* ctx, const Geom& g, const double2* hop,
     typedef typename CT<R>::V V;
     const unsigned blocks = (unsigned)((g.N + 31) / 32);
     const int thr = 32 * kReadWarps;
-    if (w) bond_currents_kets_kernel<R, true, XR><<<blocks, thr, 0, ctx->stream>>>(g, hop, (const V*)x, m, ld, w, out, m, nullptr);
-    else bond_currents_kets_kernel<R, false, XR><<<blocks, thr, 0, ctx->stream>>>(g, hop, (const V*)x, m, ld, w, out, m, nullptr);
+    if (w) bond_currents_kets_kernel<R, true, XR, false><<<blocks, thr, 0, ctx->stream>>>(g, hop, (const V*)x, m, ld, w, out, m, nullptr);
+    else bond_currents_kets_kernel<R, false, XR, false><<<blocks, thr, 0, ctx->stream>>>(g, hop, (const V*)x, m, ld, w, out, m, nullptr);
     ctx->launches++;
 }
 
@@ -693,7 +699,7 @@ static cudaError_t launch_currents_weighted(lm_ctx* ctx, const Geom& g, const do
                                             int64_t ld, const double* w, double* out, int S) {
     cudaError_t e = ensure_readout_part(ctx, (size_t)S * (XR ? 3 : 4) * (size_t)g.N);
     if (e != cudaSuccess) return e;
-    bond_currents_kets_kernel<float, true, XR><<<dim3((unsigned)((g.N + 31) / 32), (unsigned)S), 32 * kReadWarps, 0,
+    bond_currents_kets_kernel<float, true, XR, true><<<dim3((unsigned)((g.N + 31) / 32), (unsigned)S), 32 * kReadWarps, 0,
                                                  ctx->stream>>>(g, hop, x, m, ld, w, out, (m + S - 1) / S, ctx->d_ld_part);
     readout_slices_kernel<XR, false><<<(unsigned)((g.N + 127) / 128), 128, 0, ctx->stream>>>(g, hop, ctx->d_ld_part, S, nullptr,
                                                                                             out);
@@ -739,11 +745,13 @@ cudaError_t launch_bond_currents(lm_ctx* ctx, const Geom& g, int precision, int 
         if (xr) launch_currents_kets<double, true>(ctx, g, hop, x, m, ld, w, out);
         else launch_currents_kets<double, false>(ctx, g, hop, x, m, ld, w, out);
     } else {
-        if (!w) {
+        // up to four kets with a site per lane: the scalar kernel's one exchange between warps is shorter than an
+        // exchange per sum (97 x 75 sites, one ket: 10.5 against 13 us)
+        if (!w && (m > 4 || readout_wide(ctx, g, x, ld))) {
             const cudaError_t e = launch_readout_c32(ctx, g, hop, xr, (const float2*)x, m, ld, nullptr, out);
             if (e != cudaErrorMemoryAllocation) return e;
             (void)cudaGetLastError();  // no scratch for the partial sums: one block per 32 sites and all kets
-        } else if (const int S = weighted_slices(ctx, g, m); S > 1) {
+        } else if (const int S = w ? weighted_slices(ctx, g, m) : 1; S > 1) {
             const cudaError_t e = xr ? launch_currents_weighted<true>(ctx, g, hop, (const float2*)x, m, ld, w, out, S)
                                      : launch_currents_weighted<false>(ctx, g, hop, (const float2*)x, m, ld, w, out, S);
             if (e != cudaErrorMemoryAllocation) return e;
