@@ -352,7 +352,6 @@ __global__ void sum_parts_kernel(const double* __restrict__ part, int nblk, int6
     if (i >= 2 * M) return;
     const double* p = part + (int64_t)blockIdx.y * nblk * 2 * M + i;
     double v = 0.0;
-#pragma unroll 16  // that many loads under way together: with few kets this chain is all the kernel does
     for (int b = 0; b < nblk; ++b) v += p[(int64_t)b * 2 * M];
     out[(int64_t)blockIdx.y * 2 * M + i] = v;
 }
@@ -472,20 +471,24 @@ constexpr int64_t kPartPasses = 16;  // passes whose partial dots are summed by 
 // pass of 9216 x 9216 against 1.66 ms in chunks of 32).  Two kets share the table loads, so one alone costs
 // 0.8 of two; where a thread has three columns or less, its chain of loads and sums is what counts, and one ket
 // costs 0.6 (64 x 64 sites, complex x-hops, a series of 64 terms on one / two / eight kets: 295 us each, the
-// launches' pace; with two kets and at least four columns per thread 471 / 554 / 562 us).
-static void march_plan(const lm_ctx* ctx, const Geom& g, int64_t M, MarchArgs& a) {
+// launches' pace; with two kets and at least four columns per thread 471 / 554 / 562 us).  Half a wave, one block
+// per SM, costs 0.7 of one, 0.6 with the dots, whose sums at a block's end then come once per SM (256 x 256
+// sites, four kets, 64 moments 464 us, in a whole wave of half the columns 502 us).
+static void march_plan(const lm_ctx* ctx, const Geom& g, int64_t M, bool dots, MarchArgs& a) {
     const int64_t slots = 2ll * ctx->sm_count, chunks0 = (g.Ly + 255) / 256;
     double best = 1e300;
     for (int kt = 2; kt >= 1; --kt) {
         const int64_t groups = (M + kt - 1) / kt;
         for (int64_t c = chunks0; c <= std::max<int64_t>(chunks0, g.Ly / 32); ++c) {
             const int64_t rows = (g.Ly + c - 1) / c, segs = std::max<int64_t>(1, 256 / rows), chunks = (g.Ly + rows - 1) / rows;
-            // the fewest columns whose blocks make w waves, for the first w that hold them all and on
+            // the fewest columns whose blocks make w waves, for the first w that hold them all and on, as long as
+            // w waves without an idle block could still be shorter
+            const double edge = 1.0 + (c > 1 ? 0.5 / (double)rows : 0.0);
+            const double work = (double)g.Lx * (double)(chunks * groups) / (double)(slots * segs);
             const int64_t w0 = (chunks * groups + slots - 1) / slots;
-            for (int64_t w = w0; w <= std::max<int64_t>(w0, 64); ++w) {
-                const int64_t cols = (g.Lx + w * slots / (chunks * groups) * segs - 1) / (w * slots / (chunks * groups) * segs);
-                const double t = (double)w * ((double)cols + 1.5) * (1.0 + (c > 1 ? 0.5 / (double)rows : 0.0)) *
-                                 (kt == 2 ? 1.0 : cols <= 3 ? 0.6 : 0.8);
+            auto take = [&](int64_t room, double waves) {  // `room` blocks, which cost so many waves
+                const int64_t nseg = room / (chunks * groups) * segs, cols = (g.Lx + nseg - 1) / nseg;
+                const double t = waves * ((double)cols + 1.5) * edge * (kt == 2 ? 1.0 : cols <= 3 ? 0.6 : 0.8);
                 if (t < best) {
                     best = t;
                     a.kt = kt;
@@ -493,7 +496,12 @@ static void march_plan(const lm_ctx* ctx, const Geom& g, int64_t M, MarchArgs& a
                     a.segs = (int)segs;
                     a.cols = (int)cols;
                 }
-                if (cols <= 1) break;
+                return cols;
+            };
+            if (chunks * groups <= slots / 2) take(slots / 2, dots ? 0.6 : 0.7);
+            for (int64_t w = w0; w <= std::max<int64_t>(w0, 64); ++w) {
+                if ((work + 1.5 * (double)w) * edge * (kt == 2 ? 1.0 : 0.6) >= best) break;
+                if (take(w * slots, (double)w) <= 1) break;
             }
         }
     }
@@ -621,7 +629,7 @@ int lm_kpm_moments(lm_ham* h, double emin, double emax, int nmom, const lm_state
     ma.g = g;
     ma.ld = ld;
     ma.M = ma.pstride = M;
-    march_plan(ctx, g, M, ma);
+    march_plan(ctx, g, M, true, ma);
     const int64_t nblk = march_blocks(ma);
     double* part = nullptr;  // partial dots of kPartPasses passes
     auto release = [&]() {
@@ -836,7 +844,7 @@ int lm_cheb_apply(lm_ham* h, double emin, double emax, const double* coef, int n
         ma.g = g;
         ma.ld = ld;
         ma.M = M;
-        march_plan(ctx, g, M, ma);
+        march_plan(ctx, g, M, false, ma);
         ma.hop = hopd;
         ma.diag = diagd;
         ma.alpha = split(h->t1 * (2.0 / a));
