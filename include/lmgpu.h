@@ -173,7 +173,8 @@ int lm_state_download(lm_state *st, void *host, int64_t ld);
 int lm_state_copy(lm_state *dst, const lm_state *src);
 /* A new state with src's shape, kind, precision, values, weights and residual plane. */
 int lm_state_clone(const lm_state *src, lm_state **out);
-/* Current device buffer (it may change after a step) and its leading dimension. */
+/* Current device buffer (cudaMalloc memory; another one may be current after a step) and its leading
+ * dimension. */
 int lm_state_device_ptr(lm_state *st, void **ptr, int64_t *ld);
 /* Ket weights w_m, so that P = sum_m w_m |psi_m><psi_m| for the readouts; NULL = all ones. */
 int lm_state_set_weights(lm_state *st, const double *w);

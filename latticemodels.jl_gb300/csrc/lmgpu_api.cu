@@ -104,13 +104,14 @@ cudaError_t dev_malloc(lm_ctx* ctx, void** p, size_t bytes) {
 cudaError_t state_mem_alloc(lm_ctx* ctx, void** p, size_t bytes) {
     {
         std::lock_guard<std::mutex> lock(ctx->kept_mutex);
-        for (auto it = ctx->kept.begin(); it != ctx->kept.end(); ++it)
-            if (it->first == bytes) {
-                *p = it->second;
-                ctx->kept_bytes -= bytes;
-                ctx->kept.erase(it);
-                return cudaSuccess;
-            }
+        const auto it = ctx->kept_by_size.find(bytes);
+        if (it != ctx->kept_by_size.end()) {
+            *p = it->second->second;
+            ctx->kept_bytes -= bytes;
+            ctx->kept.erase(it->second);
+            ctx->kept_by_size.erase(it);
+            return cudaSuccess;
+        }
     }
     return dev_malloc(ctx, p, bytes);
 }
@@ -120,12 +121,19 @@ void state_mem_free(lm_ctx* ctx, void* p, size_t bytes) {
     std::vector<void*> drop;  // the oldest ones beyond the limit
     {
         std::lock_guard<std::mutex> lock(ctx->kept_mutex);
-        ctx->kept.emplace_back(bytes, p);
+        ctx->kept_by_size.emplace(bytes, ctx->kept.emplace(ctx->kept.end(), bytes, p));
         ctx->kept_bytes += bytes;
         while (ctx->kept_bytes > ctx->kept_max) {
-            drop.push_back(ctx->kept.front().second);
-            ctx->kept_bytes -= ctx->kept.front().first;
-            ctx->kept.pop_front();
+            const auto oldest = ctx->kept.begin();
+            const auto same = ctx->kept_by_size.equal_range(oldest->first);
+            for (auto it = same.first; it != same.second; ++it)
+                if (it->second == oldest) {
+                    ctx->kept_by_size.erase(it);
+                    break;
+                }
+            drop.push_back(oldest->second);
+            ctx->kept_bytes -= oldest->first;
+            ctx->kept.erase(oldest);
         }
     }
     if (drop.empty()) return;
@@ -138,6 +146,7 @@ void release_kept(lm_ctx* ctx) {
     {
         std::lock_guard<std::mutex> lock(ctx->kept_mutex);
         drop.swap(ctx->kept);
+        ctx->kept_by_size.clear();
         ctx->kept_bytes = 0;
     }
     cudaStreamSynchronize(ctx->stream);
@@ -146,7 +155,7 @@ void release_kept(lm_ctx* ctx) {
 }
 
 // A pool of the context's own for tables and temporaries, and the limit of the states' buffers kept for
-// reuse: up to a 64th of the device's memory each (4.4 GB) stays with the context instead of going back to
+// reuse: up to a 64th of the device's memory each (4.6 GB) stays with the context instead of going back to
 // the driver, as allocating and freeing the buffers of a 265 MB state cost 1.1 ms per Evolution.  An
 // allocation of the library that fails gives it back and tries again; lm_ctx_trim and lm_ctx_destroy give
 // it back too, and the driver takes what the pool keeps for other allocations of the process by itself.

@@ -6,6 +6,7 @@
 #include <list>
 #include <mutex>
 #include <string>
+#include <unordered_map>
 #include <utility>
 #include <vector>
 
@@ -111,6 +112,7 @@ struct lm_ctx {
     // buffers of destroyed states, oldest first, for the next state of the same size (state_alloc)
     std::mutex kept_mutex;
     std::list<std::pair<size_t, void*>> kept;
+    std::unordered_multimap<size_t, std::list<std::pair<size_t, void*>>::iterator> kept_by_size;
     size_t kept_bytes = 0, kept_max = 0;
     unsigned resident_attr = 0;         // shared-memory attributes of the lattice-resident kernels set
     unsigned long long* h_res_err = nullptr;  // timeout word of the kernels that wait (mapped host memory)
